@@ -18,7 +18,6 @@
 // arithmetic and independent of launch shape.
 #include "mvr_common.cuh"
 #include "mvr_kernels.cuh"
-#include "mvr_mbar.cuh"
 
 #include <cfloat>
 
@@ -30,6 +29,10 @@ namespace mvr {
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
 }
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::);
@@ -811,89 +814,280 @@ filter_select_kernel(DevIndex ix, uint32_t probe_topk, FilterScratch scr,
 // ---------------------------------------------------------------------
 // K3: decompress + exact MaxSim of up to kRkDocs shortlisted docs of one query.
 //
-// The docs' tokens, each doc padded to a multiple of 4 tokens, form a stream
-// of 256-token tiles; a tile is consumed in 8 chunks of 16 dimensions.  Two
-// CTAs of 256 threads per SM:
-//  warps 4-7   decoders (one warpgroup): per chunk, each thread decodes 2
-//              tokens (positions p and p + 128 of the tile) x 16 dims,
-//              x = centroid + W[bucket] (one rounded FP32 add; W from a table
-//              replicated across the 32 banks, read conflict-free), into
-//              stage i % kRkStages of a shared-memory ring [16 dims][256];
-//              the loads of chunk i + 1 are in flight while chunk i is
-//              decoded, and the next tile's tokens are located a tile ahead;
-//  warps 0-3   FMA (one warpgroup): thread (warp w, lane l) owns query tokens
-//              16(w&1)..+16 of the pass and doc tokens 128(w>>1) + 4l..+4 of
-//              the tile, so per dimension it reads 16 query values (4
-//              broadcast LDS.128) and 4 doc values (one LDS.128) for 64 FMAs.
-//              After the 8th chunk of a tile: max over the thread's valid
-//              tokens (all of one doc, thanks to the padding), then per doc a
-//              __reduce_max_sync over the lanes holding it, folded into
-//              best[query token][doc] by atomicMax.
-// Registers: the launch gives every thread 128; setmaxnreg lowers the FMA
-// warpgroup to 120 and raises the decoders to 136.
-// Queries of more than 32 tokens run in two passes (tokens 0-31, 32-63).
-// Ring handoff: mbarriers full[s] (the 128 decoder threads arrive) and
-// empty[s] (the 128 FMA threads arrive); every wait is bounded (wait_ns) and
-// a timeout sets bit 32 of *err and stops the CTA without writing scores.
-// Every dot product is the sequential __fmaf_rn chain over d = 0..127 from
-// 0.0f, so the scores are bit-identical to the canonical arithmetic.
+// The docs' tokens, doc after doc, form a stream of 128-token tiles; each of
+// the CTA's 4 warps takes every 4th tile and works alone (no barrier inside a
+// tile).  Lane l owns the tile's tokens l, l + 32, l + 64, l + 96 and all
+// query tokens of the pass (16 or 32): it decodes its own tokens in registers,
+// x = centroid + W[bucket] (one rounded FP32 add), and accumulates them with
+// fma.rn.f32x2, two query tokens per instruction (each half a rounded FP32
+// fma, so every dot product is the sequential __fmaf_rn chain over
+// d = 0..127 from 0.0f and the scores are bit-identical to the canonical
+// arithmetic).  Per dimension a lane reads NQ query values (broadcast
+// LDS.128) for 4 NQ FMAs.
+//
+// Centroid rows come through shared memory in chunks of 16 dimensions, two
+// stages per warp: 4 lanes copy a token's 64 bytes (cp.async), so a copy
+// instruction touches 8 cache lines instead of the 32 of a row per lane, and
+// the 16-byte parts are swizzled so that both the copies and the lanes' reads
+// of their own rows spread over all banks.  Residual bytes (one load per
+// token and chunk) are in registers a chunk ahead, the next tile's codes two
+// chunks ahead.
+//
+// After a tile: per doc of the tile, the max over the lane's tokens of that
+// doc and a REDUX over the warp for every query token, folded into
+// best[doc][query token] by atomicMax.  Queries of more than 32 tokens run in
+// two passes; a pass of at most 16 query tokens takes the 16-wide body.
+//
+// Bound: the FMA pipe (a token of a 32-token query is 32 cycles of an SM's 128
+// lanes), 60 % busy by the counters at 2 warps per scheduler and 255
+// registers; three warps of 3 tokens per lane spilled (12.2 ms where this
+// takes 8.8).  400 queries x 1500 docs of 70 tokens, 2 bits: 12.8 ms with
+// scalar FFMA and separate decoder warps -> 8.8 ms, 39 TFLOP/s.
 // ---------------------------------------------------------------------
-constexpr int kRkDocs = 64;       // shortlisted docs per CTA
-constexpr int kRkTile = 256;      // doc tokens per tile
-constexpr int kRkChunk = 16;      // dimensions per ring stage
-constexpr int kRkStages = 4;      // ring stages
+constexpr int kRkDocs = 64;       // most shortlisted docs per CTA
+constexpr int kRkT = 4;           // doc tokens per lane
+constexpr int kRkTile = 32 * kRkT;  // doc tokens per warp and tile
+constexpr int kRkChunk = 16;      // dimensions per stage
+constexpr int kRkStages = 2;
 constexpr int kRkQ = 32;          // query tokens per pass
-constexpr int kRkThreads = 256;   // 4 FMA warps + 4 decoder warps (two CTAs per SM)
-constexpr int kRkFma = 128;       // FMA threads
-// registers per thread after the split (setmaxnreg): the launch gives every
-// thread 128 (65,536 / 512 for the SM's two CTAs); the FMA warpgroup gives 8
-// each back and the decoder warpgroup takes them, 128 x 120 + 128 x 136 =
-// 256 x 128
-constexpr int kRkRegLaunch = 128;
-constexpr int kRkRegFma = 120;
-constexpr int kRkRegDec = 136;
-static_assert(kRkFma * kRkRegFma + (kRkThreads - kRkFma) * kRkRegDec == kRkThreads * kRkRegLaunch,
-              "register split must equal the launch allocation");
+constexpr int kRkWarps = 4;
+constexpr int kRkThreads = 32 * kRkWarps;  // two CTAs per SM, up to 255 registers a thread
+constexpr int kRkNch = kDim / kRkChunk;    // chunks per tile
 
-// CTA-local barrier of the FMA warps only (named barrier 1, kRkFma threads)
-__device__ __forceinline__ void fma_bar_sync() {
-  asm volatile("bar.sync 1, %0;\n" ::"n"(kRkFma) : "memory");
-}
+// copies of the weight table, so that lanes reading different weights of a
+// large table meet fewer bank conflicts (1 is conflict-free up to 32 entries)
+__host__ __device__ constexpr int rk_wcopies(int n_bit) { return n_bit <= 4 ? 1 : 8; }
 
 __host__ __device__ constexpr size_t rk_smem_bytes(int n_bit) {
-  return (size_t)kRkStages * kRkChunk * kRkTile * sizeof(float) +  // ring
-         (size_t)kDim * kRkQ * sizeof(float) +                      // query tokens of the pass
-         (size_t)(1 << n_bit) * 32 * sizeof(float) +                // replicated weights
-         (size_t)kMaxQueryTok * kRkDocs * sizeof(int);              // best[q][doc]
+  return (size_t)kRkWarps * kRkStages * kRkTile * kRkChunk * sizeof(float) +  // centroid chunks
+         (size_t)kDim * kRkQ * sizeof(float) +                                // query tokens
+         (size_t)(1 << n_bit) * rk_wcopies(n_bit) * sizeof(float) +           // weights
+         (size_t)kRkDocs * (kRkQ + 1) * sizeof(int);                          // best[doc][q]
+}
+
+// 4-dimension groups of a chunk per loop body.  All four unrolled miss the
+// instruction cache at 1 and 2 bits (400 queries x 1500 docs at 2 bits: 9.2,
+// 8.8 and 9.6 ms with 1, 2 and 4 groups a body), two spill at 4 bits (600
+// queries x 40 docs: 1.32, 1.59, 1.35 ms), and at 8 bits only the unrolled
+// form knows which register a group's codes are in (200 x 400: 2.12, 2.12, 1.79 ms).
+__host__ __device__ constexpr int rk_unroll(int n_bit) { return n_bit <= 2 ? 2 : n_bit == 4 ? 1 : 4; }
+
+__device__ __forceinline__ uint64_t dup_f32x2(float x) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};\n" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// What a warp needs of its CTA's docs and buffers (shared memory).
+struct RkCta {
+  const float *Qs;         // [128 dims][32 query tokens]
+  const float *wtab;       // [2^NBIT][copies]
+  float *xs;               // this warp's stages [kRkStages][128 tokens][16 dims], swizzled
+  uint32_t *codes;         // this warp's vq codes [2 tile parities][kRkTile]
+  uint64_t *toks;          // ... and token indexes
+  int *best;               // [kRkDocs][kRkQ + 1]
+  const uint32_t *d_pref;  // [nd + 1] token offsets of the docs
+  const uint64_t *d_off;   // [nd] first token of each doc
+  uint32_t nd, T;          // docs and tokens of the CTA
+};
+
+// One pass of one warp over its tiles: NQ query tokens (rows 0 .. NQ - 1 of Qs).
+template <int NBIT, int NQ>
+__device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c, uint32_t nq_pass) {
+  constexpr int CB = kRkChunk * NBIT / 8;  // residual bytes per token and chunk
+  constexpr int RW = (CB + 3) / 4;         // ... in 32-bit words
+  constexpr uint32_t MASK = (1u << NBIT) - 1u;
+  constexpr int WC = rk_wcopies(NBIT);
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t n_tiles = (c.T + kRkTile - 1) / kRkTile;
+  if (warp >= n_tiles) return;
+  const float *wt = c.wtab + (lane & (WC - 1));
+
+  uint32_t docs4 = 0, docs4_n = 0;  // doc of each of the lane's tokens, a byte each (255: none)
+  // tile tl's tokens of this lane into the buffers of parity pr (the codes by
+  // cp.async); past the last token: the last one again (loaded, never counted)
+  auto locate = [&](uint32_t tl, uint32_t pr) {
+    docs4_n = 0;
+#pragma unroll
+    for (int j = 0; j < kRkT; j++) {
+      const uint32_t g = kRkTile * tl + 32u * j + lane, gt = min(g, c.T - 1u);
+      const uint32_t d = find_seg(c.d_pref, (int)c.nd, gt);
+      docs4_n |= (g < c.T ? d : 255u) << (8 * j);
+      const uint64_t v = c.d_off[d] + (gt - c.d_pref[d]);
+      c.toks[pr * kRkTile + 32 * j + lane] = v;
+      cp_async4(&c.codes[pr * kRkTile + 32 * j + lane], ix.vq_code + v);
+    }
+    cp_async_commit();
+  };
+  uint32_t res[kRkT][RW], res_n[kRkT][RW];
+  auto load_res = [&](uint32_t ch, uint32_t pr) {
+#pragma unroll
+    for (int j = 0; j < kRkT; j++) {
+      const uint8_t *rp =
+          ix.residual + c.toks[pr * kRkTile + 32 * j + lane] * (kDim * NBIT / 8) + ch * CB;
+      if constexpr (CB == 2) {
+        res_n[j][0] = __ldg(reinterpret_cast<const unsigned short *>(rp));
+      } else if constexpr (CB == 4) {
+        res_n[j][0] = __ldg(reinterpret_cast<const uint32_t *>(rp));
+      } else if constexpr (CB == 8) {
+        const uint2 t = __ldg(reinterpret_cast<const uint2 *>(rp));
+        res_n[j][0] = t.x;
+        res_n[j][1] = t.y;
+      } else {
+        const uint4 t = __ldg(reinterpret_cast<const uint4 *>(rp));
+        res_n[j][0] = t.x;
+        res_n[j][1] = t.y;
+        res_n[j][2] = t.z;
+        res_n[j][3] = t.w;
+      }
+    }
+  };
+  // chunk ch of the tile of parity pr into stage st: lane copies 16-byte part
+  // lane % 4 of tokens lane / 4, lane / 4 + 8, ...
+  auto copy_chunk = [&](uint32_t ch, uint32_t pr, uint32_t st) {
+    const uint32_t part = lane & 3u;
+    float *dst = c.xs + st * (kRkTile * kRkChunk);
+    const float *src = ix.centroid + ch * kRkChunk + part * 4u;
+#pragma unroll
+    for (int i = 0; i < kRkTile / 8; i++) {
+      const uint32_t p = 8u * i + (lane >> 2);
+      const uint32_t cd = c.codes[pr * kRkTile + p];
+      cp_async16(dst + p * kRkChunk + ((part ^ ((p >> 1) & 3u)) << 2), src + (size_t)cd * kDim);
+    }
+    cp_async_commit();
+  };
+
+  locate(warp, 0);
+  cp_async_wait<0>();
+  __syncwarp();
+  copy_chunk(0, 0, 0);
+  load_res(0, 0);
+  uint32_t par = 0;
+  for (uint32_t tl = warp; tl < n_tiles; tl += kRkWarps) {
+    const bool more = tl + kRkWarps < n_tiles;
+    docs4 = docs4_n;
+    uint64_t acc[NQ / 2][kRkT];
+#pragma unroll
+    for (int i = 0; i < NQ / 2; i++)
+#pragma unroll
+      for (int j = 0; j < kRkT; j++) acc[i][j] = 0ull;
+#pragma unroll 1
+    for (uint32_t ch = 0; ch < (uint32_t)kRkNch; ch++) {
+#pragma unroll
+      for (int j = 0; j < kRkT; j++)
+#pragma unroll
+        for (int w = 0; w < RW; w++) res[j][w] = res_n[j][w];
+      const uint32_t st = ch & 1u;
+      cp_async_wait<0>();
+      __syncwarp();  // chunk ch landed for every lane; every lane is done with the other stage
+      if (ch + 1 < (uint32_t)kRkNch) {
+        copy_chunk(ch + 1, par, st ^ 1u);
+        load_res(ch + 1, par);
+        if (ch == kRkNch - 2 && more) locate(tl + kRkWarps, par ^ 1u);
+      } else if (more) {
+        par ^= 1u;
+        copy_chunk(0, par, st ^ 1u);
+        load_res(0, par);
+      }
+      const float *xr = c.xs + st * (kRkTile * kRkChunk) + lane * kRkChunk;
+      const float *qr = c.Qs + ch * (kRkChunk * kRkQ);
+#pragma unroll rk_unroll(NBIT)
+      for (int g = 0; g < kRkChunk / 4; g++) {
+        float x[kRkT][4];  // [token][dim of the group]
+#pragma unroll
+        for (int j = 0; j < kRkT; j++) {
+          // token 32 j + lane: (p >> 1) & 3 is (lane >> 1) & 3
+          const float4 v = *reinterpret_cast<const float4 *>(
+              xr + j * 32 * kRkChunk + (((uint32_t)g ^ ((lane >> 1) & 3u)) << 2));
+          const float cv[4] = {v.x, v.y, v.z, v.w};
+          // the group's 4 codes: bytes in order, most significant bits first
+          uint32_t bits;
+          if constexpr (NBIT == 1) bits = (res[j][0] >> (8 * (g >> 1) + 4 - 4 * (g & 1))) & 15u;
+          else if constexpr (NBIT == 2) bits = (res[j][0] >> (8 * g)) & 255u;
+          else if constexpr (NBIT == 4) bits = (g & 2 ? res[j][1] : res[j][0]) >> (16 * (g & 1));
+          else bits = g & 2 ? (g & 1 ? res[j][3] : res[j][2]) : (g & 1 ? res[j][1] : res[j][0]);
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int gbit = NBIT == 1 ? 3 - u : 8 * (u * NBIT / 8) + 8 - NBIT * (u % (8 / NBIT) + 1);
+            x[j][u] = __fadd_rn(cv[u], wt[((bits >> gbit) & MASK) * WC]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          uint64_t xx[kRkT];
+#pragma unroll
+          for (int j = 0; j < kRkT; j++) xx[j] = dup_f32x2(x[j][u]);
+          const ulonglong2 *qp = reinterpret_cast<const ulonglong2 *>(qr + (4 * g + u) * kRkQ);
+#pragma unroll
+          for (int i = 0; i < NQ / 4; i++) {
+            const ulonglong2 a = qp[i];
+#pragma unroll
+            for (int j = 0; j < kRkT; j++) {
+              acc[2 * i][j] = fma_f32x2(a.x, xx[j], acc[2 * i][j]);
+              acc[2 * i + 1][j] = fma_f32x2(a.y, xx[j], acc[2 * i + 1][j]);
+            }
+          }
+        }
+      }
+    }
+    // per doc of the tile: max over its tokens for every query token (lane q
+    // ends up with query token q's)
+    uint32_t d = __reduce_min_sync(kFull, docs4 & 0xffu);
+    const uint32_t d_last = find_seg(c.d_pref, (int)c.nd, min(c.T, kRkTile * (tl + 1)) - 1u);
+#pragma unroll 1
+    for (; d <= d_last; d++) {
+      bool in[kRkT];
+#pragma unroll
+      for (int j = 0; j < kRkT; j++) in[j] = ((docs4 >> (8 * j)) & 0xffu) == d;
+      int mine = f2si(-INFINITY);
+#pragma unroll
+      for (int i = 0; i < NQ / 2; i++) {
+        int lo = f2si(-INFINITY), hi = lo;
+#pragma unroll
+        for (int j = 0; j < kRkT; j++) {
+          if (in[j]) {
+            lo = max(lo, f2si(__uint_as_float((uint32_t)acc[i][j])));
+            hi = max(hi, f2si(__uint_as_float((uint32_t)(acc[i][j] >> 32))));
+          }
+        }
+        lo = __reduce_max_sync(kFull, lo);
+        hi = __reduce_max_sync(kFull, hi);
+        mine = lane == 2 * i ? lo : lane == 2 * i + 1 ? hi : mine;
+      }
+      if ((uint32_t)lane < nq_pass) atomicMax(&c.best[d * (kRkQ + 1) + lane], mine);
+    }
+  }
 }
 
 template <int NBIT>
 __global__ void __launch_bounds__(kRkThreads, 2)
 rerank_kernel(DevIndex ix, const float *__restrict__ q, const uint64_t *__restrict__ q_off,
               const uint32_t *__restrict__ short_id, const uint32_t *__restrict__ n_short,
-              uint32_t probe_topk, int semantics, float *__restrict__ exact,
-              unsigned *__restrict__ err, uint64_t wait_ns) {
-  constexpr int VPB = 8 / NBIT;             // values per residual byte
-  constexpr int CB = kRkChunk * NBIT / 8;   // residual bytes per token and chunk
-  constexpr int RW = (CB + 3) / 4;          // ... in 32-bit words
-  constexpr uint32_t MASK = (1u << NBIT) - 1u;
-  constexpr int NCH = kDim / kRkChunk;      // chunks per tile
+              uint32_t probe_topk, uint32_t docs, int semantics, float *__restrict__ exact) {
+  constexpr int VPB = 8 / NBIT;  // values per residual byte
+  constexpr int WC = rk_wcopies(NBIT);
   extern __shared__ __align__(16) float smem[];
-  float *ring = smem;                                       // [S][16][512]
-  float *Qs = ring + kRkStages * kRkChunk * kRkTile;        // [128 dims][32 query tokens]
-  float *wrep = Qs + kDim * kRkQ;                           // [2^NBIT][32]
-  int *best = reinterpret_cast<int *>(wrep + (1 << NBIT) * 32);  // [64 query tokens][kRkDocs]
-  __shared__ uint32_t d_len[kRkDocs], d_pp[kRkDocs + 1];
+  float *xs = smem;                                             // [warps][stages][128][16]
+  float *Qs = xs + kRkWarps * kRkStages * kRkTile * kRkChunk;   // [128 dims][32 query tokens]
+  float *wtab = Qs + kDim * kRkQ;                               // [2^NBIT][WC]
+  int *best = reinterpret_cast<int *>(wtab + (1 << NBIT) * WC);  // [kRkDocs][33]
+  __shared__ uint32_t d_len[kRkDocs], d_pref[kRkDocs + 1];
   __shared__ uint64_t d_off[kRkDocs];
-  __shared__ uint64_t full[kRkStages], empty[kRkStages];
-  __shared__ volatile int s_abort;
+  __shared__ uint32_t codes[kRkWarps][2 * kRkTile];
+  __shared__ uint64_t toks[kRkWarps][2 * kRkTile];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t b = blockIdx.y;
   const uint32_t ns = n_short[b];
-  const uint32_t d0 = blockIdx.x * kRkDocs;
+  const uint32_t d0 = blockIdx.x * docs;
   if (d0 >= ns) return;
-  const uint32_t nd = min((uint32_t)kRkDocs, ns - d0);
+  const uint32_t nd = min(docs, ns - d0);
   const uint64_t tok0 = q_off[b];
   const uint32_t nq = (uint32_t)(q_off[b + 1] - tok0);
 
@@ -902,254 +1096,59 @@ rerank_kernel(DevIndex ix, const float *__restrict__ q, const uint64_t *__restri
     d_len[tid] = ix.item_n_vec[it];
     d_off[tid] = ix.item_off[it];
   }
-  if (tid == 0) {
-    for (int s = 0; s < kRkStages; s++) {
-      mbar_init(&full[s], kRkThreads - kRkFma);
-      mbar_init(&empty[s], kRkFma);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    s_abort = 0;
-  }
-  for (int i = tid; i < (1 << NBIT) * 32; i += kRkThreads) {
+  for (int i = tid; i < (1 << NBIT) * WC; i += kRkThreads) {
     // bucket v sits in the top NBIT bits of byte v << (8 - NBIT), position 0
-    const uint32_t v = (uint32_t)i >> 5;
-    wrep[i] = ix.lut[((v << (8 - NBIT)) & 0xffu) * VPB];
+    const uint32_t v = (uint32_t)i / WC;
+    wtab[i] = ix.lut[((v << (8 - NBIT)) & 0xffu) * VPB];
   }
-  for (int i = tid; i < kMaxQueryTok * kRkDocs; i += kRkThreads) best[i] = f2si(-INFINITY);
   __syncthreads();
-  if (warp == 0) {  // padded token offsets of the docs (warp scan)
+  if (warp == 0) {  // token offsets of the docs (warp scan)
     uint32_t carry = 0;
-    if (lane == 0) d_pp[0] = 0;
+    if (lane == 0) d_pref[0] = 0;
     for (uint32_t base = 0; base < nd; base += 32) {
-      uint32_t v = base + lane < nd ? (d_len[base + lane] + 3u) & ~3u : 0u;
+      uint32_t v = base + lane < nd ? d_len[base + lane] : 0u;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t t = __shfl_up_sync(kFull, v, o);
         if (lane >= o) v += t;
       }
-      if (base + lane < nd) d_pp[base + lane + 1] = carry + v;
+      if (base + lane < nd) d_pref[base + lane + 1] = carry + v;
       carry += __shfl_sync(kFull, v, 31);
     }
   }
-  __syncthreads();
-  const uint32_t Tp = d_pp[nd];
-  const uint32_t n_tiles = (Tp + kRkTile - 1) / kRkTile;
-  const uint32_t n_pass = (nq + kRkQ - 1) / kRkQ;
-  const uint32_t total = n_tiles * NCH;  // ring chunks per pass
-
-  if (warp >= kRkFma / 32) {
-    // ---------------- decoders (kRkRegDec registers) ----------------
-    // thread pt decodes tile positions pt and pt + 256 of every chunk; the
-    // loads of chunk i + 1 are in flight while chunk i is decoded, and the
-    // tokens (codes, residual rows) of tile t + 1 are located during tile t
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kRkRegDec));
-    const uint32_t pt = (uint32_t)(tid - kRkFma);
-    uint32_t code[2], code_n[2];
-    uint64_t vix[2], vix_n[2];
-    // tile tl's tokens of this thread; past a doc's last token (padding) or
-    // past the last doc: some valid token, whose values the FMA warps mask
-    auto locate = [&](uint32_t tl, uint32_t (&cd)[2], uint64_t (&vx)[2]) {
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const uint32_t g = kRkTile * tl + (kRkTile / 2) * j + pt;
-        uint64_t v = d_off[0];
-        if (g < Tp) {
-          const uint32_t d = find_seg(d_pp, (int)nd, g);
-          v = d_off[d] + min(g - d_pp[d], d_len[d] - 1u);
-        }
-        vx[j] = v;
-        cd[j] = __ldg(ix.vq_code + v);
-      }
-    };
-    auto issue = [&](const uint32_t (&cd)[2], const uint64_t (&vx)[2], uint32_t c,
-                     float4 (&cv)[2][4], uint32_t (&rw)[2][RW]) {
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const float4 *cp = reinterpret_cast<const float4 *>(ix.centroid + (size_t)cd[j] * kDim) + 4 * c;
-#pragma unroll
-        for (int u = 0; u < 4; u++) cv[j][u] = __ldg(cp + u);
-        const uint8_t *rp = ix.residual + vx[j] * ix.bytes_per_vec + (size_t)c * CB;
-        if constexpr (CB == 2) {
-          rw[j][0] = __ldg(reinterpret_cast<const unsigned short *>(rp));
-        } else if constexpr (CB == 4) {
-          rw[j][0] = __ldg(reinterpret_cast<const uint32_t *>(rp));
-        } else if constexpr (CB == 8) {
-          const uint2 t = __ldg(reinterpret_cast<const uint2 *>(rp));
-          rw[j][0] = t.x;
-          rw[j][1] = t.y;
-        } else {
-          const uint4 t = __ldg(reinterpret_cast<const uint4 *>(rp));
-          rw[j][0] = t.x;
-          rw[j][1] = t.y;
-          rw[j][2] = t.z;
-          rw[j][3] = t.w;
-        }
-      }
-    };
-    bool ok = true;
-    uint32_t base = 0;  // ring chunk counter at the start of the pass
-    // decode chunk q of the pass (values in cv / rw) into its ring stage
-    auto put = [&](uint32_t q, const float4 (&cv)[2][4], const uint32_t (&rw)[2][RW]) {
-      const uint32_t gq = base + q;
-      const uint32_t s = gq % kRkStages;
-      if (gq >= (uint32_t)kRkStages &&
-          !__all_sync(kFull, mbar_wait_sleep(&empty[s], ((gq / kRkStages) + 1) & 1, wait_ns))) {
-        ok = false;
-        return;
-      }
-      float *xs = ring + s * (kRkChunk * kRkTile) + pt;
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const float cc[16] = {cv[j][0].x, cv[j][0].y, cv[j][0].z, cv[j][0].w,
-                              cv[j][1].x, cv[j][1].y, cv[j][1].z, cv[j][1].w,
-                              cv[j][2].x, cv[j][2].y, cv[j][2].z, cv[j][2].w,
-                              cv[j][3].x, cv[j][3].y, cv[j][3].z, cv[j][3].w};
-#pragma unroll
-        for (int kk = 0; kk < kRkChunk; kk++) {
-          // dim 16c + kk: byte kk / VPB of the chunk, most significant bits first
-          const int gbit = 8 * (kk / VPB) + 8 - NBIT * (kk % VPB + 1);
-          const uint32_t v = (rw[j][gbit >> 5] >> (gbit & 31)) & MASK;
-          xs[kk * kRkTile + (kRkTile / 2) * j] = __fadd_rn(cc[kk], wrep[v * 32 + lane]);
-        }
-      }
-      mbar_arrive(&full[s]);
-      if (__any_sync(kFull, s_abort != 0)) ok = false;
-    };
-    // the loads of chunk q + 1 (the next tile's first chunk after chunk 7)
-    auto prefetch = [&](uint32_t q, float4 (&cv)[2][4], uint32_t (&rw)[2][RW]) {
-      if (q + 1 >= total) return;
-      if ((q + 1) % NCH != 0) issue(code, vix, (q + 1) % NCH, cv, rw);
-      else issue(code_n, vix_n, 0, cv, rw);
-    };
-    float4 cva[2][4], cvb[2][4];
-    uint32_t rwa[2][RW], rwb[2][RW];
-    for (uint32_t pass = 0; ok && pass < n_pass; pass++, base += total) {
-      locate(0, code, vix);
-      issue(code, vix, 0, cva, rwa);
-      if (n_tiles > 1) locate(1, code_n, vix_n);
-      for (uint32_t q = 0; ok && q < total; q += 2) {
-        // even chunk q: values in a; a tile starts at every multiple of 8
-        if (q % NCH == 0 && q > 0) {
-          const uint32_t tl = q / NCH;
-#pragma unroll
-          for (int j = 0; j < 2; j++) {
-            code[j] = code_n[j];
-            vix[j] = vix_n[j];
-          }
-          if (tl + 1 < n_tiles) locate(tl + 1, code_n, vix_n);
-        }
-        prefetch(q, cvb, rwb);
-        put(q, cva, rwa);
-        if (!ok || q + 1 >= total) break;
-        // odd chunk q + 1: values in b
-        prefetch(q + 1, cva, rwa);
-        put(q + 1, cvb, rwb);
-      }
+  const RkCta cta{Qs, wtab, xs + warp * (kRkStages * kRkTile * kRkChunk), codes[warp], toks[warp],
+                  best, d_pref, d_off, nd, 0u};
+  float sum = 0.0f;  // doc tid's score so far (token order)
+  for (uint32_t t0 = 0; t0 < nq; t0 += kRkQ) {
+    const uint32_t np = min((uint32_t)kRkQ, nq - t0);
+    // query tokens t0 .. t0 + 31 -> Qs[dim][token] (zero past the last token)
+    for (int i = tid; i < kDim / 4 * kRkQ; i += kRkThreads) {
+      const int j = i % kRkQ, k4 = i / kRkQ;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if ((uint32_t)j < np) v = __ldg(reinterpret_cast<const float4 *>(q + (tok0 + t0 + j) * kDim) + k4);
+      Qs[(4 * k4 + 0) * kRkQ + j] = v.x;
+      Qs[(4 * k4 + 1) * kRkQ + j] = v.y;
+      Qs[(4 * k4 + 2) * kRkQ + j] = v.z;
+      Qs[(4 * k4 + 3) * kRkQ + j] = v.w;
     }
-    if (!ok && lane == 0) {
-      atomicOr(err, 32u);
-      s_abort = 1;
-    }
-  } else {
-    // ---------------- FMA warps (kRkRegFma registers) ----------------
-    // Every FMA warp executes the same sequence of named barriers (two per
-    // pass and one at the end): a warp's own failure only skips its work.
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRkRegFma));
-    const uint32_t qg = (uint32_t)warp & 1u;
-    const uint32_t tb = 128u * ((uint32_t)warp >> 1) + 4u * lane;
-    uint32_t it = 0;  // ring chunk counter (continues across tiles and passes)
-    bool ok = true;
-    for (uint32_t pass = 0; pass < n_pass; pass++) {
-      // query tokens 32 pass .. +32 -> Qs[dim][token] (zero past the last token)
-      for (int i = tid; i < kDim / 4 * kRkQ; i += kRkFma) {
-        const int j = i % kRkQ, k4 = i / kRkQ;
-        const uint32_t t = kRkQ * pass + j;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < nq) v = __ldg(reinterpret_cast<const float4 *>(q + (tok0 + t) * kDim) + k4);
-        Qs[(4 * k4 + 0) * kRkQ + j] = v.x;
-        Qs[(4 * k4 + 1) * kRkQ + j] = v.y;
-        Qs[(4 * k4 + 2) * kRkQ + j] = v.z;
-        Qs[(4 * k4 + 3) * kRkQ + j] = v.w;
-      }
-      fma_bar_sync();
-      for (uint32_t tl = 0; ok && tl < n_tiles; tl++) {
-        const uint32_t g0 = kRkTile * tl + tb;
-        int doc = -1;
-        uint32_t nval = 0;
-        if (g0 < Tp) {
-          doc = (int)find_seg(d_pp, (int)nd, g0);
-          nval = min(4u, d_len[doc] - (g0 - d_pp[doc]));
-        }
-        float acc[16][4];
-#pragma unroll
-        for (int i = 0; i < 16; i++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-        for (int c = 0; c < NCH; c++, it++) {
-          const uint32_t s = it % kRkStages;
-          if (!__all_sync(kFull, mbar_wait_sleep(&full[s], (it / kRkStages) & 1, wait_ns)) ||
-              __any_sync(kFull, s_abort != 0)) {
-            ok = false;
-            break;
-          }
-          const float *xs = ring + s * (kRkChunk * kRkTile) + tb;
-          const float *qs = Qs + (kRkChunk * c) * kRkQ + 16 * qg;
-#pragma unroll
-          for (int kk = 0; kk < kRkChunk; kk++) {
-            const float4 x = *reinterpret_cast<const float4 *>(xs + kk * kRkTile);
-            float a[16];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-              const float4 t = *reinterpret_cast<const float4 *>(qs + kk * kRkQ + 4 * u);
-              a[4 * u] = t.x;
-              a[4 * u + 1] = t.y;
-              a[4 * u + 2] = t.z;
-              a[4 * u + 3] = t.w;
-            }
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-              acc[i][0] = __fmaf_rn(a[i], x.x, acc[i][0]);
-              acc[i][1] = __fmaf_rn(a[i], x.y, acc[i][1]);
-              acc[i][2] = __fmaf_rn(a[i], x.z, acc[i][2]);
-              acc[i][3] = __fmaf_rn(a[i], x.w, acc[i][3]);
-            }
-          }
-          mbar_arrive(&empty[s]);
-        }
-        if (!ok) {
-          if (lane == 0) {
-            atomicOr(err, 32u);
-            s_abort = 1;
-          }
-          break;
-        }
-        // max over the thread's valid tokens (one doc), then over the lanes of that doc
-        const unsigned grp = __match_any_sync(kFull, doc);
-        const bool lead = lane == __ffs(grp) - 1;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-          int m = f2si(-INFINITY);
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if ((uint32_t)j < nval) m = max(m, f2si(acc[i][j]));
-          m = __reduce_max_sync(grp, m);
-          const uint32_t qt = kRkQ * pass + 16u * qg + i;
-          if (doc >= 0 && lead && qt < nq) atomicMax(&best[qt * kRkDocs + doc], m);
-        }
-      }
-      fma_bar_sync();  // Qs is reloaded by the next pass; best is complete after the last
-    }
-    if (tid < (int)nd && !s_abort) {  // FMA threads 0 .. nd - 1
+    for (int i = tid; i < (int)nd * (kRkQ + 1); i += kRkThreads) best[i] = f2si(-INFINITY);
+    __syncthreads();
+    RkCta pc = cta;
+    pc.T = d_pref[nd];
+    if (np <= 16) rk_warp_pass<NBIT, 16>(ix, pc, np);
+    else rk_warp_pass<NBIT, 32>(ix, pc, np);
+    __syncthreads();
+    if (tid < (int)nd) {
       const bool clamp = semantics == 1 && d_len[tid] < ix.max_item_n_vec;
-      float s = 0.0f;
-      for (uint32_t t = 0; t < nq; t++) {
-        float m = si2f(best[t * kRkDocs + tid]);
+      for (uint32_t t = 0; t < np; t++) {
+        float m = si2f(best[tid * (kRkQ + 1) + t]);
         if (clamp) m = fmaxf(m, 0.0f);
-        s = __fadd_rn(s, m);
+        sum = __fadd_rn(sum, m);
       }
-      exact[(size_t)b * probe_topk + d0 + tid] = s;
     }
+    __syncthreads();  // Qs and best are rewritten by the next pass
   }
+  if (tid < (int)nd) exact[(size_t)b * probe_topk + d0 + tid] = sum;
 }
 
 // ---------------------------------------------------------------------
@@ -1296,38 +1295,17 @@ topk_select_kernel(const uint32_t *__restrict__ short_id, const float *__restric
 // ---------------------------------------------------------------------
 // host-side launchers
 // ---------------------------------------------------------------------
-// The register split of rerank_kernel (setmaxnreg) hands the FMA warps' and
-// decoders' shares out of the allocation the CTA was launched with; it is
-// only valid when that allocation is kRkRegLaunch per thread (a smaller one
-// would leave setmaxnreg.inc waiting), so the library refuses to run a build
-// that compiled to another count.
-template <typename K>
-static cudaError_t check_rk_registers(K kernel) {
-  cudaFuncAttributes a;
-  const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
-  if (e != cudaSuccess) return e;
-  return a.numRegs == kRkRegLaunch ? cudaSuccess : cudaErrorInvalidKernelImage;
-}
-
 cudaError_t configure_kernels() {
   cudaError_t e = cudaFuncSetAttribute(probe_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kProbeSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(1));
   if (e != cudaSuccess) return e;
-  e = check_rk_registers(rerank_kernel<1>);
-  if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(2));
-  if (e != cudaSuccess) return e;
-  e = check_rk_registers(rerank_kernel<2>);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(4));
   if (e != cudaSuccess) return e;
-  e = check_rk_registers(rerank_kernel<4>);
-  if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(8));
-  if (e != cudaSuccess) return e;
-  e = check_rk_registers(rerank_kernel<8>);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(filter_hash_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)hash_smem_bytes(1));
@@ -1452,17 +1430,31 @@ cudaError_t launch_filter_hash(const DevIndex &ix, const uint32_t *probe_id,
   return cudaGetLastError();
 }
 
+// Shortlisted docs per CTA of the exact rerank: kRkDocs for grids that fill
+// the GPU several times over, fewer (down to the 4 whose tokens are about one
+// tile per warp) while n_query * windows stays within two waves of CTAs: a
+// wide window would leave most SMs idle (one query, 200 docs: 232 us in 4
+// CTAs, 25 us in 50).
+static uint32_t rerank_docs(uint32_t n_query, uint32_t n_docs, int n_sm) {
+  uint32_t docs = kRkDocs;
+  while (docs > 4 &&
+         (uint64_t)n_query * ((n_docs + docs / 2 - 1) / (docs / 2)) <= 4ull * (uint32_t)n_sm)
+    docs /= 2;
+  return docs;
+}
+
 cudaError_t launch_rerank(const DevIndex &ix, const float *q, const uint64_t *q_off,
                           uint32_t n_query, const uint32_t *short_id,
                           const uint32_t *n_short, uint32_t probe_topk,
-                          int semantics, float *exact, unsigned *err, cudaStream_t st,
-                          int *n_launch, uint64_t wait_ns) {
+                          int semantics, float *exact, int n_sm, cudaStream_t st,
+                          int *n_launch) {
   if (n_query == 0 || probe_topk == 0) return cudaSuccess;
-  dim3 grid((probe_topk + kRkDocs - 1) / kRkDocs, n_query);
+  const uint32_t docs = rerank_docs(n_query, probe_topk, n_sm);
+  dim3 grid((probe_topk + docs - 1) / docs, n_query);
   const size_t sm = rk_smem_bytes((int)ix.n_bit);
 #define MVR_RK(NB)                                                                              \
   rerank_kernel<NB><<<grid, kRkThreads, sm, st>>>(ix, q, q_off, short_id, n_short, probe_topk, \
-                                                  semantics, exact, err, wait_ns)
+                                                  docs, semantics, exact)
   switch (ix.n_bit) {
     case 1: MVR_RK(1); break;
     case 2: MVR_RK(2); break;

@@ -46,27 +46,4 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
   }
 }
 
-// The same bounded wait, but a thread whose phase is not complete sleeps in
-// try_wait (up to hint_ns per attempt, woken when the phase completes)
-// instead of polling: for waits that are long by design, where polling warps
-// would take issue slots from the warps they wait for.
-__device__ __forceinline__ bool mbar_wait_sleep(uint64_t *bar, uint32_t parity,
-                                                uint64_t limit_ns = kWaitNs,
-                                                uint32_t hint_ns = 20000u) {
-  const uint32_t a = smem_u32(bar);
-  uint64_t t0 = 0;
-  for (uint32_t i = 0;; i++) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity), "r"(hint_ns)
-        : "memory");
-    if (done) return true;
-    if (i == 0) t0 = global_ns();
-    else if (global_ns() - t0 > limit_ns) return false;
-  }
-}
-
 }  // namespace mvr
