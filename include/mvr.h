@@ -338,21 +338,29 @@ int mvr_unpack_buckets(mvr_index *h, const uint64_t *vec_id, uint64_t n,
  *      ResidualScalarQuantizationPackGPU.hpp:30-80) ---- */
 
 /* code[i] = argmax_c dot(vec_i, centroid_c), lowest id on ties; score[i]
- * (nullable) = that max + 1.  FP32, canonical dot order. */
+ * (nullable) = that max + 1.  FP32, canonical dot order: BF16 tensor-core
+ * scoring lists every centroid that could be the best (by a bound on its own
+ * error), the listed ones are recomputed in FP32, and vectors whose bound or
+ * list does not hold out are scanned in FP32. */
 int mvr_assign_device(const float *d_vec, uint64_t n_vec,
                       const float *d_centroid, uint32_t n_centroid,
                       uint32_t dim, uint32_t *d_code, float *d_score,
                       void *cuda_stream);
 
-/* mvr_assign_device on the tensor cores, for large builds: BF16 tcgen05
- * scoring keeps each vector's 16 best centroids per centroid split, which are
- * re-scored with the canonical FP32 dot; code[i] is the best of those (equal
- * to mvr_assign_device's unless the true best missed the BF16 candidates),
- * score[i] (nullable) its FP32 score + 1. */
+/* The same function (kept for callers of its name). */
 int mvr_assign_tc_device(const float *d_vec, uint64_t n_vec,
                          const float *d_centroid, uint32_t n_centroid,
                          uint32_t dim, uint32_t *d_code, float *d_score,
                          void *cuda_stream);
+
+/* The same with the caller's device workspace (256-byte aligned, at least
+ * mvr_assign_work_bytes of the current device) instead of one allocated and
+ * freed by the call. */
+int mvr_assign_work_bytes(uint64_t n_vec, uint32_t n_centroid, size_t *bytes);
+int mvr_assign_work_device(const float *d_vec, uint64_t n_vec,
+                           const float *d_centroid, uint32_t n_centroid,
+                           uint32_t dim, uint32_t *d_code, float *d_score,
+                           void *d_work, size_t work_bytes, void *cuda_stream);
 
 /* Packed residual bytes (MSB-first, bucket = #cutoffs <= vec - centroid):
  * out [n_vec * dim*n_bit/8]. */

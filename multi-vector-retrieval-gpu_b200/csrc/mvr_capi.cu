@@ -113,16 +113,15 @@ struct Workspace {
   uint32_t *qcnt = nullptr, *ovf = nullptr;  // [slots] hash-filter counters / overflow flags
   // per batch
   uint32_t batch_slots = 0, tok_cap = 0, np_cap = 0, short_cap = 0, topk_cap = 0;
-  size_t part_cap = 0;
+  size_t ent_cap = 0, gid_cap = 0, cnt_cap = 0, flag_cap = 0, part_cap = 0;  // centroid scoring (ProbeBufs)
+  ProbeBufs probe{};
   float *q = nullptr, *q2 = nullptr;  // query tokens (host-buffer calls: two, alternating)
-  uint32_t *probe_id = nullptr, *part_id = nullptr;
-  float *probe_s = nullptr, *part_s = nullptr;
+  uint32_t *probe_id = nullptr;
+  float *probe_s = nullptr;
   uint32_t *short_id = nullptr, *n_short = nullptr;
   float *short_approx = nullptr, *exact = nullptr;
   float *out_s = nullptr;
   uint32_t *out_id = nullptr;
-  size_t cand_cap = 0;            // tensor-core probe candidates (BF16 path)
-  uint32_t *cand = nullptr;
   uint32_t r_cap = 0;             // FP32 re-score of the top-R (BF16 path)
   uint32_t *r_id = nullptr, *n_r = nullptr;
   float *r_score = nullptr, *r_exact = nullptr;
@@ -160,6 +159,7 @@ struct mvr_index {
   void *cen_bf16 = nullptr;      // [C][128] BF16 centroid rows
   void *lut_bf16 = nullptr;      // [256][8/b] BF16 decode table
   void *cen_sw = nullptr;        // [C_pad/128][32 KB] swizzled BF16 centroid tiles
+  float *cen_bounds = nullptr;   // max |c|, max |c - bf16(c)| over the centroids
   void *cen_perm = nullptr;      // [C][64] bf16x2 centroid rows, TMEM-rerank K order (b <= 2)
   TmWeights tw_bf16{};           // weight tables of the BF16 tensor-memory MaxSim (b <= 2)
   float x_bound = 0.f;           // bound on the norm of every decoded doc token
@@ -242,18 +242,19 @@ struct mvr_index {
     ws.pr_slots = ws.pr_short = ws.pr_keep = 0;
   }
   void free_batch() {
-    for (void *p : {(void *)ws.q, (void *)ws.q2, (void *)ws.probe_id, (void *)ws.part_id, (void *)ws.probe_s,
-                    (void *)ws.part_s, (void *)ws.short_id, (void *)ws.n_short,
+    for (void *p : {(void *)ws.q, (void *)ws.q2, (void *)ws.probe_id, (void *)ws.probe_s,
+                    (void *)ws.probe.part_id, (void *)ws.probe.part_s, (void *)ws.probe.ent, (void *)ws.probe.gid,
+                    (void *)ws.probe.cnt, (void *)ws.probe.eps2, (void *)ws.probe.flags,
+                    (void *)ws.short_id, (void *)ws.n_short,
                     (void *)ws.short_approx, (void *)ws.exact, (void *)ws.out_s, (void *)ws.out_id,
-                    (void *)ws.r_id, (void *)ws.n_r, (void *)ws.r_score, (void *)ws.r_exact,
-                    (void *)ws.cand})
+                    (void *)ws.r_id, (void *)ws.n_r, (void *)ws.r_score, (void *)ws.r_exact})
       dfree(p);
-    ws.cand = nullptr;
-    ws.cand_cap = 0;
+    ws.probe = ProbeBufs{};
+    ws.ent_cap = ws.gid_cap = ws.cnt_cap = ws.flag_cap = 0;
     ws.r_id = ws.n_r = nullptr;
     ws.r_score = ws.r_exact = nullptr;
     ws.r_cap = 0;
-    ws.q = ws.q2 = nullptr; ws.probe_id = ws.part_id = nullptr; ws.probe_s = ws.part_s = nullptr;
+    ws.q = ws.q2 = nullptr; ws.probe_id = nullptr; ws.probe_s = nullptr;
     ws.short_id = ws.n_short = nullptr; ws.short_approx = ws.exact = nullptr;
     ws.out_s = nullptr; ws.out_id = nullptr;
     ws.batch_slots = ws.tok_cap = ws.np_cap = ws.short_cap = ws.topk_cap = 0;
@@ -329,29 +330,36 @@ int ensure_prune(mvr_index *h, uint32_t slots, uint32_t short_cap, uint32_t keep
 }
 
 int ensure_batch(mvr_index *h, uint32_t slots, uint32_t tok_cap, uint32_t nprobe,
-                 uint32_t short_cap, uint32_t topk, size_t part_need, uint32_t r_cap,
-                 size_t cand_need) {
+                 uint32_t short_cap, uint32_t topk, const ProbePlan &need, uint32_t r_cap) {
   Workspace &w = h->ws;
   if (w.batch_slots >= slots && w.tok_cap >= tok_cap && w.np_cap >= nprobe &&
-      w.short_cap >= short_cap && w.topk_cap >= topk && w.part_cap >= part_need &&
-      w.r_cap >= r_cap && w.cand_cap >= cand_need)
+      w.short_cap >= short_cap && w.topk_cap >= topk && w.ent_cap >= need.n_ent &&
+      w.gid_cap >= need.n_gid &&
+      w.cnt_cap >= need.n_cnt && w.flag_cap >= need.n_flag && w.part_cap >= need.n_part &&
+      w.r_cap >= r_cap)
     return MVR_OK;
   r_cap = std::max(r_cap, w.r_cap);
-  cand_need = std::max(cand_need, w.cand_cap);
   const uint32_t s = std::max(slots, w.batch_slots);
   tok_cap = std::max(tok_cap, w.tok_cap);
   nprobe = std::max(nprobe, w.np_cap);
   short_cap = std::max(short_cap, w.short_cap);
   topk = std::max(topk, w.topk_cap);
-  part_need = std::max(part_need, w.part_cap);
+  const size_t n_ent = std::max(need.n_ent, w.ent_cap), n_cnt = std::max(need.n_cnt, w.cnt_cap);
+  const size_t n_gid = std::max(need.n_gid, w.gid_cap);
+  const size_t n_flag = std::max(need.n_flag, w.flag_cap), n_part = std::max(need.n_part, w.part_cap);
   h->free_batch();
   h->ws_gen++;
   MVR_TRY(dalloc(&w.q, (size_t)tok_cap * kDim));
   MVR_TRY(dalloc(&w.q2, (size_t)tok_cap * kDim));
   MVR_TRY(dalloc(&w.probe_id, (size_t)tok_cap * nprobe));
   MVR_TRY(dalloc(&w.probe_s, (size_t)tok_cap * nprobe));
-  MVR_TRY(dalloc(&w.part_id, part_need));
-  MVR_TRY(dalloc(&w.part_s, part_need));
+  MVR_TRY(dalloc(&w.probe.ent, n_ent));
+  MVR_TRY(dalloc(&w.probe.gid, n_gid));
+  MVR_TRY(dalloc(&w.probe.cnt, n_cnt));
+  MVR_TRY(dalloc(&w.probe.eps2, (size_t)tok_cap));
+  MVR_TRY(dalloc(&w.probe.flags, n_flag));
+  MVR_TRY(dalloc(&w.probe.part_id, n_part));
+  MVR_TRY(dalloc(&w.probe.part_s, n_part));
   MVR_TRY(dalloc(&w.short_id, (size_t)s * short_cap));
   MVR_TRY(dalloc(&w.short_approx, (size_t)s * short_cap));
   MVR_TRY(dalloc(&w.exact, (size_t)s * short_cap));
@@ -362,15 +370,17 @@ int ensure_batch(mvr_index *h, uint32_t slots, uint32_t tok_cap, uint32_t nprobe
   MVR_TRY(dalloc(&w.r_score, (size_t)s * r_cap));
   MVR_TRY(dalloc(&w.r_exact, (size_t)s * r_cap));
   MVR_TRY(dalloc(&w.n_r, (size_t)s));
-  MVR_TRY(dalloc(&w.cand, cand_need));
-  w.cand_cap = cand_need;
+  w.ent_cap = n_ent;
+  w.gid_cap = n_gid;
+  w.cnt_cap = n_cnt;
+  w.flag_cap = n_flag;
   w.r_cap = r_cap;
   w.batch_slots = s;
   w.tok_cap = tok_cap;
   w.np_cap = nprobe;
   w.short_cap = short_cap;
   w.topk_cap = topk;
-  w.part_cap = part_need;
+  w.part_cap = n_part;
   return MVR_OK;
 }
 
@@ -410,10 +420,20 @@ int ensure_call(mvr_index *h, size_t n_off, size_t n_stat, size_t n_events) {
   return MVR_OK;
 }
 
-size_t part_entries(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, int *splits_out) {
-  const int splits = probe_splits(n_tok, h->dix.n_centroid_pad, h->n_sm);
-  *splits_out = splits;
-  return splits > 1 ? (size_t)splits * n_tok * nprobe : 1;
+// Buffer sizes of the centroid scoring of n_tok tokens, in chunks of probe_chunk
+// (the plans of a full chunk and of the last one).
+void probe_need(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, ProbePlan *need) {
+  auto add = [&](uint32_t T) {
+    const ProbePlan p = probe_plan(T, h->dix.n_centroid, nprobe, h->n_sm);
+    need->n_ent = std::max(need->n_ent, p.n_ent);
+    need->n_gid = std::max(need->n_gid, p.n_gid);
+    need->n_cnt = std::max(need->n_cnt, p.n_cnt);
+    need->n_flag = std::max(need->n_flag, p.n_flag);
+    need->n_part = std::max(need->n_part, p.n_part);
+  };
+  const uint32_t chunk = probe_chunk(nprobe, h->n_sm);
+  if (n_tok >= chunk) add(chunk);
+  if (n_tok % chunk) add(n_tok % chunk);
 }
 
 int check_search_args(const mvr_index *h, uint32_t n_query, uint32_t topk, uint32_t nprobe,
@@ -505,17 +525,12 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
   const uint32_t B = h->batch_cap ? h->batch_cap : default_batch(h);
   const uint32_t n_batch = (n_query + B - 1) / B;
   uint32_t tok_cap = 0;
-  size_t part_need = 1, cand_need = 1;
-  const bool tc_probe = bf16 && nprobe <= 16;  // tensor-core scoring + exact re-score
+  ProbePlan need{};
   for (uint32_t bt = 0; bt < n_batch; bt++) {
     const uint32_t s = bt * B, e = std::min(n_query, s + B);
     const uint32_t T = (uint32_t)(off[e] - off[s]);
     tok_cap = std::max(tok_cap, T);
-    int sp;
-    part_need = std::max(part_need, part_entries(h, T, nprobe, &sp));
-    uint32_t tsp;
-    if (tc_probe)
-      cand_need = std::max(cand_need, (size_t)T * probe_tc_cand_per_token(T, h->dix.n_centroid, h->n_sm, &tsp));
+    probe_need(h, T, nprobe, &need);
   }
   const uint32_t rank_stride = nq_max <= 32 ? 32u : 64u;
   // before the first search: about a third of a mean-length list's docs are
@@ -525,8 +540,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                          : 0.35 * (double)h->dix.n_ele_ivf / std::max(1u, h->dix.n_centroid);
   const uint32_t parts_max = hash_parts(nq_max, nprobe, cpe);
   MVR_TRY(ensure_scratch(h, std::min(B, n_query), rank_stride, parts_max * kHashFill));
-  MVR_TRY(ensure_batch(h, std::min(B, n_query), tok_cap, nprobe, probe_topk, topk, part_need, R,
-                       cand_need));
+  MVR_TRY(ensure_batch(h, std::min(B, n_query), tok_cap, nprobe, probe_topk, topk, need, R));
   MVR_TRY(ensure_call(h, 2 * ((size_t)n_query + n_batch), (size_t)n_query * 3,
                       (size_t)kStages * n_batch + 1));
   if (prune) MVR_TRY(ensure_prune(h, std::min(B, n_query), probe_topk, keep));
@@ -619,16 +633,15 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         qp = query + off[s] * kDim;
       }
       CUDA_TRY(rec(ev(bt, 1)));
-      if (tc_probe) {
-        uint32_t tsp;
-        probe_tc_cand_per_token(T, h->dix.n_centroid, h->n_sm, &tsp);
-        CUDA_TRY(launch_probe_tc(qp, T, h->cen_sw, h->dix.centroid, h->dix.n_centroid, nprobe,
-                                 tsp, w.cand, w.probe_id, w.probe_s, h->d_err, rs, &launches));
-      } else {
-        int splits;
-        part_entries(h, T, nprobe, &splits);
-        CUDA_TRY(launch_probe(h->dix, qp, T, nprobe, splits, w.part_id, w.part_s, w.probe_id,
-                              w.probe_s, rs, &launches));
+      const uint32_t chunk = probe_chunk(nprobe, h->n_sm);
+      for (uint32_t c = 0; c < T; c += chunk) {
+        const uint32_t n = std::min(chunk, T - c);
+        CUDA_TRY(launch_probe(qp + (size_t)c * kDim, n, h->cen_sw, h->dix.centroid,
+                              h->dix.centroid_t, h->dix.n_centroid, h->dix.n_centroid_pad,
+                              h->cen_bounds, nprobe,
+                              probe_plan(n, h->dix.n_centroid, nprobe, h->n_sm), w.probe,
+                              w.probe_id + (size_t)c * nprobe, w.probe_s + (size_t)c * nprobe,
+                              h->n_sm, h->d_err, rs, &launches));
       }
       CUDA_TRY(rec(ev(bt, 2)));
       CUDA_TRY(launch_filter_hash(h->dix, w.probe_id, w.probe_s, nprobe, qo, qo + n_off,
@@ -861,6 +874,8 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
   MVR_TRY(dalloc(&sw, (size_t)d.n_centroid_pad * 256, &h->bufs));
   CUDA_TRY(make_centroid_tiles(d.centroid, d.n_centroid, d.n_centroid_pad / 64, sw, h->stream));
   h->cen_sw = sw;
+  MVR_TRY(dalloc(&h->cen_bounds, 2, &h->bufs));
+  CUDA_TRY(make_centroid_bounds(d.centroid, d.n_centroid, h->cen_bounds, h->stream));
   if (tmem_rerank_supported(d.n_bit) || fp8_rerank_supported(d.n_bit)) {
     float wmax = 0.f;
     for (uint32_t k = 0; k < (1u << d.n_bit); k++) wmax = std::max(wmax, std::fabs(weight[k]));
@@ -1405,93 +1420,127 @@ int mvr_unpack_buckets(mvr_index *h, const uint64_t *vec_id, uint64_t n, uint8_t
   return MVR_OK;
 }
 
-int mvr_assign_device(const float *d_vec, uint64_t n_vec, const float *d_centroid,
-                      uint32_t n_centroid, uint32_t dim, uint32_t *d_code, float *d_score,
-                      void *cuda_stream) {
+// Layout of an assignment call's workspace (byte offsets, 256-aligned).
+namespace {
+struct AssignWork {
+  size_t ct, sw, bounds, err, score, ent, gid, cnt, eps2, flags, part_id, part_s, total;
+};
+int assign_sms(int *n_sm) {
+  int dev = 0;
+  *n_sm = 148;
+  CUDA_TRY(cudaGetDevice(&dev));
+  CUDA_TRY(cudaDeviceGetAttribute(n_sm, cudaDevAttrMultiProcessorCount, dev));
+  return MVR_OK;
+}
+AssignWork assign_work(uint64_t n_vec, uint32_t n_centroid, int n_sm) {
+  AssignWork w{};
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 255) & ~(size_t)255;
+    return o;
+  };
+  const uint64_t chunk = probe_chunk(1, n_sm);
+  const uint32_t first = (uint32_t)std::min(chunk, std::max<uint64_t>(n_vec, 1));
+  ProbePlan p = probe_plan(first, n_centroid, 1, n_sm);
+  const uint32_t last = (uint32_t)(n_vec % chunk);
+  if (n_vec > chunk && last) {
+    const ProbePlan l = probe_plan(last, n_centroid, 1, n_sm);
+    p.n_ent = std::max(p.n_ent, l.n_ent);
+    p.n_gid = std::max(p.n_gid, l.n_gid);
+    p.n_cnt = std::max(p.n_cnt, l.n_cnt);
+    p.n_flag = std::max(p.n_flag, l.n_flag);
+  }
+  w.ct = take((size_t)kDim * ((n_centroid + 127u) / 128u * 128u) * sizeof(float));
+  w.sw = take((size_t)((n_centroid + 127u) / 128u) * 128 * 256);
+  w.bounds = take(2 * sizeof(float));
+  w.err = take(sizeof(unsigned));
+  w.score = take(first * sizeof(float));
+  w.ent = take(p.n_ent * sizeof(float4));
+  w.gid = take(p.n_gid * sizeof(uint32_t));
+  w.cnt = take(p.n_cnt * sizeof(uint32_t));
+  w.eps2 = take(first * sizeof(float));
+  w.flags = take(p.n_flag * sizeof(uint32_t));
+  w.part_id = take(p.n_part * sizeof(uint32_t));
+  w.part_s = take(p.n_part * sizeof(float));
+  w.total = at;
+  return w;
+}
+}  // namespace
+
+int mvr_assign_work_bytes(uint64_t n_vec, uint32_t n_centroid, size_t *bytes) {
+  if (!bytes || n_centroid == 0) return set_err(MVR_ERR_INVALID_ARG, "null argument or no centroids");
+  if (mvr_device_count() == 0) return set_err(MVR_ERR_CUDA, "no CUDA device available");
+  int n_sm;
+  MVR_TRY(assign_sms(&n_sm));
+  *bytes = assign_work(n_vec, n_centroid, n_sm).total;
+  return MVR_OK;
+}
+
+int mvr_assign_work_device(const float *d_vec, uint64_t n_vec, const float *d_centroid,
+                           uint32_t n_centroid, uint32_t dim, uint32_t *d_code, float *d_score,
+                           void *d_work, size_t work_bytes, void *cuda_stream) {
   if (dim != (uint32_t)kDim) return set_err(MVR_ERR_UNSUPPORTED, "dim %u not supported", dim);
-  if (!d_vec || !d_centroid || !d_code || n_centroid == 0)
+  if (!d_vec || !d_centroid || !d_code || !d_work || n_centroid == 0)
     return set_err(MVR_ERR_INVALID_ARG, "null argument or no centroids");
   if (mvr_device_count() == 0) return set_err(MVR_ERR_CUDA, "no CUDA device available");
   cudaStream_t st = (cudaStream_t)cuda_stream;
   CUDA_TRY(configure_kernels());
-  DevIndex d{};
-  d.n_centroid = n_centroid;
-  d.n_centroid_pad = (n_centroid + 127u) / 128u * 128u;
-  float *ct;
-  MVR_TRY(dalloc(&ct, (size_t)kDim * d.n_centroid_pad));
-  std::unique_ptr<void, void (*)(void *)> cg(ct, dfree);
-  CUDA_TRY(launch_transpose_centroid(d_centroid, n_centroid, d.n_centroid_pad, ct, st));
-  d.centroid_t = ct;
-  float *score = d_score;
-  std::unique_ptr<void, void (*)(void *)> sg(nullptr, dfree);
-  if (!score) {
-    const uint64_t chunk_max = std::min<uint64_t>(n_vec, 2ull << 20);
-    MVR_TRY(dalloc(&score, chunk_max));
-    sg.reset(score);
-  }
-  int launches = 0;
-  for (uint64_t s = 0; s < n_vec; s += (2ull << 20)) {  // grid.y <= 32768
-    const uint32_t T = (uint32_t)std::min<uint64_t>(2ull << 20, n_vec - s);
-    CUDA_TRY(launch_probe(d, d_vec + s * kDim, T, 1, 1, nullptr, nullptr, d_code + s,
-                          d_score ? d_score + s : score, st, &launches));
-  }
-  CUDA_TRY(cudaStreamSynchronize(st));
-  return MVR_OK;
-}
-
-int mvr_assign_tc_device(const float *d_vec, uint64_t n_vec, const float *d_centroid,
-                         uint32_t n_centroid, uint32_t dim, uint32_t *d_code, float *d_score,
-                         void *cuda_stream) {
-  if (dim != (uint32_t)kDim) return set_err(MVR_ERR_UNSUPPORTED, "dim %u not supported", dim);
-  if (!d_vec || !d_centroid || !d_code || n_centroid == 0)
-    return set_err(MVR_ERR_INVALID_ARG, "null argument or no centroids");
-  if (mvr_device_count() == 0) return set_err(MVR_ERR_CUDA, "no CUDA device available");
-  cudaStream_t st = (cudaStream_t)cuda_stream;
   CUDA_TRY(configure_tc_kernels());
-  int dev = 0, n_sm = 148;
-  CUDA_TRY(cudaGetDevice(&dev));
-  CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-  // swizzled BF16 centroid tiles (64 centroids x 256 B each)
-  const uint32_t n_tiles = (n_centroid + 63u) / 64u;
-  uint8_t *sw;
-  MVR_TRY(dalloc(&sw, (size_t)n_tiles * 64 * 256));
-  std::unique_ptr<void, void (*)(void *)> swg(sw, dfree);
-  CUDA_TRY(make_centroid_tiles(d_centroid, n_centroid, n_tiles, sw, st));
-  // token chunks of <= 1M (probe grid.y <= 8192); candidate lists sized
-  // for the largest chunk's split count
-  const uint64_t kChunk = 1ull << 20;
-  size_t cand_need = 1;
-  for (uint64_t s = 0; s < n_vec; s += kChunk) {
-    const uint32_t T = (uint32_t)std::min<uint64_t>(kChunk, n_vec - s);
-    uint32_t sp;
-    cand_need = std::max(cand_need, (size_t)T * probe_tc_cand_per_token(T, n_centroid, n_sm, &sp));
-  }
-  uint32_t *cand;
-  MVR_TRY(dalloc(&cand, cand_need));
-  std::unique_ptr<void, void (*)(void *)> cg(cand, dfree);
-  float *score = d_score;
-  std::unique_ptr<void, void (*)(void *)> sg(nullptr, dfree);
-  if (!score) {
-    MVR_TRY(dalloc(&score, std::min<uint64_t>(std::max<uint64_t>(n_vec, 1), kChunk)));
-    sg.reset(score);
-  }
-  unsigned *err;
-  MVR_TRY(dalloc(&err, 1));
-  std::unique_ptr<void, void (*)(void *)> eg(err, dfree);
+  int n_sm;
+  MVR_TRY(assign_sms(&n_sm));
+  const AssignWork a = assign_work(n_vec, n_centroid, n_sm);
+  if (work_bytes < a.total || ((uintptr_t)d_work & 255))
+    return set_err(MVR_ERR_INVALID_ARG, "assignment workspace: %zu bytes, 256-byte aligned, needed",
+                   a.total);
+  uint8_t *base = (uint8_t *)d_work;
+  float *ct = (float *)(base + a.ct), *bounds = (float *)(base + a.bounds);
+  unsigned *err = (unsigned *)(base + a.err);
+  const uint32_t c_pad = (n_centroid + 127u) / 128u * 128u;
+  ProbeBufs w{(float4 *)(base + a.ent),   (uint32_t *)(base + a.gid),
+              (uint32_t *)(base + a.cnt), (float *)(base + a.eps2),
+              (uint32_t *)(base + a.flags), (uint32_t *)(base + a.part_id),
+              (float *)(base + a.part_s)};
+  CUDA_TRY(launch_transpose_centroid(d_centroid, n_centroid, c_pad, ct, st));
+  CUDA_TRY(make_centroid_tiles(d_centroid, n_centroid, c_pad / 64u, base + a.sw, st));
+  CUDA_TRY(make_centroid_bounds(d_centroid, n_centroid, bounds, st));
   CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
   int launches = 0;
-  for (uint64_t s = 0; s < n_vec; s += kChunk) {
-    const uint32_t T = (uint32_t)std::min<uint64_t>(kChunk, n_vec - s);
-    uint32_t sp;
-    probe_tc_cand_per_token(T, n_centroid, n_sm, &sp);
-    CUDA_TRY(launch_probe_tc(d_vec + s * kDim, T, sw, d_centroid, n_centroid, 1, sp, cand,
-                             d_code + s, d_score ? d_score + s : score, err, st, &launches));
+  const uint64_t chunk = probe_chunk(1, n_sm);
+  for (uint64_t s = 0; s < n_vec; s += chunk) {
+    const uint32_t T = (uint32_t)std::min(chunk, n_vec - s);
+    CUDA_TRY(launch_probe(d_vec + s * kDim, T, base + a.sw, d_centroid, ct, n_centroid, c_pad,
+                          bounds, 1, probe_plan(T, n_centroid, 1, n_sm), w, d_code + s,
+                          d_score ? d_score + s : (float *)(base + a.score), n_sm, err, st,
+                          &launches));
   }
   unsigned herr = 0;
   CUDA_TRY(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   if (herr) return set_err(MVR_ERR_CUDA, "tensor-core scoring gave up waiting (flags %u)", herr);
   return MVR_OK;
+}
+
+int mvr_assign_device(const float *d_vec, uint64_t n_vec, const float *d_centroid,
+                      uint32_t n_centroid, uint32_t dim, uint32_t *d_code, float *d_score,
+                      void *cuda_stream) {
+  if (dim != (uint32_t)kDim) return set_err(MVR_ERR_UNSUPPORTED, "dim %u not supported", dim);
+  if (!d_vec || !d_centroid || !d_code || n_centroid == 0)
+    return set_err(MVR_ERR_INVALID_ARG, "null argument or no centroids");
+  size_t bytes = 0;
+  MVR_TRY(mvr_assign_work_bytes(n_vec, n_centroid, &bytes));
+  uint8_t *work;
+  MVR_TRY(dalloc(&work, bytes));
+  std::unique_ptr<void, void (*)(void *)> g(work, dfree);
+  return mvr_assign_work_device(d_vec, n_vec, d_centroid, n_centroid, dim, d_code, d_score, work,
+                                bytes, cuda_stream);
+}
+
+int mvr_assign_tc_device(const float *d_vec, uint64_t n_vec, const float *d_centroid,
+                         uint32_t n_centroid, uint32_t dim, uint32_t *d_code, float *d_score,
+                         void *cuda_stream) {
+  return mvr_assign_device(d_vec, n_vec, d_centroid, n_centroid, dim, d_code, d_score,
+                           cuda_stream);
 }
 
 int mvr_pack_residual_device(const float *d_vec, uint64_t n_vec, const float *d_centroid,

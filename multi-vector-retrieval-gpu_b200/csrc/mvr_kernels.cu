@@ -3,7 +3,7 @@
 // Stage map (reference -> kernel):
 //   centroid scoring S = Q.C^T + 1 and per-token top-nprobe
 //       (GenerateVQScoreCandidatePP.hpp:118-179: cuBLAS SGEMM, thrust +1,
-//        RAFT select_k)                       -> probe_topk_kernel (+ merge)
+//        RAFT select_k)                       -> mvr_tc.cu, probe_scan_kernel
 //   IVF gather, candidate flag/compaction, max-over-probes, sum over tokens,
 //   top-probe_topk shortlist (FilterPP.hpp:19-142, 267-398)
 //                                             -> filter_kernel
@@ -66,8 +66,15 @@ __device__ __forceinline__ void warp_list_insert(float &ls, uint32_t &lid,
 }
 
 // ---------------------------------------------------------------------
-// K1: S = Q.C^T + 1 over a centroid range, running top-nprobe per token.
-// CTA = 64 tokens x (tiles_per_split * 128) centroids, 256 threads.
+// K1 fallback: exact S = Q.C^T + 1 and top-nprobe of the tokens that the
+// tensor-core scan flagged (mvr_tc.cu: a list that overflowed, a bound that is
+// not finite), by FP32 chains over every centroid.  flags[0] = their count,
+// flags[2 ..] one arrival counter per 64-token tile (zeroed by the caller),
+// flags[list_at ..] the tokens.  A persistent grid of one CTA per SM takes
+// (token tile, centroid split) items; few tiles are split over the centroids
+// so that the grid has work, and the last CTA of a tile merges its partial
+// lists.  With nothing flagged, the usual case, every CTA returns at once.
+// Item = 64 tokens x (tiles_per_split * 128) centroids, 256 threads.
 // Thread (warp w, lane l): tokens w*8..w*8+7, centroids l*4..l*4+3 of the
 // current 128-wide tile.  Qs[k][64] and double-buffered Cs[k][128] in smem.
 // ---------------------------------------------------------------------
@@ -77,29 +84,24 @@ constexpr size_t kProbeSmem =
     (size_t)(kDim * kProbeTokTile + 2 * kDim * kProbeCenTile) * sizeof(float);
 
 __global__ void __launch_bounds__(256, 1)
-probe_topk_kernel(const float *__restrict__ q, uint32_t n_tok,
-                  const float *__restrict__ ct, uint32_t n_cent,
-                  uint32_t n_cent_pad, uint32_t nprobe,
-                  uint32_t tiles_per_split, uint32_t *__restrict__ out_id,
-                  float *__restrict__ out_s) {
+probe_scan_kernel(const float *__restrict__ q, const float *__restrict__ ct, uint32_t n_cent,
+                  uint32_t n_cent_pad, uint32_t nprobe, uint32_t *__restrict__ flags,
+                  uint32_t list_at, uint32_t *__restrict__ part_id, float *__restrict__ part_s,
+                  uint32_t *__restrict__ out_id, float *__restrict__ out_s) {
   extern __shared__ __align__(16) float smem[];
   float *Qs = smem;                          // [128][64]
   float *Cs = smem + kDim * kProbeTokTile;   // [2][128][128]
+  __shared__ uint32_t s_last;
+  const uint32_t n_tok = flags[0];
+  if (n_tok == 0) return;
+  const uint32_t *list = flags + list_at;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t t0 = blockIdx.y * kProbeTokTile;
+  const int np = (int)nprobe;
   const uint32_t n_tiles = n_cent_pad / kProbeCenTile;
-  const uint32_t tile_begin = blockIdx.x * tiles_per_split;
-  const uint32_t tile_end = min(n_tiles, tile_begin + tiles_per_split);
-
-  for (int i = tid; i < kProbeTokTile * (kDim / 4); i += 256) {
-    const int t = i % kProbeTokTile, k4 = i / kProbeTokTile;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t0 + t < n_tok) v = __ldg(reinterpret_cast<const float4 *>(q + (size_t)(t0 + t) * kDim) + k4);
-    Qs[(k4 * 4 + 0) * kProbeTokTile + t] = v.x;
-    Qs[(k4 * 4 + 1) * kProbeTokTile + t] = v.y;
-    Qs[(k4 * 4 + 2) * kProbeTokTile + t] = v.z;
-    Qs[(k4 * 4 + 3) * kProbeTokTile + t] = v.w;
-  }
+  const uint32_t tok_tiles = (n_tok + kProbeTokTile - 1) / kProbeTokTile;
+  uint32_t splits = min(n_tiles, max(1u, gridDim.x / tok_tiles));
+  const uint32_t tiles_per_split = (n_tiles + splits - 1) / splits;
+  splits = (n_tiles + tiles_per_split - 1) / tiles_per_split;
 
   auto load_tile = [&](uint32_t tile, int buf) {
     float *dst = Cs + buf * kDim * kProbeCenTile;
@@ -114,106 +116,131 @@ probe_topk_kernel(const float *__restrict__ q, uint32_t n_tok,
     cp_async_commit();
   };
 
-  float Ls[8], thr_s[8];
-  uint32_t Lid[8], thr_id[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    Ls[i] = -INFINITY; Lid[i] = 0xffffffffu;
-    thr_s[i] = -INFINITY; thr_id[i] = 0xffffffffu;
-  }
-  const int np = (int)nprobe;
-
-  if (tile_begin < tile_end) load_tile(tile_begin, 0);
-  for (uint32_t tile = tile_begin; tile < tile_end; tile++) {
-    const int buf = (tile - tile_begin) & 1;
-    if (tile + 1 < tile_end) {
-      load_tile(tile + 1, buf ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+  for (uint32_t item = blockIdx.x; item < tok_tiles * splits; item += gridDim.x) {
+    const uint32_t tt = item / splits, t0 = tt * kProbeTokTile;
+    const uint32_t tile_begin = (item % splits) * tiles_per_split;
+    const uint32_t tile_end = min(n_tiles, tile_begin + tiles_per_split);
+    for (int i = tid; i < kProbeTokTile * (kDim / 4); i += 256) {
+      const int t = i % kProbeTokTile, k4 = i / kProbeTokTile;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t0 + t < n_tok)
+        v = __ldg(reinterpret_cast<const float4 *>(q + (size_t)list[t0 + t] * kDim) + k4);
+      Qs[(k4 * 4 + 0) * kProbeTokTile + t] = v.x;
+      Qs[(k4 * 4 + 1) * kProbeTokTile + t] = v.y;
+      Qs[(k4 * 4 + 2) * kProbeTokTile + t] = v.z;
+      Qs[(k4 * 4 + 3) * kProbeTokTile + t] = v.w;
     }
-    __syncthreads();
+    float Ls[8], thr_s[8];
+    uint32_t Lid[8], thr_id[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      Ls[i] = -INFINITY; Lid[i] = 0xffffffffu;
+      thr_s[i] = -INFINITY; thr_id[i] = 0xffffffffu;
+    }
 
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-    const float *qs = Qs + warp * 8;
-    const float *cs = Cs + buf * kDim * kProbeCenTile + lane * 4;
-#pragma unroll 4
-    for (int k = 0; k < kDim; k++) {
-      const float4 a0 = *reinterpret_cast<const float4 *>(qs + k * kProbeTokTile);
-      const float4 a1 = *reinterpret_cast<const float4 *>(qs + k * kProbeTokTile + 4);
-      const float4 b = *reinterpret_cast<const float4 *>(cs + k * kProbeCenTile);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bb[4] = {b.x, b.y, b.z, b.w};
+    load_tile(tile_begin, 0);
+    for (uint32_t tile = tile_begin; tile < tile_end; tile++) {
+      const int buf = (tile - tile_begin) & 1;
+      if (tile + 1 < tile_end) {
+        load_tile(tile + 1, buf ^ 1);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncthreads();
+
+      float acc[8][4];
 #pragma unroll
       for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = __fmaf_rn(a[i], bb[j], acc[i][j]);
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+      const float *qs = Qs + warp * 8;
+      const float *cs = Cs + buf * kDim * kProbeCenTile + lane * 4;
+#pragma unroll 4
+      for (int k = 0; k < kDim; k++) {
+        const float4 a0 = *reinterpret_cast<const float4 *>(qs + k * kProbeTokTile);
+        const float4 a1 = *reinterpret_cast<const float4 *>(qs + k * kProbeTokTile + 4);
+        const float4 b = *reinterpret_cast<const float4 *>(cs + k * kProbeCenTile);
+        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[i][j] = __fmaf_rn(a[i], bb[j], acc[i][j]);
+      }
+
+      const uint32_t c0 = tile * kProbeCenTile + lane * 4;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float s = __fadd_rn(acc[i][j], 1.0f);
+          const uint32_t id = c0 + j;
+          const bool cand = id < n_cent && better(s, id, thr_s[i], thr_id[i]);
+          unsigned m = __ballot_sync(kFull, cand);
+          while (m) {
+            const int src = __ffs(m) - 1;
+            m &= m - 1;
+            const float ns = __shfl_sync(kFull, s, src);
+            const uint32_t nid = __shfl_sync(kFull, id, src);
+            if (better(ns, nid, thr_s[i], thr_id[i]))
+              warp_list_insert(Ls[i], Lid[i], thr_s[i], thr_id[i], ns, nid, lane, np);
+          }
+        }
+      }
+      __syncthreads();
     }
 
-    const uint32_t c0 = tile * kProbeCenTile + lane * 4;
+    if (splits == 1) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+      for (int i = 0; i < 8; i++) {
+        const uint32_t t = t0 + warp * 8 + i;
+        if (t < n_tok && lane < np) {
+          out_id[(size_t)list[t] * nprobe + lane] = Lid[i];
+          out_s[(size_t)list[t] * nprobe + lane] = Ls[i];
+        }
+      }
+    } else {
+      // items are at most gridDim.x here: one partial slot of 64 lists each
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float s = __fadd_rn(acc[i][j], 1.0f);
-        const uint32_t id = c0 + j;
-        const bool cand = id < n_cent && better(s, id, thr_s[i], thr_id[i]);
-        unsigned m = __ballot_sync(kFull, cand);
-        while (m) {
-          const int src = __ffs(m) - 1;
-          m &= m - 1;
-          const float ns = __shfl_sync(kFull, s, src);
-          const uint32_t nid = __shfl_sync(kFull, id, src);
-          if (better(ns, nid, thr_s[i], thr_id[i]))
-            warp_list_insert(Ls[i], Lid[i], thr_s[i], thr_id[i], ns, nid, lane, np);
+      for (int i = 0; i < 8; i++) {
+        if (lane < np) {
+          const size_t at = ((size_t)item * kProbeTokTile + warp * 8 + i) * nprobe + lane;
+          part_id[at] = Lid[i];
+          part_s[at] = Ls[i];
+        }
+      }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_last = atomicAdd(flags + 2 + tt, 1u) == splits - 1 ? 1u : 0u;
+      __syncthreads();
+      if (s_last) {
+        __threadfence();
+        for (int i = 0; i < 8; i++) {
+          const uint32_t t = t0 + warp * 8 + i;
+          if (t >= n_tok) break;
+          float ls = -INFINITY, ts = -INFINITY;
+          uint32_t lid = 0xffffffffu, tid_ = 0xffffffffu;
+          for (uint32_t sp = 0; sp < splits; sp++) {
+            const size_t base =
+                (((size_t)tt * splits + sp) * kProbeTokTile + warp * 8 + i) * nprobe;
+            float ps = -INFINITY;
+            uint32_t pid = 0xffffffffu;
+            if (lane < np) { ps = __ldcg(part_s + base + lane); pid = __ldcg(part_id + base + lane); }
+            for (int e = 0; e < np; e++) {
+              const float ns = __shfl_sync(kFull, ps, e);
+              const uint32_t nid = __shfl_sync(kFull, pid, e);
+              if (!better(ns, nid, ts, tid_)) break;  // partial lists are sorted
+              warp_list_insert(ls, lid, ts, tid_, ns, nid, lane, np);
+            }
+          }
+          if (lane < np) {
+            out_id[(size_t)list[t] * nprobe + lane] = lid;
+            out_s[(size_t)list[t] * nprobe + lane] = ls;
+          }
         }
       }
     }
-    __syncthreads();
-  }
-
-  const size_t split_off = (size_t)blockIdx.x * n_tok * nprobe;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint32_t t = t0 + warp * 8 + i;
-    if (t < n_tok && lane < np) {
-      out_id[split_off + (size_t)t * nprobe + lane] = Lid[i];
-      out_s[split_off + (size_t)t * nprobe + lane] = Ls[i];
-    }
-  }
-}
-
-// Merge n_split sorted partial lists per token (one warp per token).
-__global__ void __launch_bounds__(256)
-probe_merge_kernel(const uint32_t *__restrict__ part_id,
-                   const float *__restrict__ part_s, uint32_t n_split,
-                   uint32_t n_tok, uint32_t nprobe, uint32_t *__restrict__ out_id,
-                   float *__restrict__ out_s) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t t = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (t >= n_tok) return;
-  const int np = (int)nprobe;
-  float ls = -INFINITY, thr_s = -INFINITY;
-  uint32_t lid = 0xffffffffu, thr_id = 0xffffffffu;
-  for (uint32_t sp = 0; sp < n_split; sp++) {
-    const size_t base = ((size_t)sp * n_tok + t) * nprobe;
-    float ps = -INFINITY;
-    uint32_t pid = 0xffffffffu;
-    if (lane < np) { ps = part_s[base + lane]; pid = part_id[base + lane]; }
-    for (int e = 0; e < np; e++) {
-      const float ns = __shfl_sync(kFull, ps, e);
-      const uint32_t nid = __shfl_sync(kFull, pid, e);
-      if (!better(ns, nid, thr_s, thr_id)) break;  // partial lists are sorted
-      warp_list_insert(ls, lid, thr_s, thr_id, ns, nid, lane, np);
-    }
-  }
-  if (lane < np) {
-    out_id[(size_t)t * nprobe + lane] = lid;
-    out_s[(size_t)t * nprobe + lane] = ls;
   }
 }
 
@@ -1296,7 +1323,7 @@ topk_select_kernel(const uint32_t *__restrict__ short_id, const float *__restric
 // host-side launchers
 // ---------------------------------------------------------------------
 cudaError_t configure_kernels() {
-  cudaError_t e = cudaFuncSetAttribute(probe_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(probe_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kProbeSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(1));
@@ -1320,34 +1347,14 @@ cudaError_t configure_kernels() {
                               (int)(kMaxShort * sizeof(uint64_t)));
 }
 
-int probe_splits(uint32_t n_tok, uint32_t n_cent_pad, int n_sm) {
-  const uint32_t tok_tiles = (n_tok + kProbeTokTile - 1) / kProbeTokTile;
-  const uint32_t cen_tiles = n_cent_pad / kProbeCenTile;
-  uint32_t want = (uint32_t)(2 * n_sm + tok_tiles - 1) / tok_tiles;  // ~2 waves
-  if (want < 1) want = 1;
-  if (want > cen_tiles) want = cen_tiles;
-  return (int)want;
-}
-
-cudaError_t launch_probe(const DevIndex &ix, const float *q, uint32_t n_tok,
-                         uint32_t nprobe, int n_split, uint32_t *part_id,
-                         float *part_s, uint32_t *out_id, float *out_s,
-                         cudaStream_t st, int *n_launch) {
-  const uint32_t cen_tiles = ix.n_centroid_pad / kProbeCenTile;
-  const uint32_t per = (cen_tiles + n_split - 1) / n_split;
-  const uint32_t splits = (cen_tiles + per - 1) / per;
-  dim3 grid(splits, (n_tok + kProbeTokTile - 1) / kProbeTokTile);
-  if (splits == 1) {
-    probe_topk_kernel<<<grid, 256, kProbeSmem, st>>>(q, n_tok, ix.centroid_t, ix.n_centroid,
-                                                    ix.n_centroid_pad, nprobe, per, out_id, out_s);
-    *n_launch += 1;
-    return cudaGetLastError();
-  }
-  probe_topk_kernel<<<grid, 256, kProbeSmem, st>>>(q, n_tok, ix.centroid_t, ix.n_centroid,
-                                                  ix.n_centroid_pad, nprobe, per, part_id, part_s);
-  probe_merge_kernel<<<(n_tok + 7) / 8, 256, 0, st>>>(part_id, part_s, splits, n_tok, nprobe,
-                                                      out_id, out_s);
-  *n_launch += 2;
+cudaError_t launch_probe_scan(const float *q, const float *cen_t, uint32_t n_cent,
+                              uint32_t n_cent_pad, uint32_t nprobe, uint32_t *flags,
+                              uint32_t list_at, uint32_t *part_id, float *part_s,
+                              uint32_t *out_id, float *out_s, int n_sm, cudaStream_t st,
+                              int *n_launch) {
+  probe_scan_kernel<<<n_sm, 256, kProbeSmem, st>>>(q, cen_t, n_cent, n_cent_pad, nprobe, flags,
+                                                   list_at, part_id, part_s, out_id, out_s);
+  *n_launch += 1;
   return cudaGetLastError();
 }
 

@@ -42,11 +42,13 @@ inline uint32_t hash_parts(uint32_t nq, uint32_t nprobe, double cand_per_probe) 
 cudaError_t configure_kernels();
 // ivf_part table of an index ([C][kHashParts + 1] u32)
 cudaError_t make_ivf_part(const DevIndex &ix, uint32_t *out, cudaStream_t st);
-int probe_splits(uint32_t n_tok, uint32_t n_cent_pad, int n_sm);
-cudaError_t launch_probe(const DevIndex &ix, const float *q, uint32_t n_tok,
-                         uint32_t nprobe, int n_split, uint32_t *part_id,
-                         float *part_s, uint32_t *out_id, float *out_s,
-                         cudaStream_t st, int *n_launch);
+// Exact scan of the tokens flagged in flags (see probe_scan_kernel): top
+// nprobe of each by (score desc, id asc); part_*: [n_sm * 64 * nprobe].
+cudaError_t launch_probe_scan(const float *q, const float *cen_t, uint32_t n_cent,
+                              uint32_t n_cent_pad, uint32_t nprobe, uint32_t *flags,
+                              uint32_t list_at, uint32_t *part_id, float *part_s,
+                              uint32_t *out_id, float *out_s, int n_sm, cudaStream_t st,
+                              int *n_launch);
 cudaError_t launch_filter(const DevIndex &ix, const uint32_t *probe_id,
                           const float *probe_s, uint32_t nprobe,
                           const uint64_t *q_off, uint32_t n_query,

@@ -13,6 +13,7 @@
 // tile i.  Scores are approximate (BF16 inputs); the search path re-scores the
 // best of them with the exact FP32 kernel.
 #include "mvr_common.cuh"
+#include "mvr_kernels.cuh"
 #include "mvr_tc.cuh"
 #include "mvr_mbar.cuh"
 
@@ -889,35 +890,63 @@ __global__ void perm_centroid_kernel(const float *__restrict__ cen, uint32_t n_c
 }
 
 // ---------------------------------------------------------------------
-// Centroid scoring on tensor cores.
+// Centroid scoring + per-token top-nprobe, exact, with the scan on the tensor
+// cores.
 //
-// probe_tc_kernel: CTA = 128 query tokens (operand A, M = 128, BF16
-// swizzled in smem) x a range of 64-centroid tiles (operand B, N = 64),
-// warp-specialised.  Centroid tiles are stored pre-swizzled in HBM (cen_sw,
-// 16 KB per tile, contiguous); one thread of warp 4 streams them by 1-D bulk
-// copies (cp.async.bulk, mbarrier transaction count) into a 3-stage ring and
-// issues 8 tcgen05.mma per tile into a double-buffered TMEM accumulator
-// (2 x 64 columns); commits hand D to the epilogue and free the ring stage,
-// and the epilogue releases D as soon as it has loaded it, so the MMAs of
-// tile j + 1 run while tile j is scanned.  Epilogue (warps 0-3): thread =
-// token row reads its 64 scores with tcgen05.ld (two 32-column chunks) and
-// keeps the token's best kCand of the split sorted in registers.  Every
-// mbarrier wait is bounded; a timeout sets bit 2 of *err and stops the CTA
-// after its MMAs and copies have completed.  A chunk whose max beats the list's
-// last score is staged in the thread's shared-memory row and only its
-// qualifying columns are inserted (branch-free 16-slot insertion).  Candidate
-// ids per token per split go to `cand`; probe_rescore_kernel recomputes their
-// scores exactly (canonical FP32 fma chain) and selects the top nprobe.
+// probe_tc_kernel scores 256 tokens per CTA against a range of 128-centroid
+// tiles in BF16 (FP32 accumulation) and lists every centroid that could be
+// among the token's exact top nprobe.  With eps a bound on |BF16 score - exact
+// score| of the token, the K-th best BF16 score so far less 2 eps is such a
+// test: K centroids have exact scores at or above (K-th best - eps), and a
+// centroid below the test has an exact score under that.  Rounding x to
+// BF16 leaves x - bf16(x); by Cauchy-Schwarz
+//   eps = |q - bf16(q)| max|c| + |bf16(q)| max|c - bf16(c)|
+// plus 2^-13 |q| max|c| for both sides' FP32 accumulation and 2^-22 (1 + |q|
+// max|c|) for the rounding of 1 + score: the norms of the actual rounding
+// errors, about a third of the worst case 2^-7 |q| max|c|.
+// probe_pick_kernel then recomputes the listed centroids' scores with the
+// canonical FP32 chain and selects the top nprobe, so ids and scores equal an
+// exact scan's.  A token whose list overflows its buffer, or whose bound is not
+// finite, is redone by probe_scan_kernel, an exact scan of the flagged tokens.
+//
+// Warp-specialised, one CTA per SM: each epilogue thread (warps 0-7, thread =
+// token row) writes its token as BF16 into TMEM (operand A, 64 columns per 128
+// tokens, once), so the MMAs read only the centroid tile from shared memory.
+// Centroids are stored as pre-swizzled tiles of 64 in HBM (cen_sw, 16 KB each);
+// one thread of warp 9 streams two at a time by 1-D bulk copies into a 4-stage
+// ring, and one of warp 8 issues 8 tcgen05.mma (M = 128, N = 128, K = 16) for
+// each half of the tokens into one of 3 TMEM accumulators.  N = 128 and two
+// token tiles per centroid tile, because the MMAs alone reached 1.08 PFLOP/s
+// with N = 64, and every SM reading its own tile per 128 tokens would need 18
+// TB/s of L2 at full rate.  The
+// epilogue reads 64 scores at a time (the next while these are scanned) and
+// takes the maxima of their eight 8-column groups; only a half tile whose maximum
+// passes some token's test is looked at group by group.  A passing group's 8
+// scores go straight to the token's list in global memory, and its maximum into
+// the K best group maxima, sorted in registers: K groups at or above a value
+// hold K centroids at or above it, so their K-th best serves the test.  (Testing
+// and inserting column by column took 2.2 ms for 37,888 tokens and 65,536
+// centroids at K = 8, most of it in diverged insertions.)  A list takes about
+// K (1 + ln(C / 8 K)) groups for centroids in no particular order.
+// Every mbarrier wait is bounded; a timeout
+// sets bit 2 of *err and stops the CTA after its MMAs and copies have completed.
+//
+// Bound: the MMAs and the hand-offs around them (1.1 PFLOP/s of the 1.56 that
+// the same loop reaches with no waits).  1,000,003 tokens x 65,536 centroids,
+// best one: 26.9 -> 15.0 ms; 37,888 tokens, best 8: 1.08 -> 0.69 ms; 12,800
+// tokens, best 8, by FP32 scan 6.91 -> 0.43 ms; and where each of 32 tokens has
+// 296 lists, their selection 606 -> 23 us.
 // ---------------------------------------------------------------------
-constexpr int kPtTok = 128;     // tokens per CTA (M) = epilogue threads
-constexpr int kPtCen = 64;      // centroids per tile (N)
-constexpr int kCand = 16;       // candidates kept per token per split
-constexpr int kStage = 36;      // staging row stride in floats (16 B aligned, conflict-free STS.128)
-constexpr uint32_t kPtTileBytes = kPtCen * 256;  // one swizzled BF16 centroid tile
-constexpr int kPtStages = 3;    // centroid-tile ring stages
-constexpr int kPtThreads = 160;  // 4 epilogue warps (one thread per token row) + copy / MMA warp
-constexpr size_t kPtSmem = 1024 + 32768 /*A*/ + kPtStages * kPtTileBytes /*B ring*/ +
-                           kPtTok * kStage * 4 /*stage*/;
+constexpr int kPtTok = 128;     // tokens per MMA (M)
+constexpr int kPtCtaTok = 2 * kPtTok;  // tokens per CTA = epilogue threads
+constexpr int kPtSrc = 64;      // centroids per pre-swizzled source tile
+constexpr uint32_t kPtSrcBytes = kPtSrc * 256;
+constexpr int kPtCen = 128;     // centroids per tile (N): two source tiles
+constexpr uint32_t kPtTileBytes = 2 * kPtSrcBytes;
+constexpr int kPtStages = 4;    // centroid-tile ring stages
+constexpr int kPtDStages = 3;   // accumulators in TMEM (128 columns each), after A's 2 x 64 columns
+constexpr int kPtThreads = 320;  // 8 epilogue warps (one thread per token row), MMA, copy warps
+constexpr size_t kPtSmem = 1024 + kPtStages * kPtTileBytes;
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -932,56 +961,78 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-// Insert (v, c) into a register list sorted by score descending, given v >
-// s[kCand-1].  Centroids arrive in ascending id order, so an equal score
-// already in the list has the smaller id and stays ahead (strict >).  The 16
-// comparisons are independent and are collected as bits of one integer; each
-// slot then takes its own value, its left neighbour's, or (v, c).  (Holding
-// the comparisons as 16 separate bool values under the caller's v > s[15]
-// guard was compiled into code that never wrote s[15] in some contexts with
-// nvcc 12.9; the bit-mask form is checked by the probe parity tests and a
-// per-token insert count.)
-__device__ __forceinline__ void topk_insert(float (&s)[kCand], uint32_t (&d)[kCand], float v,
-                                            uint32_t c) {
-  uint32_t bm = 0;
-#pragma unroll
-  for (int k = 0; k < kCand; k++) bm |= (v > s[k] ? 1u : 0u) << k;
-#pragma unroll
-  for (int k = kCand - 1; k >= 1; k--) {
-    const bool bk = (bm >> k) & 1u, bp = (bm >> (k - 1)) & 1u;
-    const float sk = bp ? s[k - 1] : v;
-    const uint32_t dk = bp ? d[k - 1] : c;
-    s[k] = bk ? sk : s[k];
-    d[k] = bk ? dk : d[k];
-  }
-  s[0] = (bm & 1u) ? v : s[0];
-  d[0] = (bm & 1u) ? c : d[0];
+// 64 TMEM columns of the warp's 32 lanes into r, asynchronously: r holds them
+// after tmem_wait64(r), which alone may follow as its next use.  (A kernel
+// that uses the pair must compile without spills.)
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&r)[64]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,"
+      "%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,"
+      "%56,%57,%58,%59,%60,%61,%62,%63}, [%64];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
+        "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]),
+        "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]),
+        "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]),
+        "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
+        "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]),
+        "=r"(r[62]), "=r"(r[63])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait64(uint32_t (&r)[64]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+      : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
+        "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]),
+        "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]),
+        "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]),
+        "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]),
+        "+r"(r[32]), "+r"(r[33]), "+r"(r[34]), "+r"(r[35]), "+r"(r[36]), "+r"(r[37]),
+        "+r"(r[38]), "+r"(r[39]), "+r"(r[40]), "+r"(r[41]), "+r"(r[42]), "+r"(r[43]),
+        "+r"(r[44]), "+r"(r[45]), "+r"(r[46]), "+r"(r[47]), "+r"(r[48]), "+r"(r[49]),
+        "+r"(r[50]), "+r"(r[51]), "+r"(r[52]), "+r"(r[53]), "+r"(r[54]), "+r"(r[55]),
+        "+r"(r[56]), "+r"(r[57]), "+r"(r[58]), "+r"(r[59]), "+r"(r[60]), "+r"(r[61]),
+        "+r"(r[62]), "+r"(r[63])
+      :
+      : "memory");
 }
 
-__global__ void __launch_bounds__(kPtThreads, 2)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(p));
+  return p != 0;
+}
+
+template <int K>
+__global__ void __launch_bounds__(kPtThreads, 1)
 probe_tc_kernel(const float *__restrict__ q, uint32_t n_tok, const uint8_t *__restrict__ cen_sw,
                 uint32_t n_cent, uint32_t tiles_per_split, uint32_t n_tiles,
-                uint32_t *__restrict__ cand, unsigned *__restrict__ err) {
+                const float *__restrict__ bounds, uint32_t cap, float4 *__restrict__ ent,
+                uint32_t *__restrict__ gid, uint32_t *__restrict__ cnt, float *__restrict__ eps2,
+                unsigned *__restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t *Aq = smem;                  // [2 K-blocks][128 rows][128 B]
-  uint8_t *Bc = smem + 32768;          // [kPtStages][2 K-blocks][64 rows][128 B]
-  float *stage_base = reinterpret_cast<float *>(Bc + kPtStages * kPtTileBytes);
-  __shared__ uint64_t bfull[kPtStages], bfree[kPtStages], dfull[2], dfree[2], mdone;
+  uint8_t *Bc = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ uint64_t bfull[kPtStages], bfree[kPtStages], dfull[kPtDStages], dfree[kPtDStages], mdone;
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int s_abort;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t t0 = blockIdx.y * kPtTok;
+  const uint32_t t0 = blockIdx.y * kPtCtaTok;
   const uint32_t tile_begin = blockIdx.x * tiles_per_split;
   const uint32_t tile_end = min(n_tiles, tile_begin + tiles_per_split);
   if (tile_begin >= tile_end) return;
   const uint32_t n_local = tile_end - tile_begin;
+  const uint32_t nm = n_tok - t0 > (uint32_t)kPtTok ? 2u : 1u;  // token halves in use
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                      smem_u32(&tmem_base_s)),
-                 "r"(128u));
+                 "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   if (tid == 0) {
@@ -989,7 +1040,7 @@ probe_tc_kernel(const float *__restrict__ q, uint32_t n_tok, const uint8_t *__re
       mbar_init(&bfull[s], 1);
       mbar_init(&bfree[s], 1);
     }
-    for (int d = 0; d < 2; d++) {
+    for (int d = 0; d < kPtDStages; d++) {
       mbar_init(&dfull[d], 1);
       mbar_init(&dfree[d], 4);
     }
@@ -997,190 +1048,465 @@ probe_tc_kernel(const float *__restrict__ q, uint32_t n_tok, const uint8_t *__re
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     s_abort = 0;
   }
-  // query tokens -> A (BF16, swizzled; rows >= n_tok zero)
-  for (int i = tid; i < kPtTok * 16; i += kPtThreads) {
-    const int row = i >> 4, ch = i & 15;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (t0 + row < n_tok) {
-      const float4 *src = reinterpret_cast<const float4 *>(q + (size_t)(t0 + row) * kDim + ch * 8);
-      const float4 a = __ldg(src), c = __ldg(src + 1);
-      __nv_bfloat162 p0 = __floats2bfloat162_rn(a.x, a.y), p1 = __floats2bfloat162_rn(a.z, a.w);
-      __nv_bfloat162 p2 = __floats2bfloat162_rn(c.x, c.y), p3 = __floats2bfloat162_rn(c.z, c.w);
-      v.x = *reinterpret_cast<uint32_t *>(&p0);
-      v.y = *reinterpret_cast<uint32_t *>(&p1);
-      v.z = *reinterpret_cast<uint32_t *>(&p2);
-      v.w = *reinterpret_cast<uint32_t *>(&p3);
-    }
-    *reinterpret_cast<uint4 *>(Aq + (ch >> 3) * 16384 + sw128_off(row, ch & 7)) = v;
-  }
-  fence_async_smem();  // A (generic stores) before the MMAs read it
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
+  const uint32_t lane_off = (32u * (warp & 3)) << 16;
+  constexpr uint32_t DCOL0 = 128;
+  const uint32_t half = (uint32_t)warp >> 2;  // epilogue warps: token half (M tile)
 
-  if (warp == 4) {
-    // ---------------- copies and MMA issue (one thread) ----------------
+  // the thread's token -> A (BF16 pairs, rows >= n_tok zero) and its 2 eps
+  float m2 = 0.0f;
+  if (warp < 8) {
+    const bool have = t0 + tid < n_tok;
+    const float4 *src = reinterpret_cast<const float4 *>(q + (size_t)(have ? t0 + tid : 0) * kDim);
+    float nq = 0.0f, nb = 0.0f, dq = 0.0f;
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+      uint32_t w[16];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const float4 v = have ? __ldg(src + 8 * h + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float x[4] = {v.x, v.y, v.z, v.w};
+        __nv_bfloat162 p[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float r = i & 1 ? __high2float(p[i >> 1]) : __low2float(p[i >> 1]);
+          nq = fmaf(x[i], x[i], nq);
+          nb = fmaf(r, r, nb);
+          dq = fmaf(x[i] - r, x[i] - r, dq);
+        }
+        w[2 * u] = *reinterpret_cast<uint32_t *>(&p[0]);
+        w[2 * u + 1] = *reinterpret_cast<uint32_t *>(&p[1]);
+      }
+      tmem_st16(tmem + lane_off + 64u * half + 16u * h, w);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+    const float cmax = bounds[0], dcmax = bounds[1];
+    nq = sqrtf(nq) * cmax;
+    // 2^-10 over the computed norms covers their own rounding
+    const float eps = sqrtf(dq) * cmax + sqrtf(nb) * dcmax + nq * 0x1p-13f + (1.0f + nq) * 0x1p-22f;
+    m2 = 2.0f * eps * (1.0f + 0x1p-10f);
+    if (!(nq < 1e38f)) m2 = INFINITY;  // scores beyond the lists' starting value
+    if (have && blockIdx.x == 0) eps2[t0 + tid] = m2;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+
+  if (warp == 9) {
+    // ---------------- copies (one thread) ----------------
     if (lane == 0) {
-      const uint32_t idesc = idesc_bf16(kPtTok, kPtCen);
-      const uint32_t a_base = smem_u32(Aq), b_base = smem_u32(Bc);
-      uint32_t issued = 0;  // tiles whose copy was issued
-      bool ok = true;
-      // tile j -> ring stage j % kPtStages, once the MMA that read the
-      // stage's previous tile has completed
-      auto copy = [&](uint32_t j) -> bool {
+      const uint32_t b_base = smem_u32(Bc);
+      uint32_t j = 0;
+      for (; j < n_local; j++) {  // tile j -> ring stage j % kPtStages, once its MMAs are done
         const uint32_t s = j % kPtStages;
         if (j >= (uint32_t)kPtStages &&
-            !mbar_wait(&bfree[s], ((j / kPtStages) + 1) & 1, kWaitNs))
-          return false;
-        mbar_expect_tx(&bfull[s], kPtTileBytes);
-        bulk_g2s(b_base + s * kPtTileBytes, cen_sw + (size_t)(tile_begin + j) * kPtTileBytes,
-                 kPtTileBytes, &bfull[s]);
-        issued = j + 1;
-        return true;
-      };
-      for (uint32_t j = 0; j < n_local && j + 1 < (uint32_t)kPtStages && ok; j++) ok = copy(j);
-      uint32_t j = 0;
-      for (; ok && j < n_local; j++) {
-        if (j + kPtStages - 1 < n_local && !copy(j + kPtStages - 1)) { ok = false; break; }
-        const uint32_t s = j % kPtStages, d = j & 1;
-        if (!mbar_wait(&bfull[s], (j / kPtStages) & 1, kWaitNs)) { ok = false; break; }
-        if (j >= 2 && !mbar_wait(&dfree[d], ((j >> 1) + 1) & 1, kWaitNs)) { ok = false; break; }
-        if (s_abort) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t bt = b_base + s * kPtTileBytes;
-#pragma unroll
-        for (int kk = 0; kk < 8; kk++) {
-          const uint64_t ad = sw128_desc(a_base + (kk >> 2) * 16384 + (kk & 3) * 32);
-          const uint64_t bd = sw128_desc(bt + (kk >> 2) * (kPtTileBytes / 2) + (kk & 3) * 32);
-          mma_bf16(tmem + d * kPtCen, ad, bd, idesc, kk > 0 ? 1u : 0u);
+            !mbar_wait(&bfree[s], ((j / kPtStages) + 1) & 1, kWaitNs)) {
+          atomicOr(err, 2u);
+          s_abort = 1;
+          break;
         }
-        mma_commit(&dfull[d]);
-        mma_commit(&bfree[s]);
+        if (s_abort) break;
+        mbar_expect_tx(&bfull[s], kPtTileBytes);
+        // [K half][128 rows][128 B] from two source tiles of [K half][64 rows][128 B]
+        const uint8_t *src = cen_sw + (size_t)(tile_begin + j) * kPtTileBytes;
+        const uint32_t dst = b_base + s * kPtTileBytes;
+#pragma unroll
+        for (uint32_t p = 0; p < 4; p++)
+          bulk_g2s(dst + (p & 1) * (kPtTileBytes / 2) + (p >> 1) * (kPtSrcBytes / 2),
+                   src + p * (kPtSrcBytes / 2), kPtSrcBytes / 2, &bfull[s]);
       }
+      // the copies still in flight land before the CTA may exit
+      for (uint32_t i = j > (uint32_t)kPtStages ? j - kPtStages : 0; i < j; i++)
+        mbar_wait(&bfull[i % kPtStages], (i / kPtStages) & 1);
+    }
+    __syncwarp();
+  } else if (warp == 8) {
+    // ---------------- MMA issue ----------------
+    // (the whole warp runs the loop, so that the descriptors stay in uniform
+    // registers; one elected thread issues)
+    const uint32_t idesc = idesc_bf16(kPtTok, kPtCen);
+    const uint32_t b_base = smem_u32(Bc);
+    bool ok = true;
+    uint32_t i = 0;  // accumulators filled
+    for (uint32_t j = 0; ok && j < n_local; j++) {
+      const uint32_t s = j % kPtStages;
+      ok = __all_sync(kFull, mbar_wait(&bfull[s], (j / kPtStages) & 1, kWaitNs));
+      const uint64_t bd = sw128_desc(b_base + s * kPtTileBytes);
+      for (uint32_t m = 0; ok && m < nm; m++, i++) {
+        const uint32_t d = i % kPtDStages;
+        if (i >= (uint32_t)kPtDStages)
+          ok = mbar_wait(&dfree[d], ((i / kPtDStages) + 1) & 1, kWaitNs);
+        ok = __all_sync(kFull, ok && !s_abort);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < 8; kk++)  // descriptor offsets in 16-byte units
+            mma_bf16_ta(tmem + DCOL0 + d * kPtCen, tmem + 64u * m + 8u * kk,
+                        bd + (kk >> 2) * (kPtTileBytes / 32) + (kk & 3) * 2, idesc,
+                        kk > 0 ? 1u : 0u);
+          mma_commit(&dfull[d]);
+          if (m + 1 == nm) mma_commit(&bfree[s]);
+        }
+        __syncwarp();
+      }
+    }
+    if (elect_one()) {
       if (!ok) {
         atomicOr(err, 2u);
         s_abort = 1;
       }
       mma_commit(&mdone);  // every MMA of this CTA has completed once this phase does
       mbar_wait(&mdone, 0);
-      // the copies still in flight land before the CTA may exit
-      for (uint32_t i = issued > (uint32_t)kPtStages ? issued - kPtStages : 0; i < issued; i++)
-        mbar_wait(&bfull[i % kPtStages], (i / kPtStages) & 1);
     }
     __syncwarp();
-  } else {
+  } else if (half < nm) {
     // ---------------- epilogue: thread = token row ----------------
-    float *stage = stage_base + tid * kStage;
-    float ts[kCand];     // this thread's token: best kCand scores of the split so far
-    uint32_t td[kCand];  // and their centroid ids
+    float best[K];  // best group maxima of the split so far, descending
 #pragma unroll
-    for (int k = 0; k < kCand; k++) { ts[k] = -INFINITY; td[k] = 0xffffffffu; }
-    for (uint32_t j = 0; j < n_local; j++) {
-      const uint32_t d = j & 1;
-      if (!__all_sync(kFull, mbar_wait(&dfull[d], (j >> 1) & 1, kWaitNs))) {
-        if (lane == 0) {
-          atomicOr(err, 2u);
-          s_abort = 1;
-        }
-        break;
-      }
-      tc_fence_after();
-      uint32_t r0[32], r1[32];
-      tmem_ld32(tmem + ((32u * warp) << 16) + d * kPtCen, r0);
-      tmem_ld32(tmem + ((32u * warp) << 16) + d * kPtCen + 32, r1);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&dfree[d]);
-#pragma unroll
-      for (int part = 0; part < 2; part++) {
-        const uint32_t(&r)[32] = part ? r1 : r0;
-        float mx = __uint_as_float(r[0]);
-#pragma unroll
-        for (int i = 1; i < 32; i++) mx = fmaxf(mx, __uint_as_float(r[i]));
-        const float thr = ts[kCand - 1];
-        if (__any_sync(kFull, mx > thr)) {
-          const uint32_t cbase = (tile_begin + j) * kPtCen + part * 32;
-          const uint32_t valid = cbase >= n_cent        ? 0u
-                                 : n_cent - cbase >= 32 ? 0xffffffffu
-                                                        : (1u << (n_cent - cbase)) - 1u;
-          uint32_t m4[4] = {0, 0, 0, 0};
-#pragma unroll
-          for (int i = 0; i < 32; i++) m4[i >> 3] |= (__uint_as_float(r[i]) > thr ? 1u : 0u) << i;
-          uint32_t m = ((m4[0] | m4[1]) | (m4[2] | m4[3])) & valid;
-          if (m) {
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-              reinterpret_cast<uint4 *>(stage)[i] =
-                  make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-            while (m) {
-              const int i = __ffs(m) - 1;
-              m &= m - 1;
-              const float v = stage[i];
-              if (v > ts[kCand - 1]) topk_insert(ts, td, v, cbase + i);
-            }
+    for (int k = 0; k < K; k++) best[k] = -3e38f;
+    uint32_t n = 0;
+    const size_t row = (size_t)(t0 + tid) * gridDim.x + blockIdx.x;
+    float4 *out = ent + row * cap * 2;
+    uint32_t *out_g = gid + row * cap;
+    // rows past the last token, and tokens without a finite bound, list nothing
+    // (a NaN threshold passes no test)
+    const bool live = t0 + tid < n_tok && m2 < 3.0e38f;
+    if (!live) m2 = NAN;
+    float thr = best[K - 1] - m2;
+    // the scores come in halves of 64 columns: half-tile h is columns
+    // 64 (h & 1) .. + 64 of tile h / 2
+    auto fetch = [&](uint32_t h, uint32_t (&r)[64]) -> bool {
+      const uint32_t i = (h >> 1) * nm + half, d = i % kPtDStages;
+      if (!(h & 1u)) {
+        if (!__all_sync(kFull, mbar_wait(&dfull[d], (i / kPtDStages) & 1, kWaitNs))) {
+          if (lane == 0) {
+            atomicOr(err, 2u);
+            s_abort = 1;
           }
-          __syncwarp();
+          return false;
+        }
+        tc_fence_after();
+      }
+      tmem_ld64(tmem + lane_off + DCOL0 + d * kPtCen + 64u * (h & 1u), r);
+      return true;
+    };
+    auto landed = [&](uint32_t h, uint32_t (&r)[64]) {
+      tmem_wait64(r);
+      if (h & 1u) {  // both halves read: the accumulator is free
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&dfree[((h >> 1) * nm + half) % kPtDStages]);
+      }
+    };
+    auto scan = [&](uint32_t h, uint32_t (&r)[64]) {
+      const uint32_t c0 = tile_begin * kPtCen + 64u * h;
+      if (c0 + 64u > n_cent) {  // columns past the last centroid
+#pragma unroll
+        for (int i = 0; i < 64; i++)
+          if (c0 + i >= n_cent) r[i] = 0xff800000u;
+      }
+      float gm[8];  // maxima of the tile's eight 8-column groups
+#pragma unroll
+      for (int g = 0; g < 8; g++) {
+        float m[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          m[i] = fmaxf(__uint_as_float(r[8 * g + i]), __uint_as_float(r[8 * g + 4 + i]));
+        gm[g] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+      }
+      const float mt = fmaxf(fmaxf(fmaxf(gm[0], gm[1]), fmaxf(gm[2], gm[3])),
+                             fmaxf(fmaxf(gm[4], gm[5]), fmaxf(gm[6], gm[7])));
+      if (!__any_sync(kFull, mt >= thr)) return;
+      if constexpr (K == 1) {
+        best[0] = fmaxf(best[0], mt);
+        thr = best[0] - m2;
+      }
+#pragma unroll
+      for (int g = 0; g < 8; g++) {
+        const bool hit = gm[g] >= thr;
+        if (!__any_sync(kFull, hit)) continue;
+        if (hit) {
+          if (n < cap) {
+            out[2 * n] = make_float4(__uint_as_float(r[8 * g]), __uint_as_float(r[8 * g + 1]),
+                                     __uint_as_float(r[8 * g + 2]), __uint_as_float(r[8 * g + 3]));
+            out[2 * n + 1] =
+                make_float4(__uint_as_float(r[8 * g + 4]), __uint_as_float(r[8 * g + 5]),
+                            __uint_as_float(r[8 * g + 6]), __uint_as_float(r[8 * g + 7]));
+            out_g[n] = c0 / 8u + g;
+          }
+          n++;
+        }
+        if constexpr (K > 1) {
+          // insertion without branches: slot k takes the middle of (k - 1, v, k)
+          const float v = hit ? gm[g] : -INFINITY;
+#pragma unroll
+          for (int k = K - 1; k >= 1; k--) best[k] = fmaxf(best[k], fminf(best[k - 1], v));
+          best[0] = fmaxf(best[0], v);
+          thr = best[K - 1] - m2;
         }
       }
-      if (__any_sync(kFull, s_abort != 0)) break;
+    };
+    uint32_t ra[64];
+    bool ok = fetch(0, ra);
+    if constexpr (K <= 8) {
+      // two register halves: one is read from TMEM while the other is scanned
+      uint32_t rb[64];
+      for (uint32_t h = 0; ok && h < 2 * n_local; h += 2) {
+        landed(h, ra);
+        fetch(h + 1, rb);
+        scan(h, ra);
+        landed(h + 1, rb);
+        if (h + 2 < 2 * n_local) ok = fetch(h + 2, ra);
+        scan(h + 1, rb);
+        if (__any_sync(kFull, s_abort != 0)) ok = false;
+      }
+    } else {  // longer lists leave no registers for the second
+      for (uint32_t h = 0; ok && h < 2 * n_local; h++) {
+        landed(h, ra);
+        scan(h, ra);
+        if (h + 1 < 2 * n_local) ok = fetch(h + 1, ra);
+        if (__any_sync(kFull, s_abort != 0)) ok = false;
+      }
     }
-    // this split's candidates of this token: [token][split][kCand], best first
-    if (t0 + tid < n_tok && !s_abort) {
-      uint4 *dst = reinterpret_cast<uint4 *>(cand + ((size_t)(t0 + tid) * gridDim.x + blockIdx.x) * kCand);
-#pragma unroll
-      for (int i = 0; i < kCand / 4; i++)
-        dst[i] = make_uint4(td[4 * i], td[4 * i + 1], td[4 * i + 2], td[4 * i + 3]);
-    }
+    tmem_wait64(ra);  // nothing in flight into ra past here, however the loop ended
+    if (t0 + tid < n_tok && ok) cnt[row] = live ? n : cap + 1u;
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(128u));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u));
   }
 }
 
-// One warp per token: exact FP32 scores (sequential fma over d, + 1.0f) of
-// the token's BF16 candidates, top nprobe by (score desc, id asc).
+// bounds[0] = max |c|, bounds[1] = max |c - bf16(c)| over the centroids
+// (zeroed by the caller; non-negative floats order as their bits, a NaN row
+// gives a NaN bound).  One warp per centroid.
+__global__ void centroid_bounds_kernel(const float *__restrict__ cen, uint32_t n_cent,
+                                       uint32_t *__restrict__ bounds) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= n_cent) return;
+  const float4 v = __ldg(reinterpret_cast<const float4 *>(cen + (size_t)c * kDim) + lane);
+  const float x[4] = {v.x, v.y, v.z, v.w};
+  float n2 = 0.0f, d2 = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float e = x[i] - __bfloat162float(__float2bfloat16_rn(x[i]));
+    n2 = fmaf(x[i], x[i], n2);
+    d2 = fmaf(e, e, d2);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    n2 += __shfl_xor_sync(kFull, n2, o);
+    d2 += __shfl_xor_sync(kFull, d2, o);
+  }
+  if (lane == 0) {
+    atomicMax(bounds, __float_as_uint(sqrtf(n2)) & 0x7fffffffu);
+    atomicMax(bounds + 1, __float_as_uint(sqrtf(d2)) & 0x7fffffffu);
+  }
+}
+
+// canonical FP32 score of one centroid: sequential fma over d, then + 1.0f
+__device__ __forceinline__ float exact_score(const float *qs, const float *cen, uint32_t c) {
+  const float4 *row = reinterpret_cast<const float4 *>(cen + (size_t)c * kDim);
+  float acc = 0.0f;
+#pragma unroll 8
+  for (int d4 = 0; d4 < kDim / 4; d4++) {
+    const float4 x = __ldg(row + d4);
+    const float4 a = *reinterpret_cast<const float4 *>(qs + 4 * d4);
+    acc = __fmaf_rn(a.x, x.x, acc);
+    acc = __fmaf_rn(a.y, x.y, acc);
+    acc = __fmaf_rn(a.z, x.z, acc);
+    acc = __fmaf_rn(a.w, x.w, acc);
+  }
+  return __fadd_rn(acc, 1.0f);
+}
+
+// a listed group: its 8 BF16 scores (-inf past the last centroid)
+__device__ __forceinline__ float group_max(const float4 *e) {
+  const float4 a = __ldg(e), b = __ldg(e + 1);
+  return fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+}
+// f(centroid) for those of group g at or above thr
+template <class F>
+__device__ __forceinline__ void for_reach(const float4 *e, uint32_t g, float thr, F f) {
+  const float4 a = __ldg(e), b = __ldg(e + 1);
+  const float s[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) m |= (s[i] >= thr && s[i] > -INFINITY ? 1u : 0u) << i;
+  while (m) {
+    f(8u * g + __ffs(m) - 1);
+    m &= m - 1;
+  }
+}
+
+__device__ __forceinline__ void flag_token(uint32_t *flags, uint32_t list_at, uint32_t t) {
+  flags[list_at + atomicAdd(flags, 1u)] = t;
+}
+
+// The exact best centroid of each token (nprobe 1) from its lists: 8 lanes per
+// token (a list holds about a dozen entries, two or three of them within
+// 2 eps of the best), each recomputing the entries it finds in reach.
 __global__ void __launch_bounds__(256)
-probe_rescore_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__restrict__ cen,
-                     uint32_t n_cent, const uint32_t *__restrict__ cand, uint32_t n_cand,
-                     uint32_t nprobe, uint32_t *__restrict__ out_id, float *__restrict__ out_s) {
-  __shared__ float qs[8][kDim];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t t = blockIdx.x * 8 + w;
-  if (t >= n_tok) return;
-  for (int d = lane; d < kDim; d += 32) qs[w][d] = q[(size_t)t * kDim + d];
-  __syncwarp();
+probe_pick1_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__restrict__ cen,
+                   const float4 *__restrict__ ent, const uint32_t *__restrict__ gid,
+                   const uint32_t *__restrict__ cnt, const float *__restrict__ eps2, uint32_t splits, uint32_t cap,
+                   uint32_t *__restrict__ out_id, float *__restrict__ out_s,
+                   uint32_t *__restrict__ flags, uint32_t list_at) {
+  __shared__ __align__(16) float qs[32][kDim + 4];
+  const int tid = threadIdx.x, l = tid & 7, w = tid >> 3;
+  const uint32_t tb = blockIdx.x * 32, t = tb + w;
+  for (int i = tid; i < 32 * (kDim / 4); i += 256) {
+    const int r = i >> 5, d4 = i & 31;
+    if (tb + r < n_tok)
+      *reinterpret_cast<float4 *>(&qs[r][4 * d4]) =
+          __ldg(reinterpret_cast<const float4 *>(q + (size_t)(tb + r) * kDim) + d4);
+  }
+  __syncthreads();
+  if (t >= n_tok) return;  // whole groups of 8 lanes
+  const unsigned grp = 0xffu << (8 * ((tid >> 3) & 3));
+  const float m2 = eps2[t];
+  bool over = !(m2 < 3.0e38f);
+  float b = -INFINITY;
+  for (uint32_t sp = 0; sp < splits; sp++) {
+    const size_t row = (size_t)t * splits + sp;
+    const uint32_t n = cnt[row];
+    over |= n > cap;
+    for (uint32_t e = l; e < min(n, cap); e += 8) b = fmaxf(b, group_max(ent + 2 * (row * cap + e)));
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) b = fmaxf(b, __shfl_xor_sync(grp, b, o));
+  if (over) {  // uniform over the group
+    if (l == 0) flag_token(flags, list_at, t);
+    return;
+  }
+  const float thr = b - m2;
+  float s = -INFINITY;
+  uint32_t id = 0xffffffffu;
+  for (uint32_t sp = 0; sp < splits; sp++) {
+    const size_t row = (size_t)t * splits + sp;
+    const uint32_t n = cnt[row];
+    for (uint32_t e = l; e < n; e += 8) {
+      for_reach(ent + 2 * (row * cap + e), gid[row * cap + e], thr, [&](uint32_t c) {
+        const float x = exact_score(qs[w], cen, c);
+        if (better(x, c, s, id)) { s = x; id = c; }
+      });
+    }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    const float os = __shfl_xor_sync(grp, s, o);
+    const uint32_t oi = __shfl_xor_sync(grp, id, o);
+    if (better(os, oi, s, id)) { s = os; id = oi; }
+  }
+  if (l == 0) {
+    out_id[t] = id;
+    out_s[t] = s;
+  }
+}
+
+// The exact top nprobe of each token from its lists, W warps per token (1
+// where tokens are many, 8 where each has the lists of many splits).  The
+// nprobe-th best of the threads' own maxima bounds the nprobe-th best BF16
+// score from below; the entries within 2 eps of it are recomputed exactly and
+// selected by (score desc, id asc).  More of them than fit: the token is flagged.
+template <int W>
+__global__ void __launch_bounds__(256)
+probe_pick_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__restrict__ cen,
+                  const float4 *__restrict__ ent, const uint32_t *__restrict__ gid,
+                  const uint32_t *__restrict__ cnt, const float *__restrict__ eps2, uint32_t splits, uint32_t cap, uint32_t nprobe,
+                  uint32_t *__restrict__ out_id, float *__restrict__ out_s,
+                  uint32_t *__restrict__ flags, uint32_t list_at) {
+  constexpr int G = 32 * W, TB = 8 / W;     // threads per token, tokens per block
+  constexpr uint32_t LIM = W == 1 ? 256 : 1024;  // entries recomputed per token
+  __shared__ __align__(16) float qs[TB][kDim];
+  __shared__ uint32_t c_id[TB][LIM];
+  __shared__ float c_s[TB][LIM];
+  __shared__ int wmax[W == 1 ? 1 : G];
+  __shared__ uint32_t s_n[TB], s_over[TB];
+  __shared__ float s_thr[TB];
+  const int tid = threadIdx.x, lane = tid & 31, g = tid / G, gt = tid % G, w = gt >> 5;
+  const uint32_t t = blockIdx.x * TB + g;
+  auto sync = [] {
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+  };
+  if (t >= n_tok) return;  // W = 1: whole warps; W = 8: never
+  for (int d = gt; d < kDim; d += G) qs[g][d] = q[(size_t)t * kDim + d];
+  if (gt == 0) { s_n[g] = 0; s_over[g] = eps2[t] < 3.0e38f ? 0u : 1u; }
+  sync();
+  const float m2 = eps2[t];
+  int mx = f2si(-INFINITY);
+  bool over = false;
+  for (uint32_t sp = w; sp < splits; sp += W) {
+    const size_t row = (size_t)t * splits + sp;
+    const uint32_t n = cnt[row];
+    over |= n > cap;
+    for (uint32_t e = lane; e < min(n, cap); e += 32)
+      mx = max(mx, f2si(group_max(ent + 2 * (row * cap + e))));
+  }
+  if (over) s_over[g] = 1;
+  if constexpr (W > 1) wmax[gt] = mx;
+  sync();
+  if (w == 0) {  // the nprobe-th largest of the G maxima
+    int v[W];
+#pragma unroll
+    for (int i = 0; i < W; i++) v[i] = W == 1 ? mx : wmax[32 * i + lane];
+    int kth = f2si(-INFINITY);
+    for (uint32_t k = 0; k < nprobe; k++) {
+      int m = v[0];
+#pragma unroll
+      for (int i = 1; i < W; i++) m = max(m, v[i]);
+      kth = __reduce_max_sync(kFull, m);
+      const bool mine = lane == __ffs(__ballot_sync(kFull, m == kth)) - 1;
+      bool done = false;
+#pragma unroll
+      for (int i = 0; i < W; i++)
+        if (mine && !done && v[i] == kth) { v[i] = f2si(-INFINITY); done = true; }
+    }
+    if (lane == 0) s_thr[g] = si2f(kth) - m2;
+  }
+  sync();
+  const float thr = s_thr[g];
+  if (!s_over[g]) {
+    for (uint32_t sp = w; sp < splits; sp += W) {
+      const size_t row = (size_t)t * splits + sp;
+      const uint32_t n = cnt[row];
+      for (uint32_t e = lane; e < n; e += 32) {
+        for_reach(ent + 2 * (row * cap + e), gid[row * cap + e], thr, [&](uint32_t c) {
+          const uint32_t pos = atomicAdd(&s_n[g], 1u);
+          if (pos < LIM) c_id[g][pos] = c;
+        });
+      }
+    }
+  }
+  sync();
+  const uint32_t n = s_n[g];
+  if (s_over[g] || n > LIM) {
+    if (gt == 0) flag_token(flags, list_at, t);
+    return;
+  }
+  for (uint32_t i = gt; i < n; i += G) c_s[g][i] = exact_score(qs[g], cen, c_id[g][i]);
+  sync();
+  if (w != 0) return;
   const int np = (int)nprobe;
   float ls = -INFINITY, thr_s = -INFINITY;
   uint32_t lid = 0xffffffffu, thr_id = 0xffffffffu;
-  const uint32_t *cl = cand + (size_t)t * n_cand;
-  for (uint32_t c0 = 0; c0 < n_cand; c0 += 32) {
-    const uint32_t i = c0 + lane;
-    uint32_t c = i < n_cand ? cl[i] : 0xffffffffu;
-    float s = -INFINITY;
-    if (c < n_cent) {
-      const float4 *row = reinterpret_cast<const float4 *>(cen + (size_t)c * kDim);
-      float acc = 0.0f;
-#pragma unroll 8
-      for (int d4 = 0; d4 < kDim / 4; d4++) {
-        const float4 x = __ldg(row + d4);
-        acc = __fmaf_rn(qs[w][4 * d4 + 0], x.x, acc);
-        acc = __fmaf_rn(qs[w][4 * d4 + 1], x.y, acc);
-        acc = __fmaf_rn(qs[w][4 * d4 + 2], x.z, acc);
-        acc = __fmaf_rn(qs[w][4 * d4 + 3], x.w, acc);
-      }
-      s = __fadd_rn(acc, 1.0f);
-    } else {
-      c = 0xffffffffu;
-    }
-    unsigned m = __ballot_sync(kFull, c != 0xffffffffu && better(s, c, thr_s, thr_id));
+  for (uint32_t c0 = 0; c0 < n; c0 += 32) {
+    const bool has = c0 + lane < n;
+    const float sc = has ? c_s[g][c0 + lane] : -INFINITY;
+    const uint32_t c = has ? c_id[g][c0 + lane] : 0xffffffffu;
+    unsigned m = __ballot_sync(kFull, has && better(sc, c, thr_s, thr_id));
     while (m) {
       const int src = __ffs(m) - 1;
       m &= m - 1;
-      const float ns = __shfl_sync(kFull, s, src);
+      const float ns = __shfl_sync(kFull, sc, src);
       const uint32_t nid = __shfl_sync(kFull, c, src);
       if (better(ns, nid, thr_s, thr_id)) {
         const bool ahead = lane < np && better(ls, lid, ns, nid);
@@ -1204,12 +1530,12 @@ probe_rescore_kernel(const float *__restrict__ q, uint32_t n_tok, const float *_
 // tiles (rows >= C zero)
 __global__ void swizzle_centroid_kernel(const float *__restrict__ cen, uint32_t n_cent,
                                         uint32_t n_tiles, uint8_t *__restrict__ out) {
-  const size_t n_chunks = (size_t)n_tiles * kPtCen * 16;
+  const size_t n_chunks = (size_t)n_tiles * kPtSrc * 16;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_chunks;
        i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t tile = (uint32_t)(i / (kPtCen * 16));
-    const uint32_t row = (uint32_t)((i / 16) % kPtCen), ch = (uint32_t)(i % 16);
-    const uint32_t c = tile * kPtCen + row;
+    const uint32_t tile = (uint32_t)(i / (kPtSrc * 16));
+    const uint32_t row = (uint32_t)((i / 16) % kPtSrc), ch = (uint32_t)(i % 16);
+    const uint32_t c = tile * kPtSrc + row;
     uint4 v = make_uint4(0, 0, 0, 0);
     if (c < n_cent) {
       const float *src = cen + (size_t)c * kDim + ch * 8;
@@ -1220,7 +1546,7 @@ __global__ void swizzle_centroid_kernel(const float *__restrict__ cen, uint32_t 
       v.z = *reinterpret_cast<uint32_t *>(&p2);
       v.w = *reinterpret_cast<uint32_t *>(&p3);
     }
-    *reinterpret_cast<uint4 *>(out + (size_t)tile * kPtTileBytes + (ch >> 3) * (kPtTileBytes / 2) +
+    *reinterpret_cast<uint4 *>(out + (size_t)tile * kPtSrcBytes + (ch >> 3) * (kPtSrcBytes / 2) +
                                sw128_off(row, ch & 7)) = v;
   }
 }
@@ -1231,29 +1557,92 @@ cudaError_t make_centroid_tiles(const float *cen, uint32_t n_cent, uint32_t n_ti
   return cudaGetLastError();
 }
 
-uint32_t probe_tc_cand_per_token(uint32_t n_tok, uint32_t n_cent, int n_sm, uint32_t *splits) {
-  const uint32_t n_tiles = (n_cent + kPtCen - 1) / kPtCen;
-  const uint32_t tok_tiles = (n_tok + kPtTok - 1) / kPtTok;
-  uint32_t s = (2u * (uint32_t)n_sm + tok_tiles - 1) / tok_tiles;  // ~1 wave of 2 CTAs/SM
-  s = std::max(1u, std::min(s, n_tiles));
-  const uint32_t per = (n_tiles + s - 1) / s;
-  *splits = (n_tiles + per - 1) / per;
-  return *splits * kCand;
+// Tokens per launch: whole waves of token tiles (4, 2 or 1 as the lists grow),
+// which bounds the lists' memory (at most 0.8 GB).
+uint32_t probe_chunk(uint32_t nprobe, int n_sm) {
+  return (uint32_t)n_sm * kPtCtaTok * (nprobe == 1 ? 4u : nprobe <= 8 ? 2u : 1u);
 }
 
-cudaError_t launch_probe_tc(const float *q, uint32_t n_tok, const void *cen_sw, const float *cen,
-                            uint32_t n_cent, uint32_t nprobe, uint32_t splits, uint32_t *cand,
-                            uint32_t *out_id, float *out_s, unsigned *err, cudaStream_t st,
-                            int *n_launch) {
+ProbePlan probe_plan(uint32_t n_tok, uint32_t n_cent, uint32_t nprobe, int n_sm) {
+  ProbePlan p;
   const uint32_t n_tiles = (n_cent + kPtCen - 1) / kPtCen;
-  const uint32_t per = (n_tiles + splits - 1) / splits;
-  dim3 grid(splits, (n_tok + kPtTok - 1) / kPtTok);
-  probe_tc_kernel<<<grid, kPtThreads, kPtSmem, st>>>(q, n_tok, reinterpret_cast<const uint8_t *>(cen_sw),
-                                                 n_cent, per, n_tiles, cand, err);
-  probe_rescore_kernel<<<(n_tok + 7) / 8, 256, 0, st>>>(q, n_tok, cen, n_cent, cand,
-                                                       splits * kCand, nprobe, out_id, out_s);
-  *n_launch += 2;
+  const uint32_t tok_tiles = std::max(1u, (n_tok + kPtCtaTok - 1) / kPtCtaTok);
+  // CTAs (one per SM at a time) per token tile: the count that takes the least
+  // time, waves x (centroid tiles of a CTA + 8), 8 being what a split costs:
+  // its start, and lists that fill from nothing
+  uint32_t s = 1;
+  uint64_t least = ~0ull;
+  for (uint32_t c = 1; c <= std::min(n_tiles, 2u * (uint32_t)n_sm / tok_tiles + 4u); c++) {
+    const uint64_t waves = ((uint64_t)tok_tiles * c + n_sm - 1) / n_sm;
+    const uint64_t cost = waves * ((n_tiles + c - 1) / c + 8u);
+    if (cost < least) { least = cost; s = c; }
+  }
+  p.tiles_per_split = (n_tiles + s - 1) / s;
+  p.splits = (n_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
+  p.k = 1;
+  while (p.k < nprobe) p.k *= 2;
+  // a list's expected length is k (1 + ln(C / 8 k)) groups for scores in no
+  // order, and a third more for those within 2 eps (unit vectors of 128
+  // dimensions): 87 of 160 at k = 8 and 65,536 centroids, 14 of 48 at k = 1
+  p.cap = std::min(16u * p.k + 32u, p.tiles_per_split * (kPtCen / 8u));
+  p.n_ent = (size_t)n_tok * p.splits * p.cap * 2;
+  p.n_gid = (size_t)n_tok * p.splits * p.cap;
+  p.n_cnt = (size_t)n_tok * p.splits;
+  p.list_at = 2u + (n_tok + 63u) / 64u;
+  p.n_flag = (size_t)p.list_at + n_tok;
+  p.n_part = (size_t)n_sm * 64u * nprobe;
+  return p;
+}
+
+cudaError_t make_centroid_bounds(const float *cen, uint32_t n_cent, float *bounds,
+                                 cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(bounds, 0, 2 * sizeof(float), st);
+  if (e != cudaSuccess) return e;
+  centroid_bounds_kernel<<<(n_cent + 7) / 8, 256, 0, st>>>(cen, n_cent,
+                                                           reinterpret_cast<uint32_t *>(bounds));
   return cudaGetLastError();
+}
+
+cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, const float *cen,
+                         const float *cen_t, uint32_t n_cent, uint32_t n_cent_pad,
+                         const float *bounds, uint32_t nprobe, const ProbePlan &p,
+                         const ProbeBufs &w, uint32_t *out_id, float *out_s, int n_sm,
+                         unsigned *err, cudaStream_t st, int *n_launch) {
+  const uint32_t n_tiles = (n_cent + kPtCen - 1) / kPtCen;
+  // the flagged tokens' count and the scan's per-tile counters
+  cudaError_t e = cudaMemsetAsync(w.flags, 0, p.list_at * sizeof(uint32_t), st);
+  if (e != cudaSuccess) return e;
+  dim3 grid(p.splits, (n_tok + kPtCtaTok - 1) / kPtCtaTok);
+#define MVR_PT(KK)                                                                              \
+  probe_tc_kernel<KK><<<grid, kPtThreads, kPtSmem, st>>>(                                       \
+      q, n_tok, reinterpret_cast<const uint8_t *>(cen_sw), n_cent, p.tiles_per_split, n_tiles, \
+      bounds, p.cap, w.ent, w.gid, w.cnt, w.eps2, err)
+  switch (p.k) {
+    case 1: MVR_PT(1); break;
+    case 2: MVR_PT(2); break;
+    case 4: MVR_PT(4); break;
+    case 8: MVR_PT(8); break;
+    case 16: MVR_PT(16); break;
+    case 32: MVR_PT(32); break;
+    default: return cudaErrorInvalidValue;
+  }
+#undef MVR_PT
+  if (nprobe == 1)
+    probe_pick1_kernel<<<(n_tok + 31) / 32, 256, 0, st>>>(q, n_tok, cen, w.ent, w.gid, w.cnt, w.eps2,
+                                                          p.splits, p.cap, out_id, out_s, w.flags,
+                                                          p.list_at);
+  else if (p.splits <= 8)
+    probe_pick_kernel<1><<<(n_tok + 7) / 8, 256, 0, st>>>(q, n_tok, cen, w.ent, w.gid, w.cnt, w.eps2,
+                                                          p.splits, p.cap, nprobe, out_id, out_s,
+                                                          w.flags, p.list_at);
+  else
+    probe_pick_kernel<8><<<n_tok, 256, 0, st>>>(q, n_tok, cen, w.ent, w.gid, w.cnt, w.eps2, p.splits,
+                                                p.cap, nprobe, out_id, out_s, w.flags, p.list_at);
+  *n_launch += 2;
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return launch_probe_scan(q, cen_t, n_cent, n_cent_pad, nprobe, w.flags, p.list_at, w.part_id,
+                           w.part_s, out_id, out_s, n_sm, st, n_launch);
 }
 
 // BF16 tables: centroid rows and the byte -> per-value weight table.
@@ -2036,8 +2425,12 @@ cudaError_t configure_tc_kernels() {
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(4, 64));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(probe_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPtSmem);
+#define MVR_PT_ATTR(KK)                                                                         \
+  e = cudaFuncSetAttribute(probe_tc_kernel<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
+                           (int)kPtSmem);                                                       \
   if (e != cudaSuccess) return e;
+  MVR_PT_ATTR(1) MVR_PT_ATTR(2) MVR_PT_ATTR(4) MVR_PT_ATTR(8) MVR_PT_ATTR(16) MVR_PT_ATTR(32)
+#undef MVR_PT_ATTR
   e = cudaFuncSetAttribute(rerank_tmem_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tm_smem_bytes(64));
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_tmem_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tm_smem_bytes(64));

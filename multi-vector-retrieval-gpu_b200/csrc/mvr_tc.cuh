@@ -86,14 +86,41 @@ cudaError_t launch_prune_mlp(const float *feat, const uint32_t *n_short, uint32_
                              float *pred, unsigned *err, int n_sm, cudaStream_t st,
                              int *n_launch);
 
-// tensor-core centroid scoring: candidates per token = splits * 16; the
-// centroid tiles hold 64 centroids each (n_tiles = C_pad / 64)
-uint32_t probe_tc_cand_per_token(uint32_t n_tok, uint32_t n_cent, int n_sm, uint32_t *splits);
+// pre-swizzled BF16 tiles of 64 centroids (n_tiles = C_pad / 64, an even count)
 cudaError_t make_centroid_tiles(const float *cen, uint32_t n_cent, uint32_t n_tiles, void *out,
                                 cudaStream_t st);
-cudaError_t launch_probe_tc(const float *q, uint32_t n_tok, const void *cen_sw, const float *cen,
-                            uint32_t n_cent, uint32_t nprobe, uint32_t splits, uint32_t *cand,
-                            uint32_t *out_id, float *out_s, unsigned *err, cudaStream_t st,
-                            int *n_launch);
+
+// Centroid scoring and top-nprobe per token (exact; mvr_tc.cu): how a call of
+// n_tok tokens is laid out, and the sizes of its buffers in elements.
+struct ProbePlan {
+  uint32_t tiles_per_split, splits;  // 128-centroid tiles of a CTA, CTAs per token tile
+  uint32_t k;                        // best scores kept: nprobe rounded up to a power of two
+  uint32_t cap;                      // groups listed per token and split
+  uint32_t list_at;                  // first flagged token in flags
+  size_t n_ent, n_gid, n_cnt, n_flag, n_part;
+};
+// tokens per launch at most
+uint32_t probe_chunk(uint32_t nprobe, int n_sm);
+ProbePlan probe_plan(uint32_t n_tok, uint32_t n_cent, uint32_t nprobe, int n_sm);
+struct ProbeBufs {
+  float4 *ent;        // [n_ent] listed groups of 8 centroids: their BF16 scores
+  uint32_t *gid;      // [n_gid] ... and the group's index
+  uint32_t *cnt;      // [n_cnt] their count (above cap: the list overflowed)
+  float *eps2;        // [n_tok] twice the token's BF16 error bound
+  uint32_t *flags;    // [n_flag] count of flagged tokens, scan counters, the tokens
+  uint32_t *part_id;  // [n_part] the exact scan's partial lists
+  float *part_s;
+};
+// bounds[2] of probe_tc_kernel: max |c| and max |c - bf16(c)| over the centroids
+cudaError_t make_centroid_bounds(const float *cen, uint32_t n_cent, float *bounds,
+                                 cudaStream_t st);
+// top nprobe (1..32) per token, (score desc, id asc), equal to an exact FP32
+// scan's; cen_sw: swizzled BF16 tiles (make_centroid_tiles), cen: [C][128],
+// cen_t: [128][n_cent_pad]
+cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, const float *cen,
+                         const float *cen_t, uint32_t n_cent, uint32_t n_cent_pad,
+                         const float *bounds, uint32_t nprobe, const ProbePlan &p,
+                         const ProbeBufs &w, uint32_t *out_id, float *out_s, int n_sm,
+                         unsigned *err, cudaStream_t st, int *n_launch);
 
 }  // namespace mvr

@@ -34,7 +34,7 @@ EXPORTS = (
     "mvr_kmeans_accumulate_device", "mvr_residual_quantiles_device",
     "mvr_filter_noalloc", "mvr_index_set_wait_limit",
     "mvr_mlp_work_floats", "mvr_mlp_train_step", "mvr_mlp_forward", "mvr_index_set_pruner",
-    "mvr_index_set_rerank_tile",
+    "mvr_index_set_rerank_tile", "mvr_assign_work_bytes", "mvr_assign_work_device",
 )
 
 
@@ -111,6 +111,8 @@ def lib():
         "mvr_unpack_buckets": [vp, vp, u64, vp],
         "mvr_assign_device": [vp, u64, vp, u32, u32, vp, vp, vp],
         "mvr_assign_tc_device": [vp, u64, vp, u32, u32, vp, vp, vp],
+        "mvr_assign_work_bytes": [u64, u32, C.POINTER(C.c_size_t)],
+        "mvr_assign_work_device": [vp, u64, vp, u32, u32, vp, vp, vp, C.c_size_t, vp],
         "mvr_pack_residual_device": [vp, u64, vp, u32, vp, vp, u32, vp, vp],
         "mvr_kmeans_accumulate_device": [vp, u64, u32, vp, vp, vp, vp],
         "mvr_residual_quantiles_device": [vp, u64, vp, u32, vp, u32, vp, vp, vp],

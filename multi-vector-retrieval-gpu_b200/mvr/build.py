@@ -43,23 +43,23 @@ def _p(t):
 
 
 def assign(vec, centroid, stream=None):
+    """Best centroid and its score (+ 1) per vector, FP32, lowest id on ties
+    (mvr_assign_work_device, its workspace from torch's allocator)."""
     code = torch.empty(vec.shape[0], dtype=torch.int32, device=vec.device)
     score = torch.empty(vec.shape[0], dtype=torch.float32, device=vec.device)
     st = C.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
-    check(lib().mvr_assign_device(_p(vec), vec.shape[0], _p(centroid), centroid.shape[0],
-                                  centroid.shape[1], _p(code), _p(score), st))
+    n = C.c_size_t()
+    check(lib().mvr_assign_work_bytes(vec.shape[0], centroid.shape[0], C.byref(n)))
+    work = torch.empty(n.value, dtype=torch.uint8, device=vec.device)
+    check(lib().mvr_assign_work_device(_p(vec), vec.shape[0], _p(centroid), centroid.shape[0],
+                                       centroid.shape[1], _p(code), _p(score), _p(work), n.value,
+                                       st))
     return code, score
 
 
 def assign_tc(vec, centroid, stream=None):
-    """assign() on the tensor cores (mvr_assign_tc_device): BF16 candidates,
-    exact FP32 re-score; for builds over hundreds of millions of vectors."""
-    code = torch.empty(vec.shape[0], dtype=torch.int32, device=vec.device)
-    score = torch.empty(vec.shape[0], dtype=torch.float32, device=vec.device)
-    st = C.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
-    check(lib().mvr_assign_tc_device(_p(vec), vec.shape[0], _p(centroid), centroid.shape[0],
-                                     centroid.shape[1], _p(code), _p(score), st))
-    return code, score
+    """assign() (both run on the tensor cores; kept for callers of its name)."""
+    return assign(vec, centroid, stream)
 
 
 def _ord_keys(x):

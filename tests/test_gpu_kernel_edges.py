@@ -3,9 +3,11 @@ passes, remainders, the smallest and largest of a range -- against the oracle
 (bit for bit) or a plain restatement of the same operation."""
 import numpy as np
 import pytest
+import torch
 
+import pyoracle
 from helpers import make_queries, oracle_of, tiny_index
-from mvr import SEM_BASIC, SEM_PP, Index
+from mvr import SEM_BASIC, SEM_PP, Index, build
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +43,83 @@ def test_exact_rerank_edges(n_bit):
         s, i = g.search(q, 3, 8, 130, tok_off=off)
         np.testing.assert_array_equal(i, r[1])
         np.testing.assert_array_equal(s, r[0])
+
+
+def top_scan(q, cen, nprobe):
+    """The canonical scores' top nprobe per token, by the oracle's assignment
+    with every chosen centroid's row removed in turn."""
+    left = [np.arange(len(cen))] * len(q)
+    out = np.zeros((len(q), nprobe), np.int64)
+    for k in range(nprobe):
+        for t in range(len(q)):
+            j = int(pyoracle.assign(q[t:t + 1], cen[left[t]])[0])  # lowest id on ties
+            out[t, k] = left[t][j]
+            left[t] = np.delete(left[t], j)
+    return out
+
+
+def unit(x):
+    return (x / np.linalg.norm(x, axis=1, keepdims=True)).astype(np.float32)
+
+
+def hostile(kind, n, c, rng):
+    """(vectors, centroids) for which the tensor-core scan's lists or bound give out."""
+    x, cen = unit(rng.standard_normal((n, 128))), unit(rng.standard_normal((c, 128)))
+    if kind == "rising":   # every centroid beats all before it
+        cen = (np.linspace(0.1, 1.0, c)[:, None] * unit(np.ones((1, 128)) + 0 * cen[:1])).astype(np.float32)
+        x = np.abs(x)
+    elif kind == "equal":  # one centroid many times over
+        cen = np.repeat(cen[:1], c, axis=0)
+    elif kind == "zero":
+        x[: n // 2] = 0
+    elif kind == "scale":  # sizes over which a BF16 rounding is larger than unit scores
+        x *= np.float32(10.0) ** rng.integers(-12, 12, (n, 1)).astype(np.float32)
+        cen *= np.float32(3000.0)
+    elif kind == "huge":   # norms that overflow FP32: the bound is not finite
+        x[: n // 2] *= np.float32(3e37)
+    return x, cen
+
+
+@pytest.mark.parametrize("n,c", [(1, 1), (1, 63), (127, 64), (128, 65), (129, 1000), (300, 4096),
+                                 (5000, 129)])
+def test_assign_edges(n, c):
+    rng = np.random.default_rng(n + c)
+    x, cen = unit(rng.standard_normal((n, 128))), unit(rng.standard_normal((c, 128)))
+    code, _ = build.assign(torch.from_numpy(x).cuda(), torch.from_numpy(cen).cuda())
+    np.testing.assert_array_equal(code.cpu().numpy(), pyoracle.assign(x, cen).astype(np.int64))
+
+
+@pytest.mark.parametrize("kind", ["rising", "equal", "zero", "scale", "huge"])
+@pytest.mark.parametrize("n,c", [(3, 300), (200, 2000)])
+def test_assign_hostile(kind, n, c):
+    x, cen = hostile(kind, n, c, np.random.default_rng(n))
+    code, _ = build.assign(torch.from_numpy(x).cuda(), torch.from_numpy(cen).cuda())
+    np.testing.assert_array_equal(code.cpu().numpy(), pyoracle.assign(x, cen).astype(np.int64))
+
+
+@pytest.mark.parametrize("kind", ["plain", "rising", "equal", "zero", "scale"])
+@pytest.mark.parametrize("nprobe", [1, 2, 3, 4, 7, 8, 9, 16, 17, 32])
+def test_probe_edges(kind, nprobe):
+    """Probe lists of the plain path: ids of an exact scan, for list widths at and
+    beside the powers of two, one query (many splits) and a batch (few)."""
+    base = tiny_index(n_doc=60, n_centroid=33, n_bit=2, seed=7)
+    rng = np.random.default_rng(nprobe)
+    n_cent = 700
+    q, cen = hostile(kind, 40, n_cent, rng)
+    code = pyoracle.assign(base["tokens"], cen)
+    off, size, ids = pyoracle.ivf_build(code, base["item_n_vec"], n_cent)
+    ix = dict(base, centroid=cen, vq_code=code, ivf_off=off, ivf_size=size, ivf_ids=ids)
+    want = top_scan(q[:5], cen, nprobe)
+    with gpu_index(ix) as g:
+        t = g.trace(q[:5], 5, nprobe, 20)
+        np.testing.assert_array_equal(t["probe_id"].astype(np.int64), want)
+        t = g.trace(q, 5, nprobe, 20)
+        np.testing.assert_array_equal(t["probe_id"][:5].astype(np.int64), want)
+        o = oracle_of(ix)
+        many = np.tile(q, (160, 1))
+        toff = np.arange(0, len(many) + 1, 40).astype(np.uint64)
+        r = o.search(q, toff[:2], 5, nprobe, 20)
+        s, i = g.search(many, 5, nprobe, 20, tok_off=toff)
+        for k in (0, 77, 159):
+            np.testing.assert_array_equal(i[k], r[1][0])
+            np.testing.assert_array_equal(s[k], r[0][0])
