@@ -376,8 +376,8 @@ int mvr_pack_residual_device(const float *d_vec, uint64_t n_vec,
  * FP32 subtraction), cutoff_out[c] (host, 2^n_bit - 1 values) = the
  * floor((c + 1) / 2^n_bit * N)-th smallest, weight_out[w] (host, 2^n_bit
  * values) = the floor((w + 0.5) / 2^n_bit * N)-th smallest (0-based ranks,
- * the reference's nth_element positions), selected exactly by two
- * histogram passes over order keys. */
+ * the reference's nth_element positions), selected exactly by
+ * histograms of order keys. */
 int mvr_residual_quantiles_device(const float *d_vec, uint64_t n_vec,
                                   const float *d_centroid, uint32_t dim,
                                   const uint32_t *d_code, uint32_t n_bit,

@@ -10,7 +10,7 @@ vq_sq_pack.vq_sq_ivf, script/evaluation/technique/vq_sq_pack.py:91-109):
     the reference's only in distribution.)
  3. quantile cutoffs / weights: exact order statistics of all sample residual
     coordinates, ranks floor(q * N) (ResidualScalarQuantizationPack.hpp:
-    17-99), found by bisection on the float bit patterns;
+    17-99), selected by histograms of the float bit patterns (libmvr);
  4. assignment of every token + residual packing (libmvr kernels);
  5. doc -> unique-centroid IVF lists, ascending doc ids (IVFIndex.hpp:92-166).
 Returns CUDA tensors; `to_host` gives numpy arrays for formats.write_index_dir.
@@ -94,6 +94,17 @@ def quantize_params(err_flat, n_bit):
     return np.asarray(cut, np.float32), np.asarray(w, np.float32)
 
 
+def residual_quantiles(vec, cen, code, n_bit):
+    """quantize_params of the residual errors vec - cen[code] without
+    materialising them (mvr_residual_quantiles_device)."""
+    cut, w = np.empty((1 << n_bit) - 1, np.float32), np.empty(1 << n_bit, np.float32)
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    check(lib().mvr_residual_quantiles_device(_p(vec), vec.shape[0], _p(cen), vec.shape[1],
+                                              _p(code), n_bit, C.c_void_p(cut.ctypes.data),
+                                              C.c_void_p(w.ctypes.data), st))
+    return cut, w
+
+
 def kmeans(sample, n_centroid, n_iter=20, seed=123, assign_fn=assign):
     dev = sample.device
     g = torch.Generator(device=dev).manual_seed(seed)
@@ -138,8 +149,10 @@ def train(sample, n_centroid, n_bit, kmeans_iter=20, seed=123, assign_fn=assign)
     """Centroids, quantile cutoffs and bucket weights from the k-means sample."""
     cen = kmeans(sample, n_centroid, kmeans_iter, seed, assign_fn)
     s_code, _ = assign_fn(sample, cen)
-    err = (sample - cen[s_code.long()]).reshape(-1)
-    cutoff, weight = quantize_params(err, n_bit)
+    if n_bit in (1, 2, 4, 8):
+        cutoff, weight = residual_quantiles(sample, cen, s_code, n_bit)
+    else:  # widths no codec here packs
+        cutoff, weight = quantize_params((sample - cen[s_code.long()]).reshape(-1), n_bit)
     return cen, cutoff, weight
 
 

@@ -123,3 +123,27 @@ def test_probe_edges(kind, nprobe):
         for k in (0, 77, 159):
             np.testing.assert_array_equal(i[k], r[1][0])
             np.testing.assert_array_equal(s[k], r[0][0])
+
+
+@pytest.mark.parametrize("n,n_bit,shift", [(1, 1, 0), (3, 2, 1), (1000, 2, 0), (777, 4, 3),
+                                           (4097, 8, 0)])
+def test_residual_quantiles_edges(n, n_bit, shift):
+    """Order statistics of ties, signed zeros and wide exponents, from arrays at any
+    4-byte offset, against a sort."""
+    rng = np.random.default_rng(n)
+    vec = rng.standard_normal((n, 128)).astype(np.float32) * np.float32(10.0) ** rng.integers(-9, 3, (n, 1)).astype(np.float32)
+    vec[:, ::7] = np.float32(0.25)
+    cen = np.zeros((5, 128), np.float32)
+    cen[1:, ::7] = np.float32(0.25)
+    cen[2] = -cen[2]
+    code = rng.integers(0, 5, n).astype(np.int32)
+
+    def at(a):
+        t = torch.empty(a.size + shift, device="cuda")
+        t[shift:] = torch.from_numpy(a.reshape(-1)).cuda()
+        return t[shift:].view(a.shape)
+    cut, w = build.residual_quantiles(at(vec), at(cen), torch.from_numpy(code).cuda(), n_bit)
+    e = np.sort((vec - cen[code]).reshape(-1))
+    nb = 1 << n_bit
+    np.testing.assert_array_equal(cut, [e[int(np.floor((i + 1) / nb * e.size))] for i in range(nb - 1)])
+    np.testing.assert_array_equal(w, [e[int(np.floor((i / nb + 0.5 / nb) * e.size))] for i in range(nb)])
