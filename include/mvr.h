@@ -391,6 +391,15 @@ int mvr_kmeans_accumulate_device(const float *d_vec, uint64_t n_vec,
                                  double *d_sum, uint64_t *d_count,
                                  void *cuda_stream);
 
+/* Reduction of an exhaustive MaxSim: out[q][d] = sum over query q's tokens
+ * (rows q_off[q] .. q_off[q+1] of s, leading dimension ld) of the max over doc
+ * d's tokens (columns doc_off[d] .. doc_off[d+1]); s and out float, or double
+ * with f64 != 0.  Device pointers; asynchronous on cuda_stream. */
+int mvr_segment_maxsum_device(const void *d_s, int f64, uint64_t ld,
+                              const int64_t *d_q_off, uint32_t n_query,
+                              const int64_t *d_doc_off, uint32_t n_doc,
+                              void *d_out, void *cuda_stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -24,4 +24,8 @@ cudaError_t residual_select(const float *vec, uint64_t n_vec, const float *cen,
                             const uint32_t *code, const uint64_t *rank, uint32_t n_rank,
                             float *out, cudaStream_t st);
 
+cudaError_t launch_segment_maxsum(const void *s, bool f64, uint64_t ld, const int64_t *q_off,
+                                  uint32_t n_query, const int64_t *d_off, uint32_t n_doc,
+                                  void *out, cudaStream_t st);
+
 }  // namespace mvr

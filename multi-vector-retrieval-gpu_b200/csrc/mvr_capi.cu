@@ -1592,6 +1592,15 @@ int mvr_kmeans_accumulate_device(const float *d_vec, uint64_t n_vec, uint32_t di
   return MVR_OK;
 }
 
+int mvr_segment_maxsum_device(const void *d_s, int f64, uint64_t ld, const int64_t *d_q_off,
+                              uint32_t n_query, const int64_t *d_doc_off, uint32_t n_doc,
+                              void *d_out, void *cuda_stream) {
+  if (!d_s || !d_q_off || !d_doc_off || !d_out) return set_err(MVR_ERR_INVALID_ARG, "null argument");
+  CUDA_TRY(launch_segment_maxsum(d_s, f64 != 0, ld, d_q_off, n_query, d_doc_off, n_doc, d_out,
+                                 (cudaStream_t)cuda_stream));
+  return MVR_OK;
+}
+
 size_t mvr_mlp_work_floats(uint32_t n) { return mlp_work_floats(n); }
 
 int mvr_mlp_train_step(const float *d_x, const float *d_y, uint32_t n, float *d_params,

@@ -35,6 +35,7 @@ EXPORTS = (
     "mvr_filter_noalloc", "mvr_index_set_wait_limit",
     "mvr_mlp_work_floats", "mvr_mlp_train_step", "mvr_mlp_forward", "mvr_index_set_pruner",
     "mvr_index_set_rerank_tile", "mvr_assign_work_bytes", "mvr_assign_work_device",
+    "mvr_segment_maxsum_device",
 )
 
 
@@ -116,6 +117,7 @@ def lib():
         "mvr_pack_residual_device": [vp, u64, vp, u32, vp, vp, u32, vp, vp],
         "mvr_kmeans_accumulate_device": [vp, u64, u32, vp, vp, vp, vp],
         "mvr_residual_quantiles_device": [vp, u64, vp, u32, vp, u32, vp, vp, vp],
+        "mvr_segment_maxsum_device": [vp, i32, u64, vp, u32, vp, u32, vp, vp],
         "mvr_filter_noalloc": [vp, vp, vp, u32, u32, u32, vp, vp, vp, vp],
         "mvr_index_set_wait_limit": [vp, u64],
         "mvr_mlp_train_step": [vp, vp, u32, vp, vp, vp, vp, C.c_float, u32, vp, vp],

@@ -3,8 +3,12 @@ BruteForceProgressive semantics, GPUComputeScore.hpp:193-282: score(q, d) =
 sum over query tokens of the max over doc tokens of <q_t, d_j>), in FP64 by
 default, streamed over token chunks cut at doc boundaries.  Used to measure
 recall; the search path does not call it."""
+import ctypes as C
+
 import numpy as np
 import torch
+
+from ._lib import check, lib
 
 
 def _doc_ranges(lens, chunk_tokens):
@@ -21,6 +25,32 @@ def _doc_ranges(lens, chunk_tokens):
     return out
 
 
+def _maxsum(s, q_off, lens):
+    """[n_query, n_doc]: per query token the max over each doc's columns of s
+    [tokens, doc tokens], summed over the query's tokens."""
+    n_query, nd = len(q_off) - 1, len(lens)
+    doc_off = np.zeros(nd + 1, np.int64)
+    doc_off[1:] = np.cumsum(lens)
+    if doc_off[-1] != s.shape[1]:
+        raise ValueError(f"{s.shape[1]} doc tokens for lengths that sum to {doc_off[-1]}")
+    doc_off = torch.from_numpy(doc_off).to(s.device)
+    if s.is_cuda and s.dtype in (torch.float64, torch.float32) and not s.requires_grad:
+        s = s.contiguous()
+        out = torch.empty((n_query, nd), dtype=s.dtype, device=s.device)
+        with torch.cuda.device(s.device):
+            check(lib().mvr_segment_maxsum_device(
+                C.c_void_p(s.data_ptr()), int(s.dtype == torch.float64), s.stride(0),
+                C.c_void_p(q_off.data_ptr()), n_query, C.c_void_p(doc_off.data_ptr()), nd,
+                C.c_void_p(out.data_ptr()),
+                C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        return out
+    doc_of = torch.repeat_interleave(torch.arange(nd, device=s.device), doc_off.diff())
+    m = torch.full((s.shape[0], nd), -torch.inf, dtype=s.dtype, device=s.device)
+    m.scatter_reduce_(1, doc_of.expand(s.shape[0], -1), s, reduce="amax")
+    tok_q = torch.repeat_interleave(torch.arange(n_query, device=s.device), q_off.diff())
+    return torch.zeros((n_query, nd), dtype=s.dtype, device=s.device).index_add_(0, tok_q, m)
+
+
 def exhaustive_topk_stream(q, tok_off, chunks, k, dtype=torch.float64):
     """Exhaustive top-k over docs delivered in pieces.  chunks: iterable of
     (d0, lens, tokens): consecutive doc ranges in ascending order, lens the
@@ -32,19 +62,17 @@ def exhaustive_topk_stream(q, tok_off, chunks, k, dtype=torch.float64):
     dev = q.device
     n_query = len(tok_off) - 1
     qd = q.to(dtype)
-    tok_q = torch.repeat_interleave(torch.arange(n_query, device=dev),
-                                    torch.from_numpy(np.diff(np.asarray(tok_off, np.int64))).to(dev))
+    q_off = np.asarray(tok_off, np.int64)
+    q_off = q_off - q_off[0]
+    if q_off[-1] != len(qd) or (np.diff(q_off) < 0).any():
+        raise ValueError(f"token offsets do not fit {len(qd)} query tokens")
+    q_off = torch.from_numpy(q_off).to(dev)
     best_s = torch.empty((n_query, 0), dtype=dtype, device=dev)
     best_i = torch.empty((n_query, 0), dtype=torch.int64, device=dev)
     for d0, lens, x in chunks:
         nd = len(lens)
         s = qd @ x.to(dev, dtype).T                                   # [Tq, tok]
-        doc_of = torch.repeat_interleave(torch.arange(nd, device=dev),
-                                         torch.from_numpy(np.asarray(lens, np.int64)).to(dev))
-        m = torch.full((qd.shape[0], nd), -torch.inf, dtype=dtype, device=dev)
-        m.scatter_reduce_(1, doc_of.expand(qd.shape[0], -1), s, reduce="amax")
-        per_q = torch.zeros((n_query, nd), dtype=dtype, device=dev)
-        per_q.index_add_(0, tok_q, m)
+        per_q = _maxsum(s, q_off, np.asarray(lens, np.int64))
         top = torch.sort(per_q, dim=1, descending=True, stable=True)
         kk = min(k, nd)
         cat_s = torch.cat([best_s, top.values[:, :kk]], 1)

@@ -7,7 +7,7 @@ import torch
 
 import pyoracle
 from helpers import make_queries, oracle_of, tiny_index
-from mvr import SEM_BASIC, SEM_PP, Index, build
+from mvr import SEM_BASIC, SEM_PP, Index, build, exhaustive
 
 pytestmark = pytest.mark.gpu
 
@@ -147,3 +147,22 @@ def test_residual_quantiles_edges(n, n_bit, shift):
     nb = 1 << n_bit
     np.testing.assert_array_equal(cut, [e[int(np.floor((i + 1) / nb * e.size))] for i in range(nb - 1)])
     np.testing.assert_array_equal(w, [e[int(np.floor((i / nb + 0.5 / nb) * e.size))] for i in range(nb)])
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_maxsum_edges(dtype):
+    """Max over each doc's columns, sum over each query's tokens: widths around 32 on
+    both sides, empty docs, NaN and infinities, against the torch form."""
+    lens = np.array([0, 1, 31, 32, 33, 64, 100, 0, 5], np.int64)
+    off = np.cumsum([0, 1, 31, 32, 33, 64, 0, 100])
+    g = torch.Generator(device="cuda").manual_seed(3)
+    s = torch.randn((int(off[-1]), int(lens.sum())), device="cuda", generator=g, dtype=dtype)
+    s[5, 40] = float("nan")
+    s[70, 200] = float("inf")
+    s[71, :] = -float("inf")
+    q_off = torch.from_numpy(off).cuda()
+    got = exhaustive._maxsum(s, q_off, lens)
+    want = exhaustive._maxsum(s.cpu(), q_off.cpu(), lens)
+    # sums of up to 100 terms of size ~3 in another order: 100 ulps of 512 at most
+    tol = 100 * 512 * torch.finfo(dtype).eps
+    torch.testing.assert_close(got.cpu(), want, rtol=0, atol=tol, equal_nan=True)
