@@ -299,6 +299,17 @@ __device__ __forceinline__ void filter_sync() {
   }
 }
 
+// the same for data in shared memory alone (cluster-scope ordering)
+template <int CL>
+__device__ __forceinline__ void cluster_sync() {
+  if constexpr (CL == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                 "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+}
+
 template <int CL>
 __device__ __forceinline__ uint32_t *cl_ptr(uint32_t *p, uint32_t rank) {
   if constexpr (CL == 1) {
@@ -313,94 +324,122 @@ __device__ __forceinline__ uint32_t *cl_ptr(uint32_t *p, uint32_t rank) {
 constexpr int kSelU = 8;  // candidate keys per thread in flight in the select passes
 
 // Shared-memory state of select_emit.
+constexpr uint32_t kSelBins = 4096;  // bins of a pass (12 bits of the key)
+constexpr uint32_t kSelList = 512;   // keys of the boundary bin that are ranked directly
 struct SelectSmem {
-  uint32_t (*hist)[256];  // [2][256]
-  uint32_t *digit, *need, *done;
+  uint32_t *hist;   // [kSelBins]
+  uint64_t *list;   // [kSelList], CTA 0's is the cluster's
+  uint32_t *wsum;   // [32]
+  uint32_t *bin, *need, *cnt, *n_list;
 };
+constexpr size_t kSelSmem = kSelBins * sizeof(uint32_t) + kSelList * sizeof(uint64_t);
 
-// Phases C/D of the filter: radix select of the probe_topk largest 64-bit
-// keys among key[0, n_cand) (8-bit digits, high to low, stopping once the
-// boundary digit is unique), then emission of the selected keys as the
-// (unordered) shortlist of query b.  With CL > 1 the CL CTAs of a cluster
-// each take an interleaved share of the keys and add their histograms
-// through distributed shared memory; g_sel / g_stok are CTA 0's counters.
+// Phases C/D of the filter: the probe_topk largest 64-bit keys among
+// key[0, n_cand) as the (unordered) shortlist of query b.  Radix passes of 12
+// bits, high to low, find the bin that the cut falls into, until that bin is
+// taken whole or holds at most kSelList keys; the emission pass writes every
+// key above it and collects its keys, which are then ranked among themselves.
+// Scores take 8 exponent bits, so the first pass spreads them over some 30
+// bins: plain shared atomics without the match_any that 8-bit digits needed,
+// and usually one pass before the emission instead of three.  With CL > 1 the
+// CL CTAs of a cluster each take an interleaved share of the keys and add
+// their histograms through distributed shared memory; g_sel / g_stok are CTA
+// 0's counters.  Bound: latency, two reads of the keys at one CTA per query.
+// 1,184 queries of 31,000 candidates: 465 -> 235 us; one query of 34,000: 64 ->
+// 32 us, of 1,065: 15 -> 7 us.
 template <int CL>
 __device__ void select_emit(const DevIndex &ix, const uint64_t *__restrict__ key, uint32_t n_cand,
                             uint32_t probe_topk, uint32_t b, uint32_t cr, const SelectSmem &sm,
                             uint32_t *g_sel, uint32_t *g_stok, uint32_t *__restrict__ short_id,
                             float *__restrict__ short_approx) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t cstride = CL * blockDim.x;
+  const uint32_t cstride = CL * kFilterThreads;
   const unsigned lt_mask = (1u << lane) - 1u;
-  // ---- phase C: radix select of the probe_topk largest keys ----
-  uint64_t prefix = 0, mask = 0;
-  if (n_cand > probe_topk) {
-    uint32_t need = probe_topk;
-    for (int pass = 0; pass < 8; pass++) {
-      const int shift = 56 - 8 * pass;
-      uint32_t *h = sm.hist[pass & 1];
-      for (int i = tid; i < 256; i += blockDim.x) h[i] = 0;
-      __syncthreads();
-      // kSelU keys per thread in flight
-      for (uint32_t i0 = cr * blockDim.x; i0 < n_cand; i0 += kSelU * cstride) {
-        uint64_t kv[kSelU];
+  const bool cut = n_cand > probe_topk;
+  uint64_t prefix = 0;
+  int shift = 64;  // key bits below the prefix
+  bool whole = true;
+  uint32_t need = probe_topk;
+  if (tid == 0) *sm.n_list = 0;
+  // ---- phase C: the bin that holds the cut ----
+  while (cut) {
+    const int width = min(12, shift);
+    const int up = shift;  // prefix = key >> up so far
+    shift -= width;
+    const uint32_t mask = (1u << width) - 1u;
+    for (uint32_t i = tid; i < kSelBins; i += kFilterThreads) sm.hist[i] = 0;
+    __syncthreads();
+    // kSelU keys per thread in flight
+    for (uint32_t i0 = cr * kFilterThreads; i0 < n_cand; i0 += kSelU * cstride) {
+      uint64_t kv[kSelU];
 #pragma unroll
-        for (int u = 0; u < kSelU; u++) {
-          const uint32_t i = i0 + u * cstride + tid;
-          kv[u] = i < n_cand ? key[i] : ~0ull;
-        }
-#pragma unroll
-        for (int u = 0; u < kSelU; u++) {
-          const uint32_t i = i0 + u * cstride + tid;
-          uint32_t dig = 256;
-          if (i < n_cand && (kv[u] & mask) == prefix) dig = (uint32_t)(kv[u] >> shift) & 0xffu;
-          const unsigned grp = __match_any_sync(kFull, dig);
-          if (dig < 256 && lane == __ffs(grp) - 1) atomicAdd(&h[dig], (uint32_t)__popc(grp));
-        }
+      for (int u = 0; u < kSelU; u++) {
+        const uint32_t i = i0 + u * cstride + tid;
+        kv[u] = i < n_cand ? key[i] : 0ull;
       }
-      filter_sync<CL>();  // every CTA's histogram of this pass complete
-      if (warp == 0) {
-        // lane l owns bins 255-8l .. 248-8l (high to low), summed over the cluster
-        uint32_t cnt[8], sum = 0;
 #pragma unroll
-        for (int u = 0; u < 8; u++) cnt[u] = 0;
-        for (int r = 0; r < CL; r++) {
-          const uint32_t *hr = cl_ptr<CL>(h, (uint32_t)r);
-#pragma unroll
-          for (int u = 0; u < 8; u++) cnt[u] += hr[255 - 8 * lane - u];
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) sum += cnt[u];
-        uint32_t incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t v = __shfl_up_sync(kFull, incl, o);
-          if (lane >= o) incl += v;
-        }
-        const uint32_t excl = incl - sum;
-        if (excl < need && need <= incl) {
-          uint32_t above = excl;
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            if (above < need && need <= above + cnt[u]) {
-              *sm.digit = 255 - 8 * lane - u;
-              *sm.need = need - above;
-              *sm.done = (need - above == cnt[u]) ? 1u : 0u;
-            }
-            above += cnt[u];
-          }
-        }
+      for (int u = 0; u < kSelU; u++) {
+        const uint32_t i = i0 + u * cstride + tid;
+        if (i < n_cand && (up == 64 || (kv[u] >> up) == prefix))
+          atomicAdd(&sm.hist[(uint32_t)(kv[u] >> shift) & mask], 1u);
       }
-      __syncthreads();
-      prefix |= (uint64_t)*sm.digit << shift;
-      mask |= (uint64_t)0xff << shift;
-      need = *sm.need;
-      if (*sm.done) break;
     }
+    cluster_sync<CL>();  // every CTA's histogram of this pass complete
+    // thread t owns bins 4095 - 4t .. 4092 - 4t (high to low), summed over the cluster
+    uint32_t c[4] = {0, 0, 0, 0}, sum = 0;
+    for (int r = 0; r < CL; r++) {
+      const uint32_t *hr = cl_ptr<CL>(sm.hist, (uint32_t)r);
+#pragma unroll
+      for (int u = 0; u < 4; u++) c[u] += hr[kSelBins - 1 - 4 * tid - u];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) sum += c[u];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) sm.wsum[warp] = incl;
+    __syncthreads();
+    uint32_t above = incl - sum;
+    for (int w = 0; w < warp; w++) above += sm.wsum[w];
+    if (above < need && need <= above + sum) {
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (above < need && need <= above + c[u]) {
+          *sm.bin = kSelBins - 1 - 4 * tid - u;
+          *sm.need = need - above;
+          *sm.cnt = c[u];
+        }
+        above += c[u];
+      }
+    }
+    cluster_sync<CL>();  // the result, and every CTA done with the histograms
+    prefix = (prefix << width) | *sm.bin;
+    need = *sm.need;
+    const uint32_t cnt = *sm.cnt;
+    whole = cnt == need;
+    if (whole || cnt <= kSelList) break;
   }
 
   // ---- phase D: emit the shortlist (unordered) ----
-  for (uint32_t j0 = cr * blockDim.x; j0 < n_cand; j0 += kSelU * cstride) {
+  auto emit = [&](bool sel, uint64_t k) {  // whole warps
+    const unsigned m = __ballot_sync(kFull, sel);
+    if (!m) return;
+    uint32_t base = 0;
+    if (lane == __ffs(m) - 1) base = atomicAdd(g_sel, (uint32_t)__popc(m));
+    base = __shfl_sync(kFull, base, __ffs(m) - 1);
+    const uint32_t pos = base + __popc(m & lt_mask);
+    if (sel && pos < probe_topk) {
+      short_id[(size_t)b * probe_topk + pos] = key_id(k);
+      short_approx[(size_t)b * probe_topk + pos] = key_score(k);
+    }
+  };
+  uint64_t *list = cut && !whole ? reinterpret_cast<uint64_t *>(cl_ptr<CL>((uint32_t *)sm.list, 0)) : nullptr;
+  uint32_t *g_list = cl_ptr<CL>(sm.n_list, 0);
+  if constexpr (CL > 1) cluster_sync<CL>();  // CTA 0's list counter is zero
+  for (uint32_t j0 = cr * kFilterThreads; j0 < n_cand; j0 += kSelU * cstride) {
     uint64_t kv[kSelU];
 #pragma unroll
     for (int u = 0; u < kSelU; u++) {
@@ -410,25 +449,33 @@ __device__ void select_emit(const DevIndex &ix, const uint64_t *__restrict__ key
 #pragma unroll
     for (int u = 0; u < kSelU; u++) {
       const uint32_t i = j0 + u * cstride + tid;
-      const uint64_t k = kv[u];
-      const bool sel = i < n_cand && (k & mask) >= prefix;
-      const unsigned m = __ballot_sync(kFull, sel);
-      if (m) {
-        uint32_t base = 0;
-        if (lane == __ffs(m) - 1) base = atomicAdd(g_sel, (uint32_t)__popc(m));
-        base = __shfl_sync(kFull, base, __ffs(m) - 1);
-        const uint32_t pos = base + __popc(m & lt_mask);
-        uint32_t len = 0;
-        if (sel && pos < probe_topk) {
-          short_id[(size_t)b * probe_topk + pos] = key_id(k);
-          short_approx[(size_t)b * probe_topk + pos] = key_score(k);
-          len = ix.item_n_vec[key_id(k)];
-        }
-        const uint32_t tot = __reduce_add_sync(kFull, len);
-        if (lane == 0 && tot) atomicAdd(g_stok, tot);
-      }
+      const bool in = i < n_cand;
+      const uint64_t kp = cut ? kv[u] >> shift : 1ull;
+      emit(in && (kp > prefix || (whole && kp == prefix)), kv[u]);
+      if (in && list && kp == prefix) list[atomicAdd(g_list, 1u)] = kv[u];
     }
   }
+  if (list) cluster_sync<CL>();
+  if (list && cr == 0) {  // the `need` largest of the boundary bin's keys
+    const uint32_t n = *sm.n_list;
+    const uint32_t mine = tid < kSelList ? tid : kSelList;  // kSelList <= kFilterThreads
+    if ((uint32_t)(warp * 32) < n) {
+      const bool has = mine < n;
+      const uint64_t k = has ? sm.list[mine] : 0ull;
+      uint32_t rank = 0;
+      for (uint32_t i = 0; i < n; i++) rank += sm.list[i] > k ? 1u : 0u;
+      emit(has && rank < need, k);
+    }
+  }
+  // tokens of the shortlist (after the emission: a length per emitted key
+  // there put a dependent load into every step of it)
+  cluster_sync<CL>();
+  const uint32_t n_sel = min(*(volatile uint32_t *)g_sel, probe_topk);
+  uint32_t len = 0;
+  for (uint32_t i = cr * kFilterThreads + tid; i < n_sel; i += cstride)
+    len += ix.item_n_vec[__ldcg(short_id + (size_t)b * probe_topk + i)];
+  len = __reduce_add_sync(kFull, len);
+  if (lane == 0 && len) atomicAdd(g_stok, len);
 }
 
 template <int CL>
@@ -440,14 +487,17 @@ filter_kernel(DevIndex ix, const uint32_t *__restrict__ probe_id,
               uint32_t *__restrict__ short_id, float *__restrict__ short_approx,
               uint32_t *__restrict__ n_short_out, uint32_t *__restrict__ qstat,
               uint32_t *__restrict__ only_if, int impute) {
-  __shared__ long long pfix[kMaxQueryTok * kMaxProbe];
+  // the probes' scores, offsets and sizes; the select phase reuses their space
+  constexpr int kProbes = kMaxQueryTok * kMaxProbe;
+  __shared__ __align__(16) unsigned char pool[kProbes * 20];
+  static_assert(sizeof(pool) >= kSelSmem, "select state");
+  long long *pfix = reinterpret_cast<long long *>(pool);
+  uint64_t *lof = reinterpret_cast<uint64_t *>(pool) + kProbes;
+  uint32_t *lsz = reinterpret_cast<uint32_t *>(pool) + 4 * kProbes;
   __shared__ long long impf[kMaxQueryTok];  // imputed score of an unmatched token (0: off)
   __shared__ uint32_t pref[kMaxQueryTok + 1];
-  __shared__ uint32_t lsz[kMaxQueryTok * kMaxProbe];
-  __shared__ uint64_t lof[kMaxQueryTok * kMaxProbe];
-  __shared__ uint32_t hist[2][256];
-  __shared__ uint32_t s_ncand, s_sel, s_stok;     // CTA 0's copies are the cluster's
-  __shared__ uint32_t s_digit, s_need, s_done, s_entries;
+  __shared__ uint32_t s_ncand, s_sel, s_stok, s_nlist;     // CTA 0's copies are the cluster's
+  __shared__ uint32_t s_wsum[32], s_bin, s_need, s_cnt, s_entries;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n_warp = blockDim.x >> 5;
@@ -584,7 +634,9 @@ filter_kernel(DevIndex ix, const uint32_t *__restrict__ probe_id,
   filter_sync<CL>();
 
   // ---- phases C/D: radix select + emit ----
-  SelectSmem sm{hist, &s_digit, &s_need, &s_done};
+  SelectSmem sm{reinterpret_cast<uint32_t *>(pool),
+                reinterpret_cast<uint64_t *>(pool) + kSelBins / 2, s_wsum, &s_bin, &s_need, &s_cnt,
+                &s_nlist};
   select_emit<CL>(ix, key, n_cand, probe_topk, b, cr, sm, g_sel, g_stok, short_id, short_approx);
   filter_sync<CL>();
   if (cr == 0 && tid == 0) {
@@ -650,11 +702,13 @@ filter_hash_kernel(DevIndex ix, const uint32_t *__restrict__ probe_id,
   const uint64_t tok0 = q_off[b];
   const uint32_t nq = (uint32_t)(q_off[b + 1] - tok0);
 
-  for (uint32_t i = tid; i < kHashCap; i += blockDim.x) {
-    tkey[i] = kEmpty;
-    tacc[i] = 0ull;
-#pragma unroll
-    for (int w = 0; w < MW; w++) tmask[i * MW + w] = 0u;
+  {  // 16-byte stores: keys empty, masks and scores 0
+    uint4 *t4 = reinterpret_cast<uint4 *>(hsm);
+    constexpr uint32_t kKeys4 = kHashCap / 4, kAll4 = (uint32_t)(hash_smem_bytes(MW) / 16);
+    for (uint32_t i = tid; i < kAll4; i += kFilterThreads) {
+      const uint32_t x = i < kKeys4 ? kEmpty : 0u;
+      t4[i] = make_uint4(x, x, x, x);
+    }
   }
   if (tid == 0) { s_fill = 0; s_ovf = 0; s_entries = 0; }
   for (uint32_t t = tid; t < nq; t += blockDim.x)
@@ -708,6 +762,9 @@ filter_hash_kernel(DevIndex ix, const uint32_t *__restrict__ probe_id,
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
+          // a range's share of a list is often shorter than a round (50 entries
+          // of 128 at 1M docs, 65,536 lists and 8 ranges): stop where it ends
+          if (p0 + 32u * u >= sz) break;
           const uint32_t it = its[u];
           // find or insert `it` (linear probing; the walk is bounded by the
           // table size, and a CTA stops inserting once its fill count passes
@@ -820,13 +877,14 @@ __global__ void __launch_bounds__(kFilterThreads, 1)
 filter_select_kernel(DevIndex ix, uint32_t probe_topk, FilterScratch scr,
                      uint32_t *__restrict__ short_id, float *__restrict__ short_approx,
                      uint32_t *__restrict__ n_short_out, uint32_t *__restrict__ qstat) {
-  __shared__ uint32_t hist[2][256];
-  __shared__ uint32_t s_sel, s_stok, s_digit, s_need, s_done;
+  __shared__ __align__(16) uint32_t hist[kSelBins];
+  __shared__ __align__(16) uint64_t list[kSelList];
+  __shared__ uint32_t s_wsum[32], s_sel, s_stok, s_bin, s_need, s_cnt, s_nlist;
   const uint32_t b = blockIdx.x;
   const uint32_t n_cand = scr.qcnt[b];
   if (threadIdx.x == 0) { s_sel = 0; s_stok = 0; }
   __syncthreads();
-  SelectSmem sm{hist, &s_digit, &s_need, &s_done};
+  SelectSmem sm{hist, list, s_wsum, &s_bin, &s_need, &s_cnt, &s_nlist};
   select_emit<1>(ix, scr.hkey + (size_t)b * scr.key_stride, n_cand, probe_topk, b, 0, sm, &s_sel,
                  &s_stok, short_id, short_approx);
   __syncthreads();
@@ -1415,6 +1473,9 @@ cudaError_t launch_filter_hash(const DevIndex &ix, const uint32_t *probe_id,
   else
     filter_hash_kernel<2><<<n_cta, kFilterThreads, hash_smem_bytes(2), st>>>(
         ix, probe_id, probe_s, nprobe, q_off, cta_off, n_query, scr, qstat, impute);
+  // one CTA per query also where queries are few: clusters of 4 and 8 CTAs took
+  // 18 and 42 us where it takes 7 (1,065 candidates), 38 and 79 us where it takes
+  // 32 (34,000), their histograms and counters being remote
   filter_select_kernel<<<n_query, kFilterThreads, 0, st>>>(ix, probe_topk, scr, short_id,
                                                           short_approx, n_short, qstat);
   *n_launch += 2;

@@ -166,3 +166,25 @@ def test_maxsum_edges(dtype):
     # sums of up to 100 terms of size ~3 in another order: 100 ulps of 512 at most
     tol = 100 * 512 * torch.finfo(dtype).eps
     torch.testing.assert_close(got.cpu(), want, rtol=0, atol=tol, equal_nan=True)
+
+
+@pytest.mark.parametrize("ptk", [1, 511, 512, 513, 700, 3999, 4000, 5000])
+def test_shortlist_cut_edges(ptk):
+    """The shortlist's cut among equal scores (every key of the boundary bin differs in
+    its id alone), in the middle of distinct ones, and at the candidate count."""
+    rng = np.random.default_rng(1)
+    cen = unit(rng.standard_normal((40, 128)))
+    code = np.concatenate([np.zeros(3000, np.uint32), rng.integers(1, 40, 1000).astype(np.uint32)])
+    lens = np.ones(4000, np.uint32)
+    off, size, ids = pyoracle.ivf_build(code, lens, 40)
+    ix = dict(item_n_vec=lens, centroid=cen, vq_code=code, ivf_off=off, ivf_size=size, ivf_ids=ids,
+              weight=np.array([-0.05, 0.05], np.float32), n_bit=1,
+              residual=rng.integers(0, 256, 4000 * 16).astype(np.uint8))
+    q = unit(cen[0] + 0.3 * rng.standard_normal((3, 128)))
+    r = oracle_of(ix).search_one(q, 1, 32, ptk)
+    with gpu_index(ix) as g:
+        t = g.trace(q, 1, 32, ptk)
+    o = np.argsort(r["short_id"])
+    np.testing.assert_array_equal(t["cand_id"], r["cand_id"])
+    np.testing.assert_array_equal(t["short_id"], r["short_id"][o])
+    np.testing.assert_array_equal(t["short_approx"], r["short_approx"][o])
