@@ -283,9 +283,9 @@ int mvr_index_set_pruner(mvr_index *h, const float *params, uint32_t keep,
                          float margin);
 
 /* Tile shape of the FP8 MaxSim kernel (MVR_PREC_FP8): shortlisted docs per
- * CTA, 32, 64, 128 or 256 (0: the default, 256; queries of more than 32
- * tokens use at most 128); chosen by the library's tuner
- * (mvr.tune.tune_tile).  No counterpart in the reference. */
+ * CTA, 32, 64, 128 or 256 (queries of more than 32 tokens use at most 128), or
+ * 0, the default: chosen per call from the grid it gives; set by the library's
+ * tuner (mvr.tune.tune_tile).  No counterpart in the reference. */
 int mvr_index_set_rerank_tile(mvr_index *h, uint32_t docs_per_cta);
 
 /* Failure detection (test hook; no counterpart in the reference, whose

@@ -173,7 +173,7 @@ struct mvr_index {
   // queries of the previous search call (0: none yet)
   double cand_per_probe = 0.0;
   uint64_t wait_ns = 1000000000ull;  // bound of the FP8 rerank's pipeline waits
-  uint32_t ws_docs = 256;            // shortlisted docs per CTA of the FP8 rerank
+  uint32_t ws_docs = 0;              // shortlisted docs per CTA of the FP8 rerank (0: by the grid)
   // learned pruner (mvr_index_set_pruner): BF16 weight tiles, b1/b2/w3/b3
   uint8_t *prune_wts = nullptr;
   float *prune_vecs = nullptr;
@@ -456,15 +456,16 @@ int check_search_args(const mvr_index *h, uint32_t n_query, uint32_t topk, uint3
 }
 
 int build_offsets(const uint64_t *tok_off, uint32_t n_query, uint32_t query_n_vec,
-                  std::vector<uint64_t> &off, uint32_t *nq_max) {
+                  std::vector<uint64_t> &off, uint32_t *nq_min, uint32_t *nq_max) {
   off.resize((size_t)n_query + 1);
   *nq_max = 0;
+  *nq_min = kMaxQueryTok;
   if (!tok_off) {
     if (query_n_vec == 0 || query_n_vec > (uint32_t)kMaxQueryTok)
       return set_err(MVR_ERR_INVALID_ARG, "query_n_vec must be in [1, %d], got %u", kMaxQueryTok,
                      query_n_vec);
     for (uint32_t i = 0; i <= n_query; i++) off[i] = (uint64_t)i * query_n_vec;
-    *nq_max = query_n_vec;
+    *nq_min = *nq_max = query_n_vec;
     return MVR_OK;
   }
   if (tok_off[0] != 0) return set_err(MVR_ERR_INVALID_ARG, "tok_off[0] must be 0");
@@ -472,7 +473,9 @@ int build_offsets(const uint64_t *tok_off, uint32_t n_query, uint32_t query_n_ve
     if (tok_off[i + 1] <= tok_off[i] || tok_off[i + 1] - tok_off[i] > (uint64_t)kMaxQueryTok)
       return set_err(MVR_ERR_INVALID_ARG, "query %u has %lld tokens (allowed 1..%d)", i,
                      (long long)(tok_off[i + 1] - tok_off[i]), kMaxQueryTok);
-    *nq_max = std::max(*nq_max, (uint32_t)(tok_off[i + 1] - tok_off[i]));
+    const uint32_t nq = (uint32_t)(tok_off[i + 1] - tok_off[i]);
+    *nq_min = std::min(*nq_min, nq);
+    *nq_max = std::max(*nq_max, nq);
   }
   std::memcpy(off.data(), tok_off, off.size() * sizeof(uint64_t));
   return MVR_OK;
@@ -505,8 +508,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
   uint32_t R = h->rescore ? h->rescore : 4 * topk;
   R = std::min(std::max(R, topk), probe_topk);
   std::vector<uint64_t> off;
-  uint32_t nq_max = 0;
-  MVR_TRY(build_offsets(tok_off_in, n_query, query_n_vec, off, &nq_max));
+  uint32_t nq_min = 0, nq_max = 0;
+  MVR_TRY(build_offsets(tok_off_in, n_query, query_n_vec, off, &nq_min, &nq_max));
   const bool prune = (flags & MVR_PRUNE) != 0;
   if (prune) {
     // the features come from the FP8 centroid table (2- and 4-bit indexes);
@@ -673,8 +676,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         }
         if (fp8)
           CUDA_TRY(launch_rerank_ws(h->dix, h->cen8, h->tw_fp8, qp, qo, nb, sid, nsh,
-                                    probe_topk, sem, nq_max, h->x_bound, w.exact, h->d_err, rs,
-                                    &launches, h->wait_ns, h->ws_docs));
+                                    probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact, h->d_err,
+                                    h->n_sm, rs, &launches, h->wait_ns, h->ws_docs));
         else if (h->cen_perm)
           CUDA_TRY(launch_rerank_tmem(h->dix, h->cen_perm, h->tw_bf16, qp, qo, nb, sid, nsh,
                                       probe_topk, sem, nq_max, h->x_bound, w.exact,
@@ -1237,8 +1240,7 @@ int mvr_index_set_pruner(mvr_index *h, const float *params, uint32_t keep, float
 
 int mvr_index_set_rerank_tile(mvr_index *h, uint32_t docs_per_cta) {
   if (!h) return set_err(MVR_ERR_INVALID_ARG, "null index handle");
-  if (docs_per_cta == 0) docs_per_cta = 256;
-  if (!ws_docs_supported(docs_per_cta))
+  if (docs_per_cta && !ws_docs_supported(docs_per_cta))
     return set_err(MVR_ERR_INVALID_ARG, "docs per CTA %u: 32, 64, 128 or 256", docs_per_cta);
   DeviceGuard g(h->device);
   h->ws_docs = docs_per_cta;

@@ -2623,25 +2623,50 @@ static void ws_launch_docs(uint32_t docs, const DevIndex &ix, const uint8_t *c,
                           x_bound, approx, err, st, wait_ns);
 }
 
+// Docs per CTA of the FP8 MaxSim where none is set: the size that takes the
+// least time, waves of the grid x (docs + 12), 12 docs being what a CTA costs
+// besides (its TMEM, query tile, pipeline fill; a CTA alone on an SM takes 138
+// us for 256 docs of 70 tokens).  Bulk searches keep the widest (2,368 queries x
+// 1500 docs: 9.1 ms at 256, 9.3 at 128); one query x 1500 goes from 6 CTAs to
+// 47, 138 -> 26 us, 37 queries x 1000 from 148 to 296, 147 -> 111 us.
+static uint32_t ws_auto_docs(uint32_t n_query, uint32_t probe_topk, uint32_t slots,
+                             uint32_t widest) {
+  uint32_t docs = widest;
+  uint64_t least = ~0ull;
+  for (uint32_t d = widest; d >= 32; d /= 2) {
+    const uint64_t ctas = (uint64_t)n_query * ((probe_topk + d - 1) / d);
+    const uint64_t cost = (ctas + slots - 1) / slots * (std::min(d, probe_topk) + 12u);
+    if (cost < least) { least = cost; docs = d; }
+  }
+  return docs;
+}
+
 cudaError_t launch_rerank_ws(const DevIndex &ix, const void *cen8, const TmWeights &tw,
                              const float *q, const uint64_t *q_off, uint32_t n_query,
                              const uint32_t *short_id, const uint32_t *n_short,
-                             uint32_t probe_topk, int semantics, uint32_t nq_max, float x_bound,
-                             float *approx, unsigned *err, cudaStream_t st, int *n_launch,
-                             uint64_t wait_ns, uint32_t docs) {
-  if (!fp8_rerank_supported(ix.n_bit) || !ws_docs_supported(docs)) return cudaErrorInvalidValue;
+                             uint32_t probe_topk, int semantics, uint32_t nq_min, uint32_t nq_max,
+                             float x_bound, float *approx, unsigned *err, int n_sm,
+                             cudaStream_t st, int *n_launch, uint64_t wait_ns, uint32_t set_docs) {
+  if (!fp8_rerank_supported(ix.n_bit) || (set_docs && !ws_docs_supported(set_docs)))
+    return cudaErrorInvalidValue;
   const uint8_t *c = reinterpret_cast<const uint8_t *>(cen8);
   // queries of up to 32 tokens run in the 32-column variant (two CTAs per
   // SM), longer ones in the 64-column variant (one CTA per SM); each launch
   // skips the other's queries
-  if (ix.n_bit == 4)
-    ws_launch_docs<4, 32>(docs, ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk,
-                          semantics, x_bound, approx, err, st, wait_ns);
-  else
-    ws_launch_docs<2, 32>(docs, ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk,
-                          semantics, x_bound, approx, err, st, wait_ns);
-  *n_launch += 1;
+  if (nq_min <= 32) {
+    const uint32_t docs =
+        set_docs ? set_docs : ws_auto_docs(n_query, probe_topk, 2u * (uint32_t)n_sm, 256u);
+    if (ix.n_bit == 4)
+      ws_launch_docs<4, 32>(docs, ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk,
+                            semantics, x_bound, approx, err, st, wait_ns);
+    else
+      ws_launch_docs<2, 32>(docs, ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk,
+                            semantics, x_bound, approx, err, st, wait_ns);
+    *n_launch += 1;
+  }
   if (nq_max > 32) {
+    const uint32_t docs =
+        set_docs ? set_docs : ws_auto_docs(n_query, probe_topk, (uint32_t)n_sm, 128u);
     if (ix.n_bit == 4)
       ws_launch_docs<4, 64>(docs, ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk,
                             semantics, x_bound, approx, err, st, wait_ns);

@@ -50,13 +50,14 @@ cudaError_t make_centroid_fp8(const float *cen, uint32_t n_cent, uint32_t n_bit,
 // over a shared-memory ring fed by bulk copies): cen8 as above with one zero
 // row appended (row n_centroid); the vq code array must be readable 16 bytes
 // past its last code.  wait_ns bounds every pipeline wait of the kernel (on
-// expiry it stops and sets bit 4 of *err); docs: shortlisted docs per CTA.
+// expiry it stops and sets bit 4 of *err); nq_min / nq_max: fewest and most
+// tokens of a query; set_docs: shortlisted docs per CTA (0: by the grid).
 cudaError_t launch_rerank_ws(const DevIndex &ix, const void *cen8, const TmWeights &tw,
                              const float *q, const uint64_t *q_off, uint32_t n_query,
                              const uint32_t *short_id, const uint32_t *n_short,
-                             uint32_t probe_topk, int semantics, uint32_t nq_max, float x_bound,
-                             float *approx, unsigned *err, cudaStream_t st, int *n_launch,
-                             uint64_t wait_ns, uint32_t docs);
+                             uint32_t probe_topk, int semantics, uint32_t nq_min, uint32_t nq_max,
+                             float x_bound, float *approx, unsigned *err, int n_sm,
+                             cudaStream_t st, int *n_launch, uint64_t wait_ns, uint32_t set_docs);
 // shortlisted docs per CTA the FP8 kernel is built for (32, 64, 128, 256)
 bool ws_docs_supported(uint32_t docs);
 
