@@ -132,6 +132,13 @@ struct Workspace {
   uint64_t *h_off = nullptr;    // pinned mirror
   uint32_t *qstat = nullptr;    // device [n_query][3]
   uint32_t *h_qstat = nullptr;  // pinned mirror
+  // host-buffer calls: pinned staging of the call's results (scores then ids),
+  // and for small calls of its queries behind the offsets, one copy each way
+  size_t ret_cap = 0, in_cap = 0;
+  float *ret = nullptr, *h_ret = nullptr;      // [2 * n_query * topk]
+  uint8_t *in = nullptr, *h_in = nullptr;      // offsets, then query tokens
+  const float *last_q = nullptr;               // where the last batch's tokens and offsets were
+  const uint64_t *last_off = nullptr;
   // learned pruner (MVR_PRUNE), per batch
   uint32_t pr_slots = 0, pr_short = 0, pr_keep = 0;
   float *feat = nullptr;        // [slots][short][33] features
@@ -153,7 +160,7 @@ struct mvr_index {
   std::vector<cudaEvent_t> events;
   // host-buffer calls: query copies on their own stream, one event per batch
   cudaStream_t copy_stream = nullptr;
-  std::vector<cudaEvent_t> copy_events;
+  std::vector<cudaEvent_t> copy_events, done_events;  // ... and one when its kernels are done
   uint32_t batch_cap = 0;
   uint32_t rescore = 0;          // FP32 re-score count of the BF16 path (0: 4 * topk)
   void *cen_bf16 = nullptr;      // [C][128] BF16 centroid rows
@@ -166,6 +173,7 @@ struct mvr_index {
   void *cen8 = nullptr;          // [C][128] E4M3 centroid rows, FP8-rerank K order (b = 2, 4)
   TmWeights tw_fp8{};            // E4M3 weight tables of the FP8 MaxSim (b = 2, 4)
   unsigned *d_err = nullptr;     // device error flags of the tensor-core kernels
+  unsigned long long *h_flags = nullptr;  // pinned: the flags and d_fallback of a call
   uint32_t *d_epoch = nullptr;   // stamp-epoch counter of the rank-table fallback (device)
   uint64_t epoch_used = 0;       // epochs consumed since the stamps were last cleared
   uint64_t ws_gen = 0;           // bumped whenever a workspace buffer is reallocated
@@ -194,6 +202,7 @@ struct mvr_index {
     double cand_per_probe = 0.0;  // the hash filter's layout was sized by this
     std::vector<uint64_t> off;
     int launches = 0;
+    bool timed = false;  // records the stage events
   } graph;
   Workspace ws;
 
@@ -221,8 +230,14 @@ struct mvr_index {
     dfree(ws.qstat);
     if (ws.h_off) cudaFreeHost(ws.h_off);
     if (ws.h_qstat) cudaFreeHost(ws.h_qstat);
+    dfree(ws.ret);
+    dfree(ws.in);
+    if (ws.h_ret) cudaFreeHost(ws.h_ret);
+    if (ws.h_in) cudaFreeHost(ws.h_in);
+    if (h_flags) cudaFreeHost(h_flags);
     for (auto e : events) cudaEventDestroy(e);
     for (auto e : copy_events) cudaEventDestroy(e);
+    for (auto e : done_events) cudaEventDestroy(e);
     if (copy_stream) cudaStreamSynchronize(copy_stream);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     if (stream) cudaStreamDestroy(stream);
@@ -417,6 +432,41 @@ int ensure_call(mvr_index *h, size_t n_off, size_t n_stat, size_t n_events) {
     CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     h->copy_events.push_back(e);
   }
+  while (h->done_events.size() * kStages + 1 < n_events) {
+    cudaEvent_t e;
+    CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    h->done_events.push_back(e);
+  }
+  return MVR_OK;
+}
+
+// Host-buffer calls of up to this many result (query and offset) bytes pass
+// them through pinned staging: a copy from or to pageable memory waits for the
+// stream, 10 us each for the three of a small call.
+constexpr size_t kStageRet = 64u << 20, kStageIn = 256u << 10;
+
+int ensure_stage(mvr_index *h, size_t n_ret, size_t in_bytes) {
+  Workspace &w = h->ws;
+  if (w.ret_cap < n_ret) {
+    dfree(w.ret);
+    w.ret = nullptr;
+    if (w.h_ret) cudaFreeHost(w.h_ret);
+    w.h_ret = nullptr;
+    w.ret_cap = 0;
+    MVR_TRY(dalloc(&w.ret, n_ret));
+    CUDA_TRY(cudaMallocHost((void **)&w.h_ret, n_ret * sizeof(float)));
+    w.ret_cap = n_ret;
+  }
+  if (w.in_cap < in_bytes) {
+    dfree(w.in);
+    w.in = nullptr;
+    if (w.h_in) cudaFreeHost(w.h_in);
+    w.h_in = nullptr;
+    w.in_cap = 0;
+    MVR_TRY(dalloc(&w.in, in_bytes));
+    CUDA_TRY(cudaMallocHost((void **)&w.h_in, in_bytes));
+    w.in_cap = in_bytes;
+  }
   return MVR_OK;
 }
 
@@ -548,6 +598,13 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                       (size_t)kStages * n_batch + 1));
   if (prune) MVR_TRY(ensure_prune(h, std::min(B, n_query), probe_topk, keep));
   Workspace &w = h->ws;
+  const bool timed = query_time_s || stage_s || stats;
+  const size_t n_res = (size_t)n_query * topk;
+  const bool stage_ret = host_io && 2 * n_res * sizeof(float) <= kStageRet;
+  const size_t off_bytes = (2 * ((size_t)n_query + n_batch) * sizeof(uint64_t) + 255) & ~(size_t)255;
+  const size_t in_bytes = off_bytes + (size_t)off[n_query] * kDim * sizeof(float);
+  const bool stage_in = host_io && n_batch == 1 && in_bytes <= kStageIn;
+  MVR_TRY(ensure_stage(h, stage_ret ? 2 * n_res : 0, stage_in ? in_bytes : 0));
 
   // stamp epochs this call takes (one per fallback chunk of every batch);
   // clear the stamps before the device counter could wrap
@@ -591,11 +648,21 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
   auto enqueue = [&](cudaStream_t rs, bool capturing) -> int {
     if (prune) CUDA_TRY(cudaMemsetAsync(h->d_fallback, 0, sizeof(unsigned long long), rs));
     auto rec = [&](cudaEvent_t e) {
+      if (!timed) return cudaSuccess;
       return capturing ? cudaEventRecordWithFlags(e, rs, cudaEventRecordExternal)
                        : cudaEventRecord(e, rs);
     };
-    CUDA_TRY(cudaMemcpyAsync(w.q_off, w.h_off, 2 * n_off * sizeof(uint64_t),
-                             cudaMemcpyHostToDevice, rs));
+    const uint64_t *d_off = w.q_off;
+    if (stage_in) {  // offsets and queries in one copy
+      std::memcpy(w.h_in, w.h_off, 2 * n_off * sizeof(uint64_t));
+      std::memcpy(w.h_in + off_bytes, query, in_bytes - off_bytes);
+      CUDA_TRY(cudaMemcpyAsync(w.in, w.h_in, in_bytes, cudaMemcpyHostToDevice, rs));
+      d_off = reinterpret_cast<const uint64_t *>(w.in);
+      h2d += in_bytes - off_bytes;
+    } else {
+      CUDA_TRY(cudaMemcpyAsync(w.q_off, w.h_off, 2 * n_off * sizeof(uint64_t),
+                               cudaMemcpyHostToDevice, rs));
+    }
     // host buffers: batch bt's query tokens go to device buffer bt % 2 on
     // the copy stream, one batch ahead of the kernels, once batch bt - 2
     // (the buffer's previous user) has finished
@@ -605,7 +672,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     auto copy_in = [&](uint32_t bt) -> int {
       const uint32_t s = bt * B, e = std::min(n_query, s + B);
       const uint32_t T = (uint32_t)(off[e] - off[s]);
-      if (bt >= 2) CUDA_TRY(cudaStreamWaitEvent(h->copy_stream, ev(bt - 2, 5), 0));
+      if (bt >= 2) CUDA_TRY(cudaStreamWaitEvent(h->copy_stream, h->done_events[bt - 2], 0));
       CUDA_TRY(cudaMemcpyAsync(qbuf(bt), query + off[s] * kDim, (size_t)T * kDim * sizeof(float),
                                cudaMemcpyHostToDevice, h->copy_stream));
       CUDA_TRY(cudaEventRecord(h->copy_events[bt], h->copy_stream));
@@ -621,24 +688,50 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
       const uint32_t s = bt * B, e = std::min(n_query, s + B), nb = e - s;
       CUDA_TRY(rec(ev(bt, 0)));
       const uint32_t T = (uint32_t)(off[e] - off[s]);
-      const uint64_t *qo = w.q_off + (size_t)s + bt;
+      const uint64_t *qo = d_off + (size_t)s + bt;
       const float *qp;
+      uint32_t n_part = 1;  // pieces that the queries are copied and scored in
       if (pipelined) {
         if (bt + 1 < n_batch) MVR_TRY(copy_in(bt + 1));
         CUDA_TRY(cudaStreamWaitEvent(rs, h->copy_events[bt], 0));
         qp = qbuf(bt);
+      } else if (stage_in) {
+        qp = reinterpret_cast<const float *>(w.in + off_bytes);
       } else if (host_io) {
-        CUDA_TRY(cudaMemcpyAsync(w.q, query + off[s] * kDim, (size_t)T * kDim * sizeof(float),
-                                 cudaMemcpyHostToDevice, rs));
-        h2d += (size_t)T * kDim * sizeof(float);
+        // a single batch has no other batch's kernels to hide its copy behind:
+        // pieces of it are copied while the pieces before them are scored
+        // (600 queries of 33 to 64 tokens: 15 MB, 0.8 of 9.5 ms)
+        n_part = std::max(1u, std::min(4u, T / 4096u));
         qp = w.q;
+        if (n_part > 1) {
+          CUDA_TRY(cudaEventRecord(h->ev_in, rs));  // after the caller's prior work
+          CUDA_TRY(cudaStreamWaitEvent(h->copy_stream, h->ev_in, 0));
+        }
       } else {
         qp = query + off[s] * kDim;
       }
       CUDA_TRY(rec(ev(bt, 1)));
-      const uint32_t chunk = probe_chunk(nprobe, h->n_sm);
-      for (uint32_t c = 0; c < T; c += chunk) {
+      w.last_q = qp;
+      w.last_off = qo;
+      uint32_t chunk = probe_chunk(nprobe, h->n_sm);
+      if (n_part > 1) chunk = std::min(chunk, ((T / n_part + 255u) & ~255u));
+      for (uint32_t c = 0, i = 0; c < T; c += chunk, i++) {
         const uint32_t n = std::min(chunk, T - c);
+        if (host_io && !pipelined && !stage_in) {
+          CUDA_TRY(cudaMemcpyAsync(w.q + (size_t)c * kDim, query + (off[s] + c) * kDim,
+                                   (size_t)n * kDim * sizeof(float), cudaMemcpyHostToDevice,
+                                   n_part > 1 ? h->copy_stream : rs));
+          if (n_part > 1) {
+            while (h->copy_events.size() <= i) {
+              cudaEvent_t e;
+              CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+              h->copy_events.push_back(e);
+            }
+            CUDA_TRY(cudaEventRecord(h->copy_events[i], h->copy_stream));
+            CUDA_TRY(cudaStreamWaitEvent(rs, h->copy_events[i], 0));
+          }
+          h2d += (size_t)n * kDim * sizeof(float);
+        }
         CUDA_TRY(launch_probe(qp + (size_t)c * kDim, n, h->cen_sw, h->dix.centroid,
                               h->dix.centroid_t, h->dix.n_centroid, h->dix.n_centroid_pad,
                               h->cen_bounds, nprobe,
@@ -653,8 +746,10 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                                   w.n_short, w.qstat + (size_t)s * 3, rs, &launches,
                                   (flags & MVR_CAND_IMPUTE) ? 1 : 0));
       CUDA_TRY(rec(ev(bt, 3)));
-      float *os = host_io ? w.out_s : out_s + (size_t)s * topk;
-      uint32_t *oi = host_io ? w.out_id : out_id + (size_t)s * topk;
+      float *os = stage_ret ? w.ret + (size_t)s * topk : host_io ? w.out_s : out_s + (size_t)s * topk;
+      uint32_t *oi = stage_ret ? reinterpret_cast<uint32_t *>(w.ret + n_res) + (size_t)s * topk
+                     : host_io ? w.out_id
+                               : out_id + (size_t)s * topk;
       if (bf16) {
         // tensor-core MaxSim (FP8 or BF16) over the shortlist -- with
         // MVR_PRUNE over the docs the pruner keeps -- then the exact FP32
@@ -718,7 +813,13 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                              &launches));
       }
       CUDA_TRY(rec(ev(bt, 5)));
-      if (host_io) {
+      if (pipelined) CUDA_TRY(cudaEventRecord(h->done_events[bt], rs));
+      if (stage_ret) {
+        d2h += (size_t)nb * topk * 8;
+        if (bt + 1 == n_batch)
+          CUDA_TRY(cudaMemcpyAsync(w.h_ret, w.ret, 2 * n_res * sizeof(float),
+                                   cudaMemcpyDeviceToHost, rs));
+      } else if (host_io) {
         CUDA_TRY(cudaMemcpyAsync(out_s + (size_t)s * topk, w.out_s,
                                  (size_t)nb * topk * sizeof(float), cudaMemcpyDeviceToHost, rs));
         CUDA_TRY(cudaMemcpyAsync(out_id + (size_t)s * topk, w.out_id,
@@ -742,7 +843,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     const bool same = G.exec && G.query == query && G.out_s == out_s && G.out_id == out_id &&
                       G.n_query == n_query && G.topk == topk && G.nprobe == nprobe &&
                       G.probe_topk == probe_topk && G.flags == flags && G.R == R && G.B == B &&
-                      G.gen == h->ws_gen && G.off == off && G.cand_per_probe == cpe;
+                      G.gen == h->ws_gen && G.off == off && G.cand_per_probe == cpe &&
+                      G.timed == timed;
     CUDA_TRY(cudaEventRecord(h->ev_in, st));
     CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_in, 0));
     if (!same) {
@@ -765,6 +867,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
       G.query = query; G.out_s = out_s; G.out_id = out_id; G.n_query = n_query; G.topk = topk;
       G.nprobe = nprobe; G.probe_topk = probe_topk; G.flags = flags; G.R = R; G.B = B;
       G.gen = h->ws_gen; G.off = off; G.launches = launches; G.cand_per_probe = cpe;
+      G.timed = timed;
     }
     launches = G.launches;
     CUDA_TRY(cudaEventRecord(h->ev_g0, h->stream));
@@ -775,14 +878,19 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
   }
   CUDA_TRY(cudaMemcpyAsync(w.h_qstat, w.qstat, (size_t)n_query * 3 * sizeof(uint32_t),
                            cudaMemcpyDeviceToHost, st));
-  unsigned herr = 0;
-  unsigned long long n_fallback = 0;
-  CUDA_TRY(cudaMemcpyAsync(&herr, h->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  h->h_flags[0] = h->h_flags[1] = 0;
+  CUDA_TRY(cudaMemcpyAsync(&h->h_flags[0], h->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   if (prune)
-    CUDA_TRY(cudaMemcpyAsync(&n_fallback, h->d_fallback, sizeof(n_fallback), cudaMemcpyDeviceToHost,
-                             st));
+    CUDA_TRY(cudaMemcpyAsync(&h->h_flags[1], h->d_fallback, sizeof(unsigned long long),
+                             cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   CUDA_TRY(cudaGetLastError());
+  const unsigned herr = (unsigned)h->h_flags[0];
+  const unsigned long long n_fallback = h->h_flags[1];
+  if (stage_ret) {
+    std::memcpy(out_s, w.h_ret, n_res * sizeof(float));
+    std::memcpy(out_id, w.h_ret + n_res, n_res * sizeof(uint32_t));
+  }
   if (herr) {
     CUDA_TRY(cudaMemset(h->d_err, 0, sizeof(unsigned)));
     if (herr & 16u)
@@ -801,6 +909,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     if (r > 0.0) h->cand_per_probe = r;
   }
 
+  if (!timed) return MVR_OK;
   float total_ms = 0.f, max_ms = 0.f;
   if (use_graph)  // the graph launch as a whole, bracketed outside the graph
     CUDA_TRY(cudaEventElapsedTime(&total_ms, h->ev_g0, h->ev_g1));
@@ -962,6 +1071,7 @@ int new_handle(int device, std::unique_ptr<mvr_index> &h) {
   CUDA_TRY(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
   MVR_TRY(dalloc(&h->d_err, 1));
   CUDA_TRY(cudaMemset(h->d_err, 0, sizeof(unsigned)));
+  CUDA_TRY(cudaMallocHost((void **)&h->h_flags, 2 * sizeof(unsigned long long)));
   MVR_TRY(dalloc(&h->d_epoch, 1));
   CUDA_TRY(cudaMemset(h->d_epoch, 0, sizeof(uint32_t)));
   CUDA_TRY(cudaEventCreateWithFlags(&h->ev_in, cudaEventDisableTiming));
@@ -1353,7 +1463,7 @@ int mvr_search_trace(mvr_index *h, const float *query, uint32_t nq, uint32_t top
     MVR_TRY(dalloc(&d_feat, (size_t)probe_topk * 33));
     MVR_TRY(dalloc(&d_pred, probe_topk));
     std::vector<float> f((size_t)n_short * 33), p(n_short);
-    cudaError_t e = launch_prune_features(h->dix, h->cen8, w.q, w.q_off, 1, w.short_id, w.n_short,
+    cudaError_t e = launch_prune_features(h->dix, h->cen8, w.last_q, w.last_off, 1, w.short_id, w.n_short,
                                           probe_topk, h->x_bound, d_feat, h->d_err, h->stream, &l,
                                           h->wait_ns);
     if (e == cudaSuccess && tr->short_pred)

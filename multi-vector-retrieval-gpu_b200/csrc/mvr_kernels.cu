@@ -842,8 +842,6 @@ filter_hash_kernel(DevIndex ix, const uint32_t *__restrict__ probe_id,
   }
 }
 
-__global__ void advance_epoch_kernel(uint32_t *epoch, uint32_t n) { *epoch += n; }
-
 // ivf_part[c][p] = first position of list c whose doc id is >= p * n_item / P
 // (p = 0..P): the doc-range sub-lists of the hash filter.
 __global__ void ivf_part_kernel(const uint64_t *__restrict__ ivf_off,
@@ -872,11 +870,13 @@ cudaError_t make_ivf_part(const DevIndex &ix, uint32_t *out, cudaStream_t st) {
 }
 
 // Shortlist of every query from the keys filter_hash_kernel emitted; resets
-// the query's key counter for the next batch.
+// the query's key counter for the next batch and advances the fallback's stamp
+// epoch by the launches that may follow.
 __global__ void __launch_bounds__(kFilterThreads, 1)
 filter_select_kernel(DevIndex ix, uint32_t probe_topk, FilterScratch scr,
                      uint32_t *__restrict__ short_id, float *__restrict__ short_approx,
-                     uint32_t *__restrict__ n_short_out, uint32_t *__restrict__ qstat) {
+                     uint32_t *__restrict__ n_short_out, uint32_t *__restrict__ qstat,
+                     uint32_t *__restrict__ epoch, uint32_t n_epoch) {
   __shared__ __align__(16) uint32_t hist[kSelBins];
   __shared__ __align__(16) uint64_t list[kSelList];
   __shared__ uint32_t s_wsum[32], s_sel, s_stok, s_bin, s_need, s_cnt, s_nlist;
@@ -893,6 +893,7 @@ filter_select_kernel(DevIndex ix, uint32_t probe_topk, FilterScratch scr,
     qstat[b * 3 + 0] = n_cand;
     qstat[b * 3 + 2] = s_stok;
     scr.qcnt[b] = 0;
+    if (b == 0) *epoch += n_epoch;  // the rank-table fallback's, which runs next
   }
 }
 
@@ -1477,25 +1478,24 @@ cudaError_t launch_filter_hash(const DevIndex &ix, const uint32_t *probe_id,
   // 18 and 42 us where it takes 7 (1,065 candidates), 38 and 79 us where it takes
   // 32 (34,000), their histograms and counters being remote
   filter_select_kernel<<<n_query, kFilterThreads, 0, st>>>(ix, probe_topk, scr, short_id,
-                                                          short_approx, n_short, qstat);
+                                                          short_approx, n_short, qstat, epoch,
+                                                          (n_query + fb_slots - 1) / fb_slots);
   *n_launch += 2;
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // queries whose candidates overflowed a hash table: rank-table filter, in
-  // chunks of fb_slots queries over its fb_slots scratch slots; chunk c uses
-  // stamp epoch *epoch + 1 + c, then the counter advances by the chunk count
+  // chunks of fb_slots queries over its fb_slots scratch slots; chunk c takes the
+  // stamp epoch *epoch - c of those that the select kernel advanced it by
   uint32_t c = 0;
   for (uint32_t q0 = 0; q0 < n_query; q0 += fb_slots, c++) {
     const uint32_t cnt = n_query - q0 < fb_slots ? n_query - q0 : fb_slots;
     e = launch_filter_cluster(ix, probe_id, probe_s, nprobe, q_off + q0, cnt, probe_topk, scr,
-                              epoch, 1u + c, short_id + (size_t)q0 * probe_topk,
+                              epoch, 0u - c, short_id + (size_t)q0 * probe_topk,
                               short_approx + (size_t)q0 * probe_topk, n_short + q0,
                               qstat + (size_t)q0 * 3, st, n_launch, scr.ovf + q0, impute);
     if (e != cudaSuccess) return e;
   }
-  advance_epoch_kernel<<<1, 1, 0, st>>>(epoch, c);
-  *n_launch += 1;
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 // Shortlisted docs per CTA of the exact rerank: kRkDocs for grids that fill

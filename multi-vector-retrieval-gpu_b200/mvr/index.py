@@ -158,10 +158,11 @@ class Index:
     def search(self, queries, k, nprobe, probe_topk, tok_off=None, semantics=SEM_PP,
                with_stats=False, with_stages=False):
         q, off, n_query, n_vec = _flatten_queries(queries, tok_off)
-        scores = np.zeros((n_query, k), np.float32)
-        ids = np.zeros((n_query, k), np.uint32)
-        qtime = np.zeros(n_query, np.float64)
-        st = _lib.Stats()
+        scores = np.empty((n_query, k), np.float32)
+        ids = np.empty((n_query, k), np.uint32)
+        timed = with_stats or with_stages
+        qtime = np.zeros(n_query, np.float64) if timed else None
+        st = _lib.Stats() if timed else None
         if with_stages:
             stages = np.zeros((n_query, 6), np.float64)
             check(lib().mvr_search_staged(self._h, _ptr(q), _ptr(off), n_query, n_vec, k, nprobe,
@@ -171,7 +172,7 @@ class Index:
             stages = None
             check(lib().mvr_search(self._h, _ptr(q), _ptr(off), n_query, n_vec, k, nprobe,
                                    probe_topk, semantics, _ptr(scores), _ptr(ids), _ptr(qtime),
-                                   C.byref(st)))
+                                   C.byref(st) if timed else None))
         if not with_stats:
             return scores, ids
         out = dict(st.as_dict(), query_time_s=qtime)
