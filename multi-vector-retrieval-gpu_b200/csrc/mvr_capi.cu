@@ -170,6 +170,7 @@ struct mvr_index {
   void *cen_perm = nullptr;      // [C][64] bf16x2 centroid rows, TMEM-rerank K order (b <= 2)
   TmWeights tw_bf16{};           // weight tables of the BF16 tensor-memory MaxSim (b <= 2)
   float x_bound = 0.f;           // bound on the norm of every decoded doc token
+  float w_norm = 0.f, w_err = 0.f;  // ... of a token's weights, of their BF16 rounding errors
   void *cen8 = nullptr;          // [C][128] E4M3 centroid rows, FP8-rerank K order (b = 2, 4)
   TmWeights tw_fp8{};            // E4M3 weight tables of the FP8 MaxSim (b = 2, 4)
   unsigned *d_err = nullptr;     // device error flags of the tensor-core kernels
@@ -542,7 +543,8 @@ int build_offsets(const uint64_t *tok_off, uint32_t n_query, uint32_t query_n_ve
 int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, uint32_t n_query,
                 uint32_t query_n_vec, uint32_t topk, uint32_t nprobe, uint32_t probe_topk,
                 uint32_t flags, float *out_s, uint32_t *out_id, double *query_time_s,
-                double *stage_s, mvr_stats *stats, cudaStream_t st, bool host_io) {
+                double *stage_s, mvr_stats *stats, cudaStream_t st, bool host_io,
+                bool all_exact = false /* score the whole shortlist exactly (traces) */) {
   const auto t_start = std::chrono::steady_clock::now();
   MVR_TRY(check_search_args(h, n_query, topk, nprobe, probe_topk));
   if (n_query == 0) {
@@ -572,6 +574,20 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     if (!h->prune_wts) return set_err(MVR_ERR_INVALID_ARG, "MVR_PRUNE: no pruner set");
     if (nq_max > 32) return set_err(MVR_ERR_UNSUPPORTED, "MVR_PRUNE: queries of up to 32 tokens");
   }
+  // Exact FP32 search of 1- and 2-bit codes: where a shortlist is long, the BF16
+  // pass first leaves out the docs that provably miss the top topk, and the FP32
+  // kernel scores the rest (127 of 1500 on average for the best 10).  The line: at 14
+  // and 4.8 docs' tokens per ns the pass pays for itself once it spares a third
+  // of the FP32 work, which takes a shortlist of 4 topk (361 of 1500 stay for the
+  // best 100); its launches take 60 us, the FP32 work of 7,000 docs, and its CTAs
+  // of 64 docs want a grid that fills the GPU: 32,768 docs.  Queries of up to 16
+  // tokens take the FP32 kernel's half-width body, at twice its rate.  The wider
+  // codes' BF16 kernel is no faster than the FP32 one (4.9 tokens per ns at 8 bits).
+  const bool reach = !bf16 && !prune && !all_exact && h->cen_perm && nq_max > 16 &&
+                     probe_topk / 4 >= topk &&
+                     (uint64_t)std::min(h->batch_cap ? h->batch_cap : default_batch(h), n_query) *
+                             probe_topk >= 32768;
+  if (reach) R = probe_topk;
   const uint32_t keep = prune ? std::min(h->prune_keep, probe_topk) : 0u;
   DeviceGuard g(h->device);
 
@@ -806,11 +822,24 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
           sid = w.fin_id;
           nsh = w.n_fin;
         }
-        CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, sid, nsh, probe_topk, sem, w.exact, h->n_sm, rs,
-                               &launches));
+        if (reach) {
+          CUDA_TRY(launch_rerank_tmem(h->dix, h->cen_perm, h->tw_bf16, qp, qo, nb, sid, nsh,
+                                      probe_topk, sem, nq_max, h->x_bound, w.exact, h->d_err, rs,
+                                      &launches, false));
+          CUDA_TRY(launch_maxsim_reach(qp, qo, nb, sid, w.exact, nsh, probe_topk, topk,
+                                       h->cen_bounds, h->w_norm, h->w_err, w.r_id, w.n_r, rs,
+                                       &launches));
+          CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, w.r_id, w.n_r, probe_topk, sem, w.r_exact,
+                                 h->n_sm, rs, &launches, 32));
+          sid = w.r_id;
+          nsh = w.n_r;
+        } else {
+          CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, sid, nsh, probe_topk, sem, w.exact, h->n_sm,
+                                 rs, &launches));
+        }
         CUDA_TRY(rec(ev(bt, 4)));
-        CUDA_TRY(launch_topk(sid, w.exact, nsh, nb, probe_topk, topk, os, oi, nullptr, rs,
-                             &launches));
+        CUDA_TRY(launch_topk(sid, reach ? w.r_exact : w.exact, nsh, nb, probe_topk, topk, os, oi,
+                             nullptr, rs, &launches));
       }
       CUDA_TRY(rec(ev(bt, 5)));
       if (pipelined) CUDA_TRY(cudaEventRecord(h->done_events[bt], rs));
@@ -988,6 +1017,12 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
   h->cen_sw = sw;
   MVR_TRY(dalloc(&h->cen_bounds, 2, &h->bufs));
   CUDA_TRY(make_centroid_bounds(d.centroid, d.n_centroid, h->cen_bounds, h->stream));
+  for (uint32_t k = 0; k < (1u << d.n_bit); k++) {  // (a NaN or infinite weight: infinite bounds)
+    const float root = std::sqrt((float)kDim) * (1.0f + 0x1p-10f);
+    const float e = std::fabs(weight[k] - bf16_round(weight[k]));
+    h->w_norm = std::max(h->w_norm, std::isfinite(weight[k]) ? root * std::fabs(weight[k]) : INFINITY);
+    h->w_err = std::max(h->w_err, std::isfinite(e) ? root * e : INFINITY);
+  }
   if (tmem_rerank_supported(d.n_bit) || fp8_rerank_supported(d.n_bit)) {
     float wmax = 0.f;
     for (uint32_t k = 0; k < (1u << d.n_bit); k++) wmax = std::max(wmax, std::fabs(weight[k]));
@@ -1412,7 +1447,7 @@ int mvr_search_trace(mvr_index *h, const float *query, uint32_t nq, uint32_t top
     return set_err(MVR_ERR_UNSUPPORTED, "pruner features: a 2- or 4-bit index, <= 32 tokens");
   if (tr->short_pred && !h->prune_wts) return set_err(MVR_ERR_INVALID_ARG, "no pruner set");
   MVR_TRY(search_impl(h, query, nullptr, 1, nq, topk, nprobe, probe_topk, flags, tr->topk_score,
-                      tr->topk_id, nullptr, nullptr, nullptr, h->stream, true));
+                      tr->topk_id, nullptr, nullptr, nullptr, h->stream, true, true));
   DeviceGuard g(h->device);
   Workspace &w = h->ws;
   if (tr->probe_id)

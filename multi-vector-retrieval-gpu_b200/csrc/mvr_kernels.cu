@@ -19,6 +19,9 @@
 #include "mvr_common.cuh"
 #include "mvr_kernels.cuh"
 
+#include <cuda_bf16.h>
+
+#include <algorithm>
 #include <cfloat>
 
 namespace mvr {
@@ -1238,6 +1241,141 @@ rerank_kernel(DevIndex ix, const float *__restrict__ q, const uint64_t *__restri
 }
 
 // ---------------------------------------------------------------------
+// Which shortlisted docs an exact FP32 search has to score: those whose BF16
+// MaxSim (approx) reaches the topk-th best of the query less twice a bound E on
+// |BF16 - exact MaxSim|.  topk docs have exact scores of at least (the topk-th
+// best approx - E), and a doc below the cut has an exact score under that.
+// Per query token, with X a bound on |x| and dX on |x - BF16 x| of every decoded
+// doc token x = c + W (dX: the centroids' and weights' own rounding errors, and
+// a relative 2^-8 for the rounded BF16 sum), the error of a dot product is at most
+//   |q - bf16(q)| X + |bf16(q)| dX + 2^-13 |q| X,
+// the last term for both sides' FP32 accumulation; 2^-15 max(1, 4 max|q| X)
+// covers an accumulator that starts at an offset of up to 2.04 max|q| X.  The max
+// over a doc's tokens and the clamp at 0 enlarge no error, the sum over query
+// tokens adds them up.  A bound that is not finite keeps every doc.  One CTA per
+// query, the approximate scores' order keys in shared memory.
+// ---------------------------------------------------------------------
+constexpr int kReachThreads = 512;
+__host__ __device__ constexpr size_t reach_smem(uint32_t probe_topk) {
+  return (size_t)probe_topk * sizeof(uint32_t) + 4096 * sizeof(uint32_t);
+}
+
+__global__ void __launch_bounds__(kReachThreads)
+maxsim_reach_kernel(const float *__restrict__ q, const uint64_t *__restrict__ q_off,
+                    const uint32_t *__restrict__ short_id, const float *__restrict__ approx,
+                    const uint32_t *__restrict__ n_short, uint32_t probe_topk, uint32_t topk,
+                    const float *__restrict__ cen_bounds, float w_norm, float w_err,
+                    uint32_t *__restrict__ out_id, uint32_t *__restrict__ n_out) {
+  extern __shared__ uint32_t rsm[];
+  uint32_t *ord = rsm, *hist = rsm + probe_topk;  // [probe_topk], [4096]
+  __shared__ float s_e[kMaxQueryTok], s_q[kMaxQueryTok];
+  __shared__ uint32_t s_wsum[kReachThreads / 32], s_bin, s_need, s_n;
+  __shared__ float s_thr;
+  const uint32_t b = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t n = min(n_short[b], probe_topk);
+  const uint64_t tok0 = q_off[b];
+  const uint32_t nq = (uint32_t)(q_off[b + 1] - tok0);
+  const size_t row = (size_t)b * probe_topk;
+  for (uint32_t i = tid; i < n; i += kReachThreads) ord[i] = f2ord(approx[row + i]);
+  if (tid == 0) s_n = 0;
+  const float X = (cen_bounds[0] + w_norm) * (1.0f + 0x1p-10f);
+  const float dX = cen_bounds[1] + w_err + X * 0x1.02p-8f;
+  for (uint32_t t = warp; t < nq; t += kReachThreads / 32) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(q + (tok0 + t) * kDim) + lane);
+    const float x[4] = {v.x, v.y, v.z, v.w};
+    float nn = 0.0f, nb = 0.0f, dd = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float r = __bfloat162float(__float2bfloat16_rn(x[i]));
+      nn = fmaf(x[i], x[i], nn);
+      nb = fmaf(r, r, nb);
+      dd = fmaf(x[i] - r, x[i] - r, dd);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      nn += __shfl_xor_sync(kFull, nn, o);
+      nb += __shfl_xor_sync(kFull, nb, o);
+      dd += __shfl_xor_sync(kFull, dd, o);
+    }
+    if (lane == 0) {
+      s_e[t] = sqrtf(dd) * X + sqrtf(nb) * dX + sqrtf(nn) * X * 0x1p-13f;
+      s_q[t] = sqrtf(nn);
+    }
+  }
+  __syncthreads();
+  if (n > topk) {
+    // the topk-th largest order key: radix passes of 12, 12 and 8 bits
+    uint32_t prefix = 0, need = topk;
+    int shift = 32;
+    while (shift > 0) {
+      const int up = shift, width = min(12, shift);
+      shift -= width;
+      for (uint32_t i = tid; i < 4096; i += kReachThreads) hist[i] = 0;
+      __syncthreads();
+      for (uint32_t i = tid; i < n; i += kReachThreads) {
+        const uint32_t k = ord[i];
+        if (up == 32 || (k >> up) == prefix) atomicAdd(&hist[(k >> shift) & ((1u << width) - 1u)], 1u);
+      }
+      __syncthreads();
+      uint32_t c[8], sum = 0;  // bins 4095 - 8 tid .. 4088 - 8 tid, high to low
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        c[u] = hist[4095 - 8 * tid - u];
+        sum += c[u];
+      }
+      uint32_t incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) s_wsum[warp] = incl;
+      __syncthreads();
+      uint32_t above = incl - sum;
+      for (int w = 0; w < warp; w++) above += s_wsum[w];
+      if (above < need && need <= above + sum) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          if (above < need && need <= above + c[u]) {
+            s_bin = 4095 - 8 * tid - u;
+            s_need = need - above;
+          }
+          above += c[u];
+        }
+      }
+      __syncthreads();
+      prefix = (prefix << width) | s_bin;
+      need = s_need;
+    }
+    if (tid == 0) {
+      float e = 0.0f, qm = 0.0f;
+      for (uint32_t t = 0; t < nq; t++) {
+        e += s_e[t];
+        qm = fmaxf(qm, s_q[t]);
+      }
+      e = (e + (float)nq * 0x1p-15f * fmaxf(1.0f, 4.0f * qm * X)) * (1.0f + 0x1p-10f);
+      s_thr = e < 1e30f ? __fsub_rd(ord2f(prefix), 2.0f * e) : -INFINITY;
+    }
+  } else if (tid == 0) {
+    s_thr = -INFINITY;
+  }
+  __syncthreads();
+  const float thr = s_thr;
+  for (uint32_t i0 = 0; i0 < n; i0 += kReachThreads) {
+    const uint32_t i = i0 + tid;
+    const bool keep = i < n && !(ord2f(ord[i]) < thr);
+    const unsigned m = __ballot_sync(kFull, keep);
+    uint32_t at = 0;
+    if (lane == 0 && m) at = atomicAdd(&s_n, (uint32_t)__popc(m));
+    at = __shfl_sync(kFull, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (keep) out_id[row + at] = short_id[row + i];
+  }
+  __syncthreads();
+  if (tid == 0) n_out[b] = s_n;
+}
+
+// ---------------------------------------------------------------------
 // K4: final top-k of the reranked shortlist (bitonic sort of 64-bit keys).
 // ---------------------------------------------------------------------
 __global__ void __launch_bounds__(512)
@@ -1402,6 +1540,9 @@ cudaError_t configure_kernels() {
   e = cudaFuncSetAttribute(topk_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)((kMaxShort + kMaxShort / 4) * sizeof(uint64_t)));
   if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(maxsim_reach_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)reach_smem(kMaxShort));
+  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(kMaxShort * sizeof(uint64_t)));
 }
@@ -1503,8 +1644,8 @@ cudaError_t launch_filter_hash(const DevIndex &ix, const uint32_t *probe_id,
 // tile per warp) while n_query * windows stays within two waves of CTAs: a
 // wide window would leave most SMs idle (one query, 200 docs: 232 us in 4
 // CTAs, 25 us in 50).
-static uint32_t rerank_docs(uint32_t n_query, uint32_t n_docs, int n_sm) {
-  uint32_t docs = kRkDocs;
+static uint32_t rerank_docs(uint32_t n_query, uint32_t n_docs, uint32_t most, int n_sm) {
+  uint32_t docs = most;
   while (docs > 4 &&
          (uint64_t)n_query * ((n_docs + docs / 2 - 1) / (docs / 2)) <= 4ull * (uint32_t)n_sm)
     docs /= 2;
@@ -1515,9 +1656,9 @@ cudaError_t launch_rerank(const DevIndex &ix, const float *q, const uint64_t *q_
                           uint32_t n_query, const uint32_t *short_id,
                           const uint32_t *n_short, uint32_t probe_topk,
                           int semantics, float *exact, int n_sm, cudaStream_t st,
-                          int *n_launch) {
+                          int *n_launch, uint32_t most_docs) {
   if (n_query == 0 || probe_topk == 0) return cudaSuccess;
-  const uint32_t docs = rerank_docs(n_query, probe_topk, n_sm);
+  const uint32_t docs = rerank_docs(n_query, probe_topk, std::min<uint32_t>(most_docs, kRkDocs), n_sm);
   dim3 grid((probe_topk + docs - 1) / docs, n_query);
   const size_t sm = rk_smem_bytes((int)ix.n_bit);
 #define MVR_RK(NB)                                                                              \
@@ -1531,6 +1672,19 @@ cudaError_t launch_rerank(const DevIndex &ix, const float *q, const uint64_t *q_
     default: return cudaErrorInvalidValue;
   }
 #undef MVR_RK
+  *n_launch += 1;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_maxsim_reach(const float *q, const uint64_t *q_off, uint32_t n_query,
+                                const uint32_t *short_id, const float *approx,
+                                const uint32_t *n_short, uint32_t probe_topk, uint32_t topk,
+                                const float *cen_bounds, float w_norm, float w_err,
+                                uint32_t *out_id, uint32_t *n_out, cudaStream_t st,
+                                int *n_launch) {
+  maxsim_reach_kernel<<<n_query, kReachThreads, reach_smem(probe_topk), st>>>(
+      q, q_off, short_id, approx, n_short, probe_topk, topk, cen_bounds, w_norm, w_err, out_id,
+      n_out);
   *n_launch += 1;
   return cudaGetLastError();
 }

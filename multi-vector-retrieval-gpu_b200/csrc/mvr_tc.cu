@@ -2417,6 +2417,8 @@ cudaError_t make_bf16(const float *in, size_t n, void *out, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
 cudaError_t configure_tc_kernels() {
   cudaError_t e;
   e = cudaFuncSetAttribute(rerank_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(1, 64));

@@ -6,6 +6,7 @@
 namespace mvr {
 
 cudaError_t configure_tc_kernels();
+float bf16_round(float x);  // to the nearest BF16, as the BF16 tables are rounded
 cudaError_t make_bf16(const float *in, size_t n, void *out, cudaStream_t st);
 cudaError_t launch_rerank_tc(const DevIndex &ix, const void *cen_bf16, const void *lut_bf16,
                              const float *q, const uint64_t *q_off, uint32_t n_query,

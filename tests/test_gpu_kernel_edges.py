@@ -188,3 +188,30 @@ def test_shortlist_cut_edges(ptk):
     np.testing.assert_array_equal(t["cand_id"], r["cand_id"])
     np.testing.assert_array_equal(t["short_id"], r["short_id"][o])
     np.testing.assert_array_equal(t["short_approx"], r["short_approx"][o])
+
+
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 8])
+@pytest.mark.parametrize("sem", [SEM_PP, SEM_BASIC], ids=["pp", "basic"])
+def test_exact_search_through_bf16_cut(n_bit, sem):
+    """Exact FP32 searches long enough to leave docs out by their BF16 scores return the
+    oracle's results: queries of several norms (large ones, and small ones whose
+    error is the accumulator's), ragged widths, and corpora of duplicates that all tie."""
+    rng = np.random.default_rng(n_bit)
+    ix = tiny_index(n_doc=700, n_centroid=48, n_bit=n_bit, seed=60 + n_bit)
+    dup = tiny_index(n_doc=300, n_centroid=16, n_bit=n_bit, seed=61, lengths=[7] * 300)
+    for k in ("vq_code", "residual"):  # every doc the same tokens
+        per = np.asarray(dup[k]).reshape(300, -1)
+        dup[k] = np.repeat(per[:1], 300, axis=0).reshape(np.asarray(dup[k]).shape)
+    dup["ivf_off"], dup["ivf_size"], dup["ivf_ids"] = pyoracle.ivf_build(
+        dup["vq_code"], dup["item_n_vec"], 16)
+    for x, ptk in ((ix, 400), (dup, 250)):
+        o = oracle_of(x)
+        q, off = make_queries(x, 140, (17, 64), seed=4)
+        scale = np.repeat(10.0 ** rng.integers(-6, 5, 140), np.diff(off.astype(np.int64)))
+        with gpu_index(x) as g:
+            for qq in (q, (q * scale[:, None]).astype(np.float32)):
+                for k in (1, 10, 60):
+                    r = o.search(qq, off, k, 8, ptk, sem)
+                    s, i = g.search(qq, k, 8, ptk, tok_off=off, semantics=sem)
+                    np.testing.assert_array_equal(i, r[1])
+                    np.testing.assert_array_equal(s, r[0])
