@@ -1652,24 +1652,28 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 //
 // The CTA takes DOCS docs of a query's shortlist; their tokens, doc after
 // doc, are the rows of its MMA tiles (128 rows per tile; rows past the last
-// token are zero).  Roles of the 320 threads:
+// token are zero), two CTAs per SM.  Roles of the 320 (N = 64: 448) threads:
 //  warp 0     producer: per tile, one 1-D bulk copy (cp.async.bulk, completion
 //             by mbarrier transaction count) of the residual bytes of every
-//             doc segment the tile covers, into stage i % kWsStages of a
+//             doc segment the tile covers, into the next stage of a
 //             shared-memory ring;
 //  warps 2-5  decoders, one thread per row: the row's vq code (loaded from
-//             HBM three tiles ahead), its E4M3 centroid row from L2 (one tile
-//             ahead), a tcgen05.st of that row (A_c), the residual bytes from
-//             the ring (read in a bank-conflict-free order) expanded by PRMT
-//             into E4M3 bucket weights (as rerank_tmem_kernel's FP8 decode),
-//             a tcgen05.st of those (A_r);
+//             HBM three tiles ahead); the E4M3 centroid rows copied from L2
+//             into the swizzled A_c tile of the next stage (cp.async one tile
+//             ahead, 8 lanes a row: a copy touches 4 cache lines, where a row
+//             per lane touched 32 and its loads and tcgen05.st took two thirds
+//             of the L1 data pipe); the residual bytes from the ring (read in
+//             a bank-conflict-free order) expanded by PRMT into E4M3 bucket
+//             weights (as rerank_tmem_kernel's FP8 decode), a tcgen05.st of
+//             those (A_r);
 //  warp 1     MMA: one thread issues per tile a bias MMA that writes OFF into
 //             every element of the tile's D stage (a constant A_e of 16.0 in
 //             TMEM times a B_e tile of OFF / 512, 32 products summed exactly),
 //             then 4 K-steps x 2 tcgen05.mma (kind::f8f6f4, M = 128,
-//             N = NMAX, K = 32): A_c and A_r from TMEM, the query tile B from
-//             shared memory; commits release the A stage and hand D over;
-//  warps 6-9  epilogue, one warp per 32 rows: tcgen05.ld of its rows, the D
+//             N = NMAX, K = 32): A_c from shared memory, A_r from TMEM, the
+//             query tile B from shared memory; commits release the A stages
+//             and hand D over;
+//  warps 6-   epilogue, one warp per 32 rows and 32 columns: tcgen05.ld, the D
 //             stage released at once, then for each doc its rows belong to
 //             one full-warp REDUX.MAX per query-token column (rows of other
 //             docs masked to 0), folded into the per-(doc, query token) maxima
@@ -1685,34 +1689,38 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 // error and every role stops; the producer then waits (1 s bound) for its
 // bulk copies still in flight and the MMA thread for its MMAs before TMEM
 // is freed.
+//
+// Bound: the ALU pipe (REDUX, selects and PRMT: 61 % busy, issue 63 %; the L1 data
+// pipe, 78 % with centroid rows loaded a row per lane, is at 25 %).  2,368 queries x
+// 1500 docs of 32 tokens at 2 bits: 9.05 -> 8.27 ms, 30 docs' tokens per ns; 600
+// queries of 33-64 tokens x 1500 docs at 4 bits, whose one CTA per SM became two with
+// twice the epilogue warps: 5.46 -> 3.60 ms.  Two epilogue warps per 32 rows also for
+// N = 32 (72 registers a thread): 8.9 ms; three CTAs per SM with one A_r stage: 10.8
+// ms; the maxima written by one lane's 32 atomics instead of 32 selects: 8.4 ms.
 // ---------------------------------------------------------------------
 constexpr int kWsDocs = 256;         // shortlisted docs per CTA (default; 32, 64, 128 or 256)
-constexpr int kWsStages = 4;         // shared-memory ring stages (residual bytes of one tile)
-constexpr int kWsDStages = 3;        // D stages in TMEM
-constexpr int kWsThreads = 320;
+// epilogue warps per 32 rows: the 64-column variant splits the columns in two
+__host__ __device__ constexpr int ws_groups(int nmax) { return nmax <= 32 ? 1 : 2; }
+__host__ __device__ constexpr int ws_threads(int nmax) { return 32 * (6 + 4 * ws_groups(nmax)); }
 
-__host__ __device__ constexpr int ws_astages(int nmax) { return nmax <= 32 ? 2 : 4; }
-__host__ __device__ constexpr uint32_t ws_cols(int nmax) { return nmax <= 32 ? 256u : 512u; }
+constexpr int kWsAStages = 2;        // A_r stages in TMEM
+// A_c stages: one more, so that the wait for tile i's A_r stage (the MMAs of tile
+// i - 2 done) also frees the stage of tile i + 1's copies
+constexpr int kWsCStages = kWsAStages + 1;
+// D stages in TMEM: 3, or 2 of 64 columns, so that two CTAs share an SM's 512 columns
+__host__ __device__ constexpr int ws_dstages(int nmax) { return nmax <= 32 ? 3 : 2; }
+constexpr uint32_t kWsCols = 256;    // TMEM columns of a CTA
+// ring stages of residual bytes: 4, or the 2 that two CTAs leave room for at 4 bits
+__host__ __device__ constexpr int ws_rstages(int nbit) { return nbit == 4 ? 2 : 4; }
 __host__ __device__ constexpr uint32_t ws_stage_bytes(int nbit) { return 128u * (128u * nbit / 8u); }
-// dynamic shared memory: 1 KB alignment slack + query tile + bias tile + ring;
-// the wide (NMAX = 64) variant asks for more than half an SM's shared memory
-// so that one CTA holds the SM's 512 TMEM columns alone
+constexpr uint32_t kWsCBytes = 128u * 128u;  // one A_c stage
+// dynamic shared memory: 1 KB alignment slack + query tile + bias tile + A_c
+// stages + ring
 __host__ __device__ constexpr size_t ws_smem_bytes(int nbit, int nmax) {
-  return nmax <= 32 ? 1024 + 2 * (size_t)nmax * 128 + kWsStages * (size_t)ws_stage_bytes(nbit)
-                    : 120 * 1024;
+  return 1024 + 2 * (size_t)nmax * 128 + kWsCStages * (size_t)kWsCBytes +
+         ws_rstages(nbit) * (size_t)ws_stage_bytes(nbit);
 }
 
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-      "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
-      "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]),
-      "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
-      "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
 // the same word into 8 consecutive TMEM columns of the warp's 32 lanes
 __device__ __forceinline__ void tmem_fill8(uint32_t taddr, uint32_t x) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(
@@ -1722,6 +1730,15 @@ __device__ __forceinline__ void tmem_fill8(uint32_t taddr, uint32_t x) {
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+}
+// accumulating MMA with A in shared memory
+__device__ __forceinline__ void mma_e4m3_ss(uint32_t tmem_d, uint64_t a, uint64_t b,
+                                            uint32_t idesc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(1u)
+      : "memory");
 }
 __device__ __forceinline__ void mma_e4m3_acc(uint32_t tmem_d, uint32_t tmem_a, uint64_t b,
                                              uint32_t idesc, uint32_t accum) {
@@ -1733,7 +1750,7 @@ __device__ __forceinline__ void mma_e4m3_acc(uint32_t tmem_d, uint32_t tmem_a, u
 }
 
 template <int NBIT, int NMAX, bool FEAT = false, int DOCS = kWsDocs>
-__global__ void __launch_bounds__(kWsThreads, NMAX <= 32 ? 2 : 1)
+__global__ void __launch_bounds__(ws_threads(NMAX), 2)
 rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
                  const float *__restrict__ q, const uint64_t *__restrict__ q_off,
                  const uint32_t *__restrict__ short_id, const uint32_t *__restrict__ n_short,
@@ -1742,20 +1759,22 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
   static_assert(NBIT == 2 || NBIT == 4, "FP8 decode of 2- and 4-bit codes");
   static_assert(NMAX == 32 || NMAX == 64, "query tiles of 32 or 64 rows");
   static_assert(!FEAT || NMAX == 32, "pruner features: queries of up to 32 tokens");
-  static_assert(DOCS == 32 || DOCS == 64 || DOCS == 128 || (DOCS == 256 && NMAX == 32),
-                "docs per CTA (256: the 32-column variant only, whose maxima fit static smem)");
-  constexpr int S = kWsStages, SA = ws_astages(NMAX), SD = kWsDStages;
+  static_assert(DOCS == 32 || DOCS == 64 || ((DOCS == 128 || DOCS == 256) && NMAX == 32),
+                "docs per CTA (64 at most with 64 columns: the maxima of two CTAs fit an SM)");
+  constexpr int S = ws_rstages(NBIT), SA = kWsAStages, SD = ws_dstages(NMAX), SC = kWsCStages;
+  constexpr int G = ws_groups(NMAX), CW = NMAX / G;  // column groups and their width
   constexpr uint32_t BPV = 128u * NBIT / 8u;       // residual bytes per token
   constexpr uint32_t STAGE = ws_stage_bytes(NBIT);
-  constexpr uint32_t COLS = ws_cols(NMAX);
-  constexpr uint32_t DCOL0 = 64u * SA;              // D stages after the A stages
+  constexpr uint32_t COLS = kWsCols;
+  constexpr uint32_t DCOL0 = 32u * SA;              // D stages after the A_r stages
   constexpr uint32_t ECOL = DCOL0 + NMAX * SD;      // bias operand A_e (8 columns)
   static_assert(ECOL + 8 <= COLS, "TMEM columns");
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *Bq = smem;                     // [NMAX rows][128 B] E4M3, SW128, K-major
   uint8_t *Be = smem + NMAX * 128;        // bias B operand, same layout
-  uint8_t *ring = smem + 2 * NMAX * 128;  // [S][128 rows][BPV] residual bytes
+  uint8_t *Ac = smem + 2 * NMAX * 128;    // [SC][128 rows][128 B] centroid rows, SW128, K-major
+  uint8_t *ring = Ac + SC * kWsCBytes;    // [S][128 rows][BPV] residual bytes
   __shared__ uint32_t best[DOCS * NMAX];  // [doc][query token]: bits of OFF + max
   __shared__ uint32_t s_qss, tmem_base_s;
   __shared__ float s_qinv[NMAX];
@@ -1784,7 +1803,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
   if (tid == 0) {
     for (int s = 0; s < S; s++) { mbar_init(&full[s], 1); mbar_init(&sfree[s], 4); }
     for (int s = 0; s < SA; s++) { mbar_init(&afull[s], 4); mbar_init(&afree[s], 1); }
-    for (int s = 0; s < SD; s++) { mbar_init(&dfull[s], 1); mbar_init(&dempty[s], 4); }
+    for (int s = 0; s < SD; s++) { mbar_init(&dfull[s], 1); mbar_init(&dempty[s], 4 * G); }
     mbar_init(&mdone, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     s_abort = 0;
@@ -1795,7 +1814,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
     d_len[tid] = ix.item_n_vec[it];
     d_off[tid] = ix.item_off[it];
   }
-  for (int i = tid; i < DOCS * NMAX; i += kWsThreads) best[i] = 0u;
+  for (int i = tid; i < DOCS * NMAX; i += ws_threads(NMAX)) best[i] = 0u;
   __syncthreads();
   if (warp == 0) {  // token offsets of the docs within the CTA (warp scan)
     uint32_t carry = 0;
@@ -1813,7 +1832,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
   }
   // query tokens -> B (E4M3, per-token power-of-two scales, FP8 K order,
   // swizzled, rows >= nq zero): 8 lanes per row, 16 positions each
-  for (int i = tid; i < NMAX * 8; i += kWsThreads) {
+  for (int i = tid; i < NMAX * 8; i += ws_threads(NMAX)) {
     const int row = i >> 3, ch = i & 7;
     float x[16];
     float amax = 0.0f, ss = 0.0f;
@@ -1860,7 +1879,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
   if (e_off > 21) {  // norms beyond the bias's range: report, do not guess
     if (tid == 0) atomicOr(err, 16u);
   }
-  for (int i = tid; i < NMAX * 8; i += kWsThreads) {
+  for (int i = tid; i < NMAX * 8; i += ws_threads(NMAX)) {
     const int row = i >> 3, ch = i & 7;
     const uint32_t e = ch < 2 ? (uint32_t)__nv_cvt_float_to_fp8(exp2f((float)(e_off - 5 - a_exp)),
                                                                 __NV_SATFINITE, __NV_E4M3) *
@@ -1922,7 +1941,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
     // ---------------- MMA issue ----------------
     if (lane == 0) {
       const uint32_t idesc = idesc_e4m3(128, NMAX);
-      const uint32_t b_base = smem_u32(Bq);
+      const uint32_t b_base = smem_u32(Bq), c_base = smem_u32(Ac);
       const uint64_t be_desc = sw128_desc(smem_u32(Be));
       uint32_t i = 0;
       for (; i < n_tiles; i++) {
@@ -1931,12 +1950,13 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
         if (i >= (uint32_t)SD && !mbar_wait(&dempty[sd], ((i / SD) + 1) & 1, wait_ns)) break;
         tc_fence_after();
         const uint32_t dcol = tmem + DCOL0 + NMAX * sd;
+        const uint32_t ca = c_base + (i % SC) * kWsCBytes;
         mma_e4m3_acc(dcol, tmem + ECOL, be_desc, idesc, 0u);  // D = OFF
 #pragma unroll
         for (int kk = 0; kk < 4; kk++) {  // K = 32 per MMA: centroid part, residual part
           const uint64_t bd = sw128_desc(b_base + kk * 32);
-          mma_e4m3_acc(dcol, tmem + 64u * sa + 8u * kk, bd, idesc, 1u);
-          if constexpr (!FEAT) mma_e4m3_acc(dcol, tmem + 64u * sa + 32u + 8u * kk, bd, idesc, 1u);
+          mma_e4m3_ss(dcol, sw128_desc(ca + kk * 32), bd, idesc);
+          if constexpr (!FEAT) mma_e4m3_acc(dcol, tmem + 32u * sa + 8u * kk, bd, idesc, 1u);
         }
         mma_commit(&dfull[sd]);
         mma_commit(&afree[sa]);
@@ -1963,22 +1983,28 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
       while (d_pref[dcur + 1] <= g) dcur++;
       return __ldg(ix.vq_code + d_off[dcur] + (g - d_pref[dcur]));
     };
-    uint32_t cen[32];
-    auto load_cen = [&](uint32_t code) {
-      const uint4 *cp = reinterpret_cast<const uint4 *>(cen8 + (size_t)code * kDim);
+    // the centroid rows of this warp's 32 rows of a tile -> A_c stage st, 8
+    // lanes a row (row 4u + lane / 8, 16-byte chunk lane % 8)
+    // (its offset in the swizzled tile: 1 KB per 8 rows, two patterns for u even and odd)
+    const uint32_t l3 = (uint32_t)lane >> 3, ch = lane & 7u;
+    const uint32_t c_even = smem_u32(Ac) + 4096u * qd + l3 * 128u + ((ch ^ l3) << 4);
+    const uint32_t c_odd = smem_u32(Ac) + 4096u * qd + (4u + l3) * 128u + ((ch ^ (4u + l3)) << 4);
+    auto copy_cen = [&](uint32_t code, uint32_t st) {
 #pragma unroll
       for (int u = 0; u < 8; u++) {
-        const uint4 t = __ldg(cp + u);
-        cen[4 * u] = t.x;
-        cen[4 * u + 1] = t.y;
-        cen[4 * u + 2] = t.z;
-        cen[4 * u + 3] = t.w;
+        const uint32_t cd = __shfl_sync(kFull, code, 4u * u + l3);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                         (u & 1 ? c_odd : c_even) + st * kWsCBytes + (u >> 1) * 1024u),
+                     "l"(cen8 + (size_t)cd * kDim + 16u * ch)
+                     : "memory");
       }
     };
+    auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
     // codes three tiles ahead, centroid rows one tile ahead
     const uint32_t c0 = code_of(0);
     uint32_t c1 = code_of(1), c2 = code_of(2);
-    load_cen(c0);
+    copy_cen(c0, 0);
+    commit();
     // chunk rotation of the residual reads: rows are BPV bytes apart, so a
     // wavefront's 8 lanes (rows) start in 4 (2-bit) or 2 (4-bit) bank groups
     const uint32_t rot = NBIT == 2 ? ((uint32_t)lane >> 2) & 1u : ((uint32_t)lane >> 1) & 3u;
@@ -1991,10 +2017,9 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
         break;
       }
       tc_fence_after();
-      const uint32_t acol = tmem + lane_off + 64u * sa;
-      tmem_st32(acol, cen);  // A_c: the centroid row as loaded
-      tmem_wait_st();
-      if (i + 1 < n_tiles) load_cen(c1);
+      const uint32_t acol = tmem + lane_off + 32u * sa;
+      if (i + 1 < n_tiles) copy_cen(c1, (i + 1) % SC);
+      commit();
       c1 = c2;
       c2 = code_of(i + 3);
       if constexpr (!FEAT) {
@@ -2032,19 +2057,24 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
         uint32_t out[16];
         if constexpr (NBIT == 4) {
           fp8_decode16_b4(res, tw, out);
-          tmem_st16(acol + 32u, out);
+          tmem_st16(acol, out);
           fp8_decode16_b4(res + 8, tw, out);
-          tmem_st16(acol + 48u, out);
+          tmem_st16(acol + 16u, out);
         } else {
           fp8_decode16(res, tw.w[0], out);
-          tmem_st16(acol + 32u, out);
+          tmem_st16(acol, out);
           fp8_decode16(res + 4, tw.w[0], out);
-          tmem_st16(acol + 48u, out);
+          tmem_st16(acol + 16u, out);
         }
         tmem_wait_st();
       } else {
         (void)rot;
+        (void)acol;
       }
+      // tile i's rows have landed (tile i + 1's may be on their way) and are
+      // visible to the MMAs
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      fence_async_smem();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -2053,13 +2083,14 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
       }
       if (__any_sync(kFull, s_abort != 0)) ok = false;
     }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     if (!__all_sync(kFull, ok) && lane == 0) {
       atomicOr(err, 4u);
       s_abort = 1;
     }
   } else {
-    // ---------------- epilogue: one warp per 32 rows ----------------
-    const uint32_t r = 32u * qd + lane;
+    // ---------------- epilogue: G warps per 32 rows, CW columns each ----------------
+    const uint32_t r = 32u * qd + lane, j0 = CW * ((uint32_t)(warp - 6) >> 2);
     uint32_t dcur = 0;
     bool ok = true;
     for (uint32_t i = 0; i < n_tiles; i++) {
@@ -2069,11 +2100,9 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
         break;
       }
       tc_fence_after();
-      const uint32_t dcol = tmem + lane_off + DCOL0 + NMAX * sd;
-      uint32_t v0[32];
-      tmem_ld32(dcol, v0);
-      uint32_t v1[NMAX > 32 ? 32 : 1];
-      if constexpr (NMAX > 32) tmem_ld32(dcol + 32u, v1);
+      uint32_t v0[CW];
+      if constexpr (CW == 32) tmem_ld32(tmem + lane_off + DCOL0 + NMAX * sd + j0, v0);
+      else tmem_ld16(tmem + lane_off + DCOL0 + NMAX * sd + j0, v0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&dempty[sd]);
@@ -2090,38 +2119,21 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
         const bool in = doc == gd;
         const unsigned mem = __ballot_sync(kFull, in);
         rem &= ~mem;
-        uint32_t m0 = 0u;
+        uint32_t m0 = 0u;  // lane j: column j0 + j
         if (mem == kFull) {
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
+          for (int j = 0; j < CW; j++) {
             const uint32_t m = __reduce_max_sync(kFull, v0[j]);
             m0 = lane == j ? m : m0;
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
+          for (int j = 0; j < CW; j++) {
             const uint32_t m = __reduce_max_sync(kFull, in ? v0[j] : 0u);
             m0 = lane == j ? m : m0;
           }
         }
-        if ((uint32_t)lane < nq) atomicMax(&best[gd * NMAX + lane], m0);
-        if constexpr (NMAX > 32) {
-          uint32_t m1 = 0u;
-          if (mem == kFull) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-              const uint32_t m = __reduce_max_sync(kFull, v1[j]);
-              m1 = lane == j ? m : m1;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-              const uint32_t m = __reduce_max_sync(kFull, in ? v1[j] : 0u);
-              m1 = lane == j ? m : m1;
-            }
-          }
-          if ((uint32_t)lane + 32u < nq) atomicMax(&best[gd * NMAX + 32 + lane], m1);
-        }
+        if (lane < CW && j0 + lane < nq) atomicMax(&best[gd * NMAX + j0 + lane], m0);
       }
       if (__any_sync(kFull, s_abort != 0)) {
         ok = false;
@@ -2139,7 +2151,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
     // pruner features: approx is [queries][probe_topk][33]: per query token
     // the doc's best centroid score (0 past the query's last token), then
     // log(doc length)
-    for (int i = tid; i < (int)nd * 33 && !s_abort; i += kWsThreads) {
+    for (int i = tid; i < (int)nd * 33 && !s_abort; i += ws_threads(NMAX)) {
       const int d = i / 33, t = i % 33;
       float f = 0.0f;
       if (t == 32) f = logf((float)d_len[d]);
@@ -2447,9 +2459,9 @@ cudaError_t configure_tc_kernels() {
   if (e != cudaSuccess) return e;
   MVR_WS_ATTR(2, 32, false, 32) MVR_WS_ATTR(2, 32, false, 64) MVR_WS_ATTR(2, 32, false, 128)
   MVR_WS_ATTR(2, 32, false, 256) MVR_WS_ATTR(4, 32, false, 256)
-  MVR_WS_ATTR(2, 64, false, 32) MVR_WS_ATTR(2, 64, false, 64) MVR_WS_ATTR(2, 64, false, 128)
+  MVR_WS_ATTR(2, 64, false, 32) MVR_WS_ATTR(2, 64, false, 64)
   MVR_WS_ATTR(4, 32, false, 32) MVR_WS_ATTR(4, 32, false, 64) MVR_WS_ATTR(4, 32, false, 128)
-  MVR_WS_ATTR(4, 64, false, 32) MVR_WS_ATTR(4, 64, false, 64) MVR_WS_ATTR(4, 64, false, 128)
+  MVR_WS_ATTR(4, 64, false, 32) MVR_WS_ATTR(4, 64, false, 64)
   // the pruner's feature launch: the default docs per CTA
   MVR_WS_ATTR(2, 32, true, kWsDocs) MVR_WS_ATTR(4, 32, true, kWsDocs)
 #undef MVR_WS_ATTR
@@ -2599,7 +2611,7 @@ static void ws_launch(const DevIndex &ix, const uint8_t *c, const TmWeights &tw,
                       const uint32_t *n_short, uint32_t probe_topk, int semantics, float x_bound,
                       float *approx, unsigned *err, cudaStream_t st, uint64_t wait_ns) {
   const dim3 grid((probe_topk + DOCS - 1) / DOCS, n_query);
-  rerank_ws_kernel<NB, NM, false, DOCS><<<grid, kWsThreads, ws_smem_bytes(NB, NM), st>>>(
+  rerank_ws_kernel<NB, NM, false, DOCS><<<grid, ws_threads(NM), ws_smem_bytes(NB, NM), st>>>(
       ix, c, tw, q, q_off, short_id, n_short, probe_topk, semantics, x_bound, approx, err,
       wait_ns);
 }
@@ -2613,13 +2625,14 @@ static void ws_launch_docs(uint32_t docs, const DevIndex &ix, const uint8_t *c,
   if (docs == 32)
     ws_launch<NB, NM, 32>(ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk, semantics,
                           x_bound, approx, err, st, wait_ns);
-  else if (docs == 256 && NM == 32)  // the 64-column variant's maxima would not fit: 128 there
-    ws_launch<NB, NM, NM == 32 ? 256 : 128>(ix, c, tw, q, q_off, n_query, short_id, n_short,
-                                            probe_topk, semantics, x_bound, approx, err, st,
-                                            wait_ns);
-  else if (docs >= 128)
-    ws_launch<NB, NM, 128>(ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk, semantics,
-                           x_bound, approx, err, st, wait_ns);
+  else if (docs == 256 && NM == 32)  // (the 64-column variant takes 64 docs at most)
+    ws_launch<NB, NM, NM == 32 ? 256 : 64>(ix, c, tw, q, q_off, n_query, short_id, n_short,
+                                           probe_topk, semantics, x_bound, approx, err, st,
+                                           wait_ns);
+  else if (docs == 128 && NM == 32)
+    ws_launch<NB, NM, NM == 32 ? 128 : 64>(ix, c, tw, q, q_off, n_query, short_id, n_short,
+                                           probe_topk, semantics, x_bound, approx, err, st,
+                                           wait_ns);
   else
     ws_launch<NB, NM, 64>(ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk, semantics,
                           x_bound, approx, err, st, wait_ns);
@@ -2629,7 +2642,7 @@ static void ws_launch_docs(uint32_t docs, const DevIndex &ix, const uint8_t *c,
 // least time, waves of the grid x (docs + 12), 12 docs being what a CTA costs
 // besides (its TMEM, query tile, pipeline fill; a CTA alone on an SM takes 138
 // us for 256 docs of 70 tokens).  Bulk searches keep the widest (2,368 queries x
-// 1500 docs: 9.1 ms at 256, 9.3 at 128); one query x 1500 goes from 6 CTAs to
+// 1500 docs: 8.3 ms at 256); one query x 1500 goes from 6 CTAs to
 // 47, 138 -> 26 us, 37 queries x 1000 from 148 to 296, 147 -> 111 us.
 static uint32_t ws_auto_docs(uint32_t n_query, uint32_t probe_topk, uint32_t slots,
                              uint32_t widest) {
@@ -2668,7 +2681,7 @@ cudaError_t launch_rerank_ws(const DevIndex &ix, const void *cen8, const TmWeigh
   }
   if (nq_max > 32) {
     const uint32_t docs =
-        set_docs ? set_docs : ws_auto_docs(n_query, probe_topk, (uint32_t)n_sm, 128u);
+        set_docs ? set_docs : ws_auto_docs(n_query, probe_topk, 2u * (uint32_t)n_sm, 64u);
     if (ix.n_bit == 4)
       ws_launch_docs<4, 64>(docs, ix, c, tw, q, q_off, n_query, short_id, n_short, probe_topk,
                             semantics, x_bound, approx, err, st, wait_ns);
@@ -2690,10 +2703,10 @@ cudaError_t launch_prune_features(const DevIndex &ix, const void *cen8, const fl
   const uint8_t *c = reinterpret_cast<const uint8_t *>(cen8);
   const TmWeights none{};
   if (ix.n_bit == 4)
-    rerank_ws_kernel<4, 32, true><<<grid, kWsThreads, ws_smem_bytes(4, 32), st>>>(
+    rerank_ws_kernel<4, 32, true><<<grid, ws_threads(32), ws_smem_bytes(4, 32), st>>>(
         ix, c, none, q, q_off, short_id, n_short, probe_topk, 0, x_bound, feat, err, wait_ns);
   else
-    rerank_ws_kernel<2, 32, true><<<grid, kWsThreads, ws_smem_bytes(2, 32), st>>>(
+    rerank_ws_kernel<2, 32, true><<<grid, ws_threads(32), ws_smem_bytes(2, 32), st>>>(
         ix, c, none, q, q_off, short_id, n_short, probe_topk, 0, x_bound, feat, err, wait_ns);
   *n_launch += 1;
   return cudaGetLastError();

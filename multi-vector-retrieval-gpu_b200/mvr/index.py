@@ -141,7 +141,7 @@ class Index:
 
     def set_rerank_tile(self, docs_per_cta=0):
         """Shortlisted docs per CTA of the FP8 MaxSim kernel: 32, 64, 128 or
-        256 (queries of more than 32 tokens use at most 128), or 0, the
+        256 (queries of more than 32 tokens use at most 64), or 0, the
         default: chosen per call from the grid it gives."""
         check(lib().mvr_index_set_rerank_tile(self._h, int(docs_per_cta)))
 
