@@ -123,7 +123,7 @@ struct Workspace {
   float *out_s = nullptr;
   uint32_t *out_id = nullptr;
   uint32_t r_cap = 0;             // FP32 re-score of the top-R (BF16 path)
-  uint32_t *r_id = nullptr, *n_r = nullptr;
+  uint32_t *r_id = nullptr, *n_r = nullptr, *r2_id = nullptr, *n_r2 = nullptr;
   float *r_score = nullptr, *r_exact = nullptr;
   // per call
   size_t off_cap = 0, stat_cap = 0;
@@ -263,11 +263,12 @@ struct mvr_index {
                     (void *)ws.probe.cnt, (void *)ws.probe.eps2, (void *)ws.probe.flags,
                     (void *)ws.short_id, (void *)ws.n_short,
                     (void *)ws.short_approx, (void *)ws.exact, (void *)ws.out_s, (void *)ws.out_id,
-                    (void *)ws.r_id, (void *)ws.n_r, (void *)ws.r_score, (void *)ws.r_exact})
+                    (void *)ws.r_id, (void *)ws.n_r, (void *)ws.r2_id, (void *)ws.n_r2,
+                    (void *)ws.r_score, (void *)ws.r_exact})
       dfree(p);
     ws.probe = ProbeBufs{};
     ws.ent_cap = ws.gid_cap = ws.cnt_cap = ws.flag_cap = 0;
-    ws.r_id = ws.n_r = nullptr;
+    ws.r_id = ws.n_r = ws.r2_id = ws.n_r2 = nullptr;
     ws.r_score = ws.r_exact = nullptr;
     ws.r_cap = 0;
     ws.q = ws.q2 = nullptr; ws.probe_id = nullptr; ws.probe_s = nullptr;
@@ -386,6 +387,8 @@ int ensure_batch(mvr_index *h, uint32_t slots, uint32_t tok_cap, uint32_t nprobe
   MVR_TRY(dalloc(&w.r_score, (size_t)s * r_cap));
   MVR_TRY(dalloc(&w.r_exact, (size_t)s * r_cap));
   MVR_TRY(dalloc(&w.n_r, (size_t)s));
+  MVR_TRY(dalloc(&w.r2_id, (size_t)s * r_cap));
+  MVR_TRY(dalloc(&w.n_r2, (size_t)s));
   w.ent_cap = n_ent;
   w.gid_cap = n_gid;
   w.cnt_cap = n_cnt;
@@ -588,6 +591,13 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                      (uint64_t)std::min(h->batch_cap ? h->batch_cap : default_batch(h), n_query) *
                              probe_topk >= 32768;
   if (reach) R = probe_topk;
+  // the BF16 path's best R: the same bound leaves out those of them that miss the
+  // top topk (FP8's own error is an order larger and would leave out none).  400 docs
+  // of each of 256 queries for the best 100: 3.26 -> 1.89 ms of FP32 work for 16 us.
+  // From 16,384 docs, whose FP32 work is 500 us.
+  const bool cut_r = bf16 && !fp8 && R > topk &&
+                     (uint64_t)std::min(h->batch_cap ? h->batch_cap : default_batch(h), n_query) *
+                             R >= 16384;
   const uint32_t keep = prune ? std::min(h->prune_keep, probe_topk) : 0u;
   DeviceGuard g(h->device);
 
@@ -800,10 +810,17 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         CUDA_TRY(rec(ev(bt, 4)));
         CUDA_TRY(launch_topk(sid, w.exact, nsh, nb, probe_topk, R, w.r_score, w.r_id, w.n_r, rs,
                              &launches));
-        CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, w.r_id, w.n_r, R, sem, w.r_exact, h->n_sm, rs,
+        const uint32_t *rid = w.r_id, *nr = w.n_r;
+        if (cut_r) {
+          CUDA_TRY(launch_maxsim_reach(qp, qo, nb, w.r_id, w.r_score, w.n_r, R, topk,
+                                       h->cen_bounds, h->w_norm, h->w_err, w.r2_id, w.n_r2, rs,
+                                       &launches));
+          rid = w.r2_id;
+          nr = w.n_r2;
+        }
+        CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, rid, nr, R, sem, w.r_exact, h->n_sm, rs,
                                &launches));
-        CUDA_TRY(launch_topk(w.r_id, w.r_exact, w.n_r, nb, R, topk, os, oi, nullptr, rs,
-                             &launches));
+        CUDA_TRY(launch_topk(rid, w.r_exact, nr, nb, R, topk, os, oi, nullptr, rs, &launches));
       } else {
         // exact FP32 MaxSim over the shortlist -- with MVR_PRUNE over the docs
         // the pruner keeps (its fallback: the whole shortlist)

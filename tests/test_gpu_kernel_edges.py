@@ -7,7 +7,7 @@ import torch
 
 import pyoracle
 from helpers import make_queries, oracle_of, tiny_index
-from mvr import SEM_BASIC, SEM_PP, Index, build, exhaustive
+from mvr import PREC_BF16, SEM_BASIC, SEM_PP, Index, build, exhaustive
 
 pytestmark = pytest.mark.gpu
 
@@ -215,3 +215,25 @@ def test_exact_search_through_bf16_cut(n_bit, sem):
                     s, i = g.search(qq, k, 8, ptk, tok_off=off, semantics=sem)
                     np.testing.assert_array_equal(i, r[1])
                     np.testing.assert_array_equal(s, r[0])
+
+
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 8])
+def test_bf16_rescore_cut(n_bit):
+    """BF16 searches: a batch whose re-scored lists are long enough to be cut by the
+    bound on the BF16 error returns what batches too small for the cut return."""
+    ix = tiny_index(n_doc=900, n_centroid=48, n_bit=n_bit, seed=80 + n_bit)
+    for width in ((1, 32), (20, 64)):
+        q, off = make_queries(ix, 140, width, seed=5)
+        scale = np.repeat(10.0 ** np.random.default_rng(n_bit).integers(-6, 5, 140),
+                          np.diff(off.astype(np.int64)))
+        with gpu_index(ix) as g:
+            for qq in (q, (q * scale[:, None]).astype(np.float32)):
+                for k, r, ptk in ((1, 300, 400), (10, 400, 400), (100, 130, 300)):
+                    g.set_rescore(r)
+                    for sem in (SEM_PP, SEM_BASIC):
+                        g.set_batch(20)  # 20 x 400 docs: no cut
+                        s0, i0 = g.search(qq, k, 8, ptk, tok_off=off, semantics=sem | PREC_BF16)
+                        g.set_batch(140)  # 140 x 130 docs or more: cut
+                        s1, i1 = g.search(qq, k, 8, ptk, tok_off=off, semantics=sem | PREC_BF16)
+                        np.testing.assert_array_equal(i1, i0)
+                        np.testing.assert_array_equal(s1, s0)
