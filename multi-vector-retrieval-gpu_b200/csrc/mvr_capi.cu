@@ -167,7 +167,7 @@ struct mvr_index {
   void *lut_bf16 = nullptr;      // [256][8/b] BF16 decode table
   void *cen_sw = nullptr;        // [C_pad/128][32 KB] swizzled BF16 centroid tiles
   float *cen_bounds = nullptr;   // max |c|, max |c - bf16(c)| over the centroids
-  void *cen_perm = nullptr;      // [C][64] bf16x2 centroid rows, TMEM-rerank K order (b <= 2)
+  void *cen_perm = nullptr;      // [C + 1][64] bf16x2 centroid rows, BF16 K order (b <= 2)
   TmWeights tw_bf16{};           // weight tables of the BF16 tensor-memory MaxSim (b <= 2)
   float x_bound = 0.f;           // bound on the norm of every decoded doc token
   float w_norm = 0.f, w_err = 0.f;  // ... of a token's weights, of their BF16 rounding errors
@@ -579,11 +579,11 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
   }
   // Exact FP32 search of 1- and 2-bit codes: where a shortlist is long, the BF16
   // pass first leaves out the docs that provably miss the top topk, and the FP32
-  // kernel scores the rest (127 of 1500 on average for the best 10).  The line: at 14
-  // and 4.8 docs' tokens per ns the pass pays for itself once it spares a third
-  // of the FP32 work, which takes a shortlist of 4 topk (361 of 1500 stay for the
-  // best 100); its launches take 60 us, the FP32 work of 7,000 docs, and its CTAs
-  // of 64 docs want a grid that fills the GPU: 32,768 docs.  Queries of up to 16
+  // kernel scores the rest (50 of 1500 on average for the best 10).  The line: at 22
+  // and 4.8 docs' tokens per ns the pass pays for itself once it spares a fourth
+  // of the FP32 work, which takes a shortlist of 4 topk; its launches take 60 us,
+  // the FP32 work of 7,000 docs, and its CTAs of 32 to 128 docs want a grid that
+  // fills the GPU: 32,768 docs.  Queries of up to 16
   // tokens take the FP32 kernel's half-width body, at twice its rate.  The wider
   // codes' BF16 kernel is no faster than the FP32 one (4.9 tokens per ns at 8 bits).
   const bool reach = !bf16 && !prune && !all_exact && h->cen_perm && nq_max > 16 &&
@@ -593,8 +593,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
   if (reach) R = probe_topk;
   // the BF16 path's best R: the same bound leaves out those of them that miss the
   // top topk (FP8's own error is an order larger and would leave out none).  400 docs
-  // of each of 256 queries for the best 100: 3.26 -> 1.89 ms of FP32 work for 16 us.
-  // From 16,384 docs, whose FP32 work is 500 us.
+  // of each of 500 queries for the best 100: 3.26 -> 1.42 ms of FP32 work for 16 us.
+  // From 16,384 docs, whose FP32 work is 300 us.
   const bool cut_r = bf16 && !fp8 && R > topk &&
                      (uint64_t)std::min(h->batch_cap ? h->batch_cap : default_batch(h), n_query) *
                              R >= 16384;
@@ -801,8 +801,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                                     h->n_sm, rs, &launches, h->wait_ns, h->ws_docs));
         else if (h->cen_perm)
           CUDA_TRY(launch_rerank_tmem(h->dix, h->cen_perm, h->tw_bf16, qp, qo, nb, sid, nsh,
-                                      probe_topk, sem, nq_max, h->x_bound, w.exact,
-                                      h->d_err, rs, &launches, false));
+                                      probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact,
+                                      h->d_err, h->n_sm, rs, &launches, h->wait_ns));
         else
           CUDA_TRY(launch_rerank_tc(h->dix, h->cen_bf16, h->lut_bf16, qp, qo, nb, w.short_id,
                                     w.n_short, probe_topk, sem, nq_max, w.exact, h->d_err, rs,
@@ -813,7 +813,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         const uint32_t *rid = w.r_id, *nr = w.n_r;
         if (cut_r) {
           CUDA_TRY(launch_maxsim_reach(qp, qo, nb, w.r_id, w.r_score, w.n_r, R, topk,
-                                       h->cen_bounds, h->w_norm, h->w_err, w.r2_id, w.n_r2, rs,
+                                       h->cen_bounds, h->w_norm, h->w_err,
+                                       h->cen_perm ? kBf16SplitTok : 0u, w.r2_id, w.n_r2, rs,
                                        &launches));
           rid = w.r2_id;
           nr = w.n_r2;
@@ -841,10 +842,10 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         }
         if (reach) {
           CUDA_TRY(launch_rerank_tmem(h->dix, h->cen_perm, h->tw_bf16, qp, qo, nb, sid, nsh,
-                                      probe_topk, sem, nq_max, h->x_bound, w.exact, h->d_err, rs,
-                                      &launches, false));
+                                      probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact,
+                                      h->d_err, h->n_sm, rs, &launches, h->wait_ns));
           CUDA_TRY(launch_maxsim_reach(qp, qo, nb, sid, w.exact, nsh, probe_topk, topk,
-                                       h->cen_bounds, h->w_norm, h->w_err, w.r_id, w.n_r, rs,
+                                       h->cen_bounds, h->w_norm, h->w_err, kBf16SplitTok, w.r_id, w.n_r, rs,
                                        &launches));
           CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, w.r_id, w.n_r, probe_topk, sem, w.r_exact,
                                  h->n_sm, rs, &launches, 32));
@@ -1050,7 +1051,7 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
   }
   if (tmem_rerank_supported(d.n_bit)) {
     uint32_t *cp;
-    MVR_TRY(dalloc(&cp, (size_t)d.n_centroid * 64, &h->bufs));
+    MVR_TRY(dalloc(&cp, ((size_t)d.n_centroid + 1) * 64, &h->bufs));
     CUDA_TRY(make_centroid_perm(d.centroid, d.n_centroid, d.n_bit, cp, h->stream));
     h->cen_perm = cp;
     h->tw_bf16 = make_tm_weights(d.n_bit, weight, false);

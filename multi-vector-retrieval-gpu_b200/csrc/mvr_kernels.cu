@@ -1246,10 +1246,11 @@ rerank_kernel(DevIndex ix, const float *__restrict__ q, const uint64_t *__restri
 // |BF16 - exact MaxSim|.  topk docs have exact scores of at least (the topk-th
 // best approx - E), and a doc below the cut has an exact score under that.
 // Per query token, with X a bound on |x| and dX on |x - BF16 x| of every decoded
-// doc token x = c + W (dX: the centroids' and weights' own rounding errors, and
-// a relative 2^-8 for the rounded BF16 sum), the error of a dot product is at most
+// doc token x = c + W (dX: the centroids' and weights' own rounding errors, and for
+// queries of more than split_tok tokens, whose kernel rounds the sum, a relative
+// 2^-8), the error of a dot product is at most
 //   |q - bf16(q)| X + |bf16(q)| dX + 2^-13 |q| X,
-// the last term for both sides' FP32 accumulation; 2^-15 max(1, 4 max|q| X)
+// the last term for both sides' FP32 accumulation; 2^-14 max(1, 4 max|q| X)
 // covers an accumulator that starts at an offset of up to 2.04 max|q| X.  The max
 // over a doc's tokens and the clamp at 0 enlarge no error, the sum over query
 // tokens adds them up.  A bound that is not finite keeps every doc.  One CTA per
@@ -1265,7 +1266,7 @@ maxsim_reach_kernel(const float *__restrict__ q, const uint64_t *__restrict__ q_
                     const uint32_t *__restrict__ short_id, const float *__restrict__ approx,
                     const uint32_t *__restrict__ n_short, uint32_t probe_topk, uint32_t topk,
                     const float *__restrict__ cen_bounds, float w_norm, float w_err,
-                    uint32_t *__restrict__ out_id, uint32_t *__restrict__ n_out) {
+                    uint32_t split_tok, uint32_t *__restrict__ out_id, uint32_t *__restrict__ n_out) {
   extern __shared__ uint32_t rsm[];
   uint32_t *ord = rsm, *hist = rsm + probe_topk;  // [probe_topk], [4096]
   __shared__ float s_e[kMaxQueryTok], s_q[kMaxQueryTok];
@@ -1280,7 +1281,7 @@ maxsim_reach_kernel(const float *__restrict__ q, const uint64_t *__restrict__ q_
   for (uint32_t i = tid; i < n; i += kReachThreads) ord[i] = f2ord(approx[row + i]);
   if (tid == 0) s_n = 0;
   const float X = (cen_bounds[0] + w_norm) * (1.0f + 0x1p-10f);
-  const float dX = cen_bounds[1] + w_err + X * 0x1.02p-8f;
+  const float dX = cen_bounds[1] + w_err + (nq > split_tok ? X * 0x1.02p-8f : 0.0f);
   for (uint32_t t = warp; t < nq; t += kReachThreads / 32) {
     const float4 v = __ldg(reinterpret_cast<const float4 *>(q + (tok0 + t) * kDim) + lane);
     const float x[4] = {v.x, v.y, v.z, v.w};
@@ -1354,7 +1355,7 @@ maxsim_reach_kernel(const float *__restrict__ q, const uint64_t *__restrict__ q_
         e += s_e[t];
         qm = fmaxf(qm, s_q[t]);
       }
-      e = (e + (float)nq * 0x1p-15f * fmaxf(1.0f, 4.0f * qm * X)) * (1.0f + 0x1p-10f);
+      e = (e + (float)nq * 0x1p-14f * fmaxf(1.0f, 4.0f * qm * X)) * (1.0f + 0x1p-10f);
       s_thr = e < 1e30f ? __fsub_rd(ord2f(prefix), 2.0f * e) : -INFINITY;
     }
   } else if (tid == 0) {
@@ -1680,10 +1681,10 @@ cudaError_t launch_maxsim_reach(const float *q, const uint64_t *q_off, uint32_t 
                                 const uint32_t *short_id, const float *approx,
                                 const uint32_t *n_short, uint32_t probe_topk, uint32_t topk,
                                 const float *cen_bounds, float w_norm, float w_err,
-                                uint32_t *out_id, uint32_t *n_out, cudaStream_t st,
+                                uint32_t split_tok, uint32_t *out_id, uint32_t *n_out, cudaStream_t st,
                                 int *n_launch) {
   maxsim_reach_kernel<<<n_query, kReachThreads, reach_smem(probe_topk), st>>>(
-      q, q_off, short_id, approx, n_short, probe_topk, topk, cen_bounds, w_norm, w_err, out_id,
+      q, q_off, short_id, approx, n_short, probe_topk, topk, cen_bounds, w_norm, w_err, split_tok, out_id,
       n_out);
   *n_launch += 1;
   return cudaGetLastError();

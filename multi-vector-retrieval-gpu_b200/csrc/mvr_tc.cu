@@ -364,13 +364,13 @@ rerank_tc_kernel(DevIndex ix, const __nv_bfloat16 *__restrict__ cen_bf16,
 }
 
 // ---------------------------------------------------------------------
-// rerank_tmem_kernel: BF16 MaxSim for 1- and 2-bit residual codes with the
-// doc-token operand in tensor memory.
+// rerank_tmem_kernel: BF16 MaxSim for 1- and 2-bit residual codes and queries of
+// more than 32 tokens, with the doc-token operand in tensor memory (shorter
+// queries: rerank_ws_kernel with BF).
 //
 // Per 128-token tile every thread decodes one half row (64 dims) in
 // registers and writes it to TMEM with tcgen05.st; tcgen05.mma then reads A
-// (M = 128 doc tokens, K = 128) from TMEM and B (the query tokens, N = 32 or
-// 64) from a swizzled shared-memory tile, so the decoded tile never passes
+// (M = 128 doc tokens, K = 128) from TMEM and B (the query tokens, N = 64) from a swizzled shared-memory tile, so the decoded tile never passes
 // through shared memory.  Decode of one 32-bit residual word (4*VPB dims)
 // needs no table lookups: the codes j of the four bytes are isolated with one
 // shift and mask, turned into PRMT byte selectors with one IMAD
@@ -393,9 +393,8 @@ rerank_tc_kernel(DevIndex ix, const __nv_bfloat16 *__restrict__ cen_bf16,
 constexpr int kTmTile = 128;
 constexpr int kTmDocs = 64;       // shortlisted docs per CTA
 constexpr int kTmThreads = 256;   // warp w: TMEM lane quadrant w & 3, half row w >> 2
-// TMEM columns: A[2] x 64 + D[3] x N  (N = 32: 224 -> 256, 2 CTAs per SM;
-// N = 64: 320 -> 512, one CTA per SM, enforced through the smem size)
-__host__ __device__ constexpr uint32_t tm_cols(uint32_t n_max) { return n_max <= 32 ? 256u : 512u; }
+constexpr uint32_t kTmN = 64;     // query rows of the B tile
+constexpr uint32_t kTmCols = 512; // TMEM columns: A[2] x 64 + D[3] x 64, so one CTA per SM
 
 template <int NBIT>
 __host__ __device__ constexpr uint32_t tm_dim_of(uint32_t kappa) {
@@ -404,9 +403,8 @@ __host__ __device__ constexpr uint32_t tm_dim_of(uint32_t kappa) {
   return m * WD + VPB * (r % 4) + r / 4;
 }
 
-__host__ __device__ constexpr size_t tm_smem_bytes(uint32_t n_max) {
-  return n_max <= 32 ? 1024 + (size_t)n_max * 256 : 120 * 1024;  // dynamic part: B tile
-}
+// dynamic part: the B tile, enlarged so that one CTA fits an SM
+constexpr size_t kTmSmem = 120 * 1024;
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   uint32_t d;
@@ -447,12 +445,11 @@ __device__ __forceinline__ void mma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, ui
       : "memory");
 }
 
-// 16 output columns (bf16x2) of one half row from WPS residual words
-// (WPS = 16 / (2 * VPB): 2 words for 2-bit, 1 for 1-bit) and 4 uint4 of the
-// permuted centroid row.
+// 16 output columns (bf16x2 weights) of a row from WPS residual words
+// (WPS = 16 / (2 * VPB): 2 words for 2-bit, 1 for 1-bit)
 template <int NBIT>
-__device__ __forceinline__ void tm_decode16(const uint32_t *res, const uint4 *cen, uint32_t wlo,
-                                            uint32_t whi, uint32_t (&out)[16]) {
+__device__ __forceinline__ void tm_weights16(const uint32_t *res, uint32_t wlo, uint32_t whi,
+                                             uint32_t (&out)[16]) {
   constexpr int VPB = 8 / NBIT;
   constexpr uint32_t MASK = NBIT == 2 ? 0x03030303u : 0x01010101u;
   constexpr int WPS = 16 / (2 * VPB);
@@ -467,6 +464,12 @@ __device__ __forceinline__ void tm_decode16(const uint32_t *res, const uint4 *ce
       out[wi * 2 * VPB + 2 * j + 1] = prmt(wlo, whi, t >> 16);
     }
   }
+}
+// the same added to 4 uint4 of the permuted centroid row
+template <int NBIT>
+__device__ __forceinline__ void tm_decode16(const uint32_t *res, const uint4 *cen, uint32_t wlo,
+                                            uint32_t whi, uint32_t (&out)[16]) {
+  tm_weights16<NBIT>(res, wlo, whi, out);
 #pragma unroll
   for (int c = 0; c < 4; c++) {
     out[4 * c + 0] = hadd2_u32(cen[c].x, out[4 * c + 0]);
@@ -510,13 +513,6 @@ __host__ __device__ constexpr uint32_t idesc_e4m3(int m, int n) {
   return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_e4m3_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b,
-                                            uint32_t idesc) {
-  asm volatile("tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, 1;\n" ::"r"(tmem_d),
-               "r"(tmem_a), "l"(b), "r"(idesc)
-               : "memory");
-}
-
 // 16 A_r columns (4 FP8 weights each) of one 64-dim half row from its 4
 // residual words; wtab: the 4 FP8 bucket weights in bytes 0..3.
 __device__ __forceinline__ void fp8_decode16(const uint32_t *res, uint32_t wtab,
@@ -550,24 +546,23 @@ __device__ __forceinline__ void fp8_decode16_b4(const uint32_t *res, const TmWei
   }
 }
 
-template <int NBIT, bool FP8>
-__global__ void __launch_bounds__(kTmThreads, 2)
+template <int NBIT>
+__global__ void __launch_bounds__(kTmThreads, 1)
 rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights tw,
                    const float *__restrict__ q, const uint64_t *__restrict__ q_off,
                    const uint32_t *__restrict__ short_id, const uint32_t *__restrict__ n_short,
-                   uint32_t probe_topk, int semantics, uint32_t n_max, float x_bound,
-                   float *__restrict__ approx, unsigned *__restrict__ err) {
-  static_assert(FP8 ? (NBIT == 2 || NBIT == 4) : (NBIT == 1 || NBIT == 2),
-                "BF16 decodes 1- and 2-bit codes, FP8 2- and 4-bit codes");
+                   uint32_t probe_topk, int semantics, float x_bound, float *__restrict__ approx,
+                   unsigned *__restrict__ err) {
+  static_assert(NBIT == 1 || NBIT == 2, "BF16 decode of 1- and 2-bit codes");
   constexpr int VPB = 8 / NBIT;
-  constexpr int HW = 64 / (4 * VPB);  // residual words of a 64-dim half row (8, 4 or 2)
-  constexpr int CW = FP8 ? 16 : 32;   // centroid words (TMEM columns) of a half row
+  constexpr int HW = 64 / (4 * VPB);  // residual words of a 64-dim half row (4 or 2)
+  constexpr int CW = 32;              // centroid words (TMEM columns) of a half row
+  constexpr uint32_t N = kTmN, n_cols = kTmCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t *Bq = smem;  // BF16: [2 K-blocks][n_max rows][128 B]; FP8: [n_max rows][128 B]
+  uint8_t *Bq = smem;  // [2 K-blocks][N rows][128 B]
   __shared__ uint32_t best[kTmDocs * kMaxQueryTok];        // [doc][query token], bits of OFF + max
-  __shared__ uint32_t s_qss;                               // max squared (scaled) token norm
-  __shared__ float s_qinv[kMaxQueryTok];                   // FP8: 1 / query-token scale
+  __shared__ uint32_t s_qss;                               // max squared token norm
   __shared__ __align__(16) uint32_t stage[kTmThreads / 32][16];  // per-warp epilogue staging
   __shared__ uint64_t bar[2];
   __shared__ uint32_t tmem_base_s;
@@ -580,13 +575,13 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
   const uint32_t b = blockIdx.y;
   const uint32_t ns = n_short[b];
   const uint32_t d0 = blockIdx.x * kTmDocs;
-  if (d0 >= ns) return;  // uniform: before any TMEM / barrier use
-  const uint32_t nd = min((uint32_t)kTmDocs, ns - d0);
   const uint64_t tok0 = q_off[b];
   const uint32_t nq = (uint32_t)(q_off[b + 1] - tok0);
-  const uint32_t N = nq <= 32 ? 32u : 64u;  // <= n_max (host sizes smem by the batch)
-  const uint32_t idesc = FP8 ? idesc_e4m3(kTmTile, (int)N) : idesc_bf16(kTmTile, (int)N);
-  const uint32_t n_cols = tm_cols(n_max);
+  // uniform exits before any TMEM or barrier use: no docs here, or a query of
+  // the warp-specialised kernel
+  if (d0 >= ns || nq <= 32) return;
+  const uint32_t nd = min((uint32_t)kTmDocs, ns - d0);
+  const uint32_t idesc = idesc_bf16(kTmTile, (int)N);
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
@@ -608,42 +603,6 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
   }
   for (int i = tid; i < kMaxQueryTok * kTmDocs; i += kTmThreads) best[i] = 0u;
   __syncthreads();  // s_qss
-  if constexpr (FP8) {
-    // query tokens -> B operand (E4M3, scaled per token, permuted K order,
-    // swizzled, rows >= nq zero); 8 lanes per row, 16 positions each
-    for (int i = tid; i < (int)N * 8; i += kTmThreads) {  // N * 8 is a multiple of 256
-      const int row = i >> 3, ch = i & 7;
-      float x[16];
-      float amax = 0.0f, ss = 0.0f;
-#pragma unroll
-      for (int u = 0; u < 16; u++) {
-        x[u] = (uint32_t)row < nq ? __ldg(q + (tok0 + row) * kDim + fp8_dim_of<NBIT>(16 * ch + u)) : 0.0f;
-        amax = fmaxf(amax, fabsf(x[u]));
-        ss = fmaf(x[u], x[u], ss);
-      }
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) {
-        amax = fmaxf(amax, __shfl_xor_sync(kFull, amax, o));
-        ss += __shfl_xor_sync(kFull, ss, o);
-      }
-      // power-of-two scale: largest entry into [112, 224] (1 for an all-zero row)
-      const float sc = amax > 0.0f ? exp2f(floorf(log2f(224.0f / amax))) : 1.0f;
-      uint32_t v[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(
-            make_float2(x[4 * u] * sc, x[4 * u + 1] * sc), __NV_SATFINITE, __NV_E4M3);
-        const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(
-            make_float2(x[4 * u + 2] * sc, x[4 * u + 3] * sc), __NV_SATFINITE, __NV_E4M3);
-        v[u] = (uint32_t)lo | ((uint32_t)hi << 16);
-      }
-      *reinterpret_cast<uint4 *>(Bq + sw128_off(row, ch)) = make_uint4(v[0], v[1], v[2], v[3]);
-      if ((lane & 7) == 0) {
-        atomicMax(&s_qss, __float_as_uint(ss * sc * sc));
-        if (row < kMaxQueryTok) s_qinv[row] = 1.0f / sc;
-      }
-    }
-  } else
   // query tokens -> B operand (BF16, permuted K order, swizzled, rows >= nq
   // zero); the 16 lanes of a row also sum its squares (fixed shuffle order)
   for (int i = tid; i < (int)N * 16; i += kTmThreads) {  // N * 16 is a multiple of 256
@@ -679,10 +638,9 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   const uint32_t n_tok = d_pref[nd];
-  // OFF: smallest power of two >= 1 above max |q| * |x| (margin for BF16 /
-  // FP8 rounding; FP8: scaled query tokens)
-  const float off = fmaxf(1.0f, exp2f(ceilf(log2f(sqrtf(__uint_as_float(s_qss)) * x_bound *
-                                                  (FP8 ? 1.15f : 1.02f) + 1e-30f))));
+  // OFF: smallest power of two >= 1 above max |q| * |x| (margin for BF16 rounding)
+  const float off = fmaxf(1.0f, exp2f(ceilf(log2f(sqrtf(__uint_as_float(s_qss)) * x_bound * 1.02f +
+                                                  1e-30f))));
   const uint32_t off_bits = __float_as_uint(off);
   const uint32_t n_tiles = (n_tok + kTmTile - 1) / kTmTile;
   const uint32_t b_base = smem_u32(Bq);
@@ -704,12 +662,7 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
   };
   auto load_res = [&](uint64_t v, uint32_t (&r)[HW]) {
     const uint8_t *p = ix.residual + v * ix.bytes_per_vec + hf * (HW * 4);
-    if constexpr (HW == 8) {
-      const uint4 t0 = __ldg(reinterpret_cast<const uint4 *>(p));
-      const uint4 t1 = __ldg(reinterpret_cast<const uint4 *>(p) + 1);
-      r[0] = t0.x; r[1] = t0.y; r[2] = t0.z; r[3] = t0.w;
-      r[4] = t1.x; r[5] = t1.y; r[6] = t1.z; r[7] = t1.w;
-    } else if constexpr (HW == 4) {
+    if constexpr (HW == 4) {
       const uint4 t = __ldg(reinterpret_cast<const uint4 *>(p));
       r[0] = t.x; r[1] = t.y; r[2] = t.z; r[3] = t.w;
     } else {
@@ -769,7 +722,7 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
   }
   for (uint32_t tile = 0; tile < n_tiles; tile++) {
     const int st = tile & 1;
-    // centroid half row of this tile (permuted BF16: 8 x 16 B; FP8: 4 x 16 B)
+    // centroid half row of this tile (permuted BF16: 8 x 16 B)
     uint4 cen[CW / 4];
     if (doc_c >= 0) {
       const uint4 *cp = reinterpret_cast<const uint4 *>(cen_perm + (size_t)code_c * (2 * CW) + hf * CW);
@@ -787,39 +740,17 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
     }
     if (tile > 1) epilogue(tile - 2);  // its MMA completed during the previous iteration
     if (hf == 0) tok_doc[tile % 3][row] = doc_c;
-    if constexpr (FP8) {
-      // A_c: columns 64 st + 16 hf (centroid, as loaded); A_r: + 32 (weights)
-      const uint32_t acol = tmem + lane_off + 64u * st + 16u * hf;
-      uint32_t out[16];
+    const uint32_t acol = tmem + lane_off + 64u * st + 32u * hf;
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        out[4 * u] = doc_c >= 0 ? cen[u].x : 0u;
-        out[4 * u + 1] = doc_c >= 0 ? cen[u].y : 0u;
-        out[4 * u + 2] = doc_c >= 0 ? cen[u].z : 0u;
-        out[4 * u + 3] = doc_c >= 0 ? cen[u].w : 0u;
-      }
-      tmem_st16(acol, out);
+    for (int part = 0; part < 2; part++) {
+      uint32_t out[16];
       if (doc_c >= 0) {
-        if constexpr (NBIT == 4) fp8_decode16_b4(res_c, tw, out);
-        else fp8_decode16(res_c, tw.w[0], out);
+        tm_decode16<NBIT>(res_c + part * (HW / 2), cen + part * 4, tw.w[0], tw.w[1], out);
       } else {
 #pragma unroll
         for (int u = 0; u < 16; u++) out[u] = 0u;
       }
-      tmem_st16(acol + 32u, out);
-    } else {
-      const uint32_t acol = tmem + lane_off + 64u * st + 32u * hf;
-#pragma unroll
-      for (int part = 0; part < 2; part++) {
-        uint32_t out[16];
-        if (doc_c >= 0) {
-          tm_decode16<NBIT>(res_c + part * (HW / 2), cen + part * 4, tw.w[0], tw.w[1], out);
-        } else {
-#pragma unroll
-          for (int u = 0; u < 16; u++) out[u] = 0u;
-        }
-        tmem_st16(acol + 16u * part, out);
-      }
+      tmem_st16(acol + 16u * part, out);
     }
     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
     tc_fence_before();
@@ -828,19 +759,10 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
     if (tid == 0) {
       tc_fence_after();
       const uint32_t dcol = tmem + 128u + N * (tile % 3);
-      if constexpr (FP8) {
 #pragma unroll
-        for (int kk = 0; kk < 4; kk++) {  // K = 32 per MMA; centroid part, then residual part
-          const uint64_t bd = sw128_desc(b_base + kk * 32);
-          mma_e4m3_ta(dcol, tmem + 64u * st + 8u * kk, bd, idesc);        // D starts at OFF
-          mma_e4m3_ta(dcol, tmem + 64u * st + 32u + 8u * kk, bd, idesc);
-        }
-      } else {
-#pragma unroll
-        for (int kk = 0; kk < 8; kk++) {
-          const uint64_t bd = sw128_desc(b_base + (kk >> 2) * (N * 128) + (kk & 3) * 32);
-          mma_bf16_ta(dcol, tmem + 64u * st + 8u * kk, bd, idesc, 1u);  // D starts at OFF
-        }
+      for (int kk = 0; kk < 8; kk++) {
+        const uint64_t bd = sw128_desc(b_base + (kk >> 2) * (N * 128) + (kk & 3) * 32);
+        mma_bf16_ta(dcol, tmem + 64u * st + 8u * kk, bd, idesc, 1u);  // D starts at OFF
       }
       mma_commit(&bar[st]);
     }
@@ -859,7 +781,6 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
     float s = 0.0f;
     for (uint32_t t = 0; t < nq; t++) {
       float m = __uint_as_float(best[tid * kMaxQueryTok + t]) - off;
-      if constexpr (FP8) m *= s_qinv[t];
       if (clamp) m = fmaxf(m, 0.0f);
       s += m;
     }
@@ -874,14 +795,18 @@ rerank_tmem_kernel(DevIndex ix, const uint32_t *__restrict__ cen_perm, TmWeights
 }
 
 // cen_perm[c][w] = bf16x2 of centroid c at K positions 2w, 2w+1 of the
-// rerank_tmem_kernel order.
+// K order of the BF16 kernels; row n_cent is zero.
 template <int NBIT>
 __global__ void perm_centroid_kernel(const float *__restrict__ cen, uint32_t n_cent,
                                      uint32_t *__restrict__ out) {
-  const size_t n = (size_t)n_cent * 64;
+  const size_t n = ((size_t)n_cent + 1) * 64;  // and a row of zeros
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const size_t c = i / 64;
+    if (c == n_cent) {
+      out[i] = 0u;
+      continue;
+    }
     const uint32_t w = (uint32_t)(i % 64);
     const float *row = cen + c * kDim;
     __nv_bfloat162 p = __floats2bfloat162_rn(row[tm_dim_of<NBIT>(2 * w)], row[tm_dim_of<NBIT>(2 * w + 1)]);
@@ -1664,7 +1589,7 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 //             per lane touched 32 and its loads and tcgen05.st took two thirds
 //             of the L1 data pipe); the residual bytes from the ring (read in
 //             a bank-conflict-free order) expanded by PRMT into E4M3 bucket
-//             weights (as rerank_tmem_kernel's FP8 decode), a tcgen05.st of
+//             weights, a tcgen05.st of
 //             those (A_r);
 //  warp 1     MMA: one thread issues per tile a bias MMA that writes OFF into
 //             every element of the tile's D stage (a constant A_e of 16.0 in
@@ -1684,7 +1609,10 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 // FEAT the kernel computes the learned pruner's features instead: the
 // centroid part only (no producer, residual decode or residual MMA), and
 // per doc the maxima themselves (per query token the best centroid score
-// over the doc's tokens) plus log(doc length).  Every pipeline mbarrier wait
+// over the doc's tokens) plus log(doc length).  With BF (1- and 2-bit codes)
+// centroid rows, weights and query are BF16: rows of 256 bytes in two A_c
+// stages, 64 A_r columns, 8 K-steps of K = 16 (kind::f16), A_e = 1 and OFF in K
+// position 0 of B_e.  The sum c + W[b] is not rounded.  Every pipeline mbarrier wait
 // is bounded (wait_ns, 1 s by default); on a timeout the CTA records the
 // error and every role stops; the producer then waits (1 s bound) for its
 // bulk copies still in flight and the MMA thread for its MMAs before TMEM
@@ -1697,6 +1625,8 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 // twice the epilogue warps: 5.46 -> 3.60 ms.  Two epilogue warps per 32 rows also for
 // N = 32 (72 registers a thread): 8.9 ms; three CTAs per SM with one A_r stage: 10.8
 // ms; the maxima written by one lane's 32 atomics instead of 32 selects: 8.4 ms.
+// BF against rerank_tmem_kernel at 32 columns: 400 queries x 1500 docs at 2 bits 3.13
+// -> 1.96 ms (21.6 tokens per ns), 500 x 1400 at 1 bit 3.25 -> 2.24 ms.
 // ---------------------------------------------------------------------
 constexpr int kWsDocs = 256;         // shortlisted docs per CTA (default; 32, 64, 128 or 256)
 // epilogue warps per 32 rows: the 64-column variant splits the columns in two
@@ -1705,19 +1635,20 @@ __host__ __device__ constexpr int ws_threads(int nmax) { return 32 * (6 + 4 * ws
 
 constexpr int kWsAStages = 2;        // A_r stages in TMEM
 // A_c stages: one more, so that the wait for tile i's A_r stage (the MMAs of tile
-// i - 2 done) also frees the stage of tile i + 1's copies
-constexpr int kWsCStages = kWsAStages + 1;
+// i - 2 done) also frees the stage of tile i + 1's copies; BF16 rows (32 KB a
+// stage) have room for two, and tile i + 1's copies wait for the MMAs of tile i - 1
+__host__ __device__ constexpr int ws_cstages(bool bf) { return kWsAStages + (bf ? 0 : 1); }
 // D stages in TMEM: 3, or 2 of 64 columns, so that two CTAs share an SM's 512 columns
 __host__ __device__ constexpr int ws_dstages(int nmax) { return nmax <= 32 ? 3 : 2; }
 constexpr uint32_t kWsCols = 256;    // TMEM columns of a CTA
 // ring stages of residual bytes: 4, or the 2 that two CTAs leave room for at 4 bits
 __host__ __device__ constexpr int ws_rstages(int nbit) { return nbit == 4 ? 2 : 4; }
 __host__ __device__ constexpr uint32_t ws_stage_bytes(int nbit) { return 128u * (128u * nbit / 8u); }
-constexpr uint32_t kWsCBytes = 128u * 128u;  // one A_c stage
+__host__ __device__ constexpr uint32_t ws_crow(bool bf) { return bf ? 256u : 128u; }  // A_c bytes a row
 // dynamic shared memory: 1 KB alignment slack + query tile + bias tile + A_c
 // stages + ring
-__host__ __device__ constexpr size_t ws_smem_bytes(int nbit, int nmax) {
-  return 1024 + 2 * (size_t)nmax * 128 + kWsCStages * (size_t)kWsCBytes +
+__host__ __device__ constexpr size_t ws_smem_bytes(int nbit, int nmax, bool bf = false) {
+  return 1024 + (size_t)nmax * (ws_crow(bf) + 128) + ws_cstages(bf) * (size_t)(128 * ws_crow(bf)) +
          ws_rstages(nbit) * (size_t)ws_stage_bytes(nbit);
 }
 
@@ -1749,32 +1680,36 @@ __device__ __forceinline__ void mma_e4m3_acc(uint32_t tmem_d, uint32_t tmem_a, u
       : "memory");
 }
 
-template <int NBIT, int NMAX, bool FEAT = false, int DOCS = kWsDocs>
+template <int NBIT, int NMAX, bool FEAT = false, int DOCS = kWsDocs, bool BF = false>
 __global__ void __launch_bounds__(ws_threads(NMAX), 2)
-rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
+rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen_rows, TmWeights tw,
                  const float *__restrict__ q, const uint64_t *__restrict__ q_off,
                  const uint32_t *__restrict__ short_id, const uint32_t *__restrict__ n_short,
                  uint32_t probe_topk, int semantics, float x_bound, float *__restrict__ approx,
                  unsigned *__restrict__ err, uint64_t wait_ns) {
-  static_assert(NBIT == 2 || NBIT == 4, "FP8 decode of 2- and 4-bit codes");
+  static_assert(BF ? NBIT <= 2 && NMAX == 32 && !FEAT && DOCS <= 128 : NBIT == 2 || NBIT == 4,
+                "FP8 decodes 2- and 4-bit codes, BF16 1- and 2-bit ones");
   static_assert(NMAX == 32 || NMAX == 64, "query tiles of 32 or 64 rows");
   static_assert(!FEAT || NMAX == 32, "pruner features: queries of up to 32 tokens");
   static_assert(DOCS == 32 || DOCS == 64 || ((DOCS == 128 || DOCS == 256) && NMAX == 32),
                 "docs per CTA (64 at most with 64 columns: the maxima of two CTAs fit an SM)");
-  constexpr int S = ws_rstages(NBIT), SA = kWsAStages, SD = ws_dstages(NMAX), SC = kWsCStages;
+  constexpr int S = ws_rstages(NBIT), SA = kWsAStages, SD = ws_dstages(NMAX), SC = ws_cstages(BF);
+  constexpr uint32_t CROW = ws_crow(BF), CSTAGE = 128u * CROW;  // centroid rows: bytes, a stage
+  constexpr uint32_t ACOLS = BF ? 64u : 32u;                    // TMEM columns of A_r
   constexpr int G = ws_groups(NMAX), CW = NMAX / G;  // column groups and their width
   constexpr uint32_t BPV = 128u * NBIT / 8u;       // residual bytes per token
   constexpr uint32_t STAGE = ws_stage_bytes(NBIT);
   constexpr uint32_t COLS = kWsCols;
-  constexpr uint32_t DCOL0 = 32u * SA;              // D stages after the A_r stages
+  constexpr uint32_t DCOL0 = ACOLS * SA;            // D stages after the A_r stages
   constexpr uint32_t ECOL = DCOL0 + NMAX * SD;      // bias operand A_e (8 columns)
   static_assert(ECOL + 8 <= COLS, "TMEM columns");
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t *Bq = smem;                     // [NMAX rows][128 B] E4M3, SW128, K-major
-  uint8_t *Be = smem + NMAX * 128;        // bias B operand, same layout
-  uint8_t *Ac = smem + 2 * NMAX * 128;    // [SC][128 rows][128 B] centroid rows, SW128, K-major
-  uint8_t *ring = Ac + SC * kWsCBytes;    // [S][128 rows][BPV] residual bytes
+  // E4M3: [rows][128 B], SW128, K-major; BF16: two such blocks of 64 dimensions
+  uint8_t *Bq = smem;                     // NMAX query tokens
+  uint8_t *Be = smem + NMAX * CROW;       // bias B operand, [NMAX rows][128 B]
+  uint8_t *Ac = Be + NMAX * 128;          // [SC] x 128 centroid rows
+  uint8_t *ring = Ac + SC * CSTAGE;       // [S][128 rows][BPV] residual bytes
   __shared__ uint32_t best[DOCS * NMAX];  // [doc][query token]: bits of OFF + max
   __shared__ uint32_t s_qss, tmem_base_s;
   __shared__ float s_qinv[NMAX];
@@ -1830,67 +1765,104 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
       carry += __shfl_sync(kFull, v, 31);
     }
   }
-  // query tokens -> B (E4M3, per-token power-of-two scales, FP8 K order,
-  // swizzled, rows >= nq zero): 8 lanes per row, 16 positions each
-  for (int i = tid; i < NMAX * 8; i += ws_threads(NMAX)) {
-    const int row = i >> 3, ch = i & 7;
-    float x[16];
-    float amax = 0.0f, ss = 0.0f;
+  if constexpr (BF) {
+    // query tokens -> B (BF16, the decode's K order, swizzled, rows >= nq zero):
+    // 16 lanes per row, 8 positions each
+    for (int i = tid; i < NMAX * 16; i += ws_threads(NMAX)) {  // whole warps
+      const int row = i >> 4, ch = i & 15;
+      uint32_t v[4] = {0, 0, 0, 0};
+      float ss = 0.0f;
+      if ((uint32_t)row < nq) {
+        const float *src = q + (tok0 + row) * kDim;
 #pragma unroll
-    for (int u = 0; u < 16; u++) {
-      x[u] = (uint32_t)row < nq ? __ldg(q + (tok0 + row) * kDim + fp8_dim_of<NBIT>(16 * ch + u))
-                                : 0.0f;
-      amax = fmaxf(amax, fabsf(x[u]));
-      ss = fmaf(x[u], x[u], ss);
-    }
+        for (int u = 0; u < 4; u++) {
+          const float lo = __ldg(src + tm_dim_of<NBIT>(8 * ch + 2 * u));
+          const float hi = __ldg(src + tm_dim_of<NBIT>(8 * ch + 2 * u + 1));
+          ss = fmaf(lo, lo, fmaf(hi, hi, ss));
+          __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+          v[u] = *reinterpret_cast<uint32_t *>(&p);
+        }
+      }
+      *reinterpret_cast<uint4 *>(Bq + (ch >> 3) * (NMAX * 128) + sw128_off(row, ch & 7)) =
+          make_uint4(v[0], v[1], v[2], v[3]);
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      amax = fmaxf(amax, __shfl_xor_sync(kFull, amax, o));
-      ss += __shfl_xor_sync(kFull, ss, o);
+      for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(kFull, ss, o);
+      if ((lane & 15) == 0) {
+        atomicMax(&s_qss, __float_as_uint(ss));
+        s_qinv[row] = 1.0f;
+      }
     }
-    const float sc = amax > 0.0f ? exp2f(floorf(log2f(224.0f / amax))) : 1.0f;
-    uint32_t v[4];
+  } else {
+    // query tokens -> B (E4M3, per-token power-of-two scales, FP8 K order,
+    // swizzled, rows >= nq zero): 8 lanes per row, 16 positions each
+    for (int i = tid; i < NMAX * 8; i += ws_threads(NMAX)) {
+      const int row = i >> 3, ch = i & 7;
+      float x[16];
+      float amax = 0.0f, ss = 0.0f;
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(
-          make_float2(x[4 * u] * sc, x[4 * u + 1] * sc), __NV_SATFINITE, __NV_E4M3);
-      const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(
-          make_float2(x[4 * u + 2] * sc, x[4 * u + 3] * sc), __NV_SATFINITE, __NV_E4M3);
-      v[u] = (uint32_t)lo | ((uint32_t)hi << 16);
-    }
-    *reinterpret_cast<uint4 *>(Bq + sw128_off(row, ch)) = make_uint4(v[0], v[1], v[2], v[3]);
-    if ((lane & 7) == 0) {
-      atomicMax(&s_qss, __float_as_uint(ss * sc * sc));
-      s_qinv[row] = 1.0f / sc;
+      for (int u = 0; u < 16; u++) {
+        x[u] = (uint32_t)row < nq ? __ldg(q + (tok0 + row) * kDim + fp8_dim_of<NBIT>(16 * ch + u))
+                                  : 0.0f;
+        amax = fmaxf(amax, fabsf(x[u]));
+        ss = fmaf(x[u], x[u], ss);
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(kFull, amax, o));
+        ss += __shfl_xor_sync(kFull, ss, o);
+      }
+      const float sc = amax > 0.0f ? exp2f(floorf(log2f(224.0f / amax))) : 1.0f;
+      uint32_t v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(
+            make_float2(x[4 * u] * sc, x[4 * u + 1] * sc), __NV_SATFINITE, __NV_E4M3);
+        const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(
+            make_float2(x[4 * u + 2] * sc, x[4 * u + 3] * sc), __NV_SATFINITE, __NV_E4M3);
+        v[u] = (uint32_t)lo | ((uint32_t)hi << 16);
+      }
+      *reinterpret_cast<uint4 *>(Bq + sw128_off(row, ch)) = make_uint4(v[0], v[1], v[2], v[3]);
+      if ((lane & 7) == 0) {
+        atomicMax(&s_qss, __float_as_uint(ss * sc * sc));
+        s_qinv[row] = 1.0f / sc;
+      }
     }
   }
   __syncthreads();
   const uint32_t tmem = tmem_base_s;
   const uint32_t T = d_pref[nd];                 // rows (tokens) of the CTA
   const uint32_t n_tiles = (T + 127u) / 128u;
-  const float off = fmaxf(1.0f, exp2f(ceilf(log2f(sqrtf(__uint_as_float(s_qss)) * x_bound * 1.15f +
-                                                  1e-30f))));
+  const float off = fmaxf(1.0f, exp2f(ceilf(log2f(sqrtf(__uint_as_float(s_qss)) * x_bound *
+                                                  (BF ? 1.02f : 1.15f) + 1e-30f))));
   // bias operands: OFF = 2^e = 32 * A_e * B_e with A_e = 2^a (a in [4, 8],
   // every row and K position of A_e) and B_e = 2^(e - 5 - a) >= 2^-9 in K
   // positions 0..31 of every row of the bias tile (the rest 0): both exact in
   // E4M3, the 32 products sum to OFF exactly, for OFF up to 2^21
   const int e_off = (int)log2f(off);
   const int a_exp = min(8, e_off + 4);
-  if (e_off > 21) {  // norms beyond the bias's range: report, do not guess
+  // (BF16: A_e = 1 everywhere, B_e = OFF in K position 0)
+  if (!BF && e_off > 21) {  // norms beyond the bias's range: report, do not guess
     if (tid == 0) atomicOr(err, 16u);
   }
   for (int i = tid; i < NMAX * 8; i += ws_threads(NMAX)) {
     const int row = i >> 3, ch = i & 7;
-    const uint32_t e = ch < 2 ? (uint32_t)__nv_cvt_float_to_fp8(exp2f((float)(e_off - 5 - a_exp)),
-                                                                __NV_SATFINITE, __NV_E4M3) *
-                                    0x01010101u
-                              : 0u;
-    *reinterpret_cast<uint4 *>(Be + sw128_off(row, ch)) = make_uint4(e, e, e, e);
+    uint4 v;
+    if constexpr (BF) {
+      v = make_uint4(ch == 0 ? __float_as_uint(off) >> 16 : 0u, 0u, 0u, 0u);
+    } else {
+      const uint32_t e = ch < 2 ? (uint32_t)__nv_cvt_float_to_fp8(
+                                      exp2f((float)(e_off - 5 - a_exp)), __NV_SATFINITE,
+                                      __NV_E4M3) * 0x01010101u
+                                : 0u;
+      v = make_uint4(e, e, e, e);
+    }
+    *reinterpret_cast<uint4 *>(Be + sw128_off(row, ch)) = v;
   }
   const uint32_t qd = warp & 3;  // TMEM lane quadrant of this warp
   const uint32_t lane_off = (32u * qd) << 16;
   if (warp >= 2 && warp < 6) {  // A_e = 2^a: E4M3 exponent field a + 7, mantissa 0
-    tmem_fill8(tmem + lane_off + ECOL, (uint32_t)((a_exp + 7) << 3) * 0x01010101u);
+    tmem_fill8(tmem + lane_off + ECOL,
+               BF ? 0x3f803f80u : (uint32_t)((a_exp + 7) << 3) * 0x01010101u);
     tmem_wait_st();
   }
   fence_async_smem();  // B and bias tiles (generic stores) before the MMAs read them
@@ -1940,7 +1912,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
   } else if (warp == 1) {
     // ---------------- MMA issue ----------------
     if (lane == 0) {
-      const uint32_t idesc = idesc_e4m3(128, NMAX);
+      const uint32_t idesc = BF ? idesc_bf16(128, NMAX) : idesc_e4m3(128, NMAX);
       const uint32_t b_base = smem_u32(Bq), c_base = smem_u32(Ac);
       const uint64_t be_desc = sw128_desc(smem_u32(Be));
       uint32_t i = 0;
@@ -1950,13 +1922,23 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
         if (i >= (uint32_t)SD && !mbar_wait(&dempty[sd], ((i / SD) + 1) & 1, wait_ns)) break;
         tc_fence_after();
         const uint32_t dcol = tmem + DCOL0 + NMAX * sd;
-        const uint32_t ca = c_base + (i % SC) * kWsCBytes;
-        mma_e4m3_acc(dcol, tmem + ECOL, be_desc, idesc, 0u);  // D = OFF
+        const uint32_t ca = c_base + (i % SC) * CSTAGE;
+        if constexpr (BF) {  // K = 16 per MMA
+          mma_bf16_ta(dcol, tmem + ECOL, be_desc, idesc, 0u);  // D = OFF
 #pragma unroll
-        for (int kk = 0; kk < 4; kk++) {  // K = 32 per MMA: centroid part, residual part
-          const uint64_t bd = sw128_desc(b_base + kk * 32);
-          mma_e4m3_ss(dcol, sw128_desc(ca + kk * 32), bd, idesc);
-          if constexpr (!FEAT) mma_e4m3_acc(dcol, tmem + 32u * sa + 8u * kk, bd, idesc, 1u);
+          for (int kk = 0; kk < 8; kk++) {
+            const uint64_t bd = sw128_desc(b_base + (kk >> 2) * (NMAX * 128) + (kk & 3) * 32);
+            mma_bf16(dcol, sw128_desc(ca + (kk >> 2) * 16384 + (kk & 3) * 32), bd, idesc, 1u);
+            mma_bf16_ta(dcol, tmem + ACOLS * sa + 8u * kk, bd, idesc, 1u);
+          }
+        } else {
+          mma_e4m3_acc(dcol, tmem + ECOL, be_desc, idesc, 0u);  // D = OFF
+#pragma unroll
+          for (int kk = 0; kk < 4; kk++) {  // K = 32 per MMA: centroid part, residual part
+            const uint64_t bd = sw128_desc(b_base + kk * 32);
+            mma_e4m3_ss(dcol, sw128_desc(ca + kk * 32), bd, idesc);
+            if constexpr (!FEAT) mma_e4m3_acc(dcol, tmem + ACOLS * sa + 8u * kk, bd, idesc, 1u);
+          }
         }
         mma_commit(&dfull[sd]);
         mma_commit(&afree[sa]);
@@ -1983,19 +1965,23 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
       while (d_pref[dcur + 1] <= g) dcur++;
       return __ldg(ix.vq_code + d_off[dcur] + (g - d_pref[dcur]));
     };
-    // the centroid rows of this warp's 32 rows of a tile -> A_c stage st, 8
-    // lanes a row (row 4u + lane / 8, 16-byte chunk lane % 8)
-    // (its offset in the swizzled tile: 1 KB per 8 rows, two patterns for u even and odd)
-    const uint32_t l3 = (uint32_t)lane >> 3, ch = lane & 7u;
-    const uint32_t c_even = smem_u32(Ac) + 4096u * qd + l3 * 128u + ((ch ^ l3) << 4);
-    const uint32_t c_odd = smem_u32(Ac) + 4096u * qd + (4u + l3) * 128u + ((ch ^ (4u + l3)) << 4);
+    // the centroid rows of this warp's 32 rows of a tile -> A_c stage st, a
+    // 16-byte chunk a lane: 8 lanes a row (BF16: 16, its blocks 16 KB apart), RU
+    // rows a copy; offsets in the swizzled tile repeat every 8 rows, 1 KB apart
+    constexpr uint32_t RU = 512u / CROW, NP = 8u / RU;
+    const uint32_t l_row = (uint32_t)lane / (CROW / 16u), l_ch = (uint32_t)lane % (CROW / 16u);
+    uint32_t c_off[NP];
+#pragma unroll
+    for (uint32_t p = 0; p < NP; p++)
+      c_off[p] = smem_u32(Ac) + 4096u * qd + (l_ch >> 3) * 16384u +
+                 sw128_off(RU * p + l_row, l_ch & 7u);
     auto copy_cen = [&](uint32_t code, uint32_t st) {
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const uint32_t cd = __shfl_sync(kFull, code, 4u * u + l3);
+      for (uint32_t u = 0; u < 32u / RU; u++) {
+        const uint32_t cd = __shfl_sync(kFull, code, RU * u + l_row);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
-                         (u & 1 ? c_odd : c_even) + st * kWsCBytes + (u >> 1) * 1024u),
-                     "l"(cen8 + (size_t)cd * kDim + 16u * ch)
+                         c_off[u % NP] + st * CSTAGE + (u / NP) * 1024u),
+                     "l"(cen_rows + (size_t)cd * CROW + 16u * l_ch)
                      : "memory");
       }
     };
@@ -2007,7 +1993,9 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
     commit();
     // chunk rotation of the residual reads: rows are BPV bytes apart, so a
     // wavefront's 8 lanes (rows) start in 4 (2-bit) or 2 (4-bit) bank groups
-    const uint32_t rot = NBIT == 2 ? ((uint32_t)lane >> 2) & 1u : ((uint32_t)lane >> 1) & 3u;
+    const uint32_t rot = NBIT == 1   ? 0u
+                         : NBIT == 2 ? ((uint32_t)lane >> 2) & 1u
+                                     : ((uint32_t)lane >> 1) & 3u;
     bool ok = true;
     for (uint32_t i = 0; ok && i < n_tiles; i++) {
       const uint32_t s = i % S, sa = i % SA;
@@ -2017,9 +2005,12 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
         break;
       }
       tc_fence_after();
-      const uint32_t acol = tmem + lane_off + 32u * sa;
-      if (i + 1 < n_tiles) copy_cen(c1, (i + 1) % SC);
-      commit();
+      const uint32_t acol = tmem + lane_off + ACOLS * sa;
+      const uint32_t c_next = c1;
+      if constexpr (!BF) {
+        if (i + 1 < n_tiles) copy_cen(c_next, (i + 1) % SC);
+        commit();
+      }
       c1 = c2;
       c2 = code_of(i + 3);
       if constexpr (!FEAT) {
@@ -2055,7 +2046,13 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
           res[4 * u + 3] = t[u].w;
         }
         uint32_t out[16];
-        if constexpr (NBIT == 4) {
+        if constexpr (BF) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            tm_weights16<NBIT>(res + k * (int)(BPV / 16), tw.w[0], tw.w[1], out);
+            tmem_st16(acol + 16u * k, out);
+          }
+        } else if constexpr (NBIT == 4) {
           fp8_decode16_b4(res, tw, out);
           tmem_st16(acol, out);
           fp8_decode16_b4(res + 8, tw, out);
@@ -2070,16 +2067,28 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen8, TmWeights tw,
       } else {
         (void)rot;
         (void)acol;
+        (void)c_next;
       }
       // tile i's rows have landed (tile i + 1's may be on their way) and are
       // visible to the MMAs
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      if constexpr (BF) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      else asm volatile("cp.async.wait_group 1;\n" ::: "memory");
       fence_async_smem();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&afull[sa]);
         if constexpr (!FEAT) mbar_arrive(&sfree[s]);
+      }
+      if constexpr (BF) {  // tile i + 1's stage: the MMAs of tile i - 1 done
+        if (ok && i + 1 < n_tiles) {
+          if (i + 1 >= (uint32_t)SA &&
+              !__all_sync(kFull, mbar_wait(&afree[(i + 1) % SA], (((i + 1) / SA) + 1) & 1, wait_ns)))
+            ok = false;
+          else
+            copy_cen(c_next, (i + 1) % SC);
+          commit();
+        }
       }
       if (__any_sync(kFull, s_abort != 0)) ok = false;
     }
@@ -2445,13 +2454,9 @@ cudaError_t configure_tc_kernels() {
   if (e != cudaSuccess) return e;
   MVR_PT_ATTR(1) MVR_PT_ATTR(2) MVR_PT_ATTR(4) MVR_PT_ATTR(8) MVR_PT_ATTR(16) MVR_PT_ATTR(32)
 #undef MVR_PT_ATTR
-  e = cudaFuncSetAttribute(rerank_tmem_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tm_smem_bytes(64));
+  e = cudaFuncSetAttribute(rerank_tmem_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmSmem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_tmem_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tm_smem_bytes(64));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_tmem_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tm_smem_bytes(64));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_tmem_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tm_smem_bytes(64));
+  e = cudaFuncSetAttribute(rerank_tmem_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmSmem);
   if (e != cudaSuccess) return e;
 #define MVR_WS_ATTR(NB, NM, F, D)                                                                \
   e = cudaFuncSetAttribute(rerank_ws_kernel<NB, NM, F, D>,                                       \
@@ -2465,6 +2470,14 @@ cudaError_t configure_tc_kernels() {
   // the pruner's feature launch: the default docs per CTA
   MVR_WS_ATTR(2, 32, true, kWsDocs) MVR_WS_ATTR(4, 32, true, kWsDocs)
 #undef MVR_WS_ATTR
+#define MVR_WB_ATTR(NB, D)                                                                       \
+  e = cudaFuncSetAttribute(rerank_ws_kernel<NB, 32, false, D, true>,                             \
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,                          \
+                           (int)ws_smem_bytes(NB, 32, true));                                    \
+  if (e != cudaSuccess) return e;
+  MVR_WB_ATTR(1, 32) MVR_WB_ATTR(1, 64) MVR_WB_ATTR(1, 128)
+  MVR_WB_ATTR(2, 32) MVR_WB_ATTR(2, 64) MVR_WB_ATTR(2, 128)
+#undef MVR_WB_ATTR
   e = cudaFuncSetAttribute(prune_mlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMlpSmem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(rerank_tc_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(8, 64));
@@ -2576,26 +2589,51 @@ cudaError_t make_centroid_perm(const float *cen, uint32_t n_cent, uint32_t n_bit
   return cudaGetLastError();
 }
 
+template <int NB, int DOCS>
+static void wb_launch(const DevIndex &ix, const uint8_t *c, const TmWeights &tw, const float *q,
+                      const uint64_t *q_off, uint32_t n_query, const uint32_t *short_id,
+                      const uint32_t *n_short, uint32_t probe_topk, int semantics, float x_bound,
+                      float *approx, unsigned *err, cudaStream_t st, uint64_t wait_ns) {
+  const dim3 grid((probe_topk + DOCS - 1) / DOCS, n_query);
+  rerank_ws_kernel<NB, 32, false, DOCS, true>
+      <<<grid, ws_threads(32), ws_smem_bytes(NB, 32, true), st>>>(
+          ix, c, tw, q, q_off, short_id, n_short, probe_topk, semantics, x_bound, approx, err,
+          wait_ns);
+}
+
+static uint32_t ws_auto_docs(uint32_t n_query, uint32_t probe_topk, uint32_t slots,
+                             uint32_t widest);
+
 cudaError_t launch_rerank_tmem(const DevIndex &ix, const void *cen_perm, const TmWeights &tw,
                                const float *q, const uint64_t *q_off, uint32_t n_query,
                                const uint32_t *short_id, const uint32_t *n_short,
-                               uint32_t probe_topk, int semantics, uint32_t nq_max, float x_bound,
-                               float *approx, unsigned *err, cudaStream_t st, int *n_launch,
-                               bool fp8) {
-  if (fp8 ? !fp8_rerank_supported(ix.n_bit) : !tmem_rerank_supported(ix.n_bit))
-    return cudaErrorInvalidValue;
+                               uint32_t probe_topk, int semantics, uint32_t nq_min,
+                               uint32_t nq_max, float x_bound, float *approx, unsigned *err,
+                               int n_sm, cudaStream_t st, int *n_launch, uint64_t wait_ns) {
+  if (!tmem_rerank_supported(ix.n_bit)) return cudaErrorInvalidValue;
+  if (nq_min <= 32) {  // the warp-specialised kernel; the rest take rerank_tmem_kernel
+    const uint32_t docs = ws_auto_docs(n_query, probe_topk, 2u * (uint32_t)n_sm, 128u);
+    const uint8_t *c8 = reinterpret_cast<const uint8_t *>(cen_perm);
+#define MVR_WB(NB, D)                                                                            \
+  wb_launch<NB, D>(ix, c8, tw, q, q_off, n_query, short_id, n_short, probe_topk, semantics,      \
+                   x_bound, approx, err, st, wait_ns)
+    if (ix.n_bit == 2) {
+      if (docs == 32) MVR_WB(2, 32); else if (docs == 64) MVR_WB(2, 64); else MVR_WB(2, 128);
+    } else {
+      if (docs == 32) MVR_WB(1, 32); else if (docs == 64) MVR_WB(1, 64); else MVR_WB(1, 128);
+    }
+#undef MVR_WB
+    *n_launch += 1;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || nq_max <= 32) return e;
+  }
   dim3 grid((probe_topk + kTmDocs - 1) / kTmDocs, n_query);
-  const uint32_t n_max = nq_max <= 32 ? 32u : 64u;
-  const size_t sm = tm_smem_bytes(n_max);
   const uint32_t *c = reinterpret_cast<const uint32_t *>(cen_perm);
-#define MVR_TM_LAUNCH(NB, F8)                                                                   \
-  rerank_tmem_kernel<NB, F8><<<grid, kTmThreads, sm, st>>>(ix, c, tw, q, q_off, short_id, n_short, \
-                                                           probe_topk, semantics, n_max, x_bound, \
-                                                           approx, err)
-  if (fp8 && ix.n_bit == 4) MVR_TM_LAUNCH(4, true);
-  else if (fp8) MVR_TM_LAUNCH(2, true);
-  else if (ix.n_bit == 2) MVR_TM_LAUNCH(2, false);
-  else MVR_TM_LAUNCH(1, false);
+#define MVR_TM_LAUNCH(NB)                                                                       \
+  rerank_tmem_kernel<NB><<<grid, kTmThreads, kTmSmem, st>>>(ix, c, tw, q, q_off, short_id, n_short,  \
+                                                       probe_topk, semantics, x_bound, approx, err)
+  if (ix.n_bit == 2) MVR_TM_LAUNCH(2);
+  else MVR_TM_LAUNCH(1);
 #undef MVR_TM_LAUNCH
   *n_launch += 1;
   return cudaGetLastError();

@@ -24,10 +24,12 @@ struct TmWeights {
 };
 TmWeights make_tm_weights(uint32_t n_bit, const float *weight, bool fp8);
 
-// BF16 MaxSim with the decoded doc tokens in tensor memory (1- and 2-bit
-// codes); cen_perm: [C][64] bf16x2 centroid rows in the kernel's K order
+// BF16 MaxSim of 1- and 2-bit codes on the tensor cores; cen_perm: [C + 1][64]
+// bf16x2 centroid rows in the kernels' K order, the last zero
 // (make_centroid_perm); x_bound: upper bound on the norm of every decoded
-// doc token
+// doc token.  Queries of up to kBf16SplitTok tokens: BF16 centroid and BF16
+// weights contribute separately; longer ones: their BF16-rounded sum.
+constexpr uint32_t kBf16SplitTok = 32;
 bool tmem_rerank_supported(uint32_t n_bit);
 // largest L2 norm of the centroid rows (d_tmp: one device word of scratch)
 cudaError_t max_centroid_norm(const float *cen, uint32_t n_cent, unsigned *d_tmp, float *out,
@@ -37,17 +39,15 @@ cudaError_t make_centroid_perm(const float *cen, uint32_t n_cent, uint32_t n_bit
 cudaError_t launch_rerank_tmem(const DevIndex &ix, const void *cen_perm, const TmWeights &tw,
                                const float *q, const uint64_t *q_off, uint32_t n_query,
                                const uint32_t *short_id, const uint32_t *n_short,
-                               uint32_t probe_topk, int semantics, uint32_t nq_max, float x_bound,
-                               float *approx, unsigned *err, cudaStream_t st, int *n_launch,
-                               bool fp8);
-// FP8 (E4M3) MaxSim for 2- and 4-bit codes: cen8 [C][128] E4M3 centroid
-// rows in the FP8 kernel's K order for n_bit (make_centroid_fp8); pass it as
-// cen_perm with fp8 = true
+                               uint32_t probe_topk, int semantics, uint32_t nq_min,
+                               uint32_t nq_max, float x_bound, float *approx, unsigned *err,
+                               int n_sm, cudaStream_t st, int *n_launch, uint64_t wait_ns);
+// E4M3 centroid rows [C][128] in the FP8 kernel's K order (2- and 4-bit codes)
 bool fp8_rerank_supported(uint32_t n_bit);
 cudaError_t make_centroid_fp8(const float *cen, uint32_t n_cent, uint32_t n_bit, void *out,
                               cudaStream_t st);
 
-// The same FP8 MaxSim, warp-specialised (producer / decoders / MMA / epilogue
+// FP8 (E4M3) MaxSim, warp-specialised (producer / decoders / MMA / epilogue
 // over a shared-memory ring fed by bulk copies): cen8 as above with one zero
 // row appended (row n_centroid); the vq code array must be readable 16 bytes
 // past its last code.  wait_ns bounds every pipeline wait of the kernel (on

@@ -237,3 +237,30 @@ def test_bf16_rescore_cut(n_bit):
                         s1, i1 = g.search(qq, k, 8, ptk, tok_off=off, semantics=sem | PREC_BF16)
                         np.testing.assert_array_equal(i1, i0)
                         np.testing.assert_array_equal(s1, s0)
+
+
+@pytest.mark.parametrize("n_bit", [1, 2])
+@pytest.mark.parametrize("n_query,width", [(1, (32, 32)), (3, (1, 31)), (6, (30, 36)), (150, (1, 32))])
+def test_bf16_maxsim_edges(n_bit, n_query, width):
+    """The BF16 MaxSim at its docs per CTA, doc lengths around its 128-token tiles and
+    query widths around its 32 columns: the k docs it picks have, one by one, exact
+    scores within twice the BF16 error of the exact k best.  With |x| <= X = max |c| +
+    sqrt(128) max |w|, rounding q, c and w to BF16 (2^-9 each) moves a dot product by at
+    most 2^-8 |q| X, rounding a sum c + w by as much again; 2^-11 covers the products
+    of these and the FP32 accumulation from an offset of up to 4 |q| X."""
+    lengths = (LENGTHS * 20)[:300]
+    ix = tiny_index(n_doc=300, n_centroid=48, n_bit=n_bit, seed=90 + n_bit, lengths=lengths)
+    q, off = make_queries(ix, n_query, width, seed=6)
+    X = np.linalg.norm(ix["centroid"], axis=1).max() + np.sqrt(128) * np.abs(ix["weight"]).max()
+    o, k = oracle_of(ix), 20
+    with gpu_index(ix) as g:
+        g.set_rescore(k)  # the BF16 pass alone chooses
+        for ptk in (20, 129, 300):
+            want = o.search(q, off, k, 8, ptk, SEM_PP)[0]
+            got, ids = g.search(q, k, 8, ptk, tok_off=off, semantics=SEM_PP | PREC_BF16)
+            for b in range(n_query):
+                n = np.linalg.norm(q[int(off[b]):int(off[b + 1])].astype(np.float64), axis=1).sum()
+                assert len(set(ids[b])) == k
+                assert (got[b] >= want[b] - 2 * n * X * (2.0**-7 + 2.0**-11)).all()
+                if ptk == k:
+                    np.testing.assert_array_equal(got[b], want[b])
