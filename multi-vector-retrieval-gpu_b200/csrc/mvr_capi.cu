@@ -163,11 +163,10 @@ struct mvr_index {
   std::vector<cudaEvent_t> copy_events, done_events;  // ... and one when its kernels are done
   uint32_t batch_cap = 0;
   uint32_t rescore = 0;          // FP32 re-score count of the BF16 path (0: 4 * topk)
-  void *cen_bf16 = nullptr;      // [C][128] BF16 centroid rows
-  void *lut_bf16 = nullptr;      // [256][8/b] BF16 decode table
+  void *lut_bf16 = nullptr;      // [256][8/b] BF16 decode table (b >= 4)
   void *cen_sw = nullptr;        // [C_pad/128][32 KB] swizzled BF16 centroid tiles
   float *cen_bounds = nullptr;   // max |c|, max |c - bf16(c)| over the centroids
-  void *cen_perm = nullptr;      // [C + 1][64] bf16x2 centroid rows, BF16 K order (b <= 2)
+  void *cen_perm = nullptr;      // [C + 1][128] BF16 centroid rows, BF16 K order
   TmWeights tw_bf16{};           // weight tables of the BF16 tensor-memory MaxSim (b <= 2)
   float x_bound = 0.f;           // bound on the norm of every decoded doc token
   float w_norm = 0.f, w_err = 0.f;  // ... of a token's weights, of their BF16 rounding errors
@@ -577,20 +576,23 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     if (!h->prune_wts) return set_err(MVR_ERR_INVALID_ARG, "MVR_PRUNE: no pruner set");
     if (nq_max > 32) return set_err(MVR_ERR_UNSUPPORTED, "MVR_PRUNE: queries of up to 32 tokens");
   }
-  // Exact FP32 search of 1- and 2-bit codes: where a shortlist is long, the BF16
-  // pass first leaves out the docs that provably miss the top topk, and the FP32
-  // kernel scores the rest (50 of 1500 on average for the best 10).  The line: at 22
-  // and 4.8 docs' tokens per ns the pass pays for itself once it spares a fourth
-  // of the FP32 work, which takes a shortlist of 4 topk; its launches take 60 us,
-  // the FP32 work of 7,000 docs, and its CTAs of 32 to 128 docs want a grid that
-  // fills the GPU: 32,768 docs.  Queries of up to 16
-  // tokens take the FP32 kernel's half-width body, at twice its rate.  The wider
-  // codes' BF16 kernel is no faster than the FP32 one (4.9 tokens per ns at 8 bits).
-  const bool reach = !bf16 && !prune && !all_exact && h->cen_perm && nq_max > 16 &&
+  // Exact FP32 search: where a shortlist is long, the BF16 pass first leaves out the
+  // docs that provably miss the top topk, and the FP32 kernel scores the rest.  The
+  // line: at 22 and 4.8 docs' tokens per ns (2 bits; 8.6 and 3.1 at 8 bits) the pass
+  // pays for itself once it spares a third of the FP32 work, which takes a shortlist
+  // of 4 topk; its launches take 60 us, the FP32 work of 7,000 docs, and its CTAs of
+  // 32 to 128 docs want a grid that fills the GPU: 32,768 docs.  Queries of up to 16
+  // tokens take the FP32 kernel's half-width body, at twice its rate; 4- and 8-bit
+  // codes have no faster BF16 kernel for more than 32 tokens (4.9 tokens per ns at 8
+  // bits).  200 queries x 400 docs at 8 bits: 1.80 -> 1.45 ms.
+  const bool reach = !bf16 && !prune && !all_exact && nq_max > 16 &&
+                     (h->dix.n_bit <= 2 || (nq_max <= kBf16SplitTok &&
+                                            bf16_split_supported(h->dix.n_bit, h->x_bound))) &&
                      probe_topk / 4 >= topk &&
                      (uint64_t)std::min(h->batch_cap ? h->batch_cap : default_batch(h), n_query) *
                              probe_topk >= 32768;
   if (reach) R = probe_topk;
+  const uint32_t split_tok = bf16_split_supported(h->dix.n_bit, h->x_bound) ? kBf16SplitTok : 0u;
   // the BF16 path's best R: the same bound leaves out those of them that miss the
   // top topk (FP8's own error is an order larger and would leave out none).  400 docs
   // of each of 500 queries for the best 100: 3.26 -> 1.42 ms of FP32 work for 16 us.
@@ -799,14 +801,10 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
           CUDA_TRY(launch_rerank_ws(h->dix, h->cen8, h->tw_fp8, qp, qo, nb, sid, nsh,
                                     probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact, h->d_err,
                                     h->n_sm, rs, &launches, h->wait_ns, h->ws_docs));
-        else if (h->cen_perm)
-          CUDA_TRY(launch_rerank_tmem(h->dix, h->cen_perm, h->tw_bf16, qp, qo, nb, sid, nsh,
-                                      probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact,
-                                      h->d_err, h->n_sm, rs, &launches, h->wait_ns));
         else
-          CUDA_TRY(launch_rerank_tc(h->dix, h->cen_bf16, h->lut_bf16, qp, qo, nb, w.short_id,
-                                    w.n_short, probe_topk, sem, nq_max, w.exact, h->d_err, rs,
-                                    &launches));
+          CUDA_TRY(launch_rerank_bf16(h->dix, h->cen_perm, h->lut_bf16, h->tw_bf16, qp, qo, nb, sid,
+                                      nsh, probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact,
+                                      h->d_err, h->n_sm, rs, &launches, h->wait_ns));
         CUDA_TRY(rec(ev(bt, 4)));
         CUDA_TRY(launch_topk(sid, w.exact, nsh, nb, probe_topk, R, w.r_score, w.r_id, w.n_r, rs,
                              &launches));
@@ -814,7 +812,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         if (cut_r) {
           CUDA_TRY(launch_maxsim_reach(qp, qo, nb, w.r_id, w.r_score, w.n_r, R, topk,
                                        h->cen_bounds, h->w_norm, h->w_err,
-                                       h->cen_perm ? kBf16SplitTok : 0u, w.r2_id, w.n_r2, rs,
+                                       split_tok, w.r2_id, w.n_r2, rs,
                                        &launches));
           rid = w.r2_id;
           nr = w.n_r2;
@@ -841,11 +839,11 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
           nsh = w.n_fin;
         }
         if (reach) {
-          CUDA_TRY(launch_rerank_tmem(h->dix, h->cen_perm, h->tw_bf16, qp, qo, nb, sid, nsh,
-                                      probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact,
+          CUDA_TRY(launch_rerank_bf16(h->dix, h->cen_perm, h->lut_bf16, h->tw_bf16, qp, qo, nb, sid,
+                                      nsh, probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact,
                                       h->d_err, h->n_sm, rs, &launches, h->wait_ns));
           CUDA_TRY(launch_maxsim_reach(qp, qo, nb, sid, w.exact, nsh, probe_topk, topk,
-                                       h->cen_bounds, h->w_norm, h->w_err, kBf16SplitTok, w.r_id, w.n_r, rs,
+                                       h->cen_bounds, h->w_norm, h->w_err, split_tok, w.r_id, w.n_r, rs,
                                        &launches));
           CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, w.r_id, w.n_r, probe_topk, sem, w.r_exact,
                                  h->n_sm, rs, &launches, 32));
@@ -1022,13 +1020,12 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
   MVR_TRY(dalloc(&dl, lut.size(), &h->bufs));
   CUDA_TRY(cudaMemcpy(dl, lut.data(), lut.size() * sizeof(float), cudaMemcpyHostToDevice));
   d.lut = dl;
-  uint16_t *cb, *lb;
-  MVR_TRY(dalloc(&cb, (size_t)d.n_centroid * kDim, &h->bufs));
-  MVR_TRY(dalloc(&lb, lut.size(), &h->bufs));
-  CUDA_TRY(make_bf16(d.centroid, (size_t)d.n_centroid * kDim, cb, h->stream));
-  CUDA_TRY(make_bf16(dl, lut.size(), lb, h->stream));
-  h->cen_bf16 = cb;
-  h->lut_bf16 = lb;
+  if (d.n_bit >= 4) {
+    uint16_t *lb;
+    MVR_TRY(dalloc(&lb, lut.size(), &h->bufs));
+    CUDA_TRY(make_bf16(dl, lut.size(), lb, h->stream));
+    h->lut_bf16 = lb;
+  }
   uint8_t *sw;
   MVR_TRY(dalloc(&sw, (size_t)d.n_centroid_pad * 256, &h->bufs));
   CUDA_TRY(make_centroid_tiles(d.centroid, d.n_centroid, d.n_centroid_pad / 64, sw, h->stream));
@@ -1041,7 +1038,7 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
     h->w_norm = std::max(h->w_norm, std::isfinite(weight[k]) ? root * std::fabs(weight[k]) : INFINITY);
     h->w_err = std::max(h->w_err, std::isfinite(e) ? root * e : INFINITY);
   }
-  if (tmem_rerank_supported(d.n_bit) || fp8_rerank_supported(d.n_bit)) {
+  {
     float wmax = 0.f;
     for (uint32_t k = 0; k < (1u << d.n_bit); k++) wmax = std::max(wmax, std::fabs(weight[k]));
     float cmax = 0.f;
@@ -1049,13 +1046,11 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
     CUDA_TRY(cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), h->stream));  // was scratch
     h->x_bound = cmax + std::sqrt((float)kDim) * wmax;
   }
-  if (tmem_rerank_supported(d.n_bit)) {
-    uint32_t *cp;
-    MVR_TRY(dalloc(&cp, ((size_t)d.n_centroid + 1) * 64, &h->bufs));
-    CUDA_TRY(make_centroid_perm(d.centroid, d.n_centroid, d.n_bit, cp, h->stream));
-    h->cen_perm = cp;
-    h->tw_bf16 = make_tm_weights(d.n_bit, weight, false);
-  }
+  uint32_t *cp;
+  MVR_TRY(dalloc(&cp, ((size_t)d.n_centroid + 1) * 64, &h->bufs));
+  CUDA_TRY(make_centroid_perm(d.centroid, d.n_centroid, d.n_bit, cp, h->stream));
+  h->cen_perm = cp;
+  h->tw_bf16 = make_tm_weights(d.n_bit, weight, false);
   if (fp8_rerank_supported(d.n_bit)) {
     uint8_t *c8;
     // one zero row past the last centroid: the FP8 rerank's padding rows

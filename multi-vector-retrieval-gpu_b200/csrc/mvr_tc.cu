@@ -1,7 +1,8 @@
 // mvr_tc.cu -- tensor-core (tcgen05, sm_100a) MaxSim for the mixed-precision
 // search path.
 //
-// rerank_tc_kernel scores a query's shortlisted docs with BF16 operands and
+// rerank_tc_kernel scores a query's shortlisted docs (4- and 8-bit codes, queries of
+// more than 32 tokens, or weights too large for the split form) with BF16 operands and
 // FP32 accumulation in TMEM: per 128-token tile the CTA decompresses doc tokens
 // x = centroid + W[bucket] (BF16 centroid table + BF16 decode table, one BF16
 // add) straight into a 128B-swizzled K-major shared-memory tile (operand A,
@@ -109,35 +110,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 // per-byte decode-table rows (VPB BF16 weights per residual byte).
 template <int NBIT>
 __device__ __forceinline__ uint4 decode_chunk(uint4 cen, const uint8_t *rb,
-                                              const __nv_bfloat16 *lut, const uint32_t *nib,
-                                              int lane) {
+                                              const __nv_bfloat16 *lut) {
   constexpr int VPB = 8 / NBIT;
   uint32_t w[4];
-  if constexpr (NBIT == 2) {         // 2 bytes = 4 nibbles -> 4 x (2 weights)
-    // nib[(nibble * 32 + lane)]: bf16x2 of the nibble's two codes, one copy
-    // per lane so that the 32 lanes read 32 different banks
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t byte = rb[u >> 1];
-      const uint32_t nb = (u & 1) ? (byte & 0xfu) : (byte >> 4);
-      w[u] = nib[nb * 32 + lane];
-    }
-  } else if constexpr (NBIT == 1) {  // 1 byte = 2 nibbles -> 2 x (4 weights)
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const uint32_t nb = u ? (rb[0] & 0xfu) : (rb[0] >> 4);
-      const uint2 t = reinterpret_cast<const uint2 *>(nib)[nb * 32 + lane];
-      w[2 * u] = t.x;
-      w[2 * u + 1] = t.y;
-    }
-  } else if constexpr (VPB == 8) {   // (unused) 1 byte -> 8 weights
-    const uint4 t = *reinterpret_cast<const uint4 *>(lut + rb[0] * 8);
-    w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
-  } else if constexpr (VPB == 4) {   // 2 bytes -> 2 x 4 weights
-    const uint2 t0 = *reinterpret_cast<const uint2 *>(lut + rb[0] * 4);
-    const uint2 t1 = *reinterpret_cast<const uint2 *>(lut + rb[1] * 4);
-    w[0] = t0.x; w[1] = t0.y; w[2] = t1.x; w[3] = t1.y;
-  } else if constexpr (VPB == 2) {   // 4 bytes -> 4 x 2 weights
+  if constexpr (VPB == 2) {          // 4 bytes -> 4 x 2 weights
 #pragma unroll
     for (int u = 0; u < 4; u++) w[u] = *reinterpret_cast<const uint32_t *>(lut + rb[u] * 2);
   } else {                           // 8 bytes -> 8 x 1 weight
@@ -161,7 +137,7 @@ __device__ __forceinline__ uint4 decode_chunk(uint4 cen, const uint8_t *rb,
 // Dynamic shared memory of rerank_tc_kernel for a query-token tile of N rows.
 __host__ __device__ constexpr size_t tc_smem_bytes(int nbit, uint32_t n) {
   return 1024 + 32768 /*A*/ + (size_t)n * 256 /*B*/ + 64 * kTcDocs * 4 /*best*/ +
-         (nbit <= 2 ? 16 * 32 * 4 * (nbit == 1 ? 2 : 1) : 256 * (8 / nbit) * 2) /*decode table*/;
+         256 * (8 / nbit) * 2 /*decode table*/;
 }
 
 template <int NBIT>
@@ -170,7 +146,9 @@ rerank_tc_kernel(DevIndex ix, const __nv_bfloat16 *__restrict__ cen_bf16,
                  const __nv_bfloat16 *__restrict__ lut_bf16, const float *__restrict__ q,
                  const uint64_t *__restrict__ q_off, const uint32_t *__restrict__ short_id,
                  const uint32_t *__restrict__ n_short, uint32_t probe_topk, int semantics,
-                 uint32_t n_max, float *__restrict__ approx, unsigned *__restrict__ err) {
+                 uint32_t n_max, uint32_t nq_skip, float *__restrict__ approx,
+                 unsigned *__restrict__ err) {
+  static_assert(NBIT == 4 || NBIT == 8, "4- and 8-bit codes");
   constexpr int VPB = 8 / NBIT;
   constexpr int HALF_BYTES = 64 / VPB;  // residual bytes of 64 dims
   constexpr int NRW = HALF_BYTES / 8;   // uint2 words per half row
@@ -179,8 +157,7 @@ rerank_tc_kernel(DevIndex ix, const __nv_bfloat16 *__restrict__ cen_bf16,
   uint8_t *Ad = smem;                                          // [2 K-blocks][128 rows][128 B]
   uint8_t *Bq = smem + 32768;                                  // [2 K-blocks][n_max rows][128 B]
   int *best = reinterpret_cast<int *>(Bq + n_max * 256);       // [64][kTcDocs]
-  uint32_t *nib = reinterpret_cast<uint32_t *>(best + 64 * kTcDocs);  // b<=2: [16][32](x2)
-  __nv_bfloat16 *lut = reinterpret_cast<__nv_bfloat16 *>(nib);        // b>=4: [256][VPB]
+  __nv_bfloat16 *lut = reinterpret_cast<__nv_bfloat16 *>(best + 64 * kTcDocs);  // [256][VPB]
   __shared__ uint64_t bar;
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t d_len[kTcDocs], d_pref[kTcDocs + 1];
@@ -192,10 +169,12 @@ rerank_tc_kernel(DevIndex ix, const __nv_bfloat16 *__restrict__ cen_bf16,
   const uint32_t b = blockIdx.y;
   const uint32_t ns = n_short[b];
   const uint32_t d0 = blockIdx.x * kTcDocs;
-  if (d0 >= ns) return;  // uniform: before any TMEM / barrier use
-  const uint32_t nd = min((uint32_t)kTcDocs, ns - d0);
   const uint64_t tok0 = q_off[b];
   const uint32_t nq = (uint32_t)(q_off[b + 1] - tok0);
+  // uniform exits before any TMEM or barrier use: no docs here, or a query of
+  // the warp-specialised kernel
+  if (d0 >= ns || nq <= nq_skip) return;
+  const uint32_t nd = min((uint32_t)kTcDocs, ns - d0);
   const uint32_t N = nq <= 32 ? 32u : 64u;  // <= n_max (host sizes smem by the batch)
   const uint32_t idesc = idesc_bf16(kTcTile, (int)N);
 
@@ -215,23 +194,7 @@ rerank_tc_kernel(DevIndex ix, const __nv_bfloat16 *__restrict__ cen_bf16,
     d_len[tid] = ix.item_n_vec[it];
     d_off[tid] = ix.item_off[it];
   }
-  if constexpr (NBIT <= 2) {
-    // nibble n is the top nibble of byte (n << 4): its codes' weights are the
-    // first 4 / NBIT entries of that byte's decode-table row; one copy per
-    // lane so the 32 lanes of a warp read 32 different banks
-    for (int i = tid; i < 16 * 32; i += kTcThreads) {
-      const int n = i >> 5, ln = i & 31;
-      const uint16_t *row = reinterpret_cast<const uint16_t *>(lut_bf16) + (n << 4) * VPB;
-      if constexpr (NBIT == 2) {
-        nib[n * 32 + ln] = (uint32_t)row[0] | ((uint32_t)row[1] << 16);
-      } else {
-        reinterpret_cast<uint2 *>(nib)[n * 32 + ln] =
-            make_uint2((uint32_t)row[0] | ((uint32_t)row[1] << 16), (uint32_t)row[2] | ((uint32_t)row[3] << 16));
-      }
-    }
-  } else {
-    for (int i = tid; i < 256 * VPB; i += kTcThreads) lut[i] = lut_bf16[i];
-  }
+  for (int i = tid; i < 256 * VPB; i += kTcThreads) lut[i] = lut_bf16[i];
   for (int i = tid; i < 64 * kTcDocs; i += kTcThreads) best[i] = f2si(-INFINITY);
   // query tokens -> B operand (BF16, swizzled, rows >= nq zero)
   for (int i = tid; i < (int)N * 16; i += kTcThreads) {
@@ -323,7 +286,7 @@ rerank_tc_kernel(DevIndex ix, const __nv_bfloat16 *__restrict__ cen_bf16,
 #pragma unroll
       for (int c = 0; c < 8; c++)
         *reinterpret_cast<uint4 *>(kb + sw128_off(row, c)) =
-            decode_chunk<NBIT>(__ldg(cen + c), rb + c * (8 / VPB), lut, nib, lane);
+            decode_chunk<NBIT>(__ldg(cen + c), rb + c * (8 / VPB), lut);
     } else {
 #pragma unroll
       for (int c = 0; c < 8; c++) *reinterpret_cast<uint4 *>(kb + sw128_off(row, c)) = make_uint4(0, 0, 0, 0);
@@ -398,6 +361,7 @@ constexpr uint32_t kTmCols = 512; // TMEM columns: A[2] x 64 + D[3] x 64, so one
 
 template <int NBIT>
 __host__ __device__ constexpr uint32_t tm_dim_of(uint32_t kappa) {
+  if (NBIT >= 4) return kappa;
   constexpr uint32_t VPB = 8 / NBIT, WD = 4 * VPB;
   const uint32_t m = kappa / WD, r = kappa % WD;
   return m * WD + VPB * (r % 4) + r / 4;
@@ -1609,10 +1573,11 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 // FEAT the kernel computes the learned pruner's features instead: the
 // centroid part only (no producer, residual decode or residual MMA), and
 // per doc the maxima themselves (per query token the best centroid score
-// over the doc's tokens) plus log(doc length).  With BF (1- and 2-bit codes)
-// centroid rows, weights and query are BF16: rows of 256 bytes in two A_c
+// over the doc's tokens) plus log(doc length).  With BF (codes of any
+// width) centroid rows, weights and query are BF16: rows of 256 bytes in two A_c
 // stages, 64 A_r columns, 8 K-steps of K = 16 (kind::f16), A_e = 1 and OFF in K
-// position 0 of B_e.  The sum c + W[b] is not rounded.  Every pipeline mbarrier wait
+// position 0 of B_e; 4- and 8-bit codes look their weights up in shared memory.  The
+// sum c + W[b] is not rounded.  Every pipeline mbarrier wait
 // is bounded (wait_ns, 1 s by default); on a timeout the CTA records the
 // error and every role stops; the producer then waits (1 s bound) for its
 // bulk copies still in flight and the MMA thread for its MMAs before TMEM
@@ -1626,7 +1591,8 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 // N = 32 (72 registers a thread): 8.9 ms; three CTAs per SM with one A_r stage: 10.8
 // ms; the maxima written by one lane's 32 atomics instead of 32 selects: 8.4 ms.
 // BF against rerank_tmem_kernel at 32 columns: 400 queries x 1500 docs at 2 bits 3.13
-// -> 1.96 ms (21.6 tokens per ns), 500 x 1400 at 1 bit 3.25 -> 2.24 ms.
+// -> 1.96 ms (21.6 tokens per ns), 500 x 1400 at 1 bit 3.25 -> 2.24 ms.  At 8 bits, 128
+// table reads a token in shared memory: 8.6 tokens per ns, rerank_tc_kernel 4.9.
 // ---------------------------------------------------------------------
 constexpr int kWsDocs = 256;         // shortlisted docs per CTA (default; 32, 64, 128 or 256)
 // epilogue warps per 32 rows: the 64-column variant splits the columns in two
@@ -1642,14 +1608,24 @@ __host__ __device__ constexpr int ws_cstages(bool bf) { return kWsAStages + (bf 
 __host__ __device__ constexpr int ws_dstages(int nmax) { return nmax <= 32 ? 3 : 2; }
 constexpr uint32_t kWsCols = 256;    // TMEM columns of a CTA
 // ring stages of residual bytes: 4, or the 2 that two CTAs leave room for at 4 bits
-__host__ __device__ constexpr int ws_rstages(int nbit) { return nbit == 4 ? 2 : 4; }
+// (8 bits: 1, released as soon as a tile's rows are in registers)
+__host__ __device__ constexpr int ws_rstages(int nbit) {
+  return nbit == 8 ? 1 : nbit == 4 ? 2 : 4;
+}
+// BF16 weights of 4- and 8-bit codes by residual byte (4 bits: the byte's two weights
+// in one word), kWsLutCopies interleaved copies, so that the 4 lanes that share a copy
+// meet 4 banks of their own
+constexpr uint32_t kWsLutCopies = 8;
+__host__ __device__ constexpr size_t ws_lut_bytes(int nbit, bool bf) {
+  return bf && nbit >= 4 ? 256 * 4 * kWsLutCopies : 0;
+}
 __host__ __device__ constexpr uint32_t ws_stage_bytes(int nbit) { return 128u * (128u * nbit / 8u); }
 __host__ __device__ constexpr uint32_t ws_crow(bool bf) { return bf ? 256u : 128u; }  // A_c bytes a row
 // dynamic shared memory: 1 KB alignment slack + query tile + bias tile + A_c
 // stages + ring
 __host__ __device__ constexpr size_t ws_smem_bytes(int nbit, int nmax, bool bf = false) {
   return 1024 + (size_t)nmax * (ws_crow(bf) + 128) + ws_cstages(bf) * (size_t)(128 * ws_crow(bf)) +
-         ws_rstages(nbit) * (size_t)ws_stage_bytes(nbit);
+         ws_rstages(nbit) * (size_t)ws_stage_bytes(nbit) + ws_lut_bytes(nbit, bf);
 }
 
 // the same word into 8 consecutive TMEM columns of the warp's 32 lanes
@@ -1687,8 +1663,10 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen_rows, TmWeights tw
                  const uint32_t *__restrict__ short_id, const uint32_t *__restrict__ n_short,
                  uint32_t probe_topk, int semantics, float x_bound, float *__restrict__ approx,
                  unsigned *__restrict__ err, uint64_t wait_ns) {
-  static_assert(BF ? NBIT <= 2 && NMAX == 32 && !FEAT && DOCS <= 128 : NBIT == 2 || NBIT == 4,
-                "FP8 decodes 2- and 4-bit codes, BF16 1- and 2-bit ones");
+  static_assert(BF || NBIT == 2 || NBIT == 4, "FP8 decodes 2- and 4-bit codes");
+  static_assert(!BF || (NMAX == 32 && !FEAT && DOCS <= (NBIT <= 2 ? 128 : 64)),
+                "BF16: up to 32 columns, docs per CTA that leave room for two CTAs");
+  constexpr bool LUT = BF && NBIT >= 4;  // bucket weights from a table in shared memory
   static_assert(NMAX == 32 || NMAX == 64, "query tiles of 32 or 64 rows");
   static_assert(!FEAT || NMAX == 32, "pruner features: queries of up to 32 tokens");
   static_assert(DOCS == 32 || DOCS == 64 || ((DOCS == 128 || DOCS == 256) && NMAX == 32),
@@ -1710,6 +1688,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen_rows, TmWeights tw
   uint8_t *Be = smem + NMAX * CROW;       // bias B operand, [NMAX rows][128 B]
   uint8_t *Ac = Be + NMAX * 128;          // [SC] x 128 centroid rows
   uint8_t *ring = Ac + SC * CSTAGE;       // [S][128 rows][BPV] residual bytes
+  uint32_t *lut = reinterpret_cast<uint32_t *>(ring + S * STAGE);  // LUT: [256][kWsLutCopies]
   __shared__ uint32_t best[DOCS * NMAX];  // [doc][query token]: bits of OFF + max
   __shared__ uint32_t s_qss, tmem_base_s;
   __shared__ float s_qinv[NMAX];
@@ -1750,6 +1729,19 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen_rows, TmWeights tw
     d_off[tid] = ix.item_off[it];
   }
   for (int i = tid; i < DOCS * NMAX; i += ws_threads(NMAX)) best[i] = 0u;
+  if constexpr (LUT) {
+    for (int i = tid; i < 256 * (int)kWsLutCopies; i += ws_threads(NMAX)) {
+      const uint32_t byte = (uint32_t)i / kWsLutCopies;
+      __nv_bfloat162 w;
+      if constexpr (NBIT == 4) {
+        const float2 t = __ldg(reinterpret_cast<const float2 *>(ix.lut) + byte);
+        w = __floats2bfloat162_rn(t.x, t.y);
+      } else {
+        w = __floats2bfloat162_rn(__ldg(ix.lut + byte), 0.0f);
+      }
+      lut[i] = *reinterpret_cast<uint32_t *>(&w);
+    }
+  }
   __syncthreads();
   if (warp == 0) {  // token offsets of the docs within the CTA (warp scan)
     uint32_t carry = 0;
@@ -1995,7 +1987,8 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen_rows, TmWeights tw
     // wavefront's 8 lanes (rows) start in 4 (2-bit) or 2 (4-bit) bank groups
     const uint32_t rot = NBIT == 1   ? 0u
                          : NBIT == 2 ? ((uint32_t)lane >> 2) & 1u
-                                     : ((uint32_t)lane >> 1) & 3u;
+                         : NBIT == 4 ? ((uint32_t)lane >> 1) & 3u
+                                     : (uint32_t)lane & 7u;
     bool ok = true;
     for (uint32_t i = 0; ok && i < n_tiles; i++) {
       const uint32_t s = i % S, sa = i % SA;
@@ -2045,8 +2038,29 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen_rows, TmWeights tw
           res[4 * u + 2] = t[u].z;
           res[4 * u + 3] = t[u].w;
         }
+        if constexpr (NBIT == 8) {  // the one stage goes back before the decode
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sfree[s]);
+        }
         uint32_t out[16];
-        if constexpr (BF) {
+        if constexpr (LUT) {
+          const uint32_t *lp = lut + ((uint32_t)lane & (kWsLutCopies - 1u));
+          auto at = [&](uint32_t byte) { return lp[(byte & 0xffu) * kWsLutCopies]; };
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+#pragma unroll
+            for (int u = 0; u < 16; u++) {  // column: dims 2j, 2j + 1
+              const int j = 16 * k + u;
+              if constexpr (NBIT == 4) {
+                out[u] = at(res[j >> 2] >> (8 * (j & 3)));
+              } else {
+                const uint32_t x = res[j >> 1] >> (16 * (j & 1));
+                out[u] = prmt(at(x), at(x >> 8), 0x5410u);
+              }
+            }
+            tmem_st16(acol + 16u * k, out);
+          }
+        } else if constexpr (BF) {
 #pragma unroll
           for (int k = 0; k < 4; k++) {
             tm_weights16<NBIT>(res + k * (int)(BPV / 16), tw.w[0], tw.w[1], out);
@@ -2078,7 +2092,7 @@ rerank_ws_kernel(DevIndex ix, const uint8_t *__restrict__ cen_rows, TmWeights tw
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&afull[sa]);
-        if constexpr (!FEAT) mbar_arrive(&sfree[s]);
+        if constexpr (!FEAT && NBIT != 8) mbar_arrive(&sfree[s]);
       }
       if constexpr (BF) {  // tile i + 1's stage: the MMAs of tile i - 1 done
         if (ok && i + 1 < n_tiles) {
@@ -2442,10 +2456,6 @@ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 cudaError_t configure_tc_kernels() {
   cudaError_t e;
-  e = cudaFuncSetAttribute(rerank_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(1, 64));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(2, 64));
-  if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rerank_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(4, 64));
   if (e != cudaSuccess) return e;
 #define MVR_PT_ATTR(KK)                                                                         \
@@ -2477,34 +2487,18 @@ cudaError_t configure_tc_kernels() {
   if (e != cudaSuccess) return e;
   MVR_WB_ATTR(1, 32) MVR_WB_ATTR(1, 64) MVR_WB_ATTR(1, 128)
   MVR_WB_ATTR(2, 32) MVR_WB_ATTR(2, 64) MVR_WB_ATTR(2, 128)
+  MVR_WB_ATTR(4, 32) MVR_WB_ATTR(4, 64) MVR_WB_ATTR(8, 32) MVR_WB_ATTR(8, 64)
 #undef MVR_WB_ATTR
   e = cudaFuncSetAttribute(prune_mlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMlpSmem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(rerank_tc_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(8, 64));
 }
 
-cudaError_t launch_rerank_tc(const DevIndex &ix, const void *cen_bf16, const void *lut_bf16,
-                             const float *q, const uint64_t *q_off, uint32_t n_query,
-                             const uint32_t *short_id, const uint32_t *n_short,
-                             uint32_t probe_topk, int semantics, uint32_t nq_max, float *approx,
-                             unsigned *err, cudaStream_t st, int *n_launch) {
-  dim3 grid((probe_topk + kTcDocs - 1) / kTcDocs, n_query);
-  const uint32_t n_max = nq_max <= 32 ? 32u : 64u;
-  const size_t sm = tc_smem_bytes((int)ix.n_bit, n_max);
-  const __nv_bfloat16 *c = reinterpret_cast<const __nv_bfloat16 *>(cen_bf16);
-  const __nv_bfloat16 *l = reinterpret_cast<const __nv_bfloat16 *>(lut_bf16);
-  switch (ix.n_bit) {
-    case 1: rerank_tc_kernel<1><<<grid, kTcThreads, sm, st>>>(ix, c, l, q, q_off, short_id, n_short, probe_topk, semantics, n_max, approx, err); break;
-    case 2: rerank_tc_kernel<2><<<grid, kTcThreads, sm, st>>>(ix, c, l, q, q_off, short_id, n_short, probe_topk, semantics, n_max, approx, err); break;
-    case 4: rerank_tc_kernel<4><<<grid, kTcThreads, sm, st>>>(ix, c, l, q, q_off, short_id, n_short, probe_topk, semantics, n_max, approx, err); break;
-    case 8: rerank_tc_kernel<8><<<grid, kTcThreads, sm, st>>>(ix, c, l, q, q_off, short_id, n_short, probe_topk, semantics, n_max, approx, err); break;
-    default: return cudaErrorInvalidValue;
-  }
-  *n_launch += 1;
-  return cudaGetLastError();
+// 4- and 8-bit codes: the offset that the split kernel's accumulators start at stays
+// finite for queries of any norm up to 2^66
+bool bf16_split_supported(uint32_t n_bit, float x_bound) {
+  return n_bit <= 2 || x_bound < 0x1p60f;
 }
-
-bool tmem_rerank_supported(uint32_t n_bit) { return n_bit == 1 || n_bit == 2; }
 bool fp8_rerank_supported(uint32_t n_bit) { return n_bit == 2 || n_bit == 4; }
 
 TmWeights make_tm_weights(uint32_t n_bit, const float *weight, bool fp8) {
@@ -2585,6 +2579,8 @@ cudaError_t make_centroid_perm(const float *cen, uint32_t n_cent, uint32_t n_bit
   uint32_t *o = reinterpret_cast<uint32_t *>(out);
   if (n_bit == 2) perm_centroid_kernel<2><<<592, 256, 0, st>>>(cen, n_cent, o);
   else if (n_bit == 1) perm_centroid_kernel<1><<<592, 256, 0, st>>>(cen, n_cent, o);
+  else if (n_bit == 4) perm_centroid_kernel<4><<<592, 256, 0, st>>>(cen, n_cent, o);
+  else if (n_bit == 8) perm_centroid_kernel<8><<<592, 256, 0, st>>>(cen, n_cent, o);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
@@ -2604,37 +2600,59 @@ static void wb_launch(const DevIndex &ix, const uint8_t *c, const TmWeights &tw,
 static uint32_t ws_auto_docs(uint32_t n_query, uint32_t probe_topk, uint32_t slots,
                              uint32_t widest);
 
-cudaError_t launch_rerank_tmem(const DevIndex &ix, const void *cen_perm, const TmWeights &tw,
-                               const float *q, const uint64_t *q_off, uint32_t n_query,
-                               const uint32_t *short_id, const uint32_t *n_short,
-                               uint32_t probe_topk, int semantics, uint32_t nq_min,
-                               uint32_t nq_max, float x_bound, float *approx, unsigned *err,
-                               int n_sm, cudaStream_t st, int *n_launch, uint64_t wait_ns) {
-  if (!tmem_rerank_supported(ix.n_bit)) return cudaErrorInvalidValue;
-  if (nq_min <= 32) {  // the warp-specialised kernel; the rest take rerank_tmem_kernel
-    const uint32_t docs = ws_auto_docs(n_query, probe_topk, 2u * (uint32_t)n_sm, 128u);
+cudaError_t launch_rerank_bf16(const DevIndex &ix, const void *cen_perm, const void *lut_bf16,
+                               const TmWeights &tw, const float *q, const uint64_t *q_off,
+                               uint32_t n_query, const uint32_t *short_id,
+                               const uint32_t *n_short, uint32_t probe_topk, int semantics,
+                               uint32_t nq_min, uint32_t nq_max, float x_bound, float *approx,
+                               unsigned *err, int n_sm, cudaStream_t st, int *n_launch,
+                               uint64_t wait_ns) {
+  const bool split = bf16_split_supported(ix.n_bit, x_bound);
+  if (split && nq_min <= kBf16SplitTok) {  // the longer queries take the other launch
+    const uint32_t docs =
+        ws_auto_docs(n_query, probe_topk, 2u * (uint32_t)n_sm, ix.n_bit <= 2 ? 128u : 64u);
     const uint8_t *c8 = reinterpret_cast<const uint8_t *>(cen_perm);
 #define MVR_WB(NB, D)                                                                            \
   wb_launch<NB, D>(ix, c8, tw, q, q_off, n_query, short_id, n_short, probe_topk, semantics,      \
                    x_bound, approx, err, st, wait_ns)
-    if (ix.n_bit == 2) {
-      if (docs == 32) MVR_WB(2, 32); else if (docs == 64) MVR_WB(2, 64); else MVR_WB(2, 128);
-    } else {
-      if (docs == 32) MVR_WB(1, 32); else if (docs == 64) MVR_WB(1, 64); else MVR_WB(1, 128);
+    switch (ix.n_bit) {
+      case 1:
+        if (docs == 32) MVR_WB(1, 32); else if (docs == 64) MVR_WB(1, 64); else MVR_WB(1, 128);
+        break;
+      case 2:
+        if (docs == 32) MVR_WB(2, 32); else if (docs == 64) MVR_WB(2, 64); else MVR_WB(2, 128);
+        break;
+      case 4: if (docs == 32) MVR_WB(4, 32); else MVR_WB(4, 64); break;
+      case 8: if (docs == 32) MVR_WB(8, 32); else MVR_WB(8, 64); break;
+      default: return cudaErrorInvalidValue;
     }
 #undef MVR_WB
     *n_launch += 1;
     const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || nq_max <= 32) return e;
+    if (e != cudaSuccess || nq_max <= kBf16SplitTok) return e;
   }
-  dim3 grid((probe_topk + kTmDocs - 1) / kTmDocs, n_query);
-  const uint32_t *c = reinterpret_cast<const uint32_t *>(cen_perm);
+  if (ix.n_bit <= 2) {
+    dim3 grid((probe_topk + kTmDocs - 1) / kTmDocs, n_query);
+    const uint32_t *c = reinterpret_cast<const uint32_t *>(cen_perm);
 #define MVR_TM_LAUNCH(NB)                                                                       \
-  rerank_tmem_kernel<NB><<<grid, kTmThreads, kTmSmem, st>>>(ix, c, tw, q, q_off, short_id, n_short,  \
-                                                       probe_topk, semantics, x_bound, approx, err)
-  if (ix.n_bit == 2) MVR_TM_LAUNCH(2);
-  else MVR_TM_LAUNCH(1);
+  rerank_tmem_kernel<NB><<<grid, kTmThreads, kTmSmem, st>>>(                                    \
+      ix, c, tw, q, q_off, short_id, n_short, probe_topk, semantics, x_bound, approx, err)
+    if (ix.n_bit == 2) MVR_TM_LAUNCH(2);
+    else MVR_TM_LAUNCH(1);
 #undef MVR_TM_LAUNCH
+  } else {
+    dim3 grid((probe_topk + kTcDocs - 1) / kTcDocs, n_query);
+    const uint32_t n_max = nq_max <= 32 ? 32u : 64u, skip = split ? kBf16SplitTok : 0u;
+    const size_t sm = tc_smem_bytes((int)ix.n_bit, n_max);
+    const __nv_bfloat16 *c = reinterpret_cast<const __nv_bfloat16 *>(cen_perm);
+    const __nv_bfloat16 *l = reinterpret_cast<const __nv_bfloat16 *>(lut_bf16);
+#define MVR_TC_LAUNCH(NB)                                                                       \
+  rerank_tc_kernel<NB><<<grid, kTcThreads, sm, st>>>(ix, c, l, q, q_off, short_id, n_short,     \
+                                                     probe_topk, semantics, n_max, skip, approx, err)
+    if (ix.n_bit == 4) MVR_TC_LAUNCH(4);
+    else MVR_TC_LAUNCH(8);
+#undef MVR_TC_LAUNCH
+  }
   *n_launch += 1;
   return cudaGetLastError();
 }

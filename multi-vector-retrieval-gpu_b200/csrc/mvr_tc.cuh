@@ -8,11 +8,6 @@ namespace mvr {
 cudaError_t configure_tc_kernels();
 float bf16_round(float x);  // to the nearest BF16, as the BF16 tables are rounded
 cudaError_t make_bf16(const float *in, size_t n, void *out, cudaStream_t st);
-cudaError_t launch_rerank_tc(const DevIndex &ix, const void *cen_bf16, const void *lut_bf16,
-                             const float *q, const uint64_t *q_off, uint32_t n_query,
-                             const uint32_t *short_id, const uint32_t *n_short,
-                             uint32_t probe_topk, int semantics, uint32_t nq_max, float *approx,
-                             unsigned *err, cudaStream_t st, int *n_launch);
 
 // bucket-weight tables of the tensor-memory MaxSim kernels (make_tm_weights):
 //  BF16 (1-, 2-bit): w[0] / w[1] = low / high bytes of the BF16 weights;
@@ -24,24 +19,26 @@ struct TmWeights {
 };
 TmWeights make_tm_weights(uint32_t n_bit, const float *weight, bool fp8);
 
-// BF16 MaxSim of 1- and 2-bit codes on the tensor cores; cen_perm: [C + 1][64]
-// bf16x2 centroid rows in the kernels' K order, the last zero
-// (make_centroid_perm); x_bound: upper bound on the norm of every decoded
-// doc token.  Queries of up to kBf16SplitTok tokens: BF16 centroid and BF16
-// weights contribute separately; longer ones: their BF16-rounded sum.
+// BF16 MaxSim on the tensor cores; cen_perm: [C + 1][128] BF16 centroid rows in the
+// kernels' K order, the last zero (make_centroid_perm); lut_bf16: [256][8/b] BF16
+// weights of a residual byte (4 and 8 bits); x_bound: upper bound on the norm of
+// every decoded doc token; wait_ns as launch_rerank_ws.  Queries of up to
+// kBf16SplitTok tokens: BF16 centroid and BF16 weights contribute separately, where
+// bf16_split_supported; otherwise their BF16-rounded sum.
 constexpr uint32_t kBf16SplitTok = 32;
-bool tmem_rerank_supported(uint32_t n_bit);
+bool bf16_split_supported(uint32_t n_bit, float x_bound);
 // largest L2 norm of the centroid rows (d_tmp: one device word of scratch)
 cudaError_t max_centroid_norm(const float *cen, uint32_t n_cent, unsigned *d_tmp, float *out,
                               cudaStream_t st);
 cudaError_t make_centroid_perm(const float *cen, uint32_t n_cent, uint32_t n_bit, void *out,
                                cudaStream_t st);
-cudaError_t launch_rerank_tmem(const DevIndex &ix, const void *cen_perm, const TmWeights &tw,
-                               const float *q, const uint64_t *q_off, uint32_t n_query,
-                               const uint32_t *short_id, const uint32_t *n_short,
-                               uint32_t probe_topk, int semantics, uint32_t nq_min,
-                               uint32_t nq_max, float x_bound, float *approx, unsigned *err,
-                               int n_sm, cudaStream_t st, int *n_launch, uint64_t wait_ns);
+cudaError_t launch_rerank_bf16(const DevIndex &ix, const void *cen_perm, const void *lut_bf16,
+                               const TmWeights &tw, const float *q, const uint64_t *q_off,
+                               uint32_t n_query, const uint32_t *short_id,
+                               const uint32_t *n_short, uint32_t probe_topk, int semantics,
+                               uint32_t nq_min, uint32_t nq_max, float x_bound, float *approx,
+                               unsigned *err, int n_sm, cudaStream_t st, int *n_launch,
+                               uint64_t wait_ns);
 // E4M3 centroid rows [C][128] in the FP8 kernel's K order (2- and 4-bit codes)
 bool fp8_rerank_supported(uint32_t n_bit);
 cudaError_t make_centroid_fp8(const float *cen, uint32_t n_cent, uint32_t n_bit, void *out,

@@ -239,7 +239,7 @@ def test_bf16_rescore_cut(n_bit):
                         np.testing.assert_array_equal(s1, s0)
 
 
-@pytest.mark.parametrize("n_bit", [1, 2])
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 8])
 @pytest.mark.parametrize("n_query,width", [(1, (32, 32)), (3, (1, 31)), (6, (30, 36)), (150, (1, 32))])
 def test_bf16_maxsim_edges(n_bit, n_query, width):
     """The BF16 MaxSim at its docs per CTA, doc lengths around its 128-token tiles and
@@ -264,3 +264,21 @@ def test_bf16_maxsim_edges(n_bit, n_query, width):
                 assert (got[b] >= want[b] - 2 * n * X * (2.0**-7 + 2.0**-11)).all()
                 if ptk == k:
                     np.testing.assert_array_equal(got[b], want[b])
+
+
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 8])
+def test_exact_search_through_bf16_cut_narrow(n_bit):
+    """As test_exact_search_through_bf16_cut, queries of up to 32 tokens (1 to 32 wide)."""
+    ix = tiny_index(n_doc=700, n_centroid=48, n_bit=n_bit, seed=95 + n_bit, lengths=(LENGTHS * 50)[:700])
+    o = oracle_of(ix)
+    q, off = make_queries(ix, 140, (1, 32), seed=8)
+    scale = np.repeat(10.0 ** np.random.default_rng(n_bit).integers(-6, 5, 140),
+                      np.diff(off.astype(np.int64)))
+    with gpu_index(ix) as g:
+        for qq in (q, (q * scale[:, None]).astype(np.float32)):
+            for k in (1, 10, 100):
+                for sem in (SEM_PP, SEM_BASIC):
+                    r = o.search(qq, off, k, 8, 400, sem)
+                    s, i = g.search(qq, k, 8, 400, tok_off=off, semantics=sem)
+                    np.testing.assert_array_equal(i, r[1])
+                    np.testing.assert_array_equal(s, r[0])
