@@ -165,11 +165,11 @@ struct mvr_index {
   uint32_t rescore = 0;          // FP32 re-score count of the BF16 path (0: 4 * topk)
   void *lut_bf16 = nullptr;      // [256][8/b] BF16 decode table (b >= 4)
   void *cen_sw = nullptr;        // [C_pad/128][32 KB] swizzled BF16 centroid tiles
-  float *cen_bounds = nullptr;   // max |c|, max |c - bf16(c)| over the centroids
+  // max |c|, max |c - bf16(c)| over the centroids; the same of the doc tokens' weights
+  float *bounds = nullptr;
   void *cen_perm = nullptr;      // [C + 1][128] BF16 centroid rows, BF16 K order
   TmWeights tw_bf16{};           // weight tables of the BF16 tensor-memory MaxSim (b <= 2)
   float x_bound = 0.f;           // bound on the norm of every decoded doc token
-  float w_norm = 0.f, w_err = 0.f;  // ... of a token's weights, of their BF16 rounding errors
   void *cen8 = nullptr;          // [C][128] E4M3 centroid rows, FP8-rerank K order (b = 2, 4)
   TmWeights tw_fp8{};            // E4M3 weight tables of the FP8 MaxSim (b = 2, 4)
   unsigned *d_err = nullptr;     // device error flags of the tensor-core kernels
@@ -576,27 +576,28 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     if (!h->prune_wts) return set_err(MVR_ERR_INVALID_ARG, "MVR_PRUNE: no pruner set");
     if (nq_max > 32) return set_err(MVR_ERR_UNSUPPORTED, "MVR_PRUNE: queries of up to 32 tokens");
   }
+  const uint32_t split_tok = bf16_split_supported(h->dix.n_bit, h->x_bound) ? kBf16SplitTok : 0u;
   // Exact FP32 search: where a shortlist is long, the BF16 pass first leaves out the
-  // docs that provably miss the top topk, and the FP32 kernel scores the rest.  The
+  // docs that provably miss the top topk, and the FP32 kernel scores the rest (39 of
+  // 1500 on average for the best 10, 130 of 400 for the best 100).  The
   // line: at 22 and 4.8 docs' tokens per ns (2 bits; 8.6 and 3.1 at 8 bits) the pass
   // pays for itself once it spares a third of the FP32 work, which takes a shortlist
   // of 4 topk; its launches take 60 us, the FP32 work of 7,000 docs, and its CTAs of
   // 32 to 128 docs want a grid that fills the GPU: 32,768 docs.  Queries of up to 16
   // tokens take the FP32 kernel's half-width body, at twice its rate; 4- and 8-bit
   // codes have no faster BF16 kernel for more than 32 tokens (4.9 tokens per ns at 8
-  // bits).  200 queries x 400 docs at 8 bits: 1.80 -> 1.45 ms.
+  // bits).  200 queries x 400 docs at 8 bits: 1.80 -> 1.35 ms.
   const bool reach = !bf16 && !prune && !all_exact && nq_max > 16 &&
-                     (h->dix.n_bit <= 2 || (nq_max <= kBf16SplitTok &&
-                                            bf16_split_supported(h->dix.n_bit, h->x_bound))) &&
+                     (h->dix.n_bit <= 2 || nq_max <= split_tok) &&
                      probe_topk / 4 >= topk &&
                      (uint64_t)std::min(h->batch_cap ? h->batch_cap : default_batch(h), n_query) *
                              probe_topk >= 32768;
   if (reach) R = probe_topk;
-  const uint32_t split_tok = bf16_split_supported(h->dix.n_bit, h->x_bound) ? kBf16SplitTok : 0u;
-  // the BF16 path's best R: the same bound leaves out those of them that miss the
-  // top topk (FP8's own error is an order larger and would leave out none).  400 docs
-  // of each of 500 queries for the best 100: 3.26 -> 1.42 ms of FP32 work for 16 us.
-  // From 16,384 docs, whose FP32 work is 300 us.
+  // The BF16 path's best R lose by the same bound those that miss the top topk: 400 docs
+  // of each of 500 queries for the best 100, 3.26 -> 1.38 ms of FP32 work for 16 us.
+  // From 16,384 docs, whose FP32 work is 300 us.  FP8's own error is an order larger
+  // and would leave out none, and its best 40 of 1500 are as many as BF16 scores would
+  // keep for the best 10.
   const bool cut_r = bf16 && !fp8 && R > topk &&
                      (uint64_t)std::min(h->batch_cap ? h->batch_cap : default_batch(h), n_query) *
                              R >= 16384;
@@ -762,7 +763,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         }
         CUDA_TRY(launch_probe(qp + (size_t)c * kDim, n, h->cen_sw, h->dix.centroid,
                               h->dix.centroid_t, h->dix.n_centroid, h->dix.n_centroid_pad,
-                              h->cen_bounds, nprobe,
+                              h->bounds, nprobe,
                               probe_plan(n, h->dix.n_centroid, nprobe, h->n_sm), w.probe,
                               w.probe_id + (size_t)c * nprobe, w.probe_s + (size_t)c * nprobe,
                               h->n_sm, h->d_err, rs, &launches));
@@ -810,15 +811,13 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                              &launches));
         const uint32_t *rid = w.r_id, *nr = w.n_r;
         if (cut_r) {
-          CUDA_TRY(launch_maxsim_reach(qp, qo, nb, w.r_id, w.r_score, w.n_r, R, topk,
-                                       h->cen_bounds, h->w_norm, h->w_err,
-                                       split_tok, w.r2_id, w.n_r2, rs,
-                                       &launches));
+          CUDA_TRY(launch_maxsim_reach(qp, qo, nb, w.r_id, w.r_score, w.n_r, R, topk, h->bounds,
+                                       split_tok, w.r2_id, w.n_r2, rs, &launches));
           rid = w.r2_id;
           nr = w.n_r2;
         }
         CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, rid, nr, R, sem, w.r_exact, h->n_sm, rs,
-                               &launches));
+                               &launches, cut_r ? 32 : 64));
         CUDA_TRY(launch_topk(rid, w.r_exact, nr, nb, R, topk, os, oi, nullptr, rs, &launches));
       } else {
         // exact FP32 MaxSim over the shortlist -- with MVR_PRUNE over the docs
@@ -843,8 +842,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                                       nsh, probe_topk, sem, nq_min, nq_max, h->x_bound, w.exact,
                                       h->d_err, h->n_sm, rs, &launches, h->wait_ns));
           CUDA_TRY(launch_maxsim_reach(qp, qo, nb, sid, w.exact, nsh, probe_topk, topk,
-                                       h->cen_bounds, h->w_norm, h->w_err, split_tok, w.r_id, w.n_r, rs,
-                                       &launches));
+                                       h->bounds, split_tok, w.r_id, w.n_r, rs, &launches));
           CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, w.r_id, w.n_r, probe_topk, sem, w.r_exact,
                                  h->n_sm, rs, &launches, 32));
           sid = w.r_id;
@@ -1030,14 +1028,9 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
   MVR_TRY(dalloc(&sw, (size_t)d.n_centroid_pad * 256, &h->bufs));
   CUDA_TRY(make_centroid_tiles(d.centroid, d.n_centroid, d.n_centroid_pad / 64, sw, h->stream));
   h->cen_sw = sw;
-  MVR_TRY(dalloc(&h->cen_bounds, 2, &h->bufs));
-  CUDA_TRY(make_centroid_bounds(d.centroid, d.n_centroid, h->cen_bounds, h->stream));
-  for (uint32_t k = 0; k < (1u << d.n_bit); k++) {  // (a NaN or infinite weight: infinite bounds)
-    const float root = std::sqrt((float)kDim) * (1.0f + 0x1p-10f);
-    const float e = std::fabs(weight[k] - bf16_round(weight[k]));
-    h->w_norm = std::max(h->w_norm, std::isfinite(weight[k]) ? root * std::fabs(weight[k]) : INFINITY);
-    h->w_err = std::max(h->w_err, std::isfinite(e) ? root * e : INFINITY);
-  }
+  MVR_TRY(dalloc(&h->bounds, 4, &h->bufs));
+  CUDA_TRY(make_centroid_bounds(d.centroid, d.n_centroid, h->bounds, h->stream));
+  CUDA_TRY(make_weight_bounds(d, h->bounds + 2, h->n_sm, h->stream));
   {
     float wmax = 0.f;
     for (uint32_t k = 0; k < (1u << d.n_bit); k++) wmax = std::max(wmax, std::fabs(weight[k]));

@@ -1265,8 +1265,7 @@ __global__ void __launch_bounds__(kReachThreads)
 maxsim_reach_kernel(const float *__restrict__ q, const uint64_t *__restrict__ q_off,
                     const uint32_t *__restrict__ short_id, const float *__restrict__ approx,
                     const uint32_t *__restrict__ n_short, uint32_t probe_topk, uint32_t topk,
-                    const float *__restrict__ cen_bounds, float w_norm, float w_err,
-                    uint32_t split_tok, uint32_t *__restrict__ out_id, uint32_t *__restrict__ n_out) {
+                    const float *__restrict__ bounds, uint32_t split_tok, uint32_t *__restrict__ out_id, uint32_t *__restrict__ n_out) {
   extern __shared__ uint32_t rsm[];
   uint32_t *ord = rsm, *hist = rsm + probe_topk;  // [probe_topk], [4096]
   __shared__ float s_e[kMaxQueryTok], s_q[kMaxQueryTok];
@@ -1280,8 +1279,8 @@ maxsim_reach_kernel(const float *__restrict__ q, const uint64_t *__restrict__ q_
   const size_t row = (size_t)b * probe_topk;
   for (uint32_t i = tid; i < n; i += kReachThreads) ord[i] = f2ord(approx[row + i]);
   if (tid == 0) s_n = 0;
-  const float X = (cen_bounds[0] + w_norm) * (1.0f + 0x1p-10f);
-  const float dX = cen_bounds[1] + w_err + (nq > split_tok ? X * 0x1.02p-8f : 0.0f);
+  const float X = (bounds[0] + bounds[2]) * (1.0f + 0x1p-10f);
+  const float dX = (bounds[1] + bounds[3]) * (1.0f + 0x1p-10f) + (nq > split_tok ? X * 0x1.02p-8f : 0.0f);
   for (uint32_t t = warp; t < nq; t += kReachThreads / 32) {
     const float4 v = __ldg(reinterpret_cast<const float4 *>(q + (tok0 + t) * kDim) + lane);
     const float x[4] = {v.x, v.y, v.z, v.w};
@@ -1680,12 +1679,10 @@ cudaError_t launch_rerank(const DevIndex &ix, const float *q, const uint64_t *q_
 cudaError_t launch_maxsim_reach(const float *q, const uint64_t *q_off, uint32_t n_query,
                                 const uint32_t *short_id, const float *approx,
                                 const uint32_t *n_short, uint32_t probe_topk, uint32_t topk,
-                                const float *cen_bounds, float w_norm, float w_err,
-                                uint32_t split_tok, uint32_t *out_id, uint32_t *n_out, cudaStream_t st,
-                                int *n_launch) {
+                                const float *bounds, uint32_t split_tok, uint32_t *out_id,
+                                uint32_t *n_out, cudaStream_t st, int *n_launch) {
   maxsim_reach_kernel<<<n_query, kReachThreads, reach_smem(probe_topk), st>>>(
-      q, q_off, short_id, approx, n_short, probe_topk, topk, cen_bounds, w_norm, w_err, split_tok, out_id,
-      n_out);
+      q, q_off, short_id, approx, n_short, probe_topk, topk, bounds, split_tok, out_id, n_out);
   *n_launch += 1;
   return cudaGetLastError();
 }

@@ -92,16 +92,15 @@ cudaError_t launch_rerank(const DevIndex &ix, const float *q, const uint64_t *q_
                           int *n_launch, uint32_t most_docs = 64 /* docs per CTA */);
 // The docs of each query's shortlist whose BF16 MaxSim reaches its topk-th best
 // less twice the BF16 error bound, the only ones that can be in the exact top
-// topk (maxsim_reach_kernel).  cen_bounds: max |c| and max |c - bf16(c)|;
-// w_norm / w_err: bounds on the norms of a token's weights and of their BF16
-// rounding errors; split_tok: queries of more tokens have BF16-rounded doc
-// tokens.  out_id: [n_query][probe_topk], n_out: [n_query].
+// topk (maxsim_reach_kernel).  bounds: max |c| and max |c - bf16(c)|, then the
+// largest norms of a token's weights and of their BF16 rounding errors; split_tok:
+// queries of more tokens have BF16-rounded doc tokens.  out_id:
+// [n_query][probe_topk], n_out: [n_query].
 cudaError_t launch_maxsim_reach(const float *q, const uint64_t *q_off, uint32_t n_query,
                                 const uint32_t *short_id, const float *approx,
                                 const uint32_t *n_short, uint32_t probe_topk, uint32_t topk,
-                                const float *cen_bounds, float w_norm, float w_err,
-                                uint32_t split_tok, uint32_t *out_id, uint32_t *n_out, cudaStream_t st,
-                                int *n_launch);
+                                const float *bounds, uint32_t split_tok, uint32_t *out_id,
+                                uint32_t *n_out, cudaStream_t st, int *n_launch);
 cudaError_t launch_topk(const uint32_t *short_id, const float *exact,
                         const uint32_t *n_short, uint32_t n_query,
                         uint32_t probe_topk, uint32_t topk, float *out_s,

@@ -1200,6 +1200,58 @@ __global__ void centroid_bounds_kernel(const float *__restrict__ cen, uint32_t n
   }
 }
 
+// The largest norm of a token's weights and of their BF16 rounding errors.  A lane
+// adds up 16 residual bytes from a table of each byte's sums of squares (8
+// interleaved copies), a token's n_bit lanes add theirs: 70M tokens at 2 bits, once per
+// index, 1.1 ms.  With these and not 128 times the largest weight, 8-bit searches
+// for the best 100 of 400 docs score 130 of them in FP32: 0.78 -> 0.69 ms.
+__global__ void __launch_bounds__(256)
+weight_bounds_kernel(DevIndex ix, uint32_t *__restrict__ bounds) {
+  __shared__ float2 sq[256 * 8];
+  const uint32_t vpb = 8u / ix.n_bit;
+  for (uint32_t i = threadIdx.x; i < 256 * 8; i += 256) {
+    float n2 = 0.0f, e2 = 0.0f;
+    for (uint32_t u = 0; u < vpb; u++) {
+      const float x = __ldg(ix.lut + (i >> 3) * vpb + u);
+      const float e = x - __bfloat162float(__float2bfloat16_rn(x));
+      n2 = fmaf(x, x, n2);
+      e2 = fmaf(e, e, e2);
+    }
+    sq[i] = make_float2(n2, e2);
+  }
+  __syncthreads();
+  const float2 *mine = sq + (threadIdx.x & 7u);
+  const uint64_t n = ix.n_vec * ix.n_bit;  // chunks of 16 bytes
+  const uint64_t step = (uint64_t)gridDim.x * 256;
+  uint32_t mn = 0, me = 0;
+  for (uint64_t base = (uint64_t)blockIdx.x * 256; base < n; base += step) {  // whole warps
+    const uint64_t i = base + threadIdx.x;
+    float n2 = 0.0f, e2 = 0.0f;
+    if (i < n) {
+      const uint4 t = __ldg(reinterpret_cast<const uint4 *>(ix.residual) + i);
+      const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int u = 0; u < 16; u++) {
+        const float2 s = mine[((w[u >> 2] >> (8 * (u & 3))) & 0xffu) * 8];
+        n2 += s.x;
+        e2 += s.y;
+      }
+    }
+    for (uint32_t o = 1; o < ix.n_bit; o <<= 1) {
+      n2 += __shfl_xor_sync(kFull, n2, o);
+      e2 += __shfl_xor_sync(kFull, e2, o);
+    }
+    mn = max(mn, __float_as_uint(n2) & 0x7fffffffu);  // (a NaN is the largest)
+    me = max(me, __float_as_uint(e2) & 0x7fffffffu);
+  }
+  mn = __reduce_max_sync(kFull, mn);
+  me = __reduce_max_sync(kFull, me);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(bounds, __float_as_uint(sqrtf(__uint_as_float(mn))) & 0x7fffffffu);
+    atomicMax(bounds + 1, __float_as_uint(sqrtf(__uint_as_float(me))) & 0x7fffffffu);
+  }
+}
+
 // canonical FP32 score of one centroid: sequential fma over d, then + 1.0f
 __device__ __forceinline__ float exact_score(const float *qs, const float *cen, uint32_t c) {
   const float4 *row = reinterpret_cast<const float4 *>(cen + (size_t)c * kDim);
@@ -1489,6 +1541,13 @@ cudaError_t make_centroid_bounds(const float *cen, uint32_t n_cent, float *bound
   if (e != cudaSuccess) return e;
   centroid_bounds_kernel<<<(n_cent + 7) / 8, 256, 0, st>>>(cen, n_cent,
                                                            reinterpret_cast<uint32_t *>(bounds));
+  return cudaGetLastError();
+}
+
+cudaError_t make_weight_bounds(const DevIndex &ix, float *bounds, int n_sm, cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(bounds, 0, 2 * sizeof(float), st);
+  if (e != cudaSuccess) return e;
+  weight_bounds_kernel<<<8 * n_sm, 256, 0, st>>>(ix, reinterpret_cast<uint32_t *>(bounds));
   return cudaGetLastError();
 }
 
@@ -2452,7 +2511,6 @@ cudaError_t make_bf16(const float *in, size_t n, void *out, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 cudaError_t configure_tc_kernels() {
   cudaError_t e;

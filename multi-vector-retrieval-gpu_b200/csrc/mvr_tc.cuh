@@ -6,7 +6,6 @@
 namespace mvr {
 
 cudaError_t configure_tc_kernels();
-float bf16_round(float x);  // to the nearest BF16, as the BF16 tables are rounded
 cudaError_t make_bf16(const float *in, size_t n, void *out, cudaStream_t st);
 
 // bucket-weight tables of the tensor-memory MaxSim kernels (make_tm_weights):
@@ -113,6 +112,8 @@ struct ProbeBufs {
 // bounds[2] of probe_tc_kernel: max |c| and max |c - bf16(c)| over the centroids
 cudaError_t make_centroid_bounds(const float *cen, uint32_t n_cent, float *bounds,
                                  cudaStream_t st);
+// bounds: the largest norm of a doc token's weights, and of their BF16 rounding errors
+cudaError_t make_weight_bounds(const DevIndex &ix, float *bounds, int n_sm, cudaStream_t st);
 // top nprobe (1..32) per token, (score desc, id asc), equal to an exact FP32
 // scan's; cen_sw: swizzled BF16 tiles (make_centroid_tiles), cen: [C][128],
 // cen_t: [128][n_cent_pad]
