@@ -922,6 +922,9 @@ filter_select_kernel(DevIndex ix, uint32_t probe_topk, FilterScratch scr,
 // token and chunk) are in registers a chunk ahead, the next tile's codes two
 // chunks ahead.
 //
+// With KT = 1 a tile is 32 tokens, one per lane, whose centroid rows come at once
+// (8 chunks in the space of 2 of 128 tokens): the short chain of a small grid.
+//
 // After a tile: per doc of the tile, the max over the lane's tokens of that
 // doc and a REDUX over the warp for every query token, folded into
 // best[doc][query token] by atomicMax.  Queries of more than 32 tokens run in
@@ -934,7 +937,7 @@ filter_select_kernel(DevIndex ix, uint32_t probe_topk, FilterScratch scr,
 // scalar FFMA and separate decoder warps -> 8.8 ms, 39 TFLOP/s.
 // ---------------------------------------------------------------------
 constexpr int kRkDocs = 64;       // most shortlisted docs per CTA
-constexpr int kRkT = 4;           // doc tokens per lane
+constexpr int kRkT = 4;           // doc tokens per lane (KT = 1: 1)
 constexpr int kRkTile = 32 * kRkT;  // doc tokens per warp and tile
 constexpr int kRkChunk = 16;      // dimensions per stage
 constexpr int kRkStages = 2;
@@ -986,15 +989,18 @@ struct RkCta {
 };
 
 // One pass of one warp over its tiles: NQ query tokens (rows 0 .. NQ - 1 of Qs).
-template <int NBIT, int NQ>
+template <int NBIT, int NQ, int KT>
 __device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c, uint32_t nq_pass) {
   constexpr int CB = kRkChunk * NBIT / 8;  // residual bytes per token and chunk
   constexpr int RW = (CB + 3) / 4;         // ... in 32-bit words
   constexpr uint32_t MASK = (1u << NBIT) - 1u;
+  constexpr int TILE = 32 * KT;
+  static_assert(KT == kRkT || kRkStages * kRkT == kRkNch * KT,
+                "chunks in two stages, or a whole tile of rows at once");
   constexpr int WC = rk_wcopies(NBIT);
   const int lane = threadIdx.x & 31;
   const uint32_t warp = threadIdx.x >> 5;
-  const uint32_t n_tiles = (c.T + kRkTile - 1) / kRkTile;
+  const uint32_t n_tiles = (c.T + TILE - 1) / TILE;
   if (warp >= n_tiles) return;
   const float *wt = c.wtab + (lane & (WC - 1));
 
@@ -1004,22 +1010,22 @@ __device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c,
   auto locate = [&](uint32_t tl, uint32_t pr) {
     docs4_n = 0;
 #pragma unroll
-    for (int j = 0; j < kRkT; j++) {
-      const uint32_t g = kRkTile * tl + 32u * j + lane, gt = min(g, c.T - 1u);
+    for (int j = 0; j < KT; j++) {
+      const uint32_t g = TILE * tl + 32u * j + lane, gt = min(g, c.T - 1u);
       const uint32_t d = find_seg(c.d_pref, (int)c.nd, gt);
       docs4_n |= (g < c.T ? d : 255u) << (8 * j);
       const uint64_t v = c.d_off[d] + (gt - c.d_pref[d]);
-      c.toks[pr * kRkTile + 32 * j + lane] = v;
-      cp_async4(&c.codes[pr * kRkTile + 32 * j + lane], ix.vq_code + v);
+      c.toks[pr * TILE + 32 * j + lane] = v;
+      cp_async4(&c.codes[pr * TILE + 32 * j + lane], ix.vq_code + v);
     }
     cp_async_commit();
   };
-  uint32_t res[kRkT][RW], res_n[kRkT][RW];
+  uint32_t res[KT][RW], res_n[KT][RW];
   auto load_res = [&](uint32_t ch, uint32_t pr) {
 #pragma unroll
-    for (int j = 0; j < kRkT; j++) {
+    for (int j = 0; j < KT; j++) {
       const uint8_t *rp =
-          ix.residual + c.toks[pr * kRkTile + 32 * j + lane] * (kDim * NBIT / 8) + ch * CB;
+          ix.residual + c.toks[pr * TILE + 32 * j + lane] * (kDim * NBIT / 8) + ch * CB;
       if constexpr (CB == 2) {
         res_n[j][0] = __ldg(reinterpret_cast<const unsigned short *>(rp));
       } else if constexpr (CB == 4) {
@@ -1041,12 +1047,12 @@ __device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c,
   // lane % 4 of tokens lane / 4, lane / 4 + 8, ...
   auto copy_chunk = [&](uint32_t ch, uint32_t pr, uint32_t st) {
     const uint32_t part = lane & 3u;
-    float *dst = c.xs + st * (kRkTile * kRkChunk);
+    float *dst = c.xs + st * (TILE * kRkChunk);
     const float *src = ix.centroid + ch * kRkChunk + part * 4u;
 #pragma unroll
-    for (int i = 0; i < kRkTile / 8; i++) {
+    for (int i = 0; i < TILE / 8; i++) {
       const uint32_t p = 8u * i + (lane >> 2);
-      const uint32_t cd = c.codes[pr * kRkTile + p];
+      const uint32_t cd = c.codes[pr * TILE + p];
       cp_async16(dst + p * kRkChunk + ((part ^ ((p >> 1) & 3u)) << 2), src + (size_t)cd * kDim);
     }
     cp_async_commit();
@@ -1055,42 +1061,51 @@ __device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c,
   locate(warp, 0);
   cp_async_wait<0>();
   __syncwarp();
-  copy_chunk(0, 0, 0);
-  load_res(0, 0);
+  auto copy_first = [&](uint32_t pr, uint32_t st) {  // of a tile: a chunk, or all of them
+    if constexpr (KT == kRkT) {
+      copy_chunk(0, pr, st);
+    } else {
+#pragma unroll
+      for (uint32_t ch = 0; ch < (uint32_t)kRkNch; ch++) copy_chunk(ch, pr, ch);
+    }
+    load_res(0, pr);
+  };
+  copy_first(0, 0);
   uint32_t par = 0;
   for (uint32_t tl = warp; tl < n_tiles; tl += kRkWarps) {
     const bool more = tl + kRkWarps < n_tiles;
     docs4 = docs4_n;
-    uint64_t acc[NQ / 2][kRkT];
+    uint64_t acc[NQ / 2][KT];
 #pragma unroll
     for (int i = 0; i < NQ / 2; i++)
 #pragma unroll
-      for (int j = 0; j < kRkT; j++) acc[i][j] = 0ull;
+      for (int j = 0; j < KT; j++) acc[i][j] = 0ull;
 #pragma unroll 1
     for (uint32_t ch = 0; ch < (uint32_t)kRkNch; ch++) {
 #pragma unroll
-      for (int j = 0; j < kRkT; j++)
+      for (int j = 0; j < KT; j++)
 #pragma unroll
         for (int w = 0; w < RW; w++) res[j][w] = res_n[j][w];
-      const uint32_t st = ch & 1u;
-      cp_async_wait<0>();
-      __syncwarp();  // chunk ch landed for every lane; every lane is done with the other stage
-      if (ch + 1 < (uint32_t)kRkNch) {
-        copy_chunk(ch + 1, par, st ^ 1u);
-        load_res(ch + 1, par);
-        if (ch == kRkNch - 2 && more) locate(tl + kRkWarps, par ^ 1u);
-      } else if (more) {
-        par ^= 1u;
-        copy_chunk(0, par, st ^ 1u);
-        load_res(0, par);
+      const uint32_t st = KT == kRkT ? ch & 1u : ch;
+      if (KT == kRkT || ch == 0) {
+        cp_async_wait<0>();
+        __syncwarp();  // chunk ch landed for every lane; every lane is done with the other stage
       }
-      const float *xr = c.xs + st * (kRkTile * kRkChunk) + lane * kRkChunk;
+      if (ch + 1 < (uint32_t)kRkNch) {
+        if constexpr (KT == kRkT) copy_chunk(ch + 1, par, st ^ 1u);
+        load_res(ch + 1, par);
+        if (ch == (KT == kRkT ? kRkNch - 2 : 0) && more) locate(tl + kRkWarps, par ^ 1u);
+      } else if (KT == kRkT && more) {
+        par ^= 1u;
+        copy_first(par, st ^ 1u);
+      }
+      const float *xr = c.xs + st * (TILE * kRkChunk) + lane * kRkChunk;
       const float *qr = c.Qs + ch * (kRkChunk * kRkQ);
 #pragma unroll rk_unroll(NBIT)
       for (int g = 0; g < kRkChunk / 4; g++) {
-        float x[kRkT][4];  // [token][dim of the group]
+        float x[KT][4];  // [token][dim of the group]
 #pragma unroll
-        for (int j = 0; j < kRkT; j++) {
+        for (int j = 0; j < KT; j++) {
           // token 32 j + lane: (p >> 1) & 3 is (lane >> 1) & 3
           const float4 v = *reinterpret_cast<const float4 *>(
               xr + j * 32 * kRkChunk + (((uint32_t)g ^ ((lane >> 1) & 3u)) << 2));
@@ -1109,15 +1124,15 @@ __device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c,
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          uint64_t xx[kRkT];
+          uint64_t xx[KT];
 #pragma unroll
-          for (int j = 0; j < kRkT; j++) xx[j] = dup_f32x2(x[j][u]);
+          for (int j = 0; j < KT; j++) xx[j] = dup_f32x2(x[j][u]);
           const ulonglong2 *qp = reinterpret_cast<const ulonglong2 *>(qr + (4 * g + u) * kRkQ);
 #pragma unroll
           for (int i = 0; i < NQ / 4; i++) {
             const ulonglong2 a = qp[i];
 #pragma unroll
-            for (int j = 0; j < kRkT; j++) {
+            for (int j = 0; j < KT; j++) {
               acc[2 * i][j] = fma_f32x2(a.x, xx[j], acc[2 * i][j]);
               acc[2 * i + 1][j] = fma_f32x2(a.y, xx[j], acc[2 * i + 1][j]);
             }
@@ -1125,21 +1140,27 @@ __device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c,
         }
       }
     }
+    if (KT != kRkT && more) {
+      par ^= 1u;
+      cp_async_wait<0>();
+      __syncwarp();  // the next tile's codes landed; every lane is done with this one's rows
+      copy_first(par, 0);
+    }
     // per doc of the tile: max over its tokens for every query token (lane q
     // ends up with query token q's)
     uint32_t d = __reduce_min_sync(kFull, docs4 & 0xffu);
-    const uint32_t d_last = find_seg(c.d_pref, (int)c.nd, min(c.T, kRkTile * (tl + 1)) - 1u);
+    const uint32_t d_last = find_seg(c.d_pref, (int)c.nd, min(c.T, TILE * (tl + 1)) - 1u);
 #pragma unroll 1
     for (; d <= d_last; d++) {
-      bool in[kRkT];
+      bool in[KT];
 #pragma unroll
-      for (int j = 0; j < kRkT; j++) in[j] = ((docs4 >> (8 * j)) & 0xffu) == d;
+      for (int j = 0; j < KT; j++) in[j] = ((docs4 >> (8 * j)) & 0xffu) == d;
       int mine = f2si(-INFINITY);
 #pragma unroll
       for (int i = 0; i < NQ / 2; i++) {
         int lo = f2si(-INFINITY), hi = lo;
 #pragma unroll
-        for (int j = 0; j < kRkT; j++) {
+        for (int j = 0; j < KT; j++) {
           if (in[j]) {
             lo = max(lo, f2si(__uint_as_float((uint32_t)acc[i][j])));
             hi = max(hi, f2si(__uint_as_float((uint32_t)(acc[i][j] >> 32))));
@@ -1154,7 +1175,7 @@ __device__ __forceinline__ void rk_warp_pass(const DevIndex &ix, const RkCta &c,
   }
 }
 
-template <int NBIT>
+template <int NBIT, int KT>
 __global__ void __launch_bounds__(kRkThreads, 2)
 rerank_kernel(DevIndex ix, const float *__restrict__ q, const uint64_t *__restrict__ q_off,
               const uint32_t *__restrict__ short_id, const uint32_t *__restrict__ n_short,
@@ -1224,8 +1245,8 @@ rerank_kernel(DevIndex ix, const float *__restrict__ q, const uint64_t *__restri
     __syncthreads();
     RkCta pc = cta;
     pc.T = d_pref[nd];
-    if (np <= 16) rk_warp_pass<NBIT, 16>(ix, pc, np);
-    else rk_warp_pass<NBIT, 32>(ix, pc, np);
+    if (np <= 16) rk_warp_pass<NBIT, 16, KT>(ix, pc, np);
+    else rk_warp_pass<NBIT, 32, KT>(ix, pc, np);
     __syncthreads();
     if (tid < (int)nd) {
       const bool clamp = semantics == 1 && d_len[tid] < ix.max_item_n_vec;
@@ -1523,14 +1544,15 @@ cudaError_t configure_kernels() {
   cudaError_t e = cudaFuncSetAttribute(probe_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kProbeSmem);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(1));
+#define MVR_RK_ATTR(NB, KT)                                                                     \
+  e = cudaFuncSetAttribute(rerank_kernel<NB, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                           (int)rk_smem_bytes(NB));                                             \
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(2));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(4));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rerank_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rk_smem_bytes(8));
-  if (e != cudaSuccess) return e;
+  MVR_RK_ATTR(1, 1) MVR_RK_ATTR(1, 4)
+  MVR_RK_ATTR(2, 1) MVR_RK_ATTR(2, 4)
+  MVR_RK_ATTR(4, 1) MVR_RK_ATTR(4, 4)
+  MVR_RK_ATTR(8, 1) MVR_RK_ATTR(8, 4)
+#undef MVR_RK_ATTR
   e = cudaFuncSetAttribute(filter_hash_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)hash_smem_bytes(1));
   if (e != cudaSuccess) return e;
@@ -1639,14 +1661,17 @@ cudaError_t launch_filter_hash(const DevIndex &ix, const uint32_t *probe_id,
   return cudaSuccess;
 }
 
-// Shortlisted docs per CTA of the exact rerank: kRkDocs for grids that fill
-// the GPU several times over, fewer (down to the 4 whose tokens are about one
-// tile per warp) while n_query * windows stays within two waves of CTAs: a
-// wide window would leave most SMs idle (one query, 200 docs: 232 us in 4
-// CTAs, 25 us in 50).
+// Shortlisted docs per CTA of the exact rerank: kRkDocs for grids that fill the GPU
+// several times over, fewer while n_query * windows stays within two waves of CTAs:
+// a wide window would leave most SMs idle (one query, 200 docs: 232 us in 4 CTAs,
+// 25 us in 50; 40 docs: 34 us in 10, 23 us in 40).  With up to kRkNarrow docs a CTA
+// the tiles are 32 tokens wide, so that a doc occupies its 4 warps (40 docs of 4
+// queries: 34 -> 20 us, of 16 queries: 58 -> 43 us); with 4 docs the wide tiles are
+// the faster ones (of 37 queries: 55 against 76 us).
+constexpr uint32_t kRkNarrow = 2;
 static uint32_t rerank_docs(uint32_t n_query, uint32_t n_docs, uint32_t most, int n_sm) {
   uint32_t docs = most;
-  while (docs > 4 &&
+  while (docs > 1 &&
          (uint64_t)n_query * ((n_docs + docs / 2 - 1) / (docs / 2)) <= 4ull * (uint32_t)n_sm)
     docs /= 2;
   return docs;
@@ -1661,9 +1686,14 @@ cudaError_t launch_rerank(const DevIndex &ix, const float *q, const uint64_t *q_
   const uint32_t docs = rerank_docs(n_query, probe_topk, std::min<uint32_t>(most_docs, kRkDocs), n_sm);
   dim3 grid((probe_topk + docs - 1) / docs, n_query);
   const size_t sm = rk_smem_bytes((int)ix.n_bit);
+  const bool narrow = docs <= kRkNarrow;
 #define MVR_RK(NB)                                                                              \
-  rerank_kernel<NB><<<grid, kRkThreads, sm, st>>>(ix, q, q_off, short_id, n_short, probe_topk, \
-                                                  docs, semantics, exact)
+  if (narrow)                                                                                   \
+    rerank_kernel<NB, 1><<<grid, kRkThreads, sm, st>>>(ix, q, q_off, short_id, n_short,         \
+                                                       probe_topk, docs, semantics, exact);     \
+  else                                                                                          \
+    rerank_kernel<NB, kRkT><<<grid, kRkThreads, sm, st>>>(ix, q, q_off, short_id, n_short,      \
+                                                          probe_topk, docs, semantics, exact)
   switch (ix.n_bit) {
     case 1: MVR_RK(1); break;
     case 2: MVR_RK(2); break;

@@ -282,3 +282,21 @@ def test_exact_search_through_bf16_cut_narrow(n_bit):
                     s, i = g.search(qq, k, 8, 400, tok_off=off, semantics=sem)
                     np.testing.assert_array_equal(i, r[1])
                     np.testing.assert_array_equal(s, r[0])
+
+
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 8])
+@pytest.mark.parametrize("n_query,width", [(1, (1, 1)), (1, (33, 33)), (5, (15, 18)), (16, (1, 64))])
+def test_exact_rerank_small_grids(n_bit, n_query, width):
+    """The exact rerank at one, two and a few docs per CTA (32- and 128-token tiles)."""
+    ix = tiny_index(n_doc=300, n_centroid=48, n_bit=n_bit, seed=70 + n_bit,
+                    lengths=(LENGTHS * 20)[:300])
+    o = oracle_of(ix)
+    q, off = make_queries(ix, n_query, width, seed=7)
+    with gpu_index(ix) as g:
+        for ptk in (1, 37, 74, 300):
+            for sem in (SEM_PP, SEM_BASIC):
+                k = min(ptk, 40)
+                r = o.search(q, off, k, 8, ptk, sem)
+                s, i = g.search(q, k, 8, ptk, tok_off=off, semantics=sem)
+                np.testing.assert_array_equal(i, r[1])
+                np.testing.assert_array_equal(s, r[0])
