@@ -1203,8 +1203,9 @@ __global__ void centroid_bounds_kernel(const float *__restrict__ cen, uint32_t n
 // The largest norm of a token's weights and of their BF16 rounding errors.  A lane
 // adds up 16 residual bytes: 1- and 2-bit codes by counting each, wider ones from a
 // table of each byte's sums of squares (8 interleaved copies); a token's n_bit lanes
-// add theirs.  70M tokens at 2 bits, once per index: 0.55 ms (with the table 1.1 ms).  With these and not 128 times the largest weight, 8-bit searches
-// for the best 100 of 400 docs score 130 of them in FP32: 0.78 -> 0.69 ms.
+// add theirs.  70M tokens at 2 bits, once per index: 0.55 ms (with the table 1.1
+// ms).  With these and not 128 times the largest weight, 8-bit searches for the best
+// 100 of 400 docs score 130 of them in FP32: 0.78 -> 0.69 ms.
 __global__ void __launch_bounds__(256)
 weight_bounds_kernel(DevIndex ix, uint32_t *__restrict__ bounds) {
   __shared__ float2 sq[256 * 8];
@@ -1377,7 +1378,10 @@ probe_pick1_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__r
 }
 
 // The exact top nprobe of each token from its lists, W warps per token (1
-// where tokens are many, 8 where each has the lists of many splits).  The
+// where tokens are many, 8 where each has the lists of many splits; then 16 lanes
+// read a list, each list's length one list ahead, because a list costs two loads in
+// a row: 32 tokens of 8,192 centroids 13.4 -> 9.6 us, of 65,536 23.0 -> 20.4; with 8
+// lanes 10.0 and 22.5).  The
 // nprobe-th best of the threads' own maxima bounds the nprobe-th best BF16
 // score from below; the entries within 2 eps of it are recomputed exactly and
 // selected by (score desc, id asc).  More of them than fit: the token is flagged.
@@ -1389,6 +1393,7 @@ probe_pick_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__re
                   uint32_t *__restrict__ out_id, float *__restrict__ out_s,
                   uint32_t *__restrict__ flags, uint32_t list_at) {
   constexpr int G = 32 * W, TB = 8 / W;     // threads per token, tokens per block
+  constexpr int L = W == 1 ? 32 : 16;       // lanes per list
   constexpr uint32_t LIM = W == 1 ? 256 : 1024;  // entries recomputed per token
   __shared__ __align__(16) float qs[TB][kDim];
   __shared__ uint32_t c_id[TB][LIM];
@@ -1397,6 +1402,7 @@ probe_pick_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__re
   __shared__ uint32_t s_n[TB], s_over[TB];
   __shared__ float s_thr[TB];
   const int tid = threadIdx.x, lane = tid & 31, g = tid / G, gt = tid % G, w = gt >> 5;
+  const int l0 = gt / L, el = gt % L;
   const uint32_t t = blockIdx.x * TB + g;
   auto sync = [] {
     if constexpr (W == 1) __syncwarp();
@@ -1409,13 +1415,21 @@ probe_pick_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__re
   const float m2 = eps2[t];
   int mx = f2si(-INFINITY);
   bool over = false;
-  for (uint32_t sp = w; sp < splits; sp += W) {
-    const size_t row = (size_t)t * splits + sp;
-    const uint32_t n = cnt[row];
+  // f(list's row, its length) of this thread's lists
+  auto for_lists = [&](auto f) {
+    const size_t row0 = (size_t)t * splits;
+    uint32_t n = (uint32_t)l0 < splits ? cnt[row0 + l0] : 0u;
+    for (uint32_t sp = l0; sp < splits; sp += G / L) {
+      const uint32_t ahead = sp + G / L < splits ? cnt[row0 + sp + G / L] : 0u;
+      f(row0 + sp, n);
+      n = ahead;
+    }
+  };
+  for_lists([&](size_t row, uint32_t n) {
     over |= n > cap;
-    for (uint32_t e = lane; e < min(n, cap); e += 32)
+    for (uint32_t e = el; e < min(n, cap); e += L)
       mx = max(mx, f2si(group_max(ent + 2 * (row * cap + e))));
-  }
+  });
   if (over) s_over[g] = 1;
   if constexpr (W > 1) wmax[gt] = mx;
   sync();
@@ -1440,16 +1454,14 @@ probe_pick_kernel(const float *__restrict__ q, uint32_t n_tok, const float *__re
   sync();
   const float thr = s_thr[g];
   if (!s_over[g]) {
-    for (uint32_t sp = w; sp < splits; sp += W) {
-      const size_t row = (size_t)t * splits + sp;
-      const uint32_t n = cnt[row];
-      for (uint32_t e = lane; e < n; e += 32) {
+    for_lists([&](size_t row, uint32_t n) {
+      for (uint32_t e = el; e < n; e += L) {
         for_reach(ent + 2 * (row * cap + e), gid[row * cap + e], thr, [&](uint32_t c) {
           const uint32_t pos = atomicAdd(&s_n[g], 1u);
           if (pos < LIM) c_id[g][pos] = c;
         });
       }
-    }
+    });
   }
   sync();
   const uint32_t n = s_n[g];
