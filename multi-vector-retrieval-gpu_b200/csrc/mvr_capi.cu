@@ -473,9 +473,22 @@ int ensure_stage(mvr_index *h, size_t n_ret, size_t in_bytes) {
   return MVR_OK;
 }
 
-// Buffer sizes of the centroid scoring of n_tok tokens, in chunks of probe_chunk
-// (the plans of a full chunk and of the last one).
-void probe_need(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, ProbePlan *need) {
+// Tokens per launch of the centroid scoring of n_tok tokens that arrive in n_part pieces.
+uint32_t score_chunk(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, uint32_t n_part) {
+  const uint32_t chunk = probe_chunk(nprobe, h->n_sm);
+  return n_part > 1 ? std::min(chunk, ((n_tok / n_part + 255u) & ~255u)) : chunk;
+}
+
+// Pieces that a single batch's queries are copied and scored in: it has no other
+// batch's kernels to hide its copy behind (600 queries of 33 to 64 tokens: 15 MB,
+// 0.8 of 9.5 ms)
+uint32_t copy_parts(uint32_t n_tok) { return std::max(1u, std::min(4u, n_tok / 4096u)); }
+
+// Buffer sizes of the centroid scoring of n_tok tokens in such launches: the plans of
+// a full one and of the last one (fewer tokens take more splits, so that a piece's
+// lists can be larger than the whole's)
+void probe_need(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, uint32_t n_part,
+                ProbePlan *need) {
   auto add = [&](uint32_t T) {
     const ProbePlan p = probe_plan(T, h->dix.n_centroid, nprobe, h->n_sm);
     need->n_ent = std::max(need->n_ent, p.n_ent);
@@ -484,7 +497,7 @@ void probe_need(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, ProbePlan *
     need->n_flag = std::max(need->n_flag, p.n_flag);
     need->n_part = std::max(need->n_part, p.n_part);
   };
-  const uint32_t chunk = probe_chunk(nprobe, h->n_sm);
+  const uint32_t chunk = score_chunk(h, n_tok, nprobe, n_part);
   if (n_tok >= chunk) add(chunk);
   if (n_tok % chunk) add(n_tok % chunk);
 }
@@ -612,7 +625,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     const uint32_t s = bt * B, e = std::min(n_query, s + B);
     const uint32_t T = (uint32_t)(off[e] - off[s]);
     tok_cap = std::max(tok_cap, T);
-    probe_need(h, T, nprobe, &need);
+    probe_need(h, T, nprobe, 1, &need);
+    if (host_io && n_batch == 1) probe_need(h, T, nprobe, copy_parts(T), &need);
   }
   const uint32_t rank_stride = nq_max <= 32 ? 32u : 64u;
   // before the first search: about a third of a mean-length list's docs are
@@ -727,10 +741,8 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
       } else if (stage_in) {
         qp = reinterpret_cast<const float *>(w.in + off_bytes);
       } else if (host_io) {
-        // a single batch has no other batch's kernels to hide its copy behind:
         // pieces of it are copied while the pieces before them are scored
-        // (600 queries of 33 to 64 tokens: 15 MB, 0.8 of 9.5 ms)
-        n_part = std::max(1u, std::min(4u, T / 4096u));
+        n_part = copy_parts(T);
         qp = w.q;
         if (n_part > 1) {
           CUDA_TRY(cudaEventRecord(h->ev_in, rs));  // after the caller's prior work
@@ -742,8 +754,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
       CUDA_TRY(rec(ev(bt, 1)));
       w.last_q = qp;
       w.last_off = qo;
-      uint32_t chunk = probe_chunk(nprobe, h->n_sm);
-      if (n_part > 1) chunk = std::min(chunk, ((T / n_part + 255u) & ~255u));
+      const uint32_t chunk = score_chunk(h, T, nprobe, n_part);
       for (uint32_t c = 0, i = 0; c < T; c += chunk, i++) {
         const uint32_t n = std::min(chunk, T - c);
         if (host_io && !pipelined && !stage_in) {
@@ -761,10 +772,13 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
           }
           h2d += (size_t)n * kDim * sizeof(float);
         }
+        const ProbePlan plan = probe_plan(n, h->dix.n_centroid, nprobe, h->n_sm);
+        if (plan.n_ent > w.ent_cap || plan.n_gid > w.gid_cap || plan.n_cnt > w.cnt_cap ||
+            plan.n_flag > w.flag_cap || plan.n_part > w.part_cap)
+          return set_err(MVR_ERR_CUDA, "centroid scoring: %u tokens outgrow their workspace", n);
         CUDA_TRY(launch_probe(qp + (size_t)c * kDim, n, h->cen_sw, h->dix.centroid,
                               h->dix.centroid_t, h->dix.n_centroid, h->dix.n_centroid_pad,
-                              h->bounds, nprobe,
-                              probe_plan(n, h->dix.n_centroid, nprobe, h->n_sm), w.probe,
+                              h->bounds, nprobe, plan, w.probe,
                               w.probe_id + (size_t)c * nprobe, w.probe_s + (size_t)c * nprobe,
                               h->n_sm, h->d_err, rs, &launches));
       }

@@ -300,3 +300,24 @@ def test_exact_rerank_small_grids(n_bit, n_query, width):
                 s, i = g.search(q, k, 8, ptk, tok_off=off, semantics=sem)
                 np.testing.assert_array_equal(i, r[1])
                 np.testing.assert_array_equal(s, r[0])
+
+
+@pytest.mark.parametrize("n_query", [255, 256, 300, 520])
+def test_host_queries_scored_in_pieces(n_query):
+    """Host-buffer calls large enough to be copied and scored in pieces, whose plans take
+    more splits of the centroids than the whole would: the results of small calls."""
+    rng = np.random.default_rng(n_query)
+    n_doc, n_tok, n_cen = 2000, 8, 8192
+    code = rng.integers(0, n_cen, n_doc * n_tok).astype(np.uint32)
+    lengths = np.full(n_doc, n_tok, np.uint32)
+    ivf_off, ivf_size, ivf_ids = pyoracle.ivf_build(code, lengths, n_cen)
+    cen = unit(rng.standard_normal((n_cen, 128)))
+    q = unit(rng.standard_normal((n_query * 32, 128))).reshape(n_query, 32, 128)
+    with Index.from_arrays(lengths, cen, code, ivf_off, ivf_size, ivf_ids,
+                           np.array([-0.1, -0.03, 0.03, 0.1], np.float32), 2,
+                           rng.integers(0, 256, n_doc * n_tok * 32).astype(np.uint8)) as g:
+        s, i = g.search(q, 10, 4, 100)  # the first call sizes the workspace
+        for b in range(0, n_query, 100):
+            s1, i1 = g.search(q[b:b + 100], 10, 4, 100)
+            np.testing.assert_array_equal(i[b:b + 100], i1)
+            np.testing.assert_array_equal(s[b:b + 100], s1)
