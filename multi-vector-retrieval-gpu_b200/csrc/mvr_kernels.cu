@@ -1272,7 +1272,8 @@ rerank_kernel(DevIndex ix, const float *__restrict__ q, const uint64_t *__restri
 // 2^-8), the error of a dot product is at most
 //   |q - bf16(q)| X + |bf16(q)| dX + 2^-13 |q| X,
 // the last term for both sides' FP32 accumulation; 2^-14 max(1, 4 max|q| X)
-// covers an accumulator that starts at an offset of up to 2.04 max|q| X.  The max
+// covers an accumulator that starts at an offset of up to 2.04 max|q| X (the kernels'
+// offset: at most 2 x 1.02 max|q| x_bound, which the index sets to X or less).  The max
 // over a doc's tokens and the clamp at 0 enlarge no error, the sum over query
 // tokens adds them up.  A bound that is not finite keeps every doc.  One CTA per
 // query, the approximate scores' order keys in shared memory.

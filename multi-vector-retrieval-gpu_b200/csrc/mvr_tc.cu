@@ -1664,7 +1664,9 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
 //             by shared-memory atomicMax.
 // D starts at OFF, a power of two above |q.x| for every pair of the CTA
 // (Cauchy-Schwarz with the query-token norms and the index's bound on |x|),
-// so every D value is a positive float ordered like its bit pattern.  With
+// so every D value of a token's row is a positive float ordered like its bit pattern
+// (rows past the last token decode stale ring bytes, which may hold any weight: their
+// values mean nothing, and the epilogue masks them out).  With
 // FEAT the kernel computes the learned pruner's features instead: the
 // centroid part only (no producer, residual decode or residual MMA), and
 // per doc the maxima themselves (per query token the best centroid score

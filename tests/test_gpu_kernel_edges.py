@@ -321,3 +321,40 @@ def test_host_queries_scored_in_pieces(n_query):
             s1, i1 = g.search(q[b:b + 100], 10, 4, 100)
             np.testing.assert_array_equal(i[b:b + 100], i1)
             np.testing.assert_array_equal(s[b:b + 100], s1)
+
+
+def buckets(ix):
+    """[n_vec, 128] bucket of every residual value."""
+    b = ix["n_bit"]
+    r = np.asarray(ix["residual"]).reshape(-1, 128 * b // 8, 1)
+    return ((r >> (8 - b * (np.arange(8 // b) + 1))) & ((1 << b) - 1)).reshape(-1, 128)
+
+
+def with_buckets(ix, bk, weight):
+    b = ix["n_bit"]
+    v = bk.reshape(-1, 128 * b // 8, 8 // b) << (8 - b * (np.arange(8 // b) + 1))
+    return dict(ix, residual=v.sum(2).astype(np.uint8).reshape(np.asarray(ix["residual"]).shape),
+                weight=np.asarray(weight, np.float32))
+
+
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 8])
+@pytest.mark.parametrize("width", [(17, 32), (20, 64)], ids=["narrow", "wide"])
+@pytest.mark.parametrize("large", [1e2, 1e4, 1e6])
+def test_bf16_cut_with_an_unused_large_weight(n_bit, width, large):
+    """A bucket weight far above the others that no token uses: FP32 searches cut by their
+    BF16 scores, and BF16 searches whose re-scored docs are cut, return the oracle's
+    results (the scores' offset has to follow the tokens, as the cut's bound does)."""
+    ix = tiny_index(n_doc=700, n_centroid=48, n_bit=n_bit, seed=110 + n_bit)
+    last = (1 << n_bit) - 1
+    bk = buckets(ix)
+    ix = with_buckets(ix, np.where(bk == last, last - 1, bk), np.append(ix["weight"][:-1], large))
+    o = oracle_of(ix)
+    q, off = make_queries(ix, 140, width, seed=9)
+    with gpu_index(ix) as g:
+        g.set_rescore(400)
+        for k in (1, 10, 60):
+            r = o.search(q, off, k, 8, 400, SEM_PP)
+            for prec in (0, PREC_BF16):
+                s, i = g.search(q, k, 8, 400, tok_off=off, semantics=SEM_PP | prec)
+                np.testing.assert_array_equal(i, r[1])
+                np.testing.assert_array_equal(s, r[0])
