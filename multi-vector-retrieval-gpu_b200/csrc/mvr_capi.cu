@@ -165,13 +165,15 @@ struct mvr_index {
   uint32_t rescore = 0;          // FP32 re-score count of the BF16 path (0: 4 * topk)
   void *lut_bf16 = nullptr;      // [256][8/b] BF16 decode table (b >= 4)
   void *cen_sw = nullptr;        // [C_pad/128][32 KB] swizzled BF16 centroid tiles
-  // max |c|, max |c - bf16(c)| over the centroids; the same of the doc tokens' weights
+  // max |c|, max |c - bf16(c)| over the centroids; the same of the doc tokens' weights;
+  // two words of scratch
   float *bounds = nullptr;
   void *cen_perm = nullptr;      // [C + 1][128] BF16 centroid rows, BF16 K order
   TmWeights tw_bf16{};           // weight tables of the BF16 tensor-memory MaxSim (b <= 2)
   // bounds on the norm of every decoded doc token: by the weight table (FP8, pruner
   // features), and by the weights that the tokens use (BF16; finish_index)
   float x_bound = 0.f, x_bf16 = 0.f;
+  bool bf16_split = false;       // bf16_split_supported
   void *cen8 = nullptr;          // [C][128] E4M3 centroid rows, FP8-rerank K order (b = 2, 4)
   TmWeights tw_fp8{};            // E4M3 weight tables of the FP8 MaxSim (b = 2, 4)
   unsigned *d_err = nullptr;     // device error flags of the tensor-core kernels
@@ -591,7 +593,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     if (!h->prune_wts) return set_err(MVR_ERR_INVALID_ARG, "MVR_PRUNE: no pruner set");
     if (nq_max > 32) return set_err(MVR_ERR_UNSUPPORTED, "MVR_PRUNE: queries of up to 32 tokens");
   }
-  const uint32_t split_tok = bf16_split_supported(h->dix.n_bit, h->x_bf16) ? kBf16SplitTok : 0u;
+  const uint32_t split_tok = h->bf16_split ? kBf16SplitTok : 0u;
   // Exact FP32 search: where a shortlist is long, the BF16 pass first leaves out the
   // docs that provably miss the top topk, and the FP32 kernel scores the rest (39 of
   // 1500 on average for the best 10, 130 of 400 for the best 100).  The
@@ -820,8 +822,9 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
                                     h->n_sm, rs, &launches, h->wait_ns, h->ws_docs));
         else
           CUDA_TRY(launch_rerank_bf16(h->dix, h->cen_perm, h->lut_bf16, h->tw_bf16, qp, qo, nb, sid,
-                                      nsh, probe_topk, sem, nq_min, nq_max, h->x_bf16, w.exact,
-                                      h->d_err, h->n_sm, rs, &launches, h->wait_ns));
+                                      nsh, probe_topk, sem, nq_min, nq_max, h->x_bf16,
+                                      h->bf16_split, w.exact, h->d_err, h->n_sm, rs, &launches,
+                                      h->wait_ns));
         CUDA_TRY(rec(ev(bt, 4)));
         CUDA_TRY(launch_topk(sid, w.exact, nsh, nb, probe_topk, R, w.r_score, w.r_id, w.n_r, rs,
                              &launches));
@@ -855,8 +858,9 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
         }
         if (reach) {
           CUDA_TRY(launch_rerank_bf16(h->dix, h->cen_perm, h->lut_bf16, h->tw_bf16, qp, qo, nb, sid,
-                                      nsh, probe_topk, sem, nq_min, nq_max, h->x_bf16, w.exact,
-                                      h->d_err, h->n_sm, rs, &launches, h->wait_ns));
+                                      nsh, probe_topk, sem, nq_min, nq_max, h->x_bf16,
+                                      h->bf16_split, w.exact, h->d_err, h->n_sm, rs, &launches,
+                                      h->wait_ns));
           CUDA_TRY(launch_maxsim_reach(qp, qo, nb, sid, w.exact, nsh, probe_topk, topk,
                                        h->bounds, split_tok, w.r_id, w.n_r, rs, &launches));
           CUDA_TRY(launch_rerank(h->dix, qp, qo, nb, w.r_id, w.n_r, probe_topk, sem, w.r_exact,
@@ -1044,17 +1048,16 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
   MVR_TRY(dalloc(&sw, (size_t)d.n_centroid_pad * 256, &h->bufs));
   CUDA_TRY(make_centroid_tiles(d.centroid, d.n_centroid, d.n_centroid_pad / 64, sw, h->stream));
   h->cen_sw = sw;
-  MVR_TRY(dalloc(&h->bounds, 4, &h->bufs));
+  MVR_TRY(dalloc(&h->bounds, 6, &h->bufs));
   CUDA_TRY(make_centroid_bounds(d.centroid, d.n_centroid, h->bounds, h->stream));
   CUDA_TRY(make_weight_bounds(d, h->bounds + 2, h->n_sm, h->stream));
   {
     float wmax = 0.f;
     for (uint32_t k = 0; k < (1u << d.n_bit); k++) wmax = std::max(wmax, std::fabs(weight[k]));
-    float cmax = 0.f;
-    float nb[4];
+    float cmax = 0.f, cmin = 0.f, nb[4];
     CUDA_TRY(cudaMemcpyAsync(nb, h->bounds, sizeof(nb), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(max_centroid_norm(d.centroid, d.n_centroid, h->d_err, &cmax, h->stream));  // syncs
-    CUDA_TRY(cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), h->stream));  // was scratch
+    CUDA_TRY(centroid_norm_range(d.centroid, d.n_centroid, (unsigned *)(h->bounds + 4), &cmax,
+                                 &cmin, h->stream));  // syncs
     h->x_bound = cmax + std::sqrt((float)kDim) * wmax;
     // The BF16 kernels' accumulators start at an offset above |q| x_bf16, and the
     // bound by which docs are left out (maxsim_reach_kernel) covers one of |q| X, its X
@@ -1063,6 +1066,7 @@ int finish_index(mvr_index *h, const uint32_t *item_n_vec_host, const uint32_t *
     // the offset is the table's.
     const float seen = (nb[0] + nb[2]) * (1.0f + 0x1p-10f);
     h->x_bf16 = seen < h->x_bound ? seen : h->x_bound;
+    h->bf16_split = bf16_split_supported(d.n_bit, h->x_bf16, cmin);
   }
   uint32_t *cp;
   MVR_TRY(dalloc(&cp, ((size_t)d.n_centroid + 1) * 64, &h->bufs));

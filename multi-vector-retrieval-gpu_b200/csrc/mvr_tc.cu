@@ -2,7 +2,7 @@
 // search path.
 //
 // rerank_tc_kernel scores a query's shortlisted docs (4- and 8-bit codes, queries of
-// more than 32 tokens, or weights too large for the split form) with BF16 operands and
+// more than 32 tokens, or token norms too far apart for the split form) with BF16 operands and
 // FP32 accumulation in TMEM: per 128-token tile the CTA decompresses doc tokens
 // x = centroid + W[bucket] (BF16 centroid table + BF16 decode table, one BF16
 // add) straight into a 128B-swizzled K-major shared-memory tile (operand A,
@@ -2590,10 +2590,15 @@ cudaError_t configure_tc_kernels() {
   return cudaFuncSetAttribute(rerank_tc_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes(8, 64));
 }
 
-// 4- and 8-bit codes: the offset that the split kernel's accumulators start at stays
-// finite for queries of any norm up to 2^66
-bool bf16_split_supported(uint32_t n_bit, float x_bound) {
-  return n_bit <= 2 || x_bound < 0x1p60f;
+// 4- and 8-bit codes have a kernel without an offset (rerank_tc_kernel), which rounds
+// the sum c + w instead; 1- and 2-bit codes have none.  The offset follows the largest
+// token, that rounding each token's own norm.  Scores of ordinary docs beside one token
+// of 1, 16, 32, 64, 256 and 4096 times their norm, 8 bits, 32 query tokens, rms error:
+// split 2.2e-3, 2.2e-3, 2.5e-3, 3.7e-3, 1.4e-2, 2.3e-1, rounded sum 2.6e-3 at each; so
+// the line is at 32, seen from the smallest centroid.  Below 2^60 the offset stays
+// finite for queries of any norm up to 2^66.
+bool bf16_split_supported(uint32_t n_bit, float x_bound, float c_min) {
+  return n_bit <= 2 || (x_bound < 0x1p60f && x_bound <= 32.0f * c_min);
 }
 bool fp8_rerank_supported(uint32_t n_bit) { return n_bit == 2 || n_bit == 4; }
 
@@ -2642,8 +2647,8 @@ cudaError_t make_centroid_fp8(const float *cen, uint32_t n_cent, uint32_t n_bit,
   return cudaGetLastError();
 }
 
-__global__ void centroid_norm_max_kernel(const float *__restrict__ cen, uint32_t n_cent,
-                                         unsigned *__restrict__ out) {
+__global__ void centroid_norm_range_kernel(const float *__restrict__ cen, uint32_t n_cent,
+                                           unsigned *__restrict__ out) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n_cent; c += gridDim.x * blockDim.x) {
     const float4 *row = reinterpret_cast<const float4 *>(cen + (size_t)c * kDim);
     float ss = 0.0f;
@@ -2652,22 +2657,23 @@ __global__ void centroid_norm_max_kernel(const float *__restrict__ cen, uint32_t
       ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
     }
     atomicMax(out, __float_as_uint(sqrtf(ss)));
+    if (ss > 0.0f) atomicMin(out + 1, __float_as_uint(sqrtf(ss)));
   }
 }
 
-cudaError_t max_centroid_norm(const float *cen, uint32_t n_cent, unsigned *d_tmp, float *out,
-                              cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(d_tmp, 0, sizeof(unsigned), st);
+cudaError_t centroid_norm_range(const float *cen, uint32_t n_cent, unsigned *d_tmp, float *c_max,
+                                float *c_min, cudaStream_t st) {
+  const unsigned init[2] = {0u, 0x7fffffffu};
+  unsigned bits[2] = {0u, 0u};
+  cudaError_t e = cudaMemcpyAsync(d_tmp, init, sizeof(init), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
-  centroid_norm_max_kernel<<<296, 256, 0, st>>>(cen, n_cent, d_tmp);
+  centroid_norm_range_kernel<<<296, 256, 0, st>>>(cen, n_cent, d_tmp);
   e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  unsigned bits = 0;
-  e = cudaMemcpyAsync(&bits, d_tmp, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-  if (e != cudaSuccess) return e;
-  e = cudaStreamSynchronize(st);
-  std::memcpy(out, &bits, 4);
-  return e;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(bits, d_tmp, sizeof(bits), cudaMemcpyDeviceToHost, st);
+  const cudaError_t s = cudaStreamSynchronize(st);
+  std::memcpy(c_max, &bits[0], 4);
+  std::memcpy(c_min, &bits[1], 4);
+  return e != cudaSuccess ? e : s;
 }
 
 cudaError_t make_centroid_perm(const float *cen, uint32_t n_cent, uint32_t n_bit, void *out,
@@ -2700,10 +2706,9 @@ cudaError_t launch_rerank_bf16(const DevIndex &ix, const void *cen_perm, const v
                                const TmWeights &tw, const float *q, const uint64_t *q_off,
                                uint32_t n_query, const uint32_t *short_id,
                                const uint32_t *n_short, uint32_t probe_topk, int semantics,
-                               uint32_t nq_min, uint32_t nq_max, float x_bound, float *approx,
-                               unsigned *err, int n_sm, cudaStream_t st, int *n_launch,
-                               uint64_t wait_ns) {
-  const bool split = bf16_split_supported(ix.n_bit, x_bound);
+                               uint32_t nq_min, uint32_t nq_max, float x_bound, bool split,
+                               float *approx, unsigned *err, int n_sm, cudaStream_t st,
+                               int *n_launch, uint64_t wait_ns) {
   if (split && nq_min <= kBf16SplitTok) {  // the longer queries take the other launch
     const uint32_t docs =
         ws_auto_docs(n_query, probe_topk, 2u * (uint32_t)n_sm, ix.n_bit <= 2 ? 128u : 64u);

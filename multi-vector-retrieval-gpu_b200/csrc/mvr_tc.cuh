@@ -23,21 +23,22 @@ TmWeights make_tm_weights(uint32_t n_bit, const float *weight, bool fp8);
 // weights of a residual byte (4 and 8 bits); x_bound: upper bound on the norm of
 // every decoded doc token; wait_ns as launch_rerank_ws.  Queries of up to
 // kBf16SplitTok tokens: BF16 centroid and BF16 weights contribute separately, where
-// bf16_split_supported; otherwise their BF16-rounded sum.
+// split (bf16_split_supported; c_min: the smallest non-zero centroid norm); otherwise their BF16-rounded sum.
 constexpr uint32_t kBf16SplitTok = 32;
-bool bf16_split_supported(uint32_t n_bit, float x_bound);
-// largest L2 norm of the centroid rows (d_tmp: one device word of scratch)
-cudaError_t max_centroid_norm(const float *cen, uint32_t n_cent, unsigned *d_tmp, float *out,
-                              cudaStream_t st);
+bool bf16_split_supported(uint32_t n_bit, float x_bound, float c_min);
+// largest and smallest non-zero L2 norm of the centroid rows (NaN: none); d_tmp: two
+// device words of scratch; synchronises st
+cudaError_t centroid_norm_range(const float *cen, uint32_t n_cent, unsigned *d_tmp, float *c_max,
+                                float *c_min, cudaStream_t st);
 cudaError_t make_centroid_perm(const float *cen, uint32_t n_cent, uint32_t n_bit, void *out,
                                cudaStream_t st);
 cudaError_t launch_rerank_bf16(const DevIndex &ix, const void *cen_perm, const void *lut_bf16,
                                const TmWeights &tw, const float *q, const uint64_t *q_off,
                                uint32_t n_query, const uint32_t *short_id,
                                const uint32_t *n_short, uint32_t probe_topk, int semantics,
-                               uint32_t nq_min, uint32_t nq_max, float x_bound, float *approx,
-                               unsigned *err, int n_sm, cudaStream_t st, int *n_launch,
-                               uint64_t wait_ns);
+                               uint32_t nq_min, uint32_t nq_max, float x_bound, bool split,
+                               float *approx, unsigned *err, int n_sm, cudaStream_t st,
+                               int *n_launch, uint64_t wait_ns);
 // E4M3 centroid rows [C][128] in the FP8 kernel's K order (2- and 4-bit codes)
 bool fp8_rerank_supported(uint32_t n_bit);
 cudaError_t make_centroid_fp8(const float *cen, uint32_t n_cent, uint32_t n_bit, void *out,

@@ -358,3 +358,40 @@ def test_bf16_cut_with_an_unused_large_weight(n_bit, width, large):
                 s, i = g.search(q, k, 8, 400, tok_off=off, semantics=SEM_PP | prec)
                 np.testing.assert_array_equal(i, r[1])
                 np.testing.assert_array_equal(s, r[0])
+
+
+@pytest.mark.parametrize("n_bit", [4, 8])
+@pytest.mark.parametrize("kind", ["weight", "centroid"])
+@pytest.mark.parametrize("large", [30.0, 1e3, 1e5])
+def test_bf16_scores_beside_a_large_token(n_bit, kind, large):
+    """BF16 scores of ordinary docs where one doc holds a token many times their norm:
+    within the rounding of their own values.  Rounding q, c, w and a sum c + w to BF16
+    moves a dot product by at most 2^-9 |q| (|x| + |c| + |w| + |x|), and the FP32
+    accumulation by 2^-13 |q| |x|: less than 2^-7 |q| (|c| + |w|) together."""
+    ix = tiny_index(n_doc=300, n_centroid=48, n_bit=n_bit, seed=120 + n_bit)
+    tok0 = np.concatenate([[0], np.cumsum(ix["item_n_vec"].astype(np.int64))])
+    bk, cen, weight = buckets(ix), ix["centroid"].copy(), ix["weight"].copy()
+    if kind == "weight":  # a bucket that one value of doc 0 alone uses
+        last = (1 << n_bit) - 1
+        bk = np.where(bk == last, last - 1, bk)
+        bk[0, 5], weight[last] = last, large
+        ix = with_buckets(ix, bk, weight)
+    else:                 # a centroid that doc 0's first token alone has
+        cen = np.concatenate([cen, cen[:1] * np.float32(large)])
+        code = np.asarray(ix["vq_code"]).copy()
+        code[0] = 48
+        off, size, ids = pyoracle.ivf_build(code, ix["item_n_vec"], 49)
+        ix = dict(ix, centroid=cen, vq_code=code, ivf_off=off, ivf_size=size, ivf_ids=ids)
+    c = cen[ix["vq_code"]].astype(np.float64)
+    w = ix["weight"].astype(np.float64)[bk]
+    norm = np.linalg.norm(c, axis=1) + np.linalg.norm(w, axis=1)
+    with gpu_index(ix) as g:
+        for nq in (20, 32):
+            q, _ = make_queries(ix, 1, nq, seed=nq)
+            t = g.trace(q, 10, 8, 250, SEM_PP | PREC_BF16)
+            q = q.astype(np.float64)
+            dots = q @ (c + w).T
+            for d, got in zip(t["short_id"], t["short_exact"]):
+                s = slice(tok0[d], tok0[d + 1])
+                tol = np.linalg.norm(q, axis=1).sum() * norm[s].max() * 2.0**-7
+                assert abs(got - dots[:, s].max(1).sum()) <= tol
