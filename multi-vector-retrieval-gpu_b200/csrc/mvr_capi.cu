@@ -477,12 +477,6 @@ int ensure_stage(mvr_index *h, size_t n_ret, size_t in_bytes) {
   return MVR_OK;
 }
 
-// Tokens per launch of the centroid scoring of n_tok tokens that arrive in n_part pieces.
-uint32_t score_chunk(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, uint32_t n_part) {
-  const uint32_t chunk = probe_chunk(nprobe, h->n_sm);
-  return n_part > 1 ? std::min(chunk, ((n_tok / n_part + 255u) & ~255u)) : chunk;
-}
-
 // Pieces that a single batch's queries are copied and scored in: it has no other
 // batch's kernels to hide its copy behind (600 queries of 33 to 64 tokens: 15 MB,
 // 0.8 of 9.5 ms)
@@ -501,7 +495,7 @@ void probe_need(const mvr_index *h, uint32_t n_tok, uint32_t nprobe, uint32_t n_
     need->n_flag = std::max(need->n_flag, p.n_flag);
     need->n_part = std::max(need->n_part, p.n_part);
   };
-  const uint32_t chunk = score_chunk(h, n_tok, nprobe, n_part);
+  const uint32_t chunk = score_chunk(n_tok, h->dix.n_centroid, nprobe, h->n_sm, n_part);
   if (n_tok >= chunk) add(chunk);
   if (n_tok % chunk) add(n_tok % chunk);
 }
@@ -758,7 +752,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
       CUDA_TRY(rec(ev(bt, 1)));
       w.last_q = qp;
       w.last_off = qo;
-      const uint32_t chunk = score_chunk(h, T, nprobe, n_part);
+      const uint32_t chunk = score_chunk(T, h->dix.n_centroid, nprobe, h->n_sm, n_part);
       for (uint32_t c = 0, i = 0; c < T; c += chunk, i++) {
         const uint32_t n = std::min(chunk, T - c);
         if (host_io && !pipelined && !stage_in) {
@@ -1622,7 +1616,7 @@ AssignWork assign_work(uint64_t n_vec, uint32_t n_centroid, int n_sm) {
     at += (bytes + 255) & ~(size_t)255;
     return o;
   };
-  const uint64_t chunk = probe_chunk(1, n_sm);
+  const uint64_t chunk = probe_chunk(n_vec, n_centroid, 1, n_sm);
   const uint32_t first = (uint32_t)std::min(chunk, std::max<uint64_t>(n_vec, 1));
   ProbePlan p = probe_plan(first, n_centroid, 1, n_sm);
   const uint32_t last = (uint32_t)(n_vec % chunk);
@@ -1688,7 +1682,7 @@ int mvr_assign_work_device(const float *d_vec, uint64_t n_vec, const float *d_ce
   CUDA_TRY(make_centroid_bounds(d_centroid, n_centroid, bounds, st));
   CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
   int launches = 0;
-  const uint64_t chunk = probe_chunk(1, n_sm);
+  const uint64_t chunk = probe_chunk(n_vec, n_centroid, 1, n_sm);
   for (uint64_t s = 0; s < n_vec; s += chunk) {
     const uint32_t T = (uint32_t)std::min(chunk, n_vec - s);
     CUDA_TRY(launch_probe(d_vec + s * kDim, T, base + a.sw, d_centroid, ct, n_centroid, c_pad,

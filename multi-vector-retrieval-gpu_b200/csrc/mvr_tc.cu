@@ -826,11 +826,10 @@ __global__ void perm_centroid_kernel(const float *__restrict__ cen, uint32_t n_c
 // tokens, best 8, by FP32 scan 6.91 -> 0.43 ms; and where each of 32 tokens has
 // 296 lists, their selection 606 -> 23 us.
 // ---------------------------------------------------------------------
-constexpr int kPtTok = 128;     // tokens per MMA (M)
-constexpr int kPtCtaTok = 2 * kPtTok;  // tokens per CTA = epilogue threads
+// (mvr_plan.hpp: kPtTok = 128 tokens per MMA (M), kPtCtaTok = 256 per CTA, kPtCen = 128
+// centroids per tile (N))
 constexpr int kPtSrc = 64;      // centroids per pre-swizzled source tile
 constexpr uint32_t kPtSrcBytes = kPtSrc * 256;
-constexpr int kPtCen = 128;     // centroids per tile (N): two source tiles
 constexpr uint32_t kPtTileBytes = 2 * kPtSrcBytes;
 constexpr int kPtStages = 4;    // centroid-tile ring stages
 constexpr int kPtDStages = 3;   // accumulators in TMEM (128 columns each), after A's 2 x 64 columns
@@ -1532,43 +1531,6 @@ cudaError_t make_centroid_tiles(const float *cen, uint32_t n_cent, uint32_t n_ti
                                 cudaStream_t st) {
   swizzle_centroid_kernel<<<592, 256, 0, st>>>(cen, n_cent, n_tiles, reinterpret_cast<uint8_t *>(out));
   return cudaGetLastError();
-}
-
-// Tokens per launch: whole waves of token tiles (4, 2 or 1 as the lists grow),
-// which bounds the lists' memory (at most 0.8 GB).
-uint32_t probe_chunk(uint32_t nprobe, int n_sm) {
-  return (uint32_t)n_sm * kPtCtaTok * (nprobe == 1 ? 4u : nprobe <= 8 ? 2u : 1u);
-}
-
-ProbePlan probe_plan(uint32_t n_tok, uint32_t n_cent, uint32_t nprobe, int n_sm) {
-  ProbePlan p;
-  const uint32_t n_tiles = (n_cent + kPtCen - 1) / kPtCen;
-  const uint32_t tok_tiles = std::max(1u, (n_tok + kPtCtaTok - 1) / kPtCtaTok);
-  // CTAs (one per SM at a time) per token tile: the count that takes the least
-  // time, waves x (centroid tiles of a CTA + 8), 8 being what a split costs:
-  // its start, and lists that fill from nothing
-  uint32_t s = 1;
-  uint64_t least = ~0ull;
-  for (uint32_t c = 1; c <= std::min(n_tiles, 2u * (uint32_t)n_sm / tok_tiles + 4u); c++) {
-    const uint64_t waves = ((uint64_t)tok_tiles * c + n_sm - 1) / n_sm;
-    const uint64_t cost = waves * ((n_tiles + c - 1) / c + 8u);
-    if (cost < least) { least = cost; s = c; }
-  }
-  p.tiles_per_split = (n_tiles + s - 1) / s;
-  p.splits = (n_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
-  p.k = 1;
-  while (p.k < nprobe) p.k *= 2;
-  // a list's expected length is k (1 + ln(C / 8 k)) groups for scores in no
-  // order, and a third more for those within 2 eps (unit vectors of 128
-  // dimensions): 87 of 160 at k = 8 and 65,536 centroids, 14 of 48 at k = 1
-  p.cap = std::min(16u * p.k + 32u, p.tiles_per_split * (kPtCen / 8u));
-  p.n_ent = (size_t)n_tok * p.splits * p.cap * 2;
-  p.n_gid = (size_t)n_tok * p.splits * p.cap;
-  p.n_cnt = (size_t)n_tok * p.splits;
-  p.list_at = 2u + (n_tok + 63u) / 64u;
-  p.n_flag = (size_t)p.list_at + n_tok;
-  p.n_part = (size_t)n_sm * 64u * nprobe;
-  return p;
 }
 
 cudaError_t make_centroid_bounds(const float *cen, uint32_t n_cent, float *bounds,

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "mvr_common.cuh"
+#include "mvr_plan.hpp"
 
 namespace mvr {
 
@@ -89,18 +90,7 @@ cudaError_t launch_prune_mlp(const float *feat, const uint32_t *n_short, uint32_
 cudaError_t make_centroid_tiles(const float *cen, uint32_t n_cent, uint32_t n_tiles, void *out,
                                 cudaStream_t st);
 
-// Centroid scoring and top-nprobe per token (exact; mvr_tc.cu): how a call of
-// n_tok tokens is laid out, and the sizes of its buffers in elements.
-struct ProbePlan {
-  uint32_t tiles_per_split, splits;  // 128-centroid tiles of a CTA, CTAs per token tile
-  uint32_t k;                        // best scores kept: nprobe rounded up to a power of two
-  uint32_t cap;                      // groups listed per token and split
-  uint32_t list_at;                  // first flagged token in flags
-  size_t n_ent, n_gid, n_cnt, n_flag, n_part;
-};
-// tokens per launch at most
-uint32_t probe_chunk(uint32_t nprobe, int n_sm);
-ProbePlan probe_plan(uint32_t n_tok, uint32_t n_cent, uint32_t nprobe, int n_sm);
+// Buffers of a centroid-scoring launch (probe_plan, mvr_plan.hpp)
 struct ProbeBufs {
   float4 *ent;        // [n_ent] listed groups of 8 centroids: their BF16 scores
   uint32_t *gid;      // [n_gid] ... and the group's index

@@ -395,3 +395,27 @@ def test_bf16_scores_beside_a_large_token(n_bit, kind, large):
                 s = slice(tok0[d], tok0[d + 1])
                 tol = np.linalg.norm(q, axis=1).sum() * norm[s].max() * 2.0**-7
                 assert abs(got - dots[:, s].max(1).sum()) <= tol
+
+
+@pytest.mark.parametrize("n_query", [410, 700, 1184])
+def test_probe_lists_at_their_memory_limit(n_query):
+    """Probe launches whose lists the memory limit leaves fewer splits or makes smaller
+    (32 probes of 16,384 centroids): the results of small calls."""
+    rng = np.random.default_rng(n_query)
+    n_doc, n_tok, n_cen = 2000, 8, 16384
+    code = rng.integers(0, n_cen, n_doc * n_tok).astype(np.uint32)
+    lengths = np.full(n_doc, n_tok, np.uint32)
+    ivf_off, ivf_size, ivf_ids = pyoracle.ivf_build(code, lengths, n_cen)
+    q = unit(rng.standard_normal((n_query * 32, 128))).reshape(n_query, 32, 128)
+    with Index.from_arrays(lengths, unit(rng.standard_normal((n_cen, 128))), code, ivf_off, ivf_size,
+                           ivf_ids, np.array([-0.1, -0.03, 0.03, 0.1], np.float32), 2,
+                           rng.integers(0, 256, n_doc * n_tok * 32).astype(np.uint8)) as g:
+        d = torch.from_numpy(q).cuda()  # (host queries would be scored in smaller pieces)
+        ds = torch.empty((n_query, 10), device="cuda")
+        di = torch.empty((n_query, 10), dtype=torch.int32, device="cuda")
+        g.search_device(d.data_ptr(), None, n_query, 32, 10, 32, 100, ds.data_ptr(), di.data_ptr())
+        s, i = ds.cpu().numpy(), di.cpu().numpy().view(np.uint32)
+        for b in range(0, n_query, 100):
+            s1, i1 = g.search(q[b:b + 100], 10, 32, 100)
+            np.testing.assert_array_equal(i[b:b + 100], i1)
+            np.testing.assert_array_equal(s[b:b + 100], s1)
