@@ -395,7 +395,9 @@ int mvr_kmeans_accumulate_device(const float *d_vec, uint64_t n_vec,
 /* Reduction of an exhaustive MaxSim: out[q][d] = sum over query q's tokens
  * (rows q_off[q] .. q_off[q+1] of s, leading dimension ld) of the max over doc
  * d's tokens (columns doc_off[d] .. doc_off[d+1]); s and out float, or double
- * with f64 != 0.  Device pointers; asynchronous on cuda_stream. */
+ * with f64 != 0.  Empty docs give -inf, queries without tokens 0.  Device
+ * pointers (s may be null where ld is 0: no doc has a token); asynchronous on
+ * cuda_stream. */
 int mvr_segment_maxsum_device(const void *d_s, int f64, uint64_t ld,
                               const int64_t *d_q_off, uint32_t n_query,
                               const int64_t *d_doc_off, uint32_t n_doc,

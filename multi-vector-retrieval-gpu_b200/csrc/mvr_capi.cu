@@ -1771,7 +1771,10 @@ int mvr_kmeans_accumulate_device(const float *d_vec, uint64_t n_vec, uint32_t di
 int mvr_segment_maxsum_device(const void *d_s, int f64, uint64_t ld, const int64_t *d_q_off,
                               uint32_t n_query, const int64_t *d_doc_off, uint32_t n_doc,
                               void *d_out, void *cuda_stream) {
-  if (!d_s || !d_q_off || !d_doc_off || !d_out) return set_err(MVR_ERR_INVALID_ARG, "null argument");
+  if (n_query == 0 || n_doc == 0) return MVR_OK;  // no output (empty buffers may be null)
+  // ld 0: no doc has a token, s is not read
+  if ((!d_s && ld) || !d_q_off || !d_doc_off || !d_out)
+    return set_err(MVR_ERR_INVALID_ARG, "null argument");
   CUDA_TRY(launch_segment_maxsum(d_s, f64 != 0, ld, d_q_off, n_query, d_doc_off, n_doc, d_out,
                                  (cudaStream_t)cuda_stream));
   return MVR_OK;

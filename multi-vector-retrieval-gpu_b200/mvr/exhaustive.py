@@ -34,7 +34,9 @@ def _maxsum(s, q_off, lens):
     if doc_off[-1] != s.shape[1]:
         raise ValueError(f"{s.shape[1]} doc tokens for lengths that sum to {doc_off[-1]}")
     doc_off = torch.from_numpy(doc_off).to(s.device)
-    if s.is_cuda and s.dtype in (torch.float64, torch.float32) and not s.requires_grad:
+    # (a matrix without elements has no address)
+    if (s.is_cuda and s.dtype in (torch.float64, torch.float32) and not s.requires_grad
+            and s.numel()):
         s = s.contiguous()
         out = torch.empty((n_query, nd), dtype=s.dtype, device=s.device)
         with torch.cuda.device(s.device):

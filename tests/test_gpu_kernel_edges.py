@@ -419,3 +419,19 @@ def test_probe_lists_at_their_memory_limit(n_query):
             s1, i1 = g.search(q[b:b + 100], 10, 32, 100)
             np.testing.assert_array_equal(i[b:b + 100], i1)
             np.testing.assert_array_equal(s[b:b + 100], s1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_exhaustive_of_nothing(dtype):
+    """No queries, queries without tokens, docs that are all empty, no docs: the results
+    of the torch form on the CPU."""
+    g = torch.Generator().manual_seed(4)
+    doc, q = (torch.randn((n, 128), generator=g, dtype=dtype) for n in (40, 6))
+    none = doc[:0]
+    pieces = [(0, [0, 0, 0], none), (3, [7, 0, 33], doc), (6, [], none), (6, [0], none)]
+    for qq, off in ((q, [0, 2, 2, 6]), (none, [0]), (none, [0, 0, 0])):
+        want = exhaustive.exhaustive_topk_stream(qq, off, pieces, 5, dtype)
+        got = exhaustive.exhaustive_topk_stream(qq.cuda(), off, [(d, n, x.cuda()) for d, n, x in pieces], 5, dtype)
+        np.testing.assert_array_equal(got[1], want[1])
+        # 6 terms of size ~30, products summed in another order: 128 * 6 ulps of 64
+        np.testing.assert_allclose(got[0], want[0], rtol=0, atol=128 * 6 * 64 * torch.finfo(dtype).eps)
