@@ -27,11 +27,12 @@ def _doc_ranges(lens, chunk_tokens):
 
 def _maxsum(s, q_off, lens):
     """[n_query, n_doc]: per query token the max over each doc's columns of s
-    [tokens, doc tokens], summed over the query's tokens."""
+    [tokens, doc tokens], summed over the query's tokens.  Columns past the docs' tokens
+    (a padded piece) belong to no doc."""
     n_query, nd = len(q_off) - 1, len(lens)
     doc_off = np.zeros(nd + 1, np.int64)
     doc_off[1:] = np.cumsum(lens)
-    if doc_off[-1] != s.shape[1]:
+    if doc_off[-1] > s.shape[1] or (np.asarray(lens) < 0).any():
         raise ValueError(f"{s.shape[1]} doc tokens for lengths that sum to {doc_off[-1]}")
     doc_off = torch.from_numpy(doc_off).to(s.device)
     # (a matrix without elements has no address)

@@ -435,3 +435,14 @@ def test_exhaustive_of_nothing(dtype):
         np.testing.assert_array_equal(got[1], want[1])
         # 6 terms of size ~30, products summed in another order: 128 * 6 ulps of 64
         np.testing.assert_allclose(got[0], want[0], rtol=0, atol=128 * 6 * 64 * torch.finfo(dtype).eps)
+
+
+def test_exhaustive_of_a_padded_piece():
+    """Tokens behind the last doc's count for no doc, on the GPU as on the CPU."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    s = torch.randn((70, 301), device="cuda", generator=g, dtype=torch.float64)
+    q_off, lens = torch.tensor([0, 33, 70]), np.array([40, 0, 200])
+    got = exhaustive._maxsum(s, q_off.cuda(), lens)
+    want = exhaustive._maxsum(s[:, :240].cpu(), q_off, lens)
+    # up to 37 terms of size ~4 in another order: 37 ulps of 256
+    torch.testing.assert_close(got.cpu(), want, rtol=0, atol=37 * 256 * torch.finfo(s.dtype).eps)

@@ -3,6 +3,7 @@ builder's pure-host helpers (sample selection, centroid-count formula, exact
 order statistics by bisection, IVF build), and the exhaustive ground truth
 (torch, CPU tensors here) against the oracle's FP64 exhaustive MaxSim."""
 import numpy as np
+import pytest
 import torch
 
 import pyoracle
@@ -172,3 +173,18 @@ def test_exhaustive_stream_fp32_screen_matches_fp64():
     np.testing.assert_array_equal(i32, i64)
     np.testing.assert_allclose(s32, s64, rtol=1e-5)
 
+
+
+def test_maxsum_lengths_that_cover_part_of_the_tokens():
+    """Docs' lengths may end before the piece's tokens do (a padded piece: what is behind
+    them counts for no doc); longer or negative ones are refused."""
+    g = torch.Generator().manual_seed(5)
+    s = torch.randn((6, 10), generator=g, dtype=torch.float64)
+    q_off = torch.tensor([0, 2, 6])
+    got = exhaustive._maxsum(s, q_off, np.array([4, 3]))
+    want = torch.stack([s[:, :4].max(1).values, s[:, 4:7].max(1).values], 1)
+    want = torch.stack([want[:2].sum(0), want[2:].sum(0)])
+    torch.testing.assert_close(got, want, rtol=0, atol=1e-14)
+    for lens in ([4, 7], [12], [4, -2, 5], [-1, 3]):
+        with pytest.raises((ValueError, RuntimeError)):
+            exhaustive._maxsum(s, q_off, np.array(lens))
