@@ -98,7 +98,9 @@ typedef struct {
   double stage_ms[6];     /* CUDA-event time summed over batches: query
                              copy, scoring + probe, filter, rerank (FP32 or
                              BF16 tensor-core), FP32 re-score + top-k,
-                             result copy */
+                             result copy.  Of copies that overlap scoring
+                             (several batches; a large single one, copied in
+                             pieces) the first is what a batch waits for */
   uint64_t n_prune_fallback; /* MVR_PRUNE: queries whose whole shortlist was
                                 scored (low-confidence predictions) */
 } mvr_stats;
@@ -219,7 +221,8 @@ int mvr_search(mvr_index *h, const float *query_l, const uint64_t *tok_off,
  * stage_time_s[i*6 + k], k = 0 query copy, 1 centroid scoring + probe,
  * 2 candidate filter + shortlist, 3 rerank, 4 re-score + top-k, 5 result
  * copy -- the stage columns of the reference's performance TSV
- * (IGPGPUBasic.cpp:183-204). */
+ * (IGPGPUBasic.cpp:183-204).  A single batch is copied as a whole before it is
+ * scored; of several, stage 0 is what a batch waits for. */
 int mvr_search_staged(mvr_index *h, const float *query_l,
                       const uint64_t *tok_off, uint32_t n_query,
                       uint32_t query_n_vec, uint32_t topk, uint32_t nprobe,

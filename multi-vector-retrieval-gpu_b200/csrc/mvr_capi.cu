@@ -552,7 +552,9 @@ int build_offsets(const uint64_t *tok_off, uint32_t n_query, uint32_t query_n_ve
 // stage k of a batch = events[bt*kStages+k] .. events[bt*kStages+k+1]:
 //   0 query copy, 1 centroid scoring + probe, 2 candidate filter + shortlist,
 //   3 rerank (FP32, or BF16 tensor-core), 4 FP32 re-score + top-k, 5 result copy.
-
+// Stage 0 is what of the copy the batch waits for: all of a small call's, and of a
+// single batch's where stage_s asks for stage times; of several batches, or of a single
+// one copied in pieces, what the scoring before does not hide.
 int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, uint32_t n_query,
                 uint32_t query_n_vec, uint32_t topk, uint32_t nprobe, uint32_t probe_topk,
                 uint32_t flags, float *out_s, uint32_t *out_id, double *query_time_s,
@@ -697,6 +699,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     if (stage_in) {  // offsets and queries in one copy
       std::memcpy(w.h_in, w.h_off, 2 * n_off * sizeof(uint64_t));
       std::memcpy(w.h_in + off_bytes, query, in_bytes - off_bytes);
+      CUDA_TRY(rec(ev(0, 0)));  // the copy is stage 0
       CUDA_TRY(cudaMemcpyAsync(w.in, w.h_in, in_bytes, cudaMemcpyHostToDevice, rs));
       d_off = reinterpret_cast<const uint64_t *>(w.in);
       h2d += in_bytes - off_bytes;
@@ -707,7 +710,7 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     // host buffers: batch bt's query tokens go to device buffer bt % 2 on
     // the copy stream, one batch ahead of the kernels, once batch bt - 2
     // (the buffer's previous user) has finished
-    // (a single batch has nothing to overlap: its copy stays on rs)
+    // (a single batch: copy_piece below)
     const bool pipelined = host_io && n_batch > 1;
     auto qbuf = [&](uint32_t bt) { return (bt & 1) ? w.q2 : w.q; };
     auto copy_in = [&](uint32_t bt) -> int {
@@ -727,11 +730,28 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
     }
     for (uint32_t bt = 0; bt < n_batch; bt++) {
       const uint32_t s = bt * B, e = std::min(n_query, s + B), nb = e - s;
-      CUDA_TRY(rec(ev(bt, 0)));
+      if (!stage_in) CUDA_TRY(rec(ev(bt, 0)));
       const uint32_t T = (uint32_t)(off[e] - off[s]);
       const uint64_t *qo = d_off + (size_t)s + bt;
       const float *qp;
       uint32_t n_part = 1;  // pieces that the queries are copied and scored in
+      // piece i, n tokens from token c, to w.q: on rs where it is the only one, else on
+      // the copy stream, rs waiting for it
+      auto copy_piece = [&](uint32_t c, uint32_t n, uint32_t i) -> int {
+        CUDA_TRY(cudaMemcpyAsync(w.q + (size_t)c * kDim, query + (off[s] + c) * kDim,
+                                 (size_t)n * kDim * sizeof(float), cudaMemcpyHostToDevice,
+                                 n_part > 1 ? h->copy_stream : rs));
+        h2d += (size_t)n * kDim * sizeof(float);
+        if (n_part == 1) return MVR_OK;
+        while (h->copy_events.size() <= i) {
+          cudaEvent_t e;
+          CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+          h->copy_events.push_back(e);
+        }
+        CUDA_TRY(cudaEventRecord(h->copy_events[i], h->copy_stream));
+        CUDA_TRY(cudaStreamWaitEvent(rs, h->copy_events[i], 0));
+        return MVR_OK;
+      };
       if (pipelined) {
         if (bt + 1 < n_batch) MVR_TRY(copy_in(bt + 1));
         CUDA_TRY(cudaStreamWaitEvent(rs, h->copy_events[bt], 0));
@@ -739,8 +759,9 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
       } else if (stage_in) {
         qp = reinterpret_cast<const float *>(w.in + off_bytes);
       } else if (host_io) {
-        // pieces of it are copied while the pieces before them are scored
-        n_part = copy_parts(T);
+        // pieces of it are copied while the pieces before them are scored, except where
+        // stage times are asked for: then it is copied as a whole, in stage 0
+        n_part = stage_s ? 1u : copy_parts(T);
         qp = w.q;
         if (n_part > 1) {
           CUDA_TRY(cudaEventRecord(h->ev_in, rs));  // after the caller's prior work
@@ -749,27 +770,15 @@ int search_impl(mvr_index *h, const float *query, const uint64_t *tok_off_in, ui
       } else {
         qp = query + off[s] * kDim;
       }
+      const uint32_t chunk = score_chunk(T, h->dix.n_centroid, nprobe, h->n_sm, n_part);
+      if (host_io && !pipelined && !stage_in)
+        MVR_TRY(copy_piece(0, n_part > 1 ? std::min(chunk, T) : T, 0));
       CUDA_TRY(rec(ev(bt, 1)));
       w.last_q = qp;
       w.last_off = qo;
-      const uint32_t chunk = score_chunk(T, h->dix.n_centroid, nprobe, h->n_sm, n_part);
       for (uint32_t c = 0, i = 0; c < T; c += chunk, i++) {
         const uint32_t n = std::min(chunk, T - c);
-        if (host_io && !pipelined && !stage_in) {
-          CUDA_TRY(cudaMemcpyAsync(w.q + (size_t)c * kDim, query + (off[s] + c) * kDim,
-                                   (size_t)n * kDim * sizeof(float), cudaMemcpyHostToDevice,
-                                   n_part > 1 ? h->copy_stream : rs));
-          if (n_part > 1) {
-            while (h->copy_events.size() <= i) {
-              cudaEvent_t e;
-              CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-              h->copy_events.push_back(e);
-            }
-            CUDA_TRY(cudaEventRecord(h->copy_events[i], h->copy_stream));
-            CUDA_TRY(cudaStreamWaitEvent(rs, h->copy_events[i], 0));
-          }
-          h2d += (size_t)n * kDim * sizeof(float);
-        }
+        if (n_part > 1 && c > 0) MVR_TRY(copy_piece(c, n, i));
         const ProbePlan plan = probe_plan(n, h->dix.n_centroid, nprobe, h->n_sm);
         if (plan.n_ent > w.ent_cap || plan.n_gid > w.gid_cap || plan.n_cnt > w.cnt_cap ||
             plan.n_flag > w.flag_cap || plan.n_part > w.part_cap)

@@ -446,3 +446,32 @@ def test_exhaustive_of_a_padded_piece():
     want = exhaustive._maxsum(s[:, :240].cpu(), q_off, lens)
     # up to 37 terms of size ~4 in another order: 37 ulps of 256
     torch.testing.assert_close(got.cpu(), want, rtol=0, atol=37 * 256 * torch.finfo(s.dtype).eps)
+
+
+@pytest.mark.parametrize("n_query", [15, 520])
+def test_stage_times_of_one_batch(n_query):
+    """Timed host calls of one batch: the query copy is stage 0 (it cannot be faster than
+    the bus), the stages add up to the device time, and a query's time is its batch's.  Without stage
+    times the larger call is copied in four pieces: stage 0 is the first."""
+    rng = np.random.default_rng(n_query)
+    n_doc, n_tok, n_cen = 2000, 8, 1024
+    code = rng.integers(0, n_cen, n_doc * n_tok).astype(np.uint32)
+    lengths = np.full(n_doc, n_tok, np.uint32)
+    ivf_off, ivf_size, ivf_ids = pyoracle.ivf_build(code, lengths, n_cen)
+    q = unit(rng.standard_normal((n_query * 32, 128))).reshape(n_query, 32, 128)
+    least = q.nbytes / 64e9  # 64 GB/s: what PCIe 5 x16 carries at most
+    with Index.from_arrays(lengths, unit(rng.standard_normal((n_cen, 128))), code, ivf_off, ivf_size,
+                           ivf_ids, np.array([-0.1, -0.03, 0.03, 0.1], np.float32), 2,
+                           rng.integers(0, 256, n_doc * n_tok * 32).astype(np.uint8)) as g:
+        s0, i0 = g.search(q, 10, 4, 100)
+        for _ in range(3):
+            s, i, st = g.search(q, 10, 4, 100, with_stats=True, with_stages=True)
+            stages = st["stage_time_s"]
+            np.testing.assert_array_equal(i, i0)
+            np.testing.assert_array_equal(s, s0)
+            assert st["n_batch"] == 1 and (stages[:, 0] >= least).all()
+            np.testing.assert_allclose(stages.sum(1), st["query_time_s"], rtol=0, atol=50e-6)
+            np.testing.assert_allclose(st["query_time_s"], st["device_ms"] * 1e-3, rtol=0, atol=50e-6)
+            _, _, st = g.search(q, 10, 4, 100, with_stats=True)
+            assert st["stage_ms"][0] * 1e-3 >= (least if n_query == 15 else least / 4)
+            assert abs(sum(st["stage_ms"]) - st["device_ms"]) <= 0.05
