@@ -45,12 +45,17 @@ def _p(t):
 def assign(vec, centroid, stream=None):
     """Best centroid and its score (+ 1) per vector, FP32, lowest id on ties
     (mvr_assign_work_device, its workspace from torch's allocator)."""
-    code = torch.empty(vec.shape[0], dtype=torch.int32, device=vec.device)
-    score = torch.empty(vec.shape[0], dtype=torch.float32, device=vec.device)
-    st = C.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
+    current = torch.cuda.current_stream()
+    st = C.c_void_p((current if stream is None else stream).cuda_stream)
     n = C.c_size_t()
     check(lib().mvr_assign_work_bytes(vec.shape[0], centroid.shape[0], C.byref(n)))
-    work = torch.empty(n.value, dtype=torch.uint8, device=vec.device)
+    with torch.cuda.stream(stream):  # memory that is free for the stream which writes it
+        code = torch.empty(vec.shape[0], dtype=torch.int32, device=vec.device)
+        score = torch.empty(vec.shape[0], dtype=torch.float32, device=vec.device)
+        work = torch.empty(n.value, dtype=torch.uint8, device=vec.device)
+    if stream is not None:  # the caller goes on with them on the current stream
+        code.record_stream(current)
+        score.record_stream(current)
     check(lib().mvr_assign_work_device(_p(vec), vec.shape[0], _p(centroid), centroid.shape[0],
                                        centroid.shape[1], _p(code), _p(score), _p(work), n.value,
                                        st))

@@ -475,3 +475,25 @@ def test_stage_times_of_one_batch(n_query):
             _, _, st = g.search(q, 10, 4, 100, with_stats=True)
             assert st["stage_ms"][0] * 1e-3 >= (least if n_query == 15 else least / 4)
             assert abs(sum(st["stage_ms"]) - st["device_ms"]) <= 0.05
+
+
+def test_assign_beside_pending_work():
+    """assign on a side stream while the current one still has to read a freed block as
+    large as assign's workspace: the block keeps its values, the codes are the oracle's."""
+    import ctypes as C
+
+    from mvr._lib import check, lib
+    rng = np.random.default_rng(9)
+    x, cen = unit(rng.standard_normal((5000, 128))), unit(rng.standard_normal((1000, 128)))
+    dx, dc = torch.from_numpy(x).cuda(), torch.from_numpy(cen).cuda()
+    n = C.c_size_t()
+    check(lib().mvr_assign_work_bytes(5000, 1000, C.byref(n)))
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    block = torch.full((n.value,), 171, dtype=torch.uint8, device="cuda")
+    torch.cuda._sleep(500_000_000)  # some 0.3 s
+    kept = block.clone()
+    del block
+    code, _ = build.assign(dx, dc, stream=side)
+    np.testing.assert_array_equal(code.cpu().numpy(), pyoracle.assign(x, cen).astype(np.int64))
+    assert bool((kept == 171).all())

@@ -188,3 +188,56 @@ def test_maxsum_lengths_that_cover_part_of_the_tokens():
     for lens in ([4, 7], [12], [4, -2, 5], [-1, 3]):
         with pytest.raises((ValueError, RuntimeError)):
             exhaustive._maxsum(s, q_off, np.array(lens))
+
+
+def test_assign_allocates_on_the_stream_it_runs_on(monkeypatch):
+    """build.assign on another stream than the current one: outputs and workspace come
+    from that stream's memory (a block that work on the current stream still reads may be
+    free for the current stream alone), and the outputs are recorded on the current one,
+    where the caller uses them."""
+    class Tensor:
+        shape, device = (5, 128), "cuda:0"
+
+        def data_ptr(self):
+            return 256
+
+        def record_stream(self, stream):
+            recorded.append((self, stream))
+
+    class On:
+        def __init__(self, stream):
+            self.stream = stream
+
+        def __enter__(self):
+            stack.append(self.stream)
+
+        def __exit__(self, *a):
+            stack.pop()
+
+    class Lib:
+        def mvr_assign_work_bytes(self, *a):
+            return 0
+
+        def mvr_assign_work_device(self, *a):
+            return 0
+
+    class Stream:
+        cuda_stream = 7
+
+    current, other = Stream(), Stream()
+    for given in (None, other):
+        stack, made, recorded = [None], [], []
+
+        def empty(*a, **k):
+            t = Tensor()
+            made.append((t, stack[-1]))
+            return t
+
+        monkeypatch.setattr(build.torch, "empty", empty)
+        monkeypatch.setattr(build.torch.cuda, "stream", On)
+        monkeypatch.setattr(build.torch.cuda, "current_stream", lambda *a: current)
+        monkeypatch.setattr(build, "lib", Lib)
+        out = build.assign(Tensor(), Tensor(), given)
+        assert len(made) == 3 and all(s is given for _, s in made)
+        if given is other:
+            assert {id(t) for t, s in recorded if s is current} == {id(t) for t in out}
