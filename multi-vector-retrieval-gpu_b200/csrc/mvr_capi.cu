@@ -1608,7 +1608,7 @@ int mvr_unpack_buckets(mvr_index *h, const uint64_t *vec_id, uint64_t n, uint8_t
 // Layout of an assignment call's workspace (byte offsets, 256-aligned).
 namespace {
 struct AssignWork {
-  size_t ct, sw, bounds, err, score, ent, gid, cnt, eps2, flags, part_id, part_s, total;
+  size_t ct, sw, cen, bounds, err, score, ent, gid, cnt, eps2, flags, part_id, part_s, total;
 };
 int assign_sms(int *n_sm) {
   int dev = 0;
@@ -1638,6 +1638,7 @@ AssignWork assign_work(uint64_t n_vec, uint32_t n_centroid, int n_sm) {
   }
   w.ct = take((size_t)kDim * ((n_centroid + 127u) / 128u * 128u) * sizeof(float));
   w.sw = take((size_t)((n_centroid + 127u) / 128u) * 128 * 256);
+  w.cen = take((size_t)n_centroid * kDim * sizeof(float));  // of centroids off a 16-byte boundary
   w.bounds = take(2 * sizeof(float));
   w.err = take(sizeof(unsigned));
   w.score = take(first * sizeof(float));
@@ -1686,6 +1687,11 @@ int mvr_assign_work_device(const float *d_vec, uint64_t n_vec, const float *d_ce
               (uint32_t *)(base + a.cnt), (float *)(base + a.eps2),
               (uint32_t *)(base + a.flags), (uint32_t *)(base + a.part_id),
               (float *)(base + a.part_s)};
+  if ((uintptr_t)d_centroid & 15) {  // the kernels read its rows 16 bytes at a time
+    CUDA_TRY(cudaMemcpyAsync(base + a.cen, d_centroid, (size_t)n_centroid * kDim * sizeof(float),
+                             cudaMemcpyDeviceToDevice, st));
+    d_centroid = (const float *)(base + a.cen);
+  }
   CUDA_TRY(launch_transpose_centroid(d_centroid, n_centroid, c_pad, ct, st));
   CUDA_TRY(make_centroid_tiles(d_centroid, n_centroid, c_pad / 64u, base + a.sw, st));
   CUDA_TRY(make_centroid_bounds(d_centroid, n_centroid, bounds, st));

@@ -497,3 +497,16 @@ def test_assign_beside_pending_work():
     code, _ = build.assign(dx, dc, stream=side)
     np.testing.assert_array_equal(code.cpu().numpy(), pyoracle.assign(x, cen).astype(np.int64))
     assert bool((kept == 171).all())
+
+
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_assign_centroids_at_any_offset(shift):
+    """Centroids that start at any 4-byte offset (rows of a larger buffer)."""
+    rng = np.random.default_rng(shift)
+    x, cen = unit(rng.standard_normal((700, 128))), unit(rng.standard_normal((300, 128)))
+    buf = torch.zeros(300 * 128 + shift, device="cuda")
+    buf[shift:] = torch.from_numpy(cen.reshape(-1)).cuda()
+    code, score = build.assign(torch.from_numpy(x).cuda(), buf[shift:].view(300, 128))
+    same, s = build.assign(torch.from_numpy(x).cuda(), torch.from_numpy(cen).cuda())
+    np.testing.assert_array_equal(code.cpu().numpy(), pyoracle.assign(x, cen).astype(np.int64))
+    assert torch.equal(code, same) and torch.equal(score, s)
