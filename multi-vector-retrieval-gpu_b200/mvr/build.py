@@ -154,9 +154,12 @@ def train(sample, n_centroid, n_bit, kmeans_iter=20, seed=123, assign_fn=assign)
     """Centroids, quantile cutoffs and bucket weights from the k-means sample."""
     cen = kmeans(sample, n_centroid, kmeans_iter, seed, assign_fn)
     s_code, _ = assign_fn(sample, cen)
-    if n_bit in (1, 2, 4, 8):
+    if (n_bit in (1, 2, 4, 8) and sample.is_cuda and sample.dtype == torch.float32
+            and sample.shape[1] == 128 and sample.is_contiguous()
+            and s_code.device == sample.device and s_code.dtype == torch.int32
+            and s_code.is_contiguous()):
         cutoff, weight = residual_quantiles(sample, cen, s_code, n_bit)
-    else:  # widths no codec here packs
+    else:  # samples, codes (of the caller's assign_fn) and widths that the kernels do not take
         cutoff, weight = quantize_params((sample - cen[s_code.long()]).reshape(-1), n_bit)
     return cen, cutoff, weight
 

@@ -241,3 +241,27 @@ def test_assign_allocates_on_the_stream_it_runs_on(monkeypatch):
         assert len(made) == 3 and all(s is given for _, s in made)
         if given is other:
             assert {id(t) for t, s in recorded if s is current} == {id(t) for t in out}
+
+
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 3])
+@pytest.mark.parametrize("kind", ["cpu", "strided", "int64 codes"])
+def test_train_takes_what_the_kernels_do_not(monkeypatch, kind, n_bit):
+    """train with an assign_fn of the caller's: cutoffs and weights of samples and codes
+    that the residual kernels cannot read (here on the CPU) by torch."""
+    g = torch.Generator().manual_seed(n_bit)
+    x = torch.randn((300, 256 if kind == "strided" else 128), generator=g)[:, ::2 if kind == "strided" else 1]
+
+    def nearest(v, c):
+        s, i = (v @ c.T).max(1)
+        return (i if kind == "int64 codes" else i.int()), s
+
+    def refuse(*a):
+        raise AssertionError("the kernels take CUDA float32 rows of 128")
+
+    monkeypatch.setattr(build.torch.cuda, "current_stream", lambda *a: type("S", (), {"cuda_stream": 0}))
+    monkeypatch.setattr(build, "residual_quantiles", refuse)
+    cen, cut, w = build.train(x, 5, n_bit, kmeans_iter=0, assign_fn=nearest)
+    err = np.sort((x - cen[nearest(x, cen)[0].long()]).numpy().reshape(-1))
+    n = 1 << n_bit
+    np.testing.assert_array_equal(cut, [err[int((i + 1) / n * err.size)] for i in range(n - 1)])
+    np.testing.assert_array_equal(w, [err[int((i + 0.5) / n * err.size)] for i in range(n)])
