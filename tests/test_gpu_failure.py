@@ -35,3 +35,26 @@ def test_fp8_wait_timeout_reports_error_and_handle_recovers():
             for d, sc in zip(i1[k], s1[k]):
                 if d != 0xFFFFFFFF:
                     assert sc == o.maxsim_item(q[off[k]:off[k + 1]], int(d))
+
+
+@pytest.mark.parametrize("n_bit", [2, 8])
+def test_exact_search_wait_timeout_reports_error_and_handle_recovers(n_bit):
+    """The same for exact FP32 searches long enough to be cut by their BF16 scores, whose
+    kernel has the bounded waits."""
+    ix = tiny_index(n_doc=700, n_centroid=48, n_bit=n_bit, seed=63)
+    q, off = make_queries(ix, 140, 32, seed=64)
+    want = oracle_of(ix).search(q, off, 10, 8, 400)
+    with Index.from_arrays(ix["item_n_vec"], ix["centroid"], ix["vq_code"], ix["ivf_off"],
+                           ix["ivf_size"], ix["ivf_ids"], ix["weight"], ix["n_bit"],
+                           ix["residual"]) as g:
+        q = q.reshape(140, 32, 128)
+        g.set_wait_limit(1)
+        with pytest.raises(_lib.MvrError) as e:
+            g.search(q, 10, 8, 400)
+        assert e.value.code == _lib.MVR_ERR_CUDA and "timed out" in str(e.value)
+        g.search(q[:2], 10, 8, 400)  # too short to be cut: no such wait
+        g.set_wait_limit(0)
+        for _ in range(2):
+            s, i = g.search(q, 10, 8, 400)
+            np.testing.assert_array_equal(i, want[1])
+            np.testing.assert_array_equal(s, want[0])

@@ -510,3 +510,29 @@ def test_assign_centroids_at_any_offset(shift):
     same, s = build.assign(torch.from_numpy(x).cuda(), torch.from_numpy(cen).cuda())
     np.testing.assert_array_equal(code.cpu().numpy(), pyoracle.assign(x, cen).astype(np.int64))
     assert torch.equal(code, same) and torch.equal(score, s)
+
+
+@pytest.mark.parametrize("n_bit", [1, 2, 4, 8])
+@pytest.mark.parametrize("sem", [SEM_PP, SEM_BASIC], ids=["pp", "basic"])
+def test_bf16_cut_of_equal_docs(n_bit, sem):
+    """Queries of 17 to 32 tokens, which are cut at every code width: a corpus of docs that
+    all tie, and one of distinct docs; by the launches, the cut did run."""
+    ix = tiny_index(n_doc=300, n_centroid=16, n_bit=n_bit, seed=130 + n_bit, lengths=[7] * 300)
+    dup = dict(ix)
+    for k in ("vq_code", "residual"):
+        per = np.asarray(ix[k]).reshape(300, -1)
+        dup[k] = np.repeat(per[:1], 300, axis=0).reshape(np.asarray(ix[k]).shape)
+    dup["ivf_off"], dup["ivf_size"], dup["ivf_ids"] = pyoracle.ivf_build(
+        dup["vq_code"], dup["item_n_vec"], 16)
+    q, off = make_queries(ix, 140, (17, 32), seed=4)
+    for x in (ix, dup):
+        o = oracle_of(x)
+        with gpu_index(x) as g:
+            for k in (1, 60):
+                r = o.search(q, off, k, 8, 250, sem)
+                s, i, cut = g.search(q, k, 8, 250, tok_off=off, semantics=sem, with_stats=True)
+                np.testing.assert_array_equal(i, r[1])
+                np.testing.assert_array_equal(s, r[0])
+                *_, plain = g.search(q, k, 8, 230, tok_off=off, semantics=sem, with_stats=True)
+                # 140 x 250 docs are cut, 140 x 230 are not: the BF16 MaxSim and the cut
+                assert cut["gpu_launches"] == plain["gpu_launches"] + 2
