@@ -17,6 +17,7 @@ Returns CUDA tensors; `to_host` gives numpy arrays for formats.write_index_dir.
 `build_index_stream` runs the same pipeline over a corpus generated (or read)
 one doc range at a time, with the tensor-core assignment by default.
 """
+import contextlib
 import ctypes as C
 import math
 import random
@@ -49,7 +50,8 @@ def assign(vec, centroid, stream=None):
     st = C.c_void_p((current if stream is None else stream).cuda_stream)
     n = C.c_size_t()
     check(lib().mvr_assign_work_bytes(vec.shape[0], centroid.shape[0], C.byref(n)))
-    with torch.cuda.stream(stream):  # memory that is free for the stream which writes it
+    # memory that is free for the stream which writes it
+    with contextlib.nullcontext() if stream is None else torch.cuda.stream(stream):
         code = torch.empty(vec.shape[0], dtype=torch.int32, device=vec.device)
         score = torch.empty(vec.shape[0], dtype=torch.float32, device=vec.device)
         work = torch.empty(n.value, dtype=torch.uint8, device=vec.device)
