@@ -833,7 +833,10 @@ def main():
     rerank_bytes = (4.0 + bpv) * fast["n_tok"]           # vq code + residual bytes per token
     filter_bytes = 4.0 * fast["n_ent"] + 16.0 * fast["n_cand"]  # list entries; keys out + in
     fp8_ran = bool(FAST & PREC_FP8) and w["n_bit"] in (2, 4)  # FP8 MaxSim: 2- and 4-bit codes
-    rk = "rerank_ws_kernel (FP8)" if fp8_ran else "rerank_ws_kernel (BF16)"
+    widest = int(np.max(w["n_tok"]))
+    rk = ("rerank_ws_kernel (FP8)" if fp8_ran else
+          "rerank_ws_kernel (BF16)" if widest <= 32 else
+          "rerank_ws_kernel + rerank_%s_kernel (BF16)" % ("tmem" if w["n_bit"] <= 2 else "tc"))
     kern = {1: ("probe_tc_kernel + probe_pick_kernel", "tensor", probe_flop / 1e12,
                 pk["tc_sus"], "TFLOP/s"),
             2: ("filter_hash_kernel + filter_select_kernel", "hbm", filter_bytes / 1e9, pk["hbm"],

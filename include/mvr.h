@@ -293,7 +293,8 @@ int mvr_index_set_rerank_tile(mvr_index *h, uint32_t docs_per_cta);
 
 /* Failure detection (test hook; no counterpart in the reference, whose
  * kernels have no bounded waits): the time bound of every pipeline wait of
- * the warp-specialised MaxSim kernel (FP8; BF16 for queries of up to 32 tokens),
+ * the warp-specialised MaxSim kernel (FP8; BF16 for queries of up to 32 tokens,
+ * which long exact FP32 searches run to leave docs out),
  * in ns (0 restores the default, 1 s).  A wait that runs out stops the kernel, which
  * still lets its own copies and MMAs finish and frees its tensor memory; the
  * search then fails with MVR_ERR_CUDA and the handle stays usable.  Tests set

@@ -184,7 +184,7 @@ struct mvr_index {
   // hash filter sizing: candidates per probed list, the largest over the
   // queries of the previous search call (0: none yet)
   double cand_per_probe = 0.0;
-  uint64_t wait_ns = 1000000000ull;  // bound of the FP8 rerank's pipeline waits
+  uint64_t wait_ns = 1000000000ull;  // bound of rerank_ws_kernel's pipeline waits (FP8, BF16)
   uint32_t ws_docs = 0;              // shortlisted docs per CTA of the FP8 rerank (0: by the grid)
   // learned pruner (mvr_index_set_pruner): BF16 weight tiles, b1/b2/w3/b3
   uint8_t *prune_wts = nullptr;

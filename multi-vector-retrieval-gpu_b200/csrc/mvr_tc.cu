@@ -1591,7 +1591,6 @@ cudaError_t launch_probe(const float *q, uint32_t n_tok, const void *cen_sw, con
                            w.part_s, out_id, out_s, n_sm, st, n_launch);
 }
 
-// BF16 tables: centroid rows and the byte -> per-value weight table.
 // ---------------------------------------------------------------------
 // rerank_ws_kernel<NBIT, NMAX, FEAT, DOCS>: the FP8 (E4M3) MaxSim of the
 // mixed-precision path for 2- and 4-bit codes, warp-specialised.
@@ -2784,9 +2783,8 @@ cudaError_t launch_rerank_ws(const DevIndex &ix, const void *cen8, const TmWeigh
   if (!fp8_rerank_supported(ix.n_bit) || (set_docs && !ws_docs_supported(set_docs)))
     return cudaErrorInvalidValue;
   const uint8_t *c = reinterpret_cast<const uint8_t *>(cen8);
-  // queries of up to 32 tokens run in the 32-column variant (two CTAs per
-  // SM), longer ones in the 64-column variant (one CTA per SM); each launch
-  // skips the other's queries
+  // queries of up to 32 tokens run in the 32-column variant, longer ones in the
+  // 64-column variant (two CTAs per SM both); each launch skips the other's queries
   if (nq_min <= 32) {
     const uint32_t docs =
         set_docs ? set_docs : ws_auto_docs(n_query, probe_topk, 2u * (uint32_t)n_sm, 256u);

@@ -146,8 +146,10 @@ class Index:
         check(lib().mvr_index_set_rerank_tile(self._h, int(docs_per_cta)))
 
     def set_wait_limit(self, wait_ns=0):
-        """Time bound (ns) of the pipeline waits of the FP8 MaxSim kernel; 0
-        restores the default (1 s).  A failure-detection test hook."""
+        """Time bound (ns) of the pipeline waits of the warp-specialised MaxSim
+        kernel (FP8; BF16 for queries of up to 32 tokens, which cuts long exact
+        FP32 searches too); 0 restores the default (1 s).  A
+        failure-detection test hook."""
         check(lib().mvr_index_set_wait_limit(self._h, int(wait_ns)))
 
     def set_graphs(self, enable=True):
